@@ -260,6 +260,7 @@ struct GpuExec {
     g.ly = G.ly;
     g.dx1 = G.dx1; g.dx2 = G.dx2;
     g.eos = G.eos;
+    g.fe = make_fast_eos(g.eos, g.dx1, g.dx2);
     for (int k = 0; k < 4; k++) g.bc[k] = G.bc[k];
     const int nx1 = G.nx1, nx2 = G.nx2;
     const PredictGeom pg = make_predict_geom(nx1, nx2, G.ly);

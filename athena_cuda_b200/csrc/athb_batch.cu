@@ -392,6 +392,7 @@ static InstGeom make_geom(const athb_config& c, int ly, int nt, double* state0, 
   g.dx1 = (c.x1max - c.x1min) / (double)c.nx1;
   g.dx2 = (c.x2max - c.x2min) / (double)c.nx2;
   g.eos = Eos{c.gamma, c.gamma - 1.0, c.gamma - 2.0};
+  g.fe = make_fast_eos(g.eos, g.dx1, g.dx2);
   g.bc[0] = c.bc_ix1; g.bc[1] = c.bc_ox1; g.bc[2] = c.bc_ix2; g.bc[3] = c.bc_ox2;
   const int nx1 = c.nx1, nx2 = c.nx2;
   I.nt = nt;

@@ -69,6 +69,7 @@ static GridArgs grid_args(const athb_ctx* c, int from) {
   g.ly = c->ly;
   g.dx1 = c->dx1; g.dx2 = c->dx2;
   g.eos = Eos{c->cfg.gamma, c->cfg.gamma - 1.0, c->cfg.gamma - 2.0};
+  g.fe = make_fast_eos(g.eos, g.dx1, g.dx2);
   g.bc[0] = c->cfg.bc_ix1; g.bc[1] = c->cfg.bc_ox1; g.bc[2] = c->cfg.bc_ix2; g.bc[3] = c->cfg.bc_ox2;
   return g;
 }

@@ -125,6 +125,7 @@ extern "C" int athb_integrate_noalloc(const athb_config* cfg, const double* d_in
   gs.dx1 = (cfg->x1max - cfg->x1min) / (double)nx1;
   gs.dx2 = (cfg->x2max - cfg->x2min) / (double)nx2;
   gs.eos = Eos{cfg->gamma, cfg->gamma - 1.0, cfg->gamma - 2.0};
+  gs.fe = make_fast_eos(gs.eos, gs.dx1, gs.dx2);
   gs.bc[0] = cfg->bc_ix1; gs.bc[1] = cfg->bc_ox1; gs.bc[2] = cfg->bc_ix2; gs.bc[3] = cfg->bc_ox2;
 
   k_noalloc_begin<<<1, 1, 0, s>>>(gs.st, dt, gs.dx1, gs.dx2);

@@ -151,11 +151,11 @@ __device__ __forceinline__ void predict_x(const GridArgs& g, int bx, int by) {
   const Prim1 wl = shfl_prim(0xffffffffu, wln, 1, true);  // W_L of face c
   if (lane >= 1 && c <= g.ie + 2) {
     // step 1e (src/__integrate_2d__.c:172-180)
-    const Cons1 ul = prim_to_cons(wl, b1l, g.eos);
-    const Cons1 ur = prim_to_cons(wrt, b1l, g.eos);
+    const Cons1 ul = cons_of(wl, b1l, g.eos, g.fe.r_gamma_1);
+    const Cons1 ur = cons_of(wrt, b1l, g.eos, g.fe.r_gamma_1);
     store_cons(g.scr + S_ULX * g.ps, g.ps, o, ul);
     store_cons(g.scr + S_URX * g.ps, g.ps, o, ur);
-    store_cons(g.scr + S_FX * g.ps, g.ps, o, riemann<FLUX>(ul, ur, wl, wrt, b1l, g.eos));
+    store_cons(g.scr + S_FX * g.ps, g.ps, o, face_flux<FLUX>(ul, ur, wl, wrt, b1l, g.eos, g.fe));
     if constexpr (TAPE) {
       store_prim(g.scr + T_WLNX * g.ps, g.ps, o - 1, wl);
       store_prim(g.scr + T_WRTX * g.ps, g.ps, o, wrt);
@@ -225,11 +225,11 @@ __device__ __forceinline__ void predict_y(const GridArgs& g, const PredictGeom& 
     if (k >= ja) {
       // step 2e (src/__integrate_2d__.c:233-241)
       const Prim1 wl = sh_load<NT>(sh, 3, tid);
-      const Cons1 ul = prim_to_cons(wl, b2l, g.eos);
-      const Cons1 ur = prim_to_cons(wrt, b2l, g.eos);
+      const Cons1 ul = cons_of(wl, b2l, g.eos, g.fe.r_gamma_1);
+      const Cons1 ur = cons_of(wrt, b2l, g.eos, g.fe.r_gamma_1);
       store_cons(g.scr + S_ULY * g.ps, g.ps, o, ul);
       store_cons(g.scr + S_URY * g.ps, g.ps, o, ur);
-      store_cons(g.scr + S_FY * g.ps, g.ps, o, riemann<FLUX>(ul, ur, wl, wrt, b2l, g.eos));
+      store_cons(g.scr + S_FY * g.ps, g.ps, o, face_flux<FLUX>(ul, ur, wl, wrt, b2l, g.eos, g.fe));
       if constexpr (TAPE) {
         store_prim(g.scr + T_WLNY * g.ps, g.ps, o - g.pitch, wl);
         store_prim(g.scr + T_WRTY * g.ps, g.ps, o, wrt);
@@ -368,7 +368,7 @@ __device__ __forceinline__ void correct_x(const GridArgs& g, int t, int w) {
     const long long ow = o - 1;
     const double dbx = s[P_B1I * ps + o] - s[P_B1I * ps + ow];
     const double B1 = s[P_B1C * ps + ow], B2 = s[P_B2C * ps + ow], B3 = s[P_B3C * ps + ow];
-    const double V3 = s[P_M3 * ps + ow] / s[P_D * ps + ow];
+    const double V3 = ratio(s[P_M3 * ps + ow], s[P_D * ps + ow]);
     ul.mx += st.hdtodx1 * B1 * dbx;
     ul.my += st.hdtodx1 * B2 * dbx;
     ul.mz += st.hdtodx1 * B3 * dbx;
@@ -378,7 +378,7 @@ __device__ __forceinline__ void correct_x(const GridArgs& g, int t, int w) {
   {
     const double dbx = s[P_B1I * ps + o + 1] - s[P_B1I * ps + o];
     const double B1 = s[P_B1C * ps + o], B2 = s[P_B2C * ps + o], B3 = s[P_B3C * ps + o];
-    const double V3 = s[P_M3 * ps + o] / s[P_D * ps + o];
+    const double V3 = ratio(s[P_M3 * ps + o], s[P_D * ps + o]);
     ur.mx += st.hdtodx1 * B1 * dbx;
     ur.my += st.hdtodx1 * B2 * dbx;
     ur.mz += st.hdtodx1 * B3 * dbx;
@@ -386,9 +386,9 @@ __device__ __forceinline__ void correct_x(const GridArgs& g, int t, int w) {
     ur.e += st.hdtodx1 * B3 * V3 * dbx;
   }
   // step 8b (src/__integrate_2d__.c:438-447)
-  const Prim1 wl = cons_to_prim(ul, b1f, g.eos);
-  const Prim1 wr = cons_to_prim(ur, b1f, g.eos);
-  store_cons(g.scr + S_FX2 * ps, ps, o, riemann<FLUX>(ul, ur, wl, wr, b1f, g.eos));
+  const Prim1 wl = prim_of(ul, b1f, any_recip(ul.d), g.eos);
+  const Prim1 wr = prim_of(ur, b1f, any_recip(ur.d), g.eos);
+  store_cons(g.scr + S_FX2 * ps, ps, o, face_flux<FLUX>(ul, ur, wl, wr, b1f, g.eos, g.fe));
 }
 
 template <int FLUX>
@@ -428,7 +428,7 @@ __device__ __forceinline__ void correct_y(const GridArgs& g, int t, int w) {
     const long long osn = o - g.pitch;
     const double dby = s[P_B2I * ps + o] - s[P_B2I * ps + osn];
     const double B1 = s[P_B1C * ps + osn], B2 = s[P_B2C * ps + osn], B3 = s[P_B3C * ps + osn];
-    const double V3 = s[P_M3 * ps + osn] / s[P_D * ps + osn];
+    const double V3 = ratio(s[P_M3 * ps + osn], s[P_D * ps + osn]);
     ul.mz += st.hdtodx2 * B1 * dby;
     ul.mx += st.hdtodx2 * B2 * dby;
     ul.my += st.hdtodx2 * B3 * dby;
@@ -438,7 +438,7 @@ __device__ __forceinline__ void correct_y(const GridArgs& g, int t, int w) {
   {
     const double dby = s[P_B2I * ps + o + g.pitch] - s[P_B2I * ps + o];
     const double B1 = s[P_B1C * ps + o], B2 = s[P_B2C * ps + o], B3 = s[P_B3C * ps + o];
-    const double V3 = s[P_M3 * ps + o] / s[P_D * ps + o];
+    const double V3 = ratio(s[P_M3 * ps + o], s[P_D * ps + o]);
     ur.mz += st.hdtodx2 * B1 * dby;
     ur.mx += st.hdtodx2 * B2 * dby;
     ur.my += st.hdtodx2 * B3 * dby;
@@ -446,9 +446,9 @@ __device__ __forceinline__ void correct_y(const GridArgs& g, int t, int w) {
     ur.e += st.hdtodx2 * B3 * V3 * dby;
   }
   // step 8c (src/__integrate_2d__.c:455-464)
-  const Prim1 wl = cons_to_prim(ul, b2f, g.eos);
-  const Prim1 wr = cons_to_prim(ur, b2f, g.eos);
-  store_cons(g.scr + S_FY2 * ps, ps, o, riemann<FLUX>(ul, ur, wl, wr, b2f, g.eos));
+  const Prim1 wl = prim_of(ul, b2f, any_recip(ul.d), g.eos);
+  const Prim1 wr = prim_of(ur, b2f, any_recip(ur.d), g.eos);
+  store_cons(g.scr + S_FY2 * ps, ps, o, face_flux<FLUX>(ul, ur, wl, wr, b2f, g.eos, g.fe));
 }
 
 // step 7: cell-centred emf3 at t^{n+1/2} (src/__integrate_2d__.c:402-431)
@@ -477,7 +477,7 @@ __device__ __forceinline__ void correct_e(const GridArgs& g, int t, int w) {
   const double B1c = 0.5 * (b1f_c + b1f_e);
   const double B2c = 0.5 * (b2f_c + b2f_n);
   // written to the scratch ECC plane: the t^n values were consumed by k_emf
-  g.scr[S_ECC * ps + o] = (B1c * M2 - B2c * M1) / d;
+  g.scr[S_ECC * ps + o] = ratio(B1c * M2 - B2c * M1, d);
 }
 
 template <int FLUX, int NT = kThreads>

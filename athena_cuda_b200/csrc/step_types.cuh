@@ -2,7 +2,7 @@
 // (step_kernels.cuh) and the host-side launchers.
 #pragma once
 
-#include "mhd_physics.cuh"
+#include "mhd_fast.cuh"
 
 namespace athb {
 
@@ -68,6 +68,7 @@ struct GridArgs {
   int ly;                         // rows per y-sweep march segment
   double dx1, dx2;
   Eos eos;
+  FastEos fe;                     // make_fast_eos(eos, dx1, dx2)
   int bc[4];                      // ix1, ox1, ix2, ox2
 };
 

@@ -1,0 +1,58 @@
+// Host build of mhd_fast.cuh for tests/test_fast_physics_cpu.py: each entry
+// runs the fast and the general form on the same operands and returns their
+// outputs.
+#include <cmath>
+
+#include "mhd_fast.cuh"
+
+using namespace athb;
+
+namespace {
+Prim1 prim(const double* w) { return Prim1{w[0], w[1], w[2], w[3], w[4], w[5], w[6]}; }
+void put(const Prim1& w, double* o) {
+  o[0] = w.d; o[1] = w.vx; o[2] = w.vy; o[3] = w.vz; o[4] = w.p; o[5] = w.by; o[6] = w.bz;
+}
+void put(const Cons1& u, double* o) {
+  o[0] = u.d; o[1] = u.mx; o[2] = u.my; o[3] = u.mz; o[4] = u.e; o[5] = u.by; o[6] = u.bz;
+}
+}  // namespace
+
+extern "C" {
+
+// op 0: 1/x, 1: sqrt(x), 2: y/x with the reciprocal of x, 3: 1/sqrt(x) from the root's by-product
+void fast_ops(int op, int n, const double* x, const double* y, double* fast, double* plain) {
+  for (int k = 0; k < n; k++) {
+    double h;
+    switch (op) {
+    case 0: fast[k] = recip(x[k]); plain[k] = 1.0 / x[k]; break;
+    case 1: fast[k] = root(x[k]); plain[k] = std::sqrt(x[k]); break;
+    case 2: fast[k] = quot(y[k], x[k], recip(x[k])); plain[k] = y[k] / x[k]; break;
+    default: {
+      const double g = root(x[k], h);
+      fast[k] = recip_of_root(g, h);
+      plain[k] = 1.0 / std::sqrt(x[k]);
+    }
+    }
+  }
+}
+
+// n faces: w = left and right primitive states, bx the normal field.
+void fast_flux(int hlle, int n, const double* w, const double* bx, double gamma, int* took, double* fast,
+               double* plain) {
+  const Eos eos{gamma, gamma - 1.0, gamma - 2.0};
+  for (int k = 0; k < n; k++) {
+    const Prim1 wl = prim(w + 14 * k), wr = prim(w + 14 * k + 7);
+    const Cons1 ul = prim_to_cons(wl, bx[k], eos), ur = prim_to_cons(wr, bx[k], eos);
+    Cons1 F{};
+    if (hlle) {
+      took[k] = flux_hlle_fast(ul, ur, wl, wr, bx[k], eos, F);
+      put(flux_hlle(ul, ur, wl, wr, bx[k], eos), plain + 7 * k);
+    } else {
+      took[k] = flux_roe_fast(ul, ur, wl, wr, bx[k], eos, 1.0 / eos.gamma_1, F);
+      put(flux_roe(ul, ur, wl, wr, bx[k], eos), plain + 7 * k);
+    }
+    put(F, fast + 7 * k);
+  }
+}
+
+}  // extern "C"

@@ -1,0 +1,169 @@
+"""The fast forms of the hot physics (csrc/mhd_fast.cuh), built for the host,
+against the general ones: every value they vouch for is identical, bit for
+bit, so no tolerance is involved.  The divisions and roots they are made of
+are checked on the operands closest to a rounding boundary."""
+from __future__ import annotations
+
+import ctypes as C
+import math
+import subprocess
+from fractions import Fraction
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+HERE = Path(__file__).resolve().parent
+CSRC = HERE.parent / "athena_cuda_b200" / "csrc"
+
+
+@pytest.fixture(scope="module")
+def fast(tmp_path_factory):
+    so = tmp_path_factory.mktemp("fast") / "libfast_host.so"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-mfma", "-ffp-contract=off", "-frounding-math",
+                    f"-I{CSRC}", "-o", str(so), str(HERE / "hostcheck" / "fast_host.cpp")], check=True)
+    return C.CDLL(str(so))
+
+
+def _p(a):
+    return a.ctypes.data_as(C.c_void_p)
+
+
+def _ops(lib, op, x, y=None):
+    x = np.ascontiguousarray(x, dtype=np.float64)
+    y = np.ascontiguousarray(x if y is None else y, dtype=np.float64)
+    f, g = np.empty_like(x), np.empty_like(x)
+    lib.fast_ops(op, x.size, _p(x), _p(y), _p(f), _p(g))
+    return f, g
+
+
+def _hard_denominators():
+    """Significands whose reciprocal, or a quotient by which, lies next to the
+    middle of two doubles: near powers of two, and near 2^106 / M for
+    midpoints M (the factors of 2^106 - k among them)."""
+    D = {(1 << 53) - k for k in range(1, 600)} | {(1 << 52) + k for k in range(600)}
+    rng = np.random.default_rng(5)
+    for M in rng.integers(1 << 53, 1 << 54, 4000):
+        D.add(min(max((1 << 106) // (int(M) | 1), 1 << 52), (1 << 53) - 1))
+    for f in (3, 5, 7, 11, 107, 641, 6361, 69431):
+        for k in range(1, 40):
+            D.add((1 << 53) // f * 1 + k) if (1 << 52) <= (1 << 53) // f + k < (1 << 53) else None
+    return np.array(sorted(D), dtype=np.float64)
+
+
+def test_reciprocals_correctly_rounded(fast):
+    d = _hard_denominators()
+    d = np.concatenate([d * s for s in (1.0, 2.0 ** -52, 2.0 ** -500, 2.0 ** 447)])
+    d = np.concatenate([d, 2.0 ** np.random.default_rng(1).uniform(-480, 480, 400000)])
+    f, g = _ops(fast, 0, d)
+    np.testing.assert_array_equal(f, g)
+
+
+def test_quotients_correctly_rounded(fast):
+    """a chosen so that a / d is as close to a midpoint as a 53-bit a allows:
+    a 2^54 = +-k (mod d) for small k."""
+    rng = np.random.default_rng(2)
+    A, D = [], []
+    dens = [int(x) | 1 for x in _hard_denominators()[::3]] + [int(x) | 1 for x in rng.integers(1 << 52, 1 << 53, 4000)]
+    for d in dens:
+        inv = pow(pow(2, 54, d), -1, d)
+        for k in (1, -1, 2, -2, 3, -3):
+            a = (k * inv) % d   # 2^54 a = k (mod d): a 2^54 / d is k/d off an integer
+            while 0 < a < 1 << 52:
+                a *= 2
+            if 0 < a < 1 << 53:
+                A.append(a)
+                D.append(d)
+    a, d = np.array(A, dtype=np.float64), np.array(D, dtype=np.float64)
+    for sa, sd in ((1.0, 1.0), (2.0 ** -700, 2.0 ** 60), (2.0 ** 300, 2.0 ** -400)):
+        f, g = _ops(fast, 2, d * sd, a * sa)
+        np.testing.assert_array_equal(f, g)
+    x = 2.0 ** rng.uniform(-200, 200, 400000)
+    y = rng.choice([-1.0, 0.0, 1.0], x.size, p=[.45, .1, .45]) * 2.0 ** rng.uniform(-500, 200, x.size)
+    f, g = _ops(fast, 2, x, y)
+    np.testing.assert_array_equal(f, g)
+
+
+def test_roots_correctly_rounded(fast):
+    """x = m^2 -+ k 2^-106 for midpoints m: the roots nearest to a midpoint."""
+    X = [float(1 + k * Fraction(1, 1 << 52)) for k in range(64)]
+    X += [float(4 - k * Fraction(1, 1 << 51)) for k in range(64)]
+    X += [float(2 - k * Fraction(1, 1 << 52)) for k in range(-64, 64)]
+    rng = np.random.default_rng(3)
+    for m in rng.integers(1 << 53, 1 << 54, 60000):
+        m = int(m) | 1
+        sq = m * m
+        for shift in (54, 55):
+            for a in (sq >> shift, (sq >> shift) + 1):
+                if 1 << 52 <= a < 1 << 53:
+                    X.append(math.ldexp(a, shift - 106))
+    # m^2 = r (mod 2^54) with the smallest residues r
+    for r in (1, 9, 17, 25, 33, 41, 49, (1 << 54) - 7, (1 << 54) - 15, (1 << 54) - 23, (1 << 54) - 31):
+        s = 1
+        for bit in range(3, 55):   # lift a square root of r modulo 2^bit
+            if (s * s - r) % (1 << (bit + 1)):
+                s += 1 << (bit - 1)
+            if (s * s - r) % (1 << (bit + 1)):
+                break
+        for m in {s % (1 << 54), -s % (1 << 54), (s + (1 << 53)) % (1 << 54), (-s + (1 << 53)) % (1 << 54)}:
+            m = m if m >= 1 << 53 else m + (1 << 53)
+            for a in ((m * m) >> 54, ((m * m) >> 54) + 1):
+                X.append(math.ldexp(a, -52) if a < 1 << 53 else math.ldexp(a // 2, -51))
+    x = np.array(X)
+    x = np.concatenate([x * 4.0 ** k for k in (0, -30, 200, -400)] + [2.0 ** rng.uniform(-900, 900, 400000), [0.0]])
+    f, g = _ops(fast, 1, x)
+    np.testing.assert_array_equal(f, g)
+    f, g = _ops(fast, 3, x[x > 0])
+    np.testing.assert_array_equal(f, g)
+
+
+def _states(rng, n, kind):
+    """n primitive states and normal fields: smooth O(1), strong jumps, exact
+    zeros and equal components, or magnitudes spread over many decades."""
+    w = np.empty((n, 7))
+    w[:, 0] = np.exp(rng.normal(0, 1.0 if kind == "jumps" else 0.1, n))
+    w[:, 4] = np.exp(rng.normal(0, 2.0 if kind == "jumps" else 0.1, n))
+    w[:, 1:4] = rng.normal(0, 2.0 if kind == "jumps" else 0.7, (n, 3))
+    w[:, 5:] = rng.normal(0, 1, (n, 2))
+    bx = rng.normal(0, 1, n)
+    if kind == "zeros":
+        for c in (1, 2, 3, 5, 6):
+            w[rng.random(n) < 0.4, c] = 0.0
+        w[rng.random(n) < 0.5, 0] = 1.0 - 2.0 ** -53
+        bx[rng.random(n) < 0.4] = 0.0
+        bx[rng.random(n) < 0.1] = -0.0
+    if kind == "wide":
+        w *= 2.0 ** rng.uniform(-150, 30, (n, 7))
+        w[rng.random((n, 7)) < 0.2] = 0.0
+        w[:, 0], w[:, 4] = 2.0 ** rng.uniform(-40, 40, n), 2.0 ** rng.uniform(-60, 40, n)
+        bx *= 2.0 ** rng.uniform(-158, 20, n)
+    if kind == "extreme":
+        w *= 2.0 ** rng.uniform(-1070, 500, (n, 7))
+        w[:, 0], w[:, 4] = 2.0 ** rng.uniform(-150, 150, n), 2.0 ** rng.uniform(-150, 150, n)
+        bx *= 2.0 ** rng.uniform(-1070, 200, n)
+    return w, bx
+
+
+KINDS = ["smooth", "jumps", "zeros", "wide", "extreme"]
+
+
+@pytest.mark.parametrize("hlle", [0, 1])
+@pytest.mark.parametrize("gamma", [5.0 / 3.0, 1.4, 2.5])
+@pytest.mark.parametrize("kind", KINDS)
+def test_flux_identical(fast, kind, gamma, hlle):
+    n = 40000
+    rng = np.random.default_rng(10 + KINDS.index(kind))
+    w0, b0 = _states(rng, 2 * n, kind)
+    w, bx = w0.reshape(n, 2, 7), np.ascontiguousarray(b0[:n])
+    if kind in ("smooth", "zeros"):
+        w[:, 1] = w[:, 0] * (1 + 10.0 ** rng.uniform(-16, -1, (n, 1)) * rng.normal(size=(n, 7)))
+        same = rng.random((n, 7)) < 0.2
+        w[:, 1][same] = w[:, 0][same]
+    w[rng.random(n) < 0.2, :, 1] += rng.choice([-8.0, 8.0])
+    w = np.ascontiguousarray(w)
+    took = np.zeros(n, dtype=np.int32)
+    f, g = np.empty((n, 7)), np.empty((n, 7))
+    fast.fast_flux(hlle, n, _p(w), _p(bx), C.c_double(gamma), _p(took), _p(f), _p(g))
+    ok = took.astype(bool)
+    assert ok.mean() >= {"smooth": 0.99, "zeros": 0.9, "jumps": 0.5}.get(kind, 0.0)
+    np.testing.assert_array_equal(f[ok], g[ok])
