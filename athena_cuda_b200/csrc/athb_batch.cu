@@ -37,7 +37,7 @@ namespace {
 
 constexpr int kPhases = 6;
 constexpr int kPhasedGraphMinSteps = 32;
-constexpr int kRing256Bytes = 4 * 7 * 256 * (int)sizeof(double);   // predictor ring of 256-thread units
+constexpr int kRing256Bytes = kRingDoubles * 256 * (int)sizeof(double);   // predictor ring of 256-thread units
 constexpr long long kBarrierSpins = 20000000;  // x ~64 ns sleep: ~1-2 s
 constexpr int kBatchMinBlocks = 3;  // as k_predict: 168 registers per thread
 

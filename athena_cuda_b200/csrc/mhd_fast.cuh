@@ -2,20 +2,25 @@
 // branch-free, correctly rounded divisions and square roots.
 //
 // The functions return the very bits of their counterparts in mhd_physics.cuh
-// (flux_roe, flux_hlle) whenever they report success; a caller whose
+// (plm_cell, flux_roe, flux_hlle) whenever they report success; a caller whose
 // operands lie outside the ranges below is told so and takes the general
-// function instead.  What differs is the cost:
+// function instead.  The ranges let fields and momenta be as small as they
+// come: where a field advects into a region that has none its edge decays by a
+// constant factor per cell, so wide bands of cells hold fields of 1e-50 ..
+// 1e-308, and sending those out of line made the two paths evict each other
+// from the instruction cache (field loop 2048^2 after 200 steps: predictor
+// 2.7 ms, against 1.9 ms for the code before and 1.5 ms at step 5).  Squares
+// of such fields (1e-162 .. 1e-145, the square a denormal or close to one) are
+// scaled into range before a root or a quotient and back after it, exactly;
+// wave speeds that small only count where the flow speed does not absorb them.  What differs is the cost:
 //   * a / b and sqrt(x) as the compiler emits them are each a chain of ~10
 //     dependent FP64 instructions that ends in a test and a call, so the ~150
 //     of them in a zone-cycle cut the code into short blocks that neither
 //     overlap one another nor share work.  Here they are straight-line code
 //     (below), operands with a common denominator share its reciprocal, and
 //     reciprocals of square roots start from the root's own by-product;
-//   * factors of 1/2, 1/4 and 2 that the reference multiplies by are moved
-//     through products and sums to where they cancel, and products with the
-//     sign of the normal field flip a sign bit.  Scaling by a power of two
-//     commutes exactly with rounding as long as nothing underflows, which the
-//     operand ranges exclude;
+//   * products with the sign of the normal field flip a sign bit, and sums that
+//     the reference forms twice with opposite signs are formed once;
 //   * the six intermediate-state tests of the Roe solver are replaced by one
 //     bound that covers all of them, and by division-free tests where that
 //     bound does not hold.
@@ -110,6 +115,8 @@ constexpr unsigned pow2_word(int e) { return (unsigned)(1023 + e) << 20; }
 template <int LO, int HI> ATHB_HD bool outside(double x) {
   return hi_word(x) - pow2_word(LO) >= pow2_word(HI) - pow2_word(LO);
 }
+// true unless |x| < 2^E
+template <int E> ATHB_HD bool above(double x) { return (hi_word(x) & 0x7fffffffu) >= pow2_word(E); }
 // true unless x == 0 or 2^LO <= |x| < 2^HI
 template <int LO, int HI> ATHB_HD bool outside0(double x) {
   const unsigned h = hi_word(x) & 0x7fffffffu;
@@ -173,6 +180,15 @@ ATHB_HD double any_quot(double a, double d, double r) {   // r = any_recip(d)
 
 ATHB_HD double ratio(double a, double d) { return any_quot(a, d, any_recip(d)); }
 
+// sqrt(x), h as root(), for x of any smallness: g is the root, g_scaled and h
+// belong to x * 2^200 where x < 2^-900 (scale = 2^100), else to x (scale = 1).
+ATHB_HD double small_root(double x, double& g_scaled, double& scale, double& h) {
+  const bool small = !above<-900>(x);
+  scale = small ? 0x1p+100 : 1.0;
+  g_scaled = root(small ? x * 0x1p+200 : x, h);
+  return small ? g_scaled * 0x1p-100 : g_scaled;
+}
+
 // Constants of a launch: reciprocals of the divisors that do not change, and
 // whether the divisors lie in the ranges above.
 struct FastEos {
@@ -206,6 +222,12 @@ ATHB_HD Prim1 prim_of(const Cons1& u, double bx, double di, const Eos& eos) {
   w.bz = u.bz;
   return w;
 }
+// Cell outside the fast functions: densities and pressures within 2^+-100,
+// momenta and fields below 2^100.
+ATHB_HD bool cell_outside(const Cons1& u, double bx, double p) {
+  return outside<-100, 100>(u.d) | outside<-100, 100>(p) | above<100>(u.mx) | above<100>(u.my) | above<100>(u.mz) |
+         above<100>(bx) | above<100>(u.by) | above<100>(u.bz);
+}
 ATHB_HD Cons1 cons_of(const Prim1& w, double bx, const Eos& eos, double r_gamma_1) {
   Cons1 u;
   u.d = w.d;
@@ -220,13 +242,14 @@ ATHB_HD Cons1 cons_of(const Prim1& w, double bx, const Eos& eos, double r_gamma_
 }
 
 // Direction of the transverse field: (1, 0) where it vanishes.
-ATHB_HD void field_direction(double b2, double b3, double btsq, double& bt, double& bet2, double& bet3) {
-  double h;
-  bt = root(btsq, h);
-  const bool none = bt == 0.0;
-  const double r = recip_of_root(bt, h);
-  bet2 = none ? 1.0 : quot(b2, bt, r);
-  bet3 = none ? 0.0 : quot(b3, bt, r);
+ATHB_HD void field_direction(double b2, double b3, double btsq, double& bet2, double& bet3, bool& bad) {
+  double g, scale, h;
+  (void)small_root(btsq, g, scale, h);
+  const bool none = g == 0.0;
+  const double r = recip_of_root(g, h);
+  bet2 = none ? 1.0 : quot(b2 * scale, g, r);
+  bet3 = none ? 0.0 : quot(b3 * scale, g, r);
+  bad |= above<400>(btsq) | outside0<-200, 1>(bet2) | outside0<-200, 1>(bet3);
 }
 // alpha_f, alpha_s (src/esystem_prim.c:76-91): roots of gap / span
 ATHB_HD void wave_weights(double span, double slow_gap, double fast_gap, double& af, double& as) {
@@ -239,18 +262,234 @@ ATHB_HD void wave_weights(double span, double slow_gap, double fast_gap, double&
 }
 
 // ---------------------------------------------------------------------------
+// plm_cell (src/lr_states_plm.c:95-233, src/esystem_prim.c:36-235) for three
+// cells that pass cell_outside; di = 1/w0.d, hdtodx = 0.5 * dtodx.  false:
+// outside the ranges, the states are not valid.
+// ---------------------------------------------------------------------------
+// Projections of v on the left eigenvectors; rows n and 6-n share their parts.
+struct PrimLeft {
+  double l01, l02, l03, l04, l05, l06;   // rows 0 and 6
+  double b2, b3, l15, l16;               // rows 1 and 5
+  double l21, l22, l23, l24, l25, l26;   // rows 2 and 4
+  double l34;
+};
+ATHB_HD void project(const PrimLeft& L, const double v[7], double a[7]) {
+  {
+    const double t = L.l01 * v[1] + L.l02 * v[2] + L.l03 * v[3];
+    const double p4 = L.l04 * v[4], p5 = L.l05 * v[5], p6 = L.l06 * v[6];
+    a[0] = t + p4 + p5 + p6;
+    a[6] = p4 - t + p5 + p6;
+  }
+  {
+    const double t = L.b2 * v[3] - L.b3 * v[2];
+    const double p5 = L.l15 * v[5], p6 = L.l16 * v[6];
+    a[1] = t - p5 + p6;
+    a[5] = p6 - (t + p5);
+  }
+  {
+    const double t = L.l21 * v[1] - L.l22 * v[2] - L.l23 * v[3];
+    const double p4 = L.l24 * v[4], p5 = L.l25 * v[5], p6 = L.l26 * v[6];
+    a[2] = t + p4 - p5 - p6;
+    a[4] = p4 - t - p5 - p6;
+  }
+  a[3] = v[0] - L.l34 * v[4];
+}
+
+ATHB_HD bool plm_cell_fast(const Prim1& wm, const Prim1& w0, const Prim1& wp, double di, double bxc, double hdtodx,
+                           const Eos& eos, Prim1& wl_next, Prim1& wr_this) {
+  bool bad = false;
+  // eigensystem of the cell
+  PrimLeft L;
+  double ev[7], R00, R02, R10, R12, R20, R21, R22, R30, R31, R32, R40, R42, R50, R51, R52, R60, R61, R62;
+  {
+    const double d = w0.d, v1 = w0.vx, b2 = w0.by, b3 = w0.bz;
+    const double btsq = b2 * b2 + b3 * b3;
+    const double vaxsq = bxc * bxc * di;
+    const double asq = eos.gamma * w0.p * di;
+    const double ct2 = btsq * di;
+    const double tsum = vaxsq + ct2 + asq;
+    const double tdif = vaxsq + ct2 - asq;
+    const double cf2_cs2 = root(tdif * tdif + 4.0 * asq * ct2);
+    const double cfsq = 0.5 * (tsum + cf2_cs2);
+    double hcf, ha, hd;
+    const double cf = root(cfsq, hcf);
+    const double csnum = asq * vaxsq;
+    const double cssq = quot(csnum, cfsq, recip_from(cfsq, 4.0 * (hcf * hcf)));
+    const double cs = root(cssq);
+    const double vax = root(vaxsq);
+    const bool tiny_waves = outside0<-960, 500>(csnum) | outside0<-960, 500>(vaxsq) | outside0<-960, 500>(cssq);
+    double bet2, bet3, alpha_f, alpha_s;
+    field_direction(b2, b3, btsq, bet2, bet3, bad);
+    wave_weights(cf2_cs2, asq - cssq, cfsq - asq, alpha_f, alpha_s);
+    // slow and Alfven speeds below 2^-480 that do not show beside v1, nor in
+    // a slow wave of weight 0, need no exact value
+    bad |= tiny_waves && !(alpha_s == 0.0 && above<-300>(v1) && !above<400>(vaxsq));
+    const double sqrtd = root(d, hd);
+    const double a = root(asq, ha);
+    const unsigned s = bxc < 0. ? 0x80000000u : 0u;
+    const double qf = flip(cf * alpha_f, s), qs = flip(cs * alpha_s, s);
+    const double af = a * alpha_f * sqrtd, as = a * alpha_s * sqrtd;
+    ev[0] = v1 - cf; ev[1] = v1 - vax; ev[2] = v1 - cs; ev[3] = v1;
+    ev[4] = v1 + cs; ev[5] = v1 + vax; ev[6] = v1 + cf;
+    R00 = d * alpha_f;        R02 = d * alpha_s;
+    R10 = -cf * alpha_f;      R12 = -cs * alpha_s;
+    R20 = qs * bet2;          R21 = -bet3;      R22 = -qf * bet2;
+    R30 = qs * bet3;          R31 = bet2;       R32 = -qf * bet3;
+    const double dasq = d * asq;
+    R40 = dasq * alpha_f;     R42 = dasq * alpha_s;
+    const double bet2s = flip(bet2, s), bet3s = flip(bet3, s);
+    R50 = as * bet2;          R51 = -bet3s * sqrtd;  R52 = -af * bet2;
+    R60 = as * bet3;          R61 = bet2s * sqrtd;   R62 = -af * bet3;
+    L.l34 = recip_from(asq, 4.0 * (ha * ha));
+    const double na = 0.5 * L.l34;
+    const double nqf = na * qf, nqs = na * qs;
+    const double afp = na * af * di, asp = na * as * di;
+    const double rs = recip_of_root(sqrtd, hd);
+    L.l01 = -na * cf * alpha_f; L.l02 = nqs * bet2; L.l03 = nqs * bet3;
+    L.l04 = na * alpha_f * di;  L.l05 = asp * bet2; L.l06 = asp * bet3;
+    L.b2 = 0.5 * bet2; L.b3 = 0.5 * bet3;
+    L.l15 = quot(0.5 * bet3s, sqrtd, rs); L.l16 = quot(0.5 * bet2s, sqrtd, rs);
+    L.l21 = -na * cs * alpha_s; L.l22 = nqf * bet2; L.l23 = nqf * bet3;
+    L.l24 = na * alpha_s * di;  L.l25 = afp * bet2; L.l26 = afp * bet3;
+  }
+
+  const double Wm[7] = {wm.d, wm.vx, wm.vy, wm.vz, wm.p, wm.by, wm.bz};
+  const double W0[7] = {w0.d, w0.vx, w0.vy, w0.vz, w0.p, w0.by, w0.bz};
+  const double Wp[7] = {wp.d, wp.vx, wp.vy, wp.vz, wp.p, wp.by, wp.bz};
+
+  // Steps 2-4.
+  double da[7];
+  {
+    double dl[7], dr[7], dc[7], dg[7];
+#pragma unroll
+    for (int n = 0; n < 7; n++) {
+      dl[n] = W0[n] - Wm[n];
+      dr[n] = Wp[n] - W0[n];
+      dc[n] = Wp[n] - Wm[n];
+      const double prod = dl[n] * dr[n], sum = dl[n] + dr[n], size = fabs(sum);
+      if (n < 5) {
+        // 2 dl dr / (dl + dr) as 2 (dl dr / (dl + dr)): with the product zero or
+        // at least 2^-960 the halves are exact
+        const double g = with_sign(quot(prod, size, recip(size)), sum);
+        dg[n] = (int)hi_word(prod) > 0 ? g + g : 0.0;
+        bad |= outside0<-960, 500>(prod);
+      } else {
+        const double num = 2.0 * dl[n] * dr[n];
+        const bool small = !above<-960>(num);
+        const double g = with_sign(quot(small ? num * 0x1p+200 : num, size, recip(size)), sum);
+        dg[n] = prod > 0.0 ? (small ? g * 0x1p-200 : g) : 0.0;
+        bad |= above<500>(prod);
+      }
+    }
+    double al[7], ar[7], ac[7], ag[7];
+    project(L, dl, al);
+    project(L, dr, ar);
+    project(L, dc, ac);
+    project(L, dg, ag);
+#pragma unroll
+    for (int n = 0; n < 7; n++) {
+      const double x = 2.0 * rmin(fabs(al[n]), fabs(ar[n]));
+      const double y = rmin(0.5 * fabs(ac[n]), fabs(ag[n]));
+      da[n] = al[n] * ar[n] > 0.0 ? with_sign(rmin(x, y), ac[n]) : 0.0;
+    }
+  }
+
+  // Step 5: primitive slopes.
+  double dWm[7];
+  dWm[0] = da[0] * R00 + da[2] * R02 + da[3] + da[4] * R02 + da[6] * R00;
+  dWm[1] = da[0] * R10 + da[2] * R12 - da[4] * R12 - da[6] * R10;
+  dWm[2] = da[0] * R20 + da[1] * R21 + da[2] * R22 - da[4] * R22 - da[5] * R21 - da[6] * R20;
+  dWm[3] = da[0] * R30 + da[1] * R31 + da[2] * R32 - da[4] * R32 - da[5] * R31 - da[6] * R30;
+  dWm[4] = da[0] * R40 + da[2] * R42 + da[4] * R42 + da[6] * R40;
+  dWm[5] = da[0] * R50 + da[1] * R51 + da[2] * R52 + da[4] * R52 + da[5] * R51 + da[6] * R50;
+  dWm[6] = da[0] * R60 + da[1] * R61 + da[2] * R62 + da[4] * R62 + da[5] * R61 + da[6] * R60;
+
+  // Steps 7 and 8.
+  double dW[7], pWl[7], pWr[7];
+  const double qx = rmax(ev[6], 0.0) * hdtodx, qy = rmin(ev[0], 0.0) * hdtodx;
+#pragma unroll
+  for (int n = 0; n < 7; n++) {
+    const double half = 0.5 * dWm[n];
+    double l = W0[n] - half, r = W0[n] + half;
+    const bool cm = W0[n] < Wm[n], cp = W0[n] < Wp[n];
+    l = rmax(cm ? W0[n] : Wm[n], l);
+    l = rmin(cm ? Wm[n] : W0[n], l);
+    r = rmax(cp ? W0[n] : Wp[n], r);
+    r = rmin(cp ? Wp[n] : W0[n], r);
+    dW[n] = r - l;
+    pWl[n] = r - qx * dW[n];
+    pWr[n] = l - qy * dW[n];
+  }
+
+  // Step 9: the waves that do not reach the interface.  h is the left row
+  // times dtodx / 2; rows n and 6-n differ in the sign of their first half.
+  const double h01 = L.l01 * hdtodx, h02 = L.l02 * hdtodx, h03 = L.l03 * hdtodx;
+  const double h04 = L.l04 * hdtodx, h05 = L.l05 * hdtodx, h06 = L.l06 * hdtodx;
+  const double h12 = L.b3 * hdtodx, h13 = L.b2 * hdtodx, h15 = L.l15 * hdtodx, h16 = L.l16 * hdtodx;
+  const double h21 = L.l21 * hdtodx, h22 = L.l22 * hdtodx, h23 = L.l23 * hdtodx;
+  const double h24 = L.l24 * hdtodx, h25 = L.l25 * hdtodx, h26 = L.l26 * hdtodx;
+  const double h34 = L.l34 * hdtodx;
+  auto strength = [&](int n, double dev) {
+    if (n == 0 || n == 6) {
+      const double t = h01 * dev * dW[1] + h02 * dev * dW[2] + h03 * dev * dW[3];
+      const double t4 = h04 * dev * dW[4], t5 = h05 * dev * dW[5], t6 = h06 * dev * dW[6];
+      return (n == 0 ? t + t4 : t4 - t) + t5 + t6;
+    }
+    if (n == 1 || n == 5) {
+      const double t = h13 * dev * dW[3] - h12 * dev * dW[2];
+      const double t5 = h15 * dev * dW[5], t6 = h16 * dev * dW[6];
+      return n == 1 ? t - t5 + t6 : t6 - (t + t5);
+    }
+    if (n == 2 || n == 4) {
+      const double t = h21 * dev * dW[1] - h22 * dev * dW[2] - h23 * dev * dW[3];
+      const double t4 = h24 * dev * dW[4], t5 = h25 * dev * dW[5], t6 = h26 * dev * dW[6];
+      return (n == 2 ? t + t4 : t4 - t) - t5 - t6;
+    }
+    return hdtodx * dev * dW[0] - h34 * dev * dW[4];
+  };
+  auto add = [&](int n, double qa, double p[7]) {
+    const double sg = n > 3 ? -qa : qa;   // columns n and 6-n share rows up to sign
+    if (n == 0 || n == 6) {
+      p[0] += qa * R00; p[1] += sg * R10; p[2] += sg * R20; p[3] += sg * R30;
+      p[4] += qa * R40; p[5] += qa * R50; p[6] += qa * R60;
+    } else if (n == 1 || n == 5) {
+      p[2] += sg * R21; p[3] += sg * R31; p[5] += qa * R51; p[6] += qa * R61;
+    } else if (n == 2 || n == 4) {
+      p[0] += qa * R02; p[1] += sg * R12; p[2] += sg * R22; p[3] += sg * R32;
+      p[4] += qa * R42; p[5] += qa * R52; p[6] += qa * R62;
+    } else {
+      p[0] += qa;
+    }
+  };
+#pragma unroll
+  for (int n = 0; n < 6; n++)
+    if (ev[n] > 0.) add(n, strength(n, ev[6] - ev[n]), pWl);
+#pragma unroll
+  for (int n = 0; n < 7; n++)
+    if (ev[n] < 0.) {
+      if (n != 0) add(n, strength(n, ev[0] - ev[n]), pWr);
+      add(n, -strength(n, ev[n] - ev[6]), pWl);
+    }
+
+  wl_next.d = pWl[0]; wl_next.vx = pWl[1]; wl_next.vy = pWl[2]; wl_next.vz = pWl[3];
+  wl_next.p = pWl[4]; wl_next.by = pWl[5]; wl_next.bz = pWl[6];
+  wr_this.d = pWr[0]; wr_this.vx = pWr[1]; wr_this.vy = pWr[2]; wr_this.vz = pWr[3];
+  wr_this.p = pWr[4]; wr_this.by = pWr[5]; wr_this.bz = pWr[6];
+  return !bad;
+}
+
+// ---------------------------------------------------------------------------
 // Roe averages and wave speeds (src/flux_roe.c:91-114, src/esystem_roe.c:68-144)
 // of a face, and by-products of their roots.  Sets bad when an operand lies
 // outside the ranges of the fast operations.
 // ---------------------------------------------------------------------------
 struct FaceRoots {
-  double rd;      // 1/droe
-  double h_a;     // 1/(2 sqrt(twid_asq)) to about an ulp
-  double twid_a;
+  double rd;         // 1/droe
+  bool tiny_waves;   // slow or Alfven speeds below 2^-480 and not zero
 };
 ATHB_HD void face_averages(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, const Prim1& Wr, double Bxi,
                            const Eos& eos, RoeAvg& r, RoeSpeeds& s, FaceRoots& f, bool& bad) {
-  bad |= outside<-100, 100>(Wl.d) | outside<-100, 100>(Wr.d) | outside0<-160, 100>(Bxi);
+  bad |= outside<-100, 100>(Wl.d) | outside<-100, 100>(Wr.d) | above<100>(Bxi);
   double hl, hr;
   r.sqrtdl = root(Wl.d, hl);
   r.sqrtdr = root(Wr.d, hr);
@@ -263,10 +502,10 @@ ATHB_HD void face_averages(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
   r.v3 = (r.sqrtdl * Wl.vz + r.sqrtdr * Wr.vz) * r.isdlpdr;
   r.b2 = (r.sqrtdr * Wl.by + r.sqrtdl * Wr.by) * r.isdlpdr;
   r.b3 = (r.sqrtdr * Wl.bz + r.sqrtdl * Wr.bz) * r.isdlpdr;
-  bad |= outside0<-160, 100>(r.b2) | outside0<-160, 100>(r.b3);
+  bad |= above<100>(r.b2) | above<100>(r.b3);
   const double dby = Wl.by - Wr.by, dbz = Wl.bz - Wr.bz;
   const double db2 = 0.5 * (dby * dby + dbz * dbz), ss2 = ss * ss;
-  bad |= outside0<-700, 300>(db2);
+  const bool tiny_jump = outside0<-900, 300>(db2);
   r.x = quot(db2, ss2, recip_from(ss2, r.isdlpdr * r.isdlpdr));
   r.y = quot(0.5 * (Wl.d + Wr.d), r.droe, f.rd);
   const double bx2 = Bxi * Bxi;
@@ -292,9 +531,15 @@ ATHB_HD void face_averages(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
   s.cfsq = 0.5 * (tsum + cf2_cs2);
   double hf;
   s.cf = root(s.cfsq, hf);
-  s.cssq = quot(s.twid_asq * s.vaxsq, s.cfsq, recip_from(s.cfsq, 4.0 * (hf * hf)));
+  const double csnum = s.twid_asq * s.vaxsq;
+  s.cssq = quot(csnum, s.cfsq, recip_from(s.cfsq, 4.0 * (hf * hf)));
   s.cs = root(s.cssq);
   s.vax = root(s.vaxsq);
+  f.tiny_waves = outside0<-960, 500>(csnum) | outside0<-960, 500>(s.vaxsq) | outside0<-960, 500>(s.cssq);
+  // x below 2^-700 does not show beside the squared velocity, nor in the
+  // sound speed
+  bad |= tiny_jump && !(above<-300>(s.vsq) && !above<300>(db2));
+  bad |= above<500>(s.vaxsq);
 }
 
 // flux_hlle (src/flux_hlle.c:60-199); false: outside the ranges, F not set.
@@ -306,12 +551,15 @@ ATHB_HD bool flux_hlle_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, c
   FaceRoots f;
   face_averages(Ul, Ur, Wl, Wr, Bxi, eos, r, s, f, bad);
   const double ev0 = r.v1 - s.cf, ev6 = r.v1 + s.cf;
+  const double bx2 = Bxi * Bxi;
+  bad |= above<300>(bx2);
   auto side_speed = [&](const Cons1& U, const Prim1& W) {
     const double rd = recip(W.d);
     const double bt2 = U.by * U.by + U.bz * U.bz;
-    bad |= outside<-200, 300>(W.p) | outside0<-700, 300>(bt2);
+    // squares below 2^-960 do not show beside the sound speed
+    bad |= outside<-200, 300>(W.p) | above<300>(bt2);
     const double asq = quot(eos.gamma * W.p, W.d, rd);
-    const double vaxsq = quot(Bxi * Bxi, W.d, rd);
+    const double vaxsq = quot(bx2, W.d, rd);
     const double ct2 = quot(bt2, W.d, rd);
     const double qsq = vaxsq + ct2 + asq;
     const double tmp = vaxsq + ct2 - asq;
@@ -325,7 +573,7 @@ ATHB_HD bool flux_hlle_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, c
   const double width = bp - bm, mid = 0.5 * (bp + bm);
   bad |= outside<-300, 400>(width) | outside0<-700, 400>(mid);
   const double t = quot(mid, width, recip(width));
-  const double wl = Wl.vx - bm, wr = Wr.vx - bp, bx2 = Bxi * Bxi;
+  const double wl = Wl.vx - bm, wr = Wr.vx - bp;
   auto mean = [&](double a, double b) { return 0.5 * (a + b) + (a - b) * t; };
   F.d = mean(Ul.mx - bm * Ul.d, Ur.mx - bp * Ur.d);
   F.mx = mean(Ul.mx * wl + Wl.p - 0.5 * (bx2 - Wl.by * Wl.by - Wl.bz * Wl.bz),
@@ -357,15 +605,17 @@ ATHB_HD bool flux_roe_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
   // Eigenvector scalars (src/esystem_roe.c:91-291).
   const double v1 = r.v1, v2 = r.v2, v3 = r.v3, b2 = r.b2, b3 = r.b3, d = r.droe;
   const double cf = s.cf, cs = s.cs, vsq = s.vsq, hp = s.hp;
-  double bt, bet2, bet3, hg, hd, ha, af, as;
-  field_direction(b2, b3, s.btsq, bt, bet2, bet3);
-  const double bt_star = root(s.bt_starsq);
+  double bet2, bet3, hg, hd, ha, af, as;
+  field_direction(b2, b3, s.btsq, bet2, bet3, bad);
+  double g_, scale_, h_;
+  const double bt_star = small_root(s.bt_starsq, g_, scale_, h_);
   const double sg = root(s.gfac, hg);
   const double rsg = recip_of_root(sg, hg);
   const double bet2s = quot(bet2, sg, rsg), bet3s = quot(bet3, sg, rsg);
   const double bet_starsq = bet2s * bet2s + bet3s * bet3s;
   const double vbet = v2 * bet2s + v3 * bet3s;
   wave_weights(s.cfsq - s.cssq, s.twid_asq - s.cssq, s.cfsq - s.twid_asq, af, as);
+  bad |= f.tiny_waves && !(as == 0.0 && above<-300>(v1));
   const double sqrtd = root(d, hd);
   const double isqrtd = recip_of_root(sqrtd, hd);
   const unsigned sgn = Bxi < 0. ? 0x80000000u : 0u;
@@ -374,7 +624,7 @@ ATHB_HD bool flux_roe_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
   const double afp = twid_a * af * isqrtd, asp = twid_a * as * isqrtd;
   const double afpbb = afp * bt_star * bet_starsq, aspbb = asp * bt_star * bet_starsq;
   const double g2x = eos.gamma_2 * r.x;
-  bad |= outside0<-800, 400>(g2x);
+  bad |= above<400>(g2x);   // below 2^-900: see tiny_jump
   const double gx = quot(g2x, eos.gamma_1, r_gamma_1);
   const double bet2n = flip(bet2, sgn), bet3n = flip(bet3, sgn);
 
@@ -482,30 +732,30 @@ ATHB_HD bool flux_roe_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
       bad |= !(u[0] > 0.0) || !((u[4] - k) * u[0] - m2 > 1.0e-12 * (u[4] * u[0]));
     }
   }
-  // Step 8 from twice the mean of the side fluxes (src/flux_roe.c:252).
+  // Step 8 (src/flux_roe.c:252).
   const Cons1 Fl = side_flux(Ul, Wl, Bxi, r.pbl), Fr = side_flux(Ur, Wr, Bxi, r.pbr);
-  double G[7] = {Fl.d + Fr.d, Fl.mx + Fr.mx, Fl.my + Fr.my, Fl.mz + Fr.mz, Fl.e + Fr.e, Fl.by + Fr.by,
-                 Fl.bz + Fr.bz};
+  double G[7] = {0.5 * (Fl.d + Fr.d), 0.5 * (Fl.mx + Fr.mx), 0.5 * (Fl.my + Fr.my), 0.5 * (Fl.mz + Fr.mz),
+                 0.5 * (Fl.e + Fr.e), 0.5 * (Fl.by + Fr.by), 0.5 * (Fl.bz + Fr.bz)};
   const double evs[7] = {ev0, v1 - s.vax, ev2, v1, ev4, v1 + s.vax, ev6};
 #pragma unroll
   for (int n = 0; n < 7; n++) {
-    const double c = fabs(evs[n]) * a[n];
+    const double c = 0.5 * fabs(evs[n]) * a[n];
 #pragma unroll
     for (int k = 0; k < 7; k++)
       if ((roe_right_mask(n) >> k) & 1) G[k] -= (n == 3 && k == 0) ? c : c * C[n][k];
   }
-  F.d = 0.5 * G[0]; F.mx = 0.5 * G[1]; F.my = 0.5 * G[2]; F.mz = 0.5 * G[3]; F.e = 0.5 * G[4];
-  F.by = 0.5 * G[5]; F.bz = 0.5 * G[6];
+  F.d = G[0]; F.mx = G[1]; F.my = G[2]; F.mz = G[3]; F.e = G[4]; F.by = G[5]; F.bz = G[6];
   return !bad;
 }
 
-// The general functions out of line, for the operands the fast ones refuse.
+// The general function out of line, for the faces the fast one refuses.
 template <int FLUX>
 ATHB_COLD void riemann_general(const Cons1* ul, const Cons1* ur, const Prim1* wl, const Prim1* wr, double bxi,
                                const Eos* eos, Cons1* F) {
   *F = riemann<FLUX>(*ul, *ur, *wl, *wr, bxi, *eos);
 }
-// Face flux: riemann<FLUX> by the fast functions where they apply (ok: the
+
+// Face flux: riemann<FLUX> by the fast functions where they apply (fe.ok: the
 // launch's constants lie in their ranges).
 template <int FLUX>
 ATHB_HD Cons1 face_flux(const Cons1& ul, const Cons1& ur, const Prim1& wl, const Prim1& wr, double bxi,

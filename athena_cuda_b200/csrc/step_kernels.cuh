@@ -38,23 +38,47 @@ __device__ __forceinline__ long long off(const GridArgs& g, int j, int i) {
 // ---------------------------------------------------------------------------
 // Slice loads
 // ---------------------------------------------------------------------------
-// x-sweep conserved vector (d, M1, M2, M3, E, B2c, B3c), normal field B1c
-// (src/__integrate_2d__.c:130-139)
-__device__ __forceinline__ Prim1 prim_x(const GridArgs& g, const double* s, long long o) {
+// Conserved vector of a cell in the sweep's frame and its normal field.
+// x-sweep (DIR 0): (d, M1, M2, M3, E, B2c, B3c), B1c (src/__integrate_2d__.c:130-139);
+// y-sweep (DIR 1): (d, M2, M3, M1, E, B3c, B1c), B2c (src/__integrate_2d__.c:191-201)
+template <int DIR>
+__device__ __forceinline__ Cons1 load_cell(const GridArgs& g, long long o, double& bn) {
+  const double* s = g.in;
   Cons1 u;
-  u.d = s[P_D * g.ps + o]; u.mx = s[P_M1 * g.ps + o]; u.my = s[P_M2 * g.ps + o];
-  u.mz = s[P_M3 * g.ps + o]; u.e = s[P_E * g.ps + o];
-  u.by = s[P_B2C * g.ps + o]; u.bz = s[P_B3C * g.ps + o];
-  return cons_to_prim(u, s[P_B1C * g.ps + o], g.eos);
+  u.d = s[P_D * g.ps + o];
+  u.mx = s[(DIR ? P_M2 : P_M1) * g.ps + o]; u.my = s[(DIR ? P_M3 : P_M2) * g.ps + o];
+  u.mz = s[(DIR ? P_M1 : P_M3) * g.ps + o]; u.e = s[P_E * g.ps + o];
+  u.by = s[(DIR ? P_B3C : P_B2C) * g.ps + o]; u.bz = s[(DIR ? P_B1C : P_B3C) * g.ps + o];
+  bn = s[(DIR ? P_B2C : P_B1C) * g.ps + o];
+  return u;
 }
-// y-sweep conserved vector (d, M2, M3, M1, E, B3c, B1c), normal field B2c
-// (src/__integrate_2d__.c:191-201)
-__device__ __forceinline__ Prim1 prim_y(const GridArgs& g, const double* s, long long o) {
-  Cons1 u;
-  u.d = s[P_D * g.ps + o]; u.mx = s[P_M2 * g.ps + o]; u.my = s[P_M3 * g.ps + o];
-  u.mz = s[P_M1 * g.ps + o]; u.e = s[P_E * g.ps + o];
-  u.by = s[P_B3C * g.ps + o]; u.bz = s[P_B1C * g.ps + o];
-  return cons_to_prim(u, s[P_B2C * g.ps + o], g.eos);
+// Primitive state of a cell with 1/d; bad: set when the cell lies outside the
+// ranges of the fast functions (the values are then not used).
+template <int DIR>
+__device__ __forceinline__ Prim1 load_prim(const GridArgs& g, long long o, double& bn, double& di, bool& bad) {
+  const Cons1 u = load_cell<DIR>(g, o, bn);
+  di = recip(u.d);
+  const Prim1 w = prim_of(u, bn, di, g.eos);
+  bad = cell_outside(u, bn, w.p);
+  return w;
+}
+// The PLM states of one cell, source terms included, by the general functions
+// and from global memory: cells outside the ranges of the fast ones.
+template <int DIR>
+static __device__ __noinline__ void plm_states_general(const GridArgs* gp, long long o, Prim1* wln, Prim1* wrt) {
+  const GridArgs& g = *gp;
+  const StepState& st = *g.st;
+  const long long P = DIR ? g.pitch : 1;
+  double bm, b0, bp;
+  const Cons1 um = load_cell<DIR>(g, o - P, bm), u0 = load_cell<DIR>(g, o, b0), up = load_cell<DIR>(g, o + P, bp);
+  plm_cell(cons_to_prim(um, bm, g.eos), cons_to_prim(u0, b0, g.eos), cons_to_prim(up, bp, g.eos), b0,
+           DIR ? st.dtodx2 : st.dtodx1, g.eos, *wln, *wrt);
+  const double* bi = g.in + (DIR ? P_B2I : P_B1I) * g.ps;
+  const double src = ((DIR ? u0.mz : u0.my) / u0.d) * (bi[o + P] - bi[o]) / (DIR ? g.dx2 : g.dx1);
+  double& l = DIR ? wln->bz : wln->by;
+  double& r = DIR ? wrt->bz : wrt->by;
+  l += st.hdt * src;
+  r += st.hdt * src;
 }
 
 __device__ __forceinline__ Prim1 shfl_prim(unsigned mask, const Prim1& w, int delta, bool up) {
@@ -132,21 +156,34 @@ __device__ __forceinline__ void predict_x(const GridArgs& g, int bx, int by) {
   const double* s = g.in;
   const long long o = off(g, j, ce);
 
-  const Prim1 w0 = prim_x(g, s, o);
+  double bn, di, b_, d_;
+  bool bad, bad2 = false;
+  const Prim1 w0 = load_prim<0>(g, o, bn, di, bad);
   Prim1 wm = shfl_prim(0xffffffffu, w0, 1, true);
   Prim1 wp = shfl_prim(0xffffffffu, w0, 1, false);
-  if (lane == 0) wm = prim_x(g, s, o - 1);
-  if (lane == 31) wp = prim_x(g, s, o + 1);
+  if (lane == 0 || lane == 31) {
+    const Prim1 w = load_prim<0>(g, lane == 0 ? o - 1 : o + 1, b_, d_, bad2);
+    if (lane == 0) wm = w; else wp = w;
+  }
 
   Prim1 wln, wrt;
-  plm_cell(wm, w0, wp, s[P_B1C * g.ps + o], st.dtodx1, g.eos, wln, wrt);
-
-  // "MHD source terms" for 0.5*dt (src/__integrate_2d__.c:156-164)
-  const double d0 = s[P_D * g.ps + o];
   const double b1l = s[P_B1I * g.ps + o], b1r = s[P_B1I * g.ps + o + 1];
-  const double src = (s[P_M2 * g.ps + o] / d0) * (b1r - b1l) / g.dx1;
-  wln.by += st.hdt * src;
-  wrt.by += st.hdt * src;
+  // a cell outside the fast ranges sends its whole row segment out of line,
+  // so that its neighbours need not know
+  bool fast = !__any_sync(0xffffffffu, bad || bad2) && g.fe.ok && !outside<-100, 100>(st.hdtodx1);
+  if (fast) fast = plm_cell_fast(wm, w0, wp, di, bn, st.hdtodx1, g.eos, wln, wrt);
+  if (fast) {
+    // "MHD source terms" for 0.5*dt (src/__integrate_2d__.c:156-164)
+    const double src = any_quot(any_quot(s[P_M2 * g.ps + o], w0.d, di) * (b1r - b1l), g.dx1, g.fe.r_dx1);
+    wln.by += st.hdt * src;
+    wrt.by += st.hdt * src;
+  } else {
+    const GridArgs gg = g;
+    Prim1 l, r;
+    plm_states_general<0>(&gg, o, &l, &r);
+    wln = l;
+    wrt = r;
+  }
 
   const Prim1 wl = shfl_prim(0xffffffffu, wln, 1, true);  // W_L of face c
   if (lane >= 1 && c <= g.ie + 2) {
@@ -164,21 +201,24 @@ __device__ __forceinline__ void predict_x(const GridArgs& g, int bx, int by) {
   // step 3: emf3_cc at t^n on [is-2,ie+2] x [js-2,je+2] (src/__integrate_2d__.c:249-255)
   if ((lane >= 1 || bx == 0) && c <= g.ie + 2) {
     g.scr[S_ECC * g.ps + o] =
-        (s[P_B1C * g.ps + o] * s[P_M2 * g.ps + o] - s[P_B2C * g.ps + o] * s[P_M1 * g.ps + o]) / d0;
+        ratio(s[P_B1C * g.ps + o] * s[P_M2 * g.ps + o] - s[P_B2C * g.ps + o] * s[P_M1 * g.ps + o],
+              s[P_D * g.ps + o]);
   }
 }
 
-// The y role carries three cell states and one face state from row to row;
-// they live in a per-thread ring in shared memory rather than in registers.
+// The y role carries three cell states (with 1/d) and one face state from row
+// to row; they live in a per-thread ring in shared memory rather than in
+// registers.
+constexpr int kRingDoubles = 3 * 8 + 7;   // per thread
 template <int NT = kThreads>
 __device__ __forceinline__ void sh_store(double* sh, int slot, int tid, const Prim1& w) {
-  double* p = sh + slot * 7 * NT + tid;
+  double* p = sh + slot * 8 * NT + tid;
   p[0 * NT] = w.d; p[1 * NT] = w.vx; p[2 * NT] = w.vy; p[3 * NT] = w.vz;
   p[4 * NT] = w.p; p[5 * NT] = w.by; p[6 * NT] = w.bz;
 }
 template <int NT = kThreads>
 __device__ __forceinline__ Prim1 sh_load(const double* sh, int slot, int tid) {
-  const double* p = sh + slot * 7 * NT + tid;
+  const double* p = sh + slot * 8 * NT + tid;
   Prim1 w;
   w.d = p[0 * NT]; w.vx = p[1 * NT]; w.vy = p[2 * NT]; w.vz = p[3 * NT];
   w.p = p[4 * NT]; w.by = p[5 * NT]; w.bz = p[6 * NT];
@@ -188,11 +228,11 @@ __device__ __forceinline__ Prim1 sh_load(const double* sh, int slot, int tid) {
 template <int FLUX, bool TAPE = false, int NT = kThreads>
 __device__ __forceinline__ void predict_y(const GridArgs& g, const PredictGeom& pg, int b) {
   // slots 0..2: prims of rows k-1, k, k+1 (ring); slot 3: W_L of face k.
-  // Above 128 threads the ring (4 x 7 x NT doubles) exceeds the 48 KB of
+  // Above 128 threads the ring exceeds the 48 KB of
   // static shared memory: the launch supplies it as dynamic shared memory.
   double* sh;
   if constexpr (NT <= 128) {
-    __shared__ double sh_static[4 * 7 * NT];
+    __shared__ double sh_static[kRingDoubles * NT];
     sh = sh_static;
   } else {
     extern __shared__ double sh_dynamic[];
@@ -207,21 +247,40 @@ __device__ __forceinline__ void predict_y(const GridArgs& g, const PredictGeom& 
   const int jb = min(ja + g.ly - 1, g.je + 2);
   const double* s = g.in;
 
-  sh_store<NT>(sh, 0, tid, prim_y(g, s, off(g, ja - 2, i)));
-  sh_store<NT>(sh, 1, tid, prim_y(g, s, off(g, ja - 1, i)));
+  double bn, bnext, di;
+  bool bad_m, bad_0, bad_p;   // rows k-1, k, k+1 outside the fast ranges
+  sh_store<NT>(sh, 0, tid, load_prim<1>(g, off(g, ja - 2, i), bn, di, bad_m));
+  sh_store<NT>(sh, 1, tid, load_prim<1>(g, off(g, ja - 1, i), bn, di, bad_0));
+  sh[(1 * 8 + 7) * NT + tid] = di;
+  const bool plain = g.fe.ok && !outside<-100, 100>(st.hdtodx2);
   int r0 = 0;  // ring slot of row k-1
   for (int k = ja - 1; k <= jb; k++) {
     const long long o = off(g, k, i);
     const int r1 = r0 == 2 ? 0 : r0 + 1, r2 = r1 == 2 ? 0 : r1 + 1;
-    sh_store<NT>(sh, r2, tid, prim_y(g, s, o + g.pitch));
+    const Prim1 wp = load_prim<1>(g, o + g.pitch, bnext, di, bad_p);
+    sh_store<NT>(sh, r2, tid, wp);
+    const double d0i = sh[(r1 * 8 + 7) * NT + tid];
+    sh[(r2 * 8 + 7) * NT + tid] = di;
     Prim1 wln, wrt;
-    plm_cell(sh_load<NT>(sh, r0, tid), sh_load<NT>(sh, r1, tid), sh_load<NT>(sh, r2, tid), s[P_B2C * g.ps + o],
-             st.dtodx2, g.eos, wln, wrt);
-    // "MHD source terms" for 0.5*dt (src/__integrate_2d__.c:216-224)
     const double b2l = s[P_B2I * g.ps + o], b2r = s[P_B2I * g.ps + o + g.pitch];
-    const double src = (s[P_M1 * g.ps + o] / s[P_D * g.ps + o]) * (b2r - b2l) / g.dx2;
-    wln.bz += st.hdt * src;
-    wrt.bz += st.hdt * src;
+    bool fast = plain && !(bad_m || bad_0 || bad_p);
+    const Prim1 w0 = sh_load<NT>(sh, r1, tid);
+    if (fast) fast = plm_cell_fast(sh_load<NT>(sh, r0, tid), w0, wp, d0i, bn, st.hdtodx2, g.eos, wln, wrt);
+    if (fast) {
+      // "MHD source terms" for 0.5*dt (src/__integrate_2d__.c:216-224)
+      const double src = any_quot(any_quot(s[P_M1 * g.ps + o], w0.d, d0i) * (b2r - b2l), g.dx2, g.fe.r_dx2);
+      wln.bz += st.hdt * src;
+      wrt.bz += st.hdt * src;
+    } else {
+      const GridArgs gg = g;
+      Prim1 l, r;
+      plm_states_general<1>(&gg, o, &l, &r);
+      wln = l;
+      wrt = r;
+    }
+    bad_m = bad_0;
+    bad_0 = bad_p;
+    bn = bnext;
     if (k >= ja) {
       // step 2e (src/__integrate_2d__.c:233-241)
       const Prim1 wl = sh_load<NT>(sh, 3, tid);
@@ -240,6 +299,12 @@ __device__ __forceinline__ void predict_y(const GridArgs& g, const PredictGeom& 
   }
 }
 
+// k_predict is bound by the FP64 pipe's latency and by instruction fetch (3
+// warps per scheduler, ~1500 straight-line FP64 instructions per cell and
+// role).  Branch-free divisions, roots and PLM (mhd_fast.cuh), measured on B200:
+// field loop 2048^2 1.90 -> 1.33 ms, blast 1024^2 0.645 -> 0.408 ms (FP64 pipe 38%
+// -> 55% busy), blast 200x300 53 -> 38 us.
+//
 // Resident blocks per SM the heavy kernels are compiled for (register caps of
 // 168 and 128 per thread): measured faster on B200 than the uncapped 255
 // registers and 2 blocks per SM despite the spills they cause.

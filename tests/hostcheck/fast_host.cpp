@@ -36,6 +36,31 @@ void fast_ops(int op, int n, const double* x, const double* y, double* fast, dou
   }
 }
 
+// n cells: w = 3 primitive states (m, 0, p) of 7 each, bx = their normal
+// fields (3 each); out: 14 values of each form.  took[k]: the fast form
+// vouches for them.
+void fast_plm(int n, const double* w, const double* bx, const double* dtodx, double gamma, int* took, double* fast,
+              double* plain) {
+  const Eos eos{gamma, gamma - 1.0, gamma - 2.0};
+  for (int k = 0; k < n; k++) {
+    Prim1 p[3];
+    bool bad = false;
+    for (int c = 0; c < 3; c++) {
+      p[c] = prim(w + 21 * k + 7 * c);
+      Cons1 u = prim_to_cons(p[c], bx[3 * k + c], eos);
+      bad |= cell_outside(u, bx[3 * k + c], p[c].p);
+    }
+    Prim1 l, r;
+    plm_cell(p[0], p[1], p[2], bx[3 * k + 1], dtodx[k], eos, l, r);
+    put(l, plain + 14 * k);
+    put(r, plain + 14 * k + 7);
+    const bool done = plm_cell_fast(p[0], p[1], p[2], recip(p[1].d), bx[3 * k + 1], 0.5 * dtodx[k], eos, l, r);
+    took[k] = !bad && done;
+    put(l, fast + 14 * k);
+    put(r, fast + 14 * k + 7);
+  }
+}
+
 // n faces: w = left and right primitive states, bx the normal field.
 void fast_flux(int hlle, int n, const double* w, const double* bx, double gamma, int* took, double* fast,
                double* plain) {

@@ -141,10 +141,41 @@ def _states(rng, n, kind):
         w *= 2.0 ** rng.uniform(-1070, 500, (n, 7))
         w[:, 0], w[:, 4] = 2.0 ** rng.uniform(-150, 150, n), 2.0 ** rng.uniform(-150, 150, n)
         bx *= 2.0 ** rng.uniform(-1070, 200, n)
+    if kind in ("edge", "still"):   # where a field fades out: all of it tiny, denormals included
+        scale = 2.0 ** rng.uniform(-1072, -140, n)
+        w[:, 5:] *= scale[:, None] * 2.0 ** rng.uniform(-30, 0, (n, 2))
+        bx *= scale
+        if kind == "still":         # in a uniform flow
+            w[:, :5] = [1.0, 2.0, 1.0, 0.0, 1.0]
+            w[:, 1] = rng.choice([2.0, 1.0, 0.0, -1.0], n)
     return w, bx
 
 
-KINDS = ["smooth", "jumps", "zeros", "wide", "extreme"]
+KINDS = ["smooth", "jumps", "zeros", "wide", "extreme", "edge", "still"]
+
+
+@pytest.mark.parametrize("gamma", [5.0 / 3.0, 1.4, 2.5])
+@pytest.mark.parametrize("kind", KINDS)
+def test_plm_identical(fast, kind, gamma):
+    n = 20000
+    rng = np.random.default_rng(KINDS.index(kind))
+    w0, b0 = _states(rng, 3 * n, kind)
+    w, bx = w0.reshape(n, 3, 7), b0.reshape(n, 3)
+    if kind in ("smooth", "zeros"):   # neighbours close, some components equal
+        w[:, 1] = w[:, 0] * (1 + 1e-3 * rng.normal(size=(n, 7)))
+        w[:, 2] = w[:, 1] * (1 + 1e-3 * rng.normal(size=(n, 7)))
+        same = rng.random((n, 7)) < 0.2
+        w[:, 2][same] = w[:, 1][same]
+    w[rng.random(n) < 0.3, :, 1] += rng.choice([-8.0, 8.0])   # supersonic cells
+    w, bx = np.ascontiguousarray(w), np.ascontiguousarray(bx)
+    dtodx = np.ascontiguousarray(rng.uniform(0.05, 0.4, n))
+    took = np.zeros(n, dtype=np.int32)
+    f, g = np.empty((n, 14)), np.empty((n, 14))
+    fast.fast_plm(n, _p(w), _p(bx), _p(dtodx), C.c_double(gamma), _p(took), _p(f), _p(g))
+    ok = took.astype(bool)
+    assert ok.mean() >= {"extreme": 0.0, "wide": 0.3, "edge": 0.8, "still": 0.8}.get(kind, 0.95)
+    assert kind != "extreme" or not ok.all()
+    np.testing.assert_array_equal(f[ok], g[ok])
 
 
 @pytest.mark.parametrize("hlle", [0, 1])
@@ -165,5 +196,5 @@ def test_flux_identical(fast, kind, gamma, hlle):
     f, g = np.empty((n, 7)), np.empty((n, 7))
     fast.fast_flux(hlle, n, _p(w), _p(bx), C.c_double(gamma), _p(took), _p(f), _p(g))
     ok = took.astype(bool)
-    assert ok.mean() >= {"smooth": 0.99, "zeros": 0.9, "jumps": 0.5}.get(kind, 0.0)
+    assert ok.mean() >= {"smooth": 0.99, "zeros": 0.9, "jumps": 0.5, "still": 0.7}.get(kind, 0.0)
     np.testing.assert_array_equal(f[ok], g[ok])
