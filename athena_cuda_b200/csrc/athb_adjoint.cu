@@ -269,14 +269,8 @@ struct GpuExec {
     k_emf<<<blocks((long long)(nx1 + 3) * (nx2 + 3), kThreads), kThreads, 0, s>>>(g, G.is - 1, G.js - 1, nx1 + 3,
                                                                                    nx2 + 3, S_FX, S_FY);
     if (taped) copy(d.tape + (size_t)T_EMF0 * G.ps, d.tape + (size_t)S_EMF * G.ps, (size_t)G.ps);
-    CorrectGeom cgm;
-    cgm.xw = nx1 + 1; cgm.xn = nx2 + 3;
-    cgm.yw = nx1 + 3; cgm.yn = nx2 + 1;
-    cgm.ew = nx1 + 3; cgm.en = nx2 + 3;
-    cgm.xb = blocks((long long)cgm.xw * cgm.xn, kThreads);
-    cgm.yb = blocks((long long)cgm.yw * cgm.yn, kThreads);
-    cgm.eb = blocks((long long)cgm.ew * cgm.en, kThreads);
-    k_correct<FLUX><<<cgm.xb + cgm.yb + cgm.eb, kThreads, 0, s>>>(g, cgm);
+    const CorrectGeom cgm = make_correct_geom(nx1, nx2);
+    k_correct<FLUX><<<cgm.blocks, kThreads, 0, s>>>(g, cgm);
     k_emf<<<blocks((long long)(nx1 + 1) * (nx2 + 1), kThreads), kThreads, 0, s>>>(g, G.is, G.js, nx1 + 1, nx2 + 1,
                                                                                    S_FX2, S_FY2);
     const int n = nx1 * nx2;

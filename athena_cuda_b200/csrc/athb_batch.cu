@@ -39,7 +39,7 @@ constexpr int kPhases = 6;
 constexpr int kPhasedGraphMinSteps = 32;
 constexpr int kRing256Bytes = kRingDoubles * 256 * (int)sizeof(double);   // predictor ring of 256-thread units
 constexpr long long kBarrierSpins = 20000000;  // x ~64 ns sleep: ~1-2 s
-constexpr int kBatchMinBlocks = 3;  // as k_predict: 168 registers per thread
+constexpr int kBatchMinBlocks = 3;  // 168 registers per thread: all phases share one budget
 
 struct InstGeom {
   GridArgs g;  // g.in = state[0], g.out = state[1]
@@ -103,7 +103,7 @@ __host__ __device__ inline int item_count(const InstGeom& I, int seg) {
   case kSegPredictY: return I.pg.ny_blocks;
   case kSegPredictX: return I.pg.nx_blocks;
   case kSegEmfHalf: return bf((long long)(I.nx1 + 3) * (I.nx2 + 3));
-  case kSegCorrect: return I.cg.xb + I.cg.yb + I.cg.eb;
+  case kSegCorrect: return I.cg.blocks;
   case kSegEmfFull: return bf((long long)(I.nx1 + 1) * (I.nx2 + 1));
   case kSegUpdate: return bf((long long)I.nx1 * I.nx2);
   default: return bf(I.nframe);
@@ -372,11 +372,6 @@ struct athb_batch {
                        __FILE__, __LINE__);                                               \
   } while (0)
 
-static int pick_ly(int nx1, int nx2) {
-  long long ly = ((long long)(nx1 + 4) * (nx2 + 3)) / (148LL * 512);
-  return (int)std::max(4LL, std::min(64LL, ly));
-}
-
 // Geometry of instance k (same rules as the single-grid launcher).
 static InstGeom make_geom(const athb_config& c, int ly, int nt, double* state0, double* state1, double* scr,
                           StepState* st) {
@@ -397,13 +392,7 @@ static InstGeom make_geom(const athb_config& c, int ly, int nt, double* state0, 
   const int nx1 = c.nx1, nx2 = c.nx2;
   I.nt = nt;
   I.pg = make_predict_geom(nx1, nx2, ly, nt);
-  I.cg.xw = nx1 + 1; I.cg.xn = nx2 + 3;
-  I.cg.yw = nx1 + 3; I.cg.yn = nx2 + 1;
-  I.cg.ew = nx1 + 3; I.cg.en = nx2 + 3;
-  auto bf = [nt](long long n) { return (int)((n + nt - 1) / nt); };
-  I.cg.xb = bf((long long)I.cg.xw * I.cg.xn);
-  I.cg.yb = bf((long long)I.cg.yw * I.cg.yn);
-  I.cg.eb = bf((long long)I.cg.ew * I.cg.en);
+  I.cg = make_correct_geom(nx1, nx2, nt);
   I.nx1 = nx1; I.nx2 = nx2; I.sx = sx; I.sy = sy;
   I.nframe = g.js * sx + (sy - g.je - 1) * sx + nx2 * 2 * g.is;
   return I;
@@ -509,7 +498,11 @@ extern "C" int athb_batch_create(int n, const athb_config* cfgs, athb_batch** ou
   b->device = cfgs[0].device;
   b->cfg.assign(cfgs, cfgs + n);
   b->ly.resize(n);
-  for (int k = 0; k < n; k++) b->ly[k] = pick_ly(cfgs[k].nx1, cfgs[k].nx2);
+  // the marches of all instances share the GPU: the rule of a single grid on
+  // all of them together
+  long long faces = 0;
+  for (int k = 0; k < n; k++) faces += (long long)(cfgs[k].nx1 + 4) * (cfgs[k].nx2 + 3);
+  for (int k = 0; k < n; k++) b->ly[k] = march_rows(faces);
   // one pool: per instance two state buffers and the scratch planes
   std::vector<size_t> base(n);
   size_t total = 0;

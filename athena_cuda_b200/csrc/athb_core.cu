@@ -112,14 +112,7 @@ extern "C" int athb_create(const athb_config* cfg, athb_ctx** out) {
   c->dx1 = (cfg->x1max - cfg->x1min) / (double)cfg->nx1;
   c->dx2 = (cfg->x2max - cfg->x2min) / (double)cfg->nx2;
   c->x1_0 = cfg->x1min; c->x2_0 = cfg->x2min;
-  {
-    // rows per column march: short marches on small grids, where the step
-    // is latency-bound and more threads shorten it (64^2 and 128^2 run
-    // fastest at 1, 200x300 at 2-3), else enough marches for ~512 threads
-    // per SM (measured on B200, blast and field loop)
-    const long long cf = (long long)(cfg->nx1 + 4) * (cfg->nx2 + 3);
-    c->ly = cf < 40000 ? 1 : cf < 100000 ? 2 : (int)std::max(4LL, std::min(64LL, cf / (148LL * 512)));
-  }
+  c->ly = march_rows((long long)(cfg->nx1 + 4) * (cfg->nx2 + 3));
   cudaError_t e = cudaSetDevice(cfg->device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   const size_t state_bytes = sizeof(double) * (size_t)c->ps * NSTATE;
@@ -288,18 +281,12 @@ int athb_launch_integrate_split(athb_ctx* c, int from, cudaEvent_t* ev) {
       g, c->is - 1, c->js - 1, nx1 + 3, nx2 + 3, S_FX, S_FY);
   CUDA_TRY(cudaGetLastError());
 
-  CorrectGeom cg;
-  cg.xw = nx1 + 1; cg.xn = nx2 + 3;
-  cg.yw = nx1 + 3; cg.yn = nx2 + 1;
-  cg.ew = nx1 + 3; cg.en = nx2 + 3;
-  cg.xb = blocks_for((long long)cg.xw * cg.xn);
-  cg.yb = blocks_for((long long)cg.yw * cg.yn);
-  cg.eb = blocks_for((long long)cg.ew * cg.en);
+  const CorrectGeom cg = make_correct_geom(nx1, nx2);
   MARK(2);
   if (hlle)
-    k_correct<kFluxHlle><<<cg.xb + cg.yb + cg.eb, kThreads, 0, c->stream>>>(g, cg);
+    k_correct<kFluxHlle><<<cg.blocks, kThreads, 0, c->stream>>>(g, cg);
   else
-    k_correct<kFluxRoe><<<cg.xb + cg.yb + cg.eb, kThreads, 0, c->stream>>>(g, cg);
+    k_correct<kFluxRoe><<<cg.blocks, kThreads, 0, c->stream>>>(g, cg);
   CUDA_TRY(cudaGetLastError());
 
   MARK(3);

@@ -135,15 +135,9 @@ extern "C" int athb_integrate_noalloc(const athb_config* cfg, const double* d_in
   else k_predict<kFluxRoe><<<pg.nx_blocks + pg.ny_blocks, kThreads, 0, s>>>(gs, pg);
   k_emf<<<blocks_of((long long)(nx1 + 3) * (nx2 + 3)), kThreads, 0, s>>>(gs, gs.is - 1, gs.js - 1, nx1 + 3, nx2 + 3,
                                                                            S_FX, S_FY);
-  CorrectGeom cg;
-  cg.xw = nx1 + 1; cg.xn = nx2 + 3;
-  cg.yw = nx1 + 3; cg.yn = nx2 + 1;
-  cg.ew = nx1 + 3; cg.en = nx2 + 3;
-  cg.xb = blocks_of((long long)cg.xw * cg.xn);
-  cg.yb = blocks_of((long long)cg.yw * cg.yn);
-  cg.eb = blocks_of((long long)cg.ew * cg.en);
-  if (cfg->flux == ATHB_FLUX_HLLE) k_correct<kFluxHlle><<<cg.xb + cg.yb + cg.eb, kThreads, 0, s>>>(gs, cg);
-  else k_correct<kFluxRoe><<<cg.xb + cg.yb + cg.eb, kThreads, 0, s>>>(gs, cg);
+  const CorrectGeom cg = make_correct_geom(nx1, nx2);
+  if (cfg->flux == ATHB_FLUX_HLLE) k_correct<kFluxHlle><<<cg.blocks, kThreads, 0, s>>>(gs, cg);
+  else k_correct<kFluxRoe><<<cg.blocks, kThreads, 0, s>>>(gs, cg);
   k_emf<<<blocks_of((long long)(nx1 + 1) * (nx2 + 1)), kThreads, 0, s>>>(gs, gs.is, gs.js, nx1 + 1, nx2 + 1, S_FX2,
                                                                            S_FY2);
   const int n = nx1 * nx2;

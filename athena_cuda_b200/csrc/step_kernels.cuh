@@ -305,17 +305,29 @@ __device__ __forceinline__ void predict_y(const GridArgs& g, const PredictGeom& 
 // field loop 2048^2 1.90 -> 1.33 ms, blast 1024^2 0.645 -> 0.408 ms (FP64 pipe 38%
 // -> 55% busy), blast 200x300 53 -> 38 us.
 //
-// Resident blocks per SM the heavy kernels are compiled for (register caps of
-// 168 and 128 per thread): measured faster on B200 than the uncapped 255
-// registers and 2 blocks per SM despite the spills they cause.
-#ifndef ATHB_PREDICT_MIN_BLOCKS
-#define ATHB_PREDICT_MIN_BLOCKS 3
-#endif
-#ifndef ATHB_CORRECT_MIN_BLOCKS
-#define ATHB_CORRECT_MIN_BLOCKS 4
-#endif
-constexpr int kPredictMinBlocks = ATHB_PREDICT_MIN_BLOCKS;
-constexpr int kCorrectMinBlocks = ATHB_CORRECT_MIN_BLOCKS;
+// Resident blocks per SM the heavy kernels are compiled for.  k_predict keeps
+// 255 registers per thread and 2 blocks (8 warps) per SM: with the branches
+// gone its warps have independent FP64 work of their own, and the spills of 3
+// blocks (168 registers) cost more than the third block hides (field loop 2048^2
+// 1.275 against 1.331 ms, blast 1024^2 0.387 against 0.409; 4 blocks 1.70 and
+// 0.49 ms).  k_correct waits on memory as well and does best at 4 blocks of
+// 128 registers (2048^2: 0.612 ms; 3 blocks 0.658, 5 blocks 0.793).
+constexpr int kPredictMinBlocks = 2;
+constexpr int kCorrectMinBlocks = 4;
+
+// Rows per role-Y march for `faces` role-Y faces: as many marches as threads
+// are resident (148 SMs x 2 blocks x 128 threads) in one wave, or in as many
+// equal waves as keep a march at 56 rows or fewer.  Each march repeats one PLM
+// cell of its neighbour, so longer is cheaper until slots are left empty:
+// 1024^2 (28 rows) 379 us against 386 at 14 and 432 at 2; 512 x 384 (6) 85
+// against 98 at 10; 200 x 300 (2) 37 against 42 at 1 or 3.
+inline int march_rows(long long faces) {
+  constexpr long long kSlots = 148LL * kPredictMinBlocks * kThreads;
+  constexpr int kMaxRows = 56;
+  const long long rows = (faces + kSlots - 1) / kSlots;           // in one wave
+  const long long waves = (rows + kMaxRows - 1) / kMaxRows;
+  return (int)((rows + waves - 1) / waves);
+}
 
 // Block b of the predictor: the long role-Y column marches (ly rows each)
 // come first and the short role-X row segments (31 faces) last, so the
@@ -393,8 +405,20 @@ struct CorrectGeom {
   int xw, xn;   // role X: faces [is, ie+1] x [js-1, je+1]
   int yw, yn;   // role Y: faces [is-1, ie+1] x [js, je+1]
   int ew, en;   // role E: cells [is-1, ie+1] x [js-1, je+1]
-  int xb, yb, eb;
+  int xb, yb, eb, blocks;   // blocks of each role and of all
 };
+inline CorrectGeom make_correct_geom(int nx1, int nx2, int nt = kThreads) {
+  CorrectGeom cg;
+  cg.xw = nx1 + 1; cg.xn = nx2 + 3;
+  cg.yw = nx1 + 3; cg.yn = nx2 + 1;
+  cg.ew = nx1 + 3; cg.en = nx2 + 3;
+  auto bf = [nt](long long n) { return (int)((n + nt - 1) / nt); };
+  cg.xb = bf((long long)cg.xw * cg.xn);
+  cg.yb = bf((long long)cg.yw * cg.yn);
+  cg.eb = bf((long long)cg.ew * cg.en);
+  cg.blocks = cg.xb + cg.yb + cg.eb;
+  return cg;
+}
 
 template <int FLUX>
 __device__ __forceinline__ void correct_x(const GridArgs& g, int t, int w) {
