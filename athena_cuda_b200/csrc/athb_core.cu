@@ -261,9 +261,10 @@ int athb_launch_cfl(athb_ctx* c, int buf) {
   return ATHB_OK;
 }
 
-// The integrator proper: reads state[from], writes the interior of state[from^1].
+// The integrator proper: reads state[from], writes the interior of
+// state[from^1]; final: also ends the step (finalize_state, mode 1).
 // With ev != nullptr, events ev[0..5] bracket the five kernels.
-int athb_launch_integrate_split(athb_ctx* c, int from, cudaEvent_t* ev) {
+static int launch_integrate(athb_ctx* c, int from, int final, cudaEvent_t* ev) {
 #define MARK(k) do { if (ev) CUDA_TRY(cudaEventRecord(ev[k], c->stream)); } while (0)
   GridArgs g = grid_args(c, from);
   const int nx1 = c->cfg.nx1, nx2 = c->cfg.nx2;
@@ -296,39 +297,35 @@ int athb_launch_integrate_split(athb_ctx* c, int from, cudaEvent_t* ev) {
 
   MARK(4);
   const int n = nx1 * nx2;
-  k_update<<<blocks_for(n), kThreads, 0, c->stream>>>(g, nx1, n);
+  k_update<<<blocks_for(n), kThreads, 0, c->stream>>>(g, nx1, n, final);
   CUDA_TRY(cudaGetLastError());
   MARK(5);
   return ATHB_OK;
 #undef MARK
 }
 
-int athb_launch_integrate(athb_ctx* c, int from) { return athb_launch_integrate_split(c, from, nullptr); }
+int athb_launch_integrate(athb_ctx* c, int from) { return launch_integrate(c, from, 0, nullptr); }
 
 // Per-kernel timing of the loop step (CUDA events on the context's stream
-// between consecutive launches).  Kernel order: predict, emf(half), correct,
-// emf(full), update, finalize, ghost.
+// between consecutive launches): predict, emf(half), correct, emf(full),
+// update, finalize, ghost; the end of the step runs inside the update kernel and
+// reads 0.
 extern "C" int athb_profile_steps(athb_ctx* c, int nsteps, double* ms_out) {
   if (!c || nsteps < 1 || !ms_out) return athb_fail(ATHB_ERR_ARG, "bad arguments");
   CUDA_TRY(cudaSetDevice(c->cfg.device));
-  constexpr int K = 7;
+  constexpr int K = 6;
+  constexpr int slot[K] = {0, 1, 2, 3, 4, 6};
   std::vector<cudaEvent_t> ev((size_t)nsteps * (K + 1));
   for (auto& e : ev) CUDA_TRY(cudaEventCreate(&e));
-  for (int k = 0; k < K; k++) ms_out[k] = 0.0;
+  for (int k = 0; k < 7; k++) ms_out[k] = 0.0;
   int rc = ATHB_OK;
   for (int s = 0; s < nsteps && rc == ATHB_OK; s++) {
     cudaEvent_t* e = &ev[(size_t)s * (K + 1)];
-    const int from = c->cur;
-    GridArgs g = grid_args(c, from);
-    const int nx1 = c->cfg.nx1, nx2 = c->cfg.nx2;
-    rc = athb_launch_integrate_split(c, from, e);
+    rc = launch_integrate(c, c->cur, 1, e);
+    if (rc == ATHB_OK) rc = athb_launch_ghost(c, c->cur ^ 1);
     if (rc) break;
-    k_finalize<<<1, 1, 0, c->stream>>>(c->st, c->dx1, c->dx2, 1);
-    CUDA_TRY(cudaEventRecord(e[6], c->stream));
-    rc = athb_launch_ghost(c, from ^ 1);
-    CUDA_TRY(cudaEventRecord(e[7], c->stream));
+    CUDA_TRY(cudaEventRecord(e[K], c->stream));
     c->cur ^= 1;
-    (void)g; (void)nx1; (void)nx2;
   }
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   for (int s = 0; s < nsteps && rc == ATHB_OK; s++) {
@@ -336,21 +333,17 @@ extern "C" int athb_profile_steps(athb_ctx* c, int nsteps, double* ms_out) {
     for (int k = 0; k < K; k++) {
       float ms = 0.f;
       CUDA_TRY(cudaEventElapsedTime(&ms, e[k], e[k + 1]));
-      ms_out[k] += ms;
+      ms_out[slot[k]] += ms / nsteps;
     }
   }
   for (auto& e : ev) cudaEventDestroy(e);
-  for (int k = 0; k < K; k++) ms_out[k] /= nsteps;
   return rc;
 }
 
 // One iteration of the reference main loop (src/main.c:229-307) on the device.
 static int launch_loop_step(athb_ctx* c, int from) {
-  int rc = athb_launch_integrate(c, from);
-  if (rc) return rc;
-  k_finalize<<<1, 1, 0, c->stream>>>(c->st, c->dx1, c->dx2, 1);
-  CUDA_TRY(cudaGetLastError());
-  return athb_launch_ghost(c, from ^ 1);
+  const int rc = launch_integrate(c, from, 1, nullptr);
+  return rc ? rc : athb_launch_ghost(c, from ^ 1);
 }
 
 static int build_graph(athb_ctx* c, int from) {

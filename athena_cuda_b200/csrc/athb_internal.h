@@ -41,7 +41,6 @@ int athb_fail(int code, const char* fmt, ...);
 int athb_ctx_validate(const athb_config* cfg);
 int athb_set_clock(athb_ctx* c, double dt, double time, int nstep);
 int athb_launch_integrate(athb_ctx* c, int from);
-int athb_launch_integrate_split(athb_ctx* c, int from, cudaEvent_t* ev);
 int athb_launch_ghost(athb_ctx* c, int buf);
 int athb_launch_ghost_phase(athb_ctx* c, int buf, int mode, int sides);
 int athb_launch_cfl(athb_ctx* c, int buf);

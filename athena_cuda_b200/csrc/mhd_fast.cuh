@@ -110,7 +110,7 @@ ATHB_HD double with_sign(double x, double y) {
 // ---------------------------------------------------------------------------
 // Operand ranges, from the exponent bits alone
 // ---------------------------------------------------------------------------
-constexpr unsigned pow2_word(int e) { return (unsigned)(1023 + e) << 20; }
+ATHB_HD constexpr unsigned pow2_word(int e) { return (unsigned)(1023 + e) << 20; }
 // true unless 2^LO <= x < 2^HI (negative values and NaN are outside)
 template <int LO, int HI> ATHB_HD bool outside(double x) {
   return hi_word(x) - pow2_word(LO) >= pow2_word(HI) - pow2_word(LO);

@@ -19,7 +19,8 @@
 //               role E: 7             (cell-centred EMF at t^{n+1/2})
 //   k_emf_full  step 9 corner EMF
 //   k_update    steps 9 (CT), 11a, 11b, 13 + new_dt per cell (src/new_dt.c)
-//               with warp-shuffle / block max and one 64-bit atomicMax
+//               with warp-shuffle / block max and one 64-bit atomicMax; in the
+//               main loop its last block does k_finalize's work
 //   k_finalize  time += dt, nstep++, dt rule (src/new_dt.c:93-97), tlim clamp
 //               (src/main.c:230-232)
 //   k_ghost     set_bvals (src/set_bvals.c:114-1031) for both directions in
@@ -625,14 +626,73 @@ __device__ __forceinline__ void block_max_to(double v, unsigned long long* dst, 
   }
 }
 
-__device__ __forceinline__ double update_cell(const GridArgs& g, int nx1, int ncell, int t);
-
 // ---------------------------------------------------------------------------
 // k_update: CT on the face fields, conservative update, cell-centred B and the
-// per-cell CFL rate.  One thread per interior cell.
+// per-cell CFL rate, one thread per interior cell; in the main loop (final != 0)
+// its last block also ends the step.
+//
+// On a large grid it streams (2048^2: 4.7 TB/s); on a small one it is latency:
+// every load comes before the first store, as a store to one plane holds back
+// the loads behind it, and the last block to finish advances the clock in place
+// of a launch of its own.
 // ---------------------------------------------------------------------------
-static __global__ void __launch_bounds__(kThreads) k_update(GridArgs g, int nx1, int ncell) {
+// CT, conservative update and cell-centred field of interior cell t; returns
+// the cell's CFL rate (0 for t >= ncell).
+__device__ __forceinline__ double update_cell(const GridArgs& g, int nx1, int ncell, int t) {
   const StepState& st = *g.st;
+  if (t >= ncell) return 0.0;
+  const int j = g.js + t / nx1, i = g.is + t % nx1;
+  const long long ps = g.ps, o = off(g, j, i), P = g.pitch;
+  const double* s = g.in;
+  double* out = g.out;
+  const double* emf = g.scr + S_EMF * ps;
+  const double* fx = g.scr + S_FX2 * ps;
+  const double* fy = g.scr + S_FY2 * ps;
+  const double dtodx1 = st.dtodx1, dtodx2 = st.dtodx2;
+  const double e00 = emf[o], e01 = emf[o + 1], e10 = emf[o + P], e11 = emf[o + P + 1];
+  double b1 = s[P_B1I * ps + o], b1e = s[P_B1I * ps + o + 1];
+  double b2 = s[P_B2I * ps + o], b2n = s[P_B2I * ps + o + P];
+  double d = s[P_D * ps + o], m1 = s[P_M1 * ps + o], m2 = s[P_M2 * ps + o];
+  double m3 = s[P_M3 * ps + o], e = s[P_E * ps + o], b3c = s[P_B3C * ps + o];
+  const double x0 = fx[0 * ps + o + 1] - fx[0 * ps + o], x1 = fx[1 * ps + o + 1] - fx[1 * ps + o],
+               x2 = fx[2 * ps + o + 1] - fx[2 * ps + o], x3 = fx[3 * ps + o + 1] - fx[3 * ps + o],
+               x4 = fx[4 * ps + o + 1] - fx[4 * ps + o], x6 = fx[6 * ps + o + 1] - fx[6 * ps + o];
+  const double y0 = fy[0 * ps + o + P] - fy[0 * ps + o], y1 = fy[1 * ps + o + P] - fy[1 * ps + o],
+               y2 = fy[2 * ps + o + P] - fy[2 * ps + o], y3 = fy[3 * ps + o + P] - fy[3 * ps + o],
+               y4 = fy[4 * ps + o + P] - fy[4 * ps + o], y5 = fy[5 * ps + o + P] - fy[5 * ps + o];
+  // step 9: CT for a full step (src/__integrate_2d__.c:476-485)
+  b1 -= dtodx2 * (e10 - e00);
+  b1e -= dtodx2 * (e11 - e01);
+  b2 += dtodx1 * (e01 - e00);
+  b2n += dtodx1 * (e11 - e10);
+  // step 11a (src/__integrate_2d__.c:491-501)
+  d -= dtodx1 * x0; m1 -= dtodx1 * x1; m2 -= dtodx1 * x2;
+  m3 -= dtodx1 * x3; e -= dtodx1 * x4; b3c -= dtodx1 * x6;
+  // step 11b (src/__integrate_2d__.c:508-518); the B1c/B2c updates of 11a/11b
+  // are overwritten by step 13 and are not formed
+  d -= dtodx2 * y0; m1 -= dtodx2 * y3; m2 -= dtodx2 * y1;
+  m3 -= dtodx2 * y2; e -= dtodx2 * y4; b3c -= dtodx2 * y5;
+  out[P_B1I * ps + o] = b1;
+  if (i == g.ie) out[P_B1I * ps + o + 1] = b1e;
+  out[P_B2I * ps + o] = b2;
+  if (j == g.je) out[P_B2I * ps + o + P] = b2n;
+  out[P_D * ps + o] = d;
+  out[P_M1 * ps + o] = m1;
+  out[P_M2 * ps + o] = m2;
+  out[P_M3 * ps + o] = m3;
+  out[P_E * ps + o] = e;
+  // step 13 (src/__integrate_2d__.c:526-534)
+  out[P_B1C * ps + o] = 0.5 * (b1 + b1e);
+  out[P_B2C * ps + o] = 0.5 * (b2 + b2n);
+  out[P_B3C * ps + o] = b3c;
+  out[P_B3I * ps + o] = b3c;
+  return cell_dti(d, m1, m2, m3, e, g.eos, g.dx1, g.dx2);
+}
+
+__device__ __forceinline__ void finalize_state(StepState& st, double dx1, double dx2, int mode);
+
+static __global__ void __launch_bounds__(kThreads) k_update(GridArgs g, int nx1, int ncell, int final) {
+  StepState& st = *g.st;
   const int t = blockIdx.x * kThreads + threadIdx.x;
   if (st.done) {
     // the loop has ended: carry the state over unchanged so that the buffer
@@ -646,63 +706,15 @@ static __global__ void __launch_bounds__(kThreads) k_update(GridArgs g, int nx1,
     }
     return;
   }
-  block_max_to(update_cell(g, nx1, ncell, t), &g.st->max_dti_bits, &g.st->flags);
-}
-
-// CT, conservative update and cell-centred field of interior cell t; returns
-// the cell's CFL rate (0 for t >= ncell).
-__device__ __forceinline__ double update_cell(const GridArgs& g, int nx1, int ncell, int t) {
-  const StepState& st = *g.st;
-  double dti = 0.0;
-  if (t < ncell) {
-    const int j = g.js + t / nx1, i = g.is + t % nx1;
-    const long long ps = g.ps, o = off(g, j, i), P = g.pitch;
-    const double* s = g.in;
-    double* out = g.out;
-    const double* emf = g.scr + S_EMF * ps;
-    const double* fx = g.scr + S_FX2 * ps;
-    const double* fy = g.scr + S_FY2 * ps;
-    const double dtodx1 = st.dtodx1, dtodx2 = st.dtodx2;
-    // step 9: CT for a full step (src/__integrate_2d__.c:476-485)
-    const double e00 = emf[o], e01 = emf[o + 1], e10 = emf[o + P], e11 = emf[o + P + 1];
-    const double b1 = s[P_B1I * ps + o] - dtodx2 * (e10 - e00);
-    const double b1e = s[P_B1I * ps + o + 1] - dtodx2 * (e11 - e01);
-    const double b2 = s[P_B2I * ps + o] + dtodx1 * (e01 - e00);
-    const double b2n = s[P_B2I * ps + o + P] + dtodx1 * (e11 - e10);
-    out[P_B1I * ps + o] = b1;
-    if (i == g.ie) out[P_B1I * ps + o + 1] = b1e;
-    out[P_B2I * ps + o] = b2;
-    if (j == g.je) out[P_B2I * ps + o + P] = b2n;
-    // step 11a (src/__integrate_2d__.c:491-501)
-    double d = s[P_D * ps + o], m1 = s[P_M1 * ps + o], m2 = s[P_M2 * ps + o];
-    double m3 = s[P_M3 * ps + o], e = s[P_E * ps + o], b3c = s[P_B3C * ps + o];
-    d -= dtodx1 * (fx[0 * ps + o + 1] - fx[0 * ps + o]);
-    m1 -= dtodx1 * (fx[1 * ps + o + 1] - fx[1 * ps + o]);
-    m2 -= dtodx1 * (fx[2 * ps + o + 1] - fx[2 * ps + o]);
-    m3 -= dtodx1 * (fx[3 * ps + o + 1] - fx[3 * ps + o]);
-    e -= dtodx1 * (fx[4 * ps + o + 1] - fx[4 * ps + o]);
-    b3c -= dtodx1 * (fx[6 * ps + o + 1] - fx[6 * ps + o]);
-    // step 11b (src/__integrate_2d__.c:508-518); the B1c/B2c updates of 11a/11b
-    // are overwritten by step 13 and are not formed
-    d -= dtodx2 * (fy[0 * ps + o + P] - fy[0 * ps + o]);
-    m1 -= dtodx2 * (fy[3 * ps + o + P] - fy[3 * ps + o]);
-    m2 -= dtodx2 * (fy[1 * ps + o + P] - fy[1 * ps + o]);
-    m3 -= dtodx2 * (fy[2 * ps + o + P] - fy[2 * ps + o]);
-    e -= dtodx2 * (fy[4 * ps + o + P] - fy[4 * ps + o]);
-    b3c -= dtodx2 * (fy[5 * ps + o + P] - fy[5 * ps + o]);
-    out[P_D * ps + o] = d;
-    out[P_M1 * ps + o] = m1;
-    out[P_M2 * ps + o] = m2;
-    out[P_M3 * ps + o] = m3;
-    out[P_E * ps + o] = e;
-    // step 13 (src/__integrate_2d__.c:526-534)
-    out[P_B1C * ps + o] = 0.5 * (b1 + b1e);
-    out[P_B2C * ps + o] = 0.5 * (b2 + b2n);
-    out[P_B3C * ps + o] = b3c;
-    out[P_B3I * ps + o] = b3c;
-    dti = cell_dti(d, m1, m2, m3, e, g.eos, g.dx1, g.dx2);
+  block_max_to(update_cell(g, nx1, ncell, t), &st.max_dti_bits, &st.flags);
+  if (final && threadIdx.x == 0) {
+    __threadfence();   // this block's maximum before its arrival
+    if (atomicAdd(&st.arrived, 1u) == gridDim.x - 1) {
+      __threadfence();
+      st.arrived = 0u;
+      finalize_state(st, g.dx1, g.dx2, 1);
+    }
   }
-  return dti;
 }
 
 // Standalone CFL reduction over the interior of the step's input buffer
@@ -865,24 +877,33 @@ __device__ __forceinline__ void ghost_item(const GridArgs& g, int sx, int sy, in
     const int k = u % side;
     i = k < g.is ? k : g.ie + 1 + (k - g.is);
   }
+  // all loads before the first store: the planes are one array to the
+  // compiler, and a store would hold back the loads behind it
   double* s = g.out;
   const long long ps = g.ps, o = off(g, j, i);
   int sj, si;
-  bool f1, f2;
-  if (ghost_src(g, 0, j, i, mode, sides, sj, si, f1, f2)) {
+  bool f1, f2, f_;
+  double v[9], b1 = 0.0, b2 = 0.0;
+  const bool on0 = ghost_src(g, 0, j, i, mode, sides, sj, si, f1, f2);
+  if (on0) {
     const long long so = off(g, sj, si);
 #pragma unroll
-    for (int p = 0; p < 8; p++) {
-      double v = s[p * ps + so];
-      if ((p == P_M1 && f1) || (p == P_M2 && f2)) v = -v;  // reflecting walls
-      s[p * ps + o] = v;
-    }
-    s[P_B3I * ps + o] = s[P_B3I * ps + so];
+    for (int p = 0; p < 8; p++) v[p] = s[p * ps + so];
+    v[8] = s[P_B3I * ps + so];
   }
-  if (ghost_src(g, 1, j, i, mode, sides, sj, si, f1, f2))
-    s[P_B1I * ps + o] = s[P_B1I * ps + off(g, sj, si)];
-  if (ghost_src(g, 2, j, i, mode, sides, sj, si, f1, f2))
-    s[P_B2I * ps + o] = s[P_B2I * ps + off(g, sj, si)];
+  const bool on1 = ghost_src(g, 1, j, i, mode, sides, sj, si, f_, f_);
+  if (on1) b1 = s[P_B1I * ps + off(g, sj, si)];
+  const bool on2 = ghost_src(g, 2, j, i, mode, sides, sj, si, f_, f_);
+  if (on2) b2 = s[P_B2I * ps + off(g, sj, si)];
+  if (on0) {
+    if (f1) v[P_M1] = -v[P_M1];   // reflecting walls
+    if (f2) v[P_M2] = -v[P_M2];
+#pragma unroll
+    for (int p = 0; p < 8; p++) s[p * ps + o] = v[p];
+    s[P_B3I * ps + o] = v[8];
+  }
+  if (on1) s[P_B1I * ps + o] = b1;
+  if (on2) s[P_B2I * ps + o] = b2;
 }
 
 static __global__ void __launch_bounds__(kThreads) k_ghost(GridArgs g, int sx, int sy, int nframe, int mode,

@@ -368,7 +368,7 @@ def ours(a) -> None:
             "warmup": a.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f64",
             "data": "synthetic (field-loop initial condition, src/field_loop.c)",
-            "config": config_dict(a), "gpu_launches": 7 * a.steps * ws, "roofline": roofline,
+            "config": config_dict(a), "gpu_launches": 6 * a.steps * ws, "roofline": roofline,
             "clocks": clk.summary()}
 
     if not a.no_e2e:
