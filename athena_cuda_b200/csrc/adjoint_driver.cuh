@@ -128,16 +128,41 @@ template <int STAGE, int FLUX> struct AdjFn {
   }
 };
 
+// One pass of the ghost fold over bands of places, all planes in one launch:
+// item (k, m) is plane k / n1 and place (k % n1, m) of the bands.  A band pair
+// is the first nlo places from lo and the rest up to hi.
+struct Bands {
+  int n, nlo, lo, hi;
+  ATHB_MEM int at(int k) const { return k < nlo ? lo + k : hi + 1 - n + k; }
+};
 struct FoldFn {
   double* l;
   long long ps;
   int pitch;
   GhostGeom g;
-  int pass;   // 2: x2 rows, 1: x1 columns, 0: clear the frame
-  ATHB_MEM void operator()(int j, int i) const {
-    if (pass == 2) fold_x2(l, ps, pitch, g, j, i);
-    else if (pass == 1) fold_x1(l, ps, pitch, g, j, i);
-    else clear_frame(l, ps, pitch, g, j, i);
+  int pass;      // 2: x2 rows, 1: x1 columns, 0: clear the frame
+  Bands rows;    // rows visited (pass 0: unused)
+  Bands cols;
+  ATHB_MEM void operator()(int k, int m) const {
+    if (pass == 0) {   // m runs over the frame: whole rows below and above, then the columns beside the rows between
+      const int nrows = g.js + g.sy - g.je - 1, ncols = g.is + g.sx - g.ie - 1;
+      const int u = m - nrows * g.sx;
+      int j, i;
+      if (u < 0) {
+        j = m / g.sx;
+        i = m % g.sx;
+        if (j >= g.js) j += g.je + 1 - g.js;
+      } else {
+        j = g.js + u / ncols;
+        i = u % ncols;
+        if (i >= g.is) i += g.ie + 1 - g.is;
+      }
+      clear_frame(l, ps, pitch, g, k, j, i);
+      return;
+    }
+    const int p = k / rows.n, j = rows.at(k % rows.n), i = cols.at(m);
+    if (pass == 2) fold_x2(l, ps, pitch, g, p, j, i);
+    else fold_x1(l, ps, pitch, g, p, j, i);
   }
 };
 
@@ -552,24 +577,18 @@ template <class Exec> struct AdjointDriver {
     const GhostGeom gg = ghost_geom();
     constexpr int kBand = kNghostA + 2;
     const int is = G.is, ie = G.ie, js = G.js, je = G.je;
-    if (2 * kBand >= je + 2 - js) {
-      x.items(GenRange{0, G.sx - 1, js, je + 1}, FoldFn{l, G.ps, G.pitch, gg, 2});
-    } else {
-      x.items(GenRange{0, G.sx - 1, js, js + kBand - 1}, FoldFn{l, G.ps, G.pitch, gg, 2});
-      x.items(GenRange{0, G.sx - 1, je + 2 - kBand, je + 1}, FoldFn{l, G.ps, G.pitch, gg, 2});
-    }
-    if (2 * kBand >= ie + 2 - is) {
-      x.items(GenRange{is, ie + 1, js, je + 1}, FoldFn{l, G.ps, G.pitch, gg, 1});
-    } else {
-      x.items(GenRange{is, is + kBand - 1, js, je + 1}, FoldFn{l, G.ps, G.pitch, gg, 1});
-      x.items(GenRange{ie + 2 - kBand, ie + 1, js, je + 1}, FoldFn{l, G.ps, G.pitch, gg, 1});
-    }
-    // the frame: rows below js and above je (B2i's row je+1 is kept by the
-    // functor), the columns left of is and right of ie on the rows between
-    x.items(GenRange{0, G.sx - 1, 0, js - 1}, FoldFn{l, G.ps, G.pitch, gg, 0});
-    x.items(GenRange{0, G.sx - 1, je + 1, G.sy - 1}, FoldFn{l, G.ps, G.pitch, gg, 0});
-    x.items(GenRange{0, is - 1, js, je}, FoldFn{l, G.ps, G.pitch, gg, 0});
-    x.items(GenRange{ie + 1, G.sx - 1, js, je}, FoldFn{l, G.ps, G.pitch, gg, 0});
+    // the two bands of [lo, hi] next to its ends (all of it where they meet)
+    auto bands = [](int lo, int hi) {
+      const int n = hi - lo + 1;
+      return 2 * kBand >= n ? Bands{n, n, lo, hi} : Bands{2 * kBand, kBand, lo, hi};
+    };
+    const Bands rows = bands(js, je + 1), cols = bands(is, ie + 1);
+    const Bands all_rows{je + 2 - js, je + 2 - js, js, je + 1}, all_cols{G.sx, G.sx, 0, G.sx - 1};
+    x.items(GenRange{0, all_cols.n - 1, 0, NSTATE * rows.n - 1}, FoldFn{l, G.ps, G.pitch, gg, 2, rows, all_cols});
+    x.items(GenRange{0, cols.n - 1, 0, NSTATE * all_rows.n - 1}, FoldFn{l, G.ps, G.pitch, gg, 1, all_rows, cols});
+    // the frame (B2i's row je+1 and B1i's column ie+1 are kept by the functor)
+    const int frame = (js + G.sy - je - 1) * G.sx + (is + G.sx - ie - 1) * (je + 1 - js);
+    x.items(GenRange{0, frame - 1, 0, NSTATE - 1}, FoldFn{l, G.ps, G.pitch, gg, 0, rows, cols});
   }
 
   // Reverse step n: S^n in S[cur].  lam[lc] holds the adjoint of S^{n+1}

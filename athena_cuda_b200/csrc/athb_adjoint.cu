@@ -55,12 +55,11 @@ template <int STAGE, int FLUX> struct ItemMinBlocks<AdjFn<STAGE, FLUX>> {
 };
 
 template <class F>
-__global__ void __launch_bounds__(kItemThreads, ItemMinBlocks<F>::value) k_items(GenRange r, long long n, F f) {
-  const long long t = (long long)blockIdx.x * kItemThreads + threadIdx.x;
+__global__ void __launch_bounds__(kItemThreads, ItemMinBlocks<F>::value) k_items(GenRange r, unsigned n, F f) {
+  const unsigned t = blockIdx.x * kItemThreads + threadIdx.x;   // 32 bits: a 64-bit division costs a small stage dearly
   if (t >= n) return;
-  int j, i;
-  range_item(r, t, j, i);
-  f(j, i);
+  const unsigned w = (unsigned)(r.i1 - r.i0 + 1);
+  f(r.j0 + (int)(t / w), r.i0 + (int)(t % w));
 }
 
 template <class F>
@@ -222,7 +221,8 @@ struct GpuExec {
   template <class F> void items(const GenRange& r, const F& f) {
     const long long n = range_count(r);
     if (n <= 0 || err != cudaSuccess) return;
-    k_items<F><<<blocks(n, kItemThreads), kItemThreads, 0, s>>>(r, n, f);
+    if (n > INT_MAX) { note(cudaErrorInvalidValue); return; }   // grids hold at most 2^30 cells
+    k_items<F><<<blocks(n, kItemThreads), kItemThreads, 0, s>>>(r, (unsigned)n, f);
   }
   template <class F> void single(const F& f) {
     if (err != cudaSuccess) return;

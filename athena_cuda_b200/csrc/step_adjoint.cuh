@@ -68,26 +68,49 @@ struct AdjArgs {
   double dx1, dx2;
   Eos eos;
   ATHB_MEM long long o(int j, int i) const { return (long long)j * pitch + i; }
-  ATHB_MEM double s(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return in[p * ps + off]; }
-  ATHB_MEM double t(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return tape[p * ps + off]; }
-  ATHB_MEM double lo(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return lout[p * ps + off]; }
+  ATHB_MEM double s(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return ro(in + p * ps + off); }
+  ATHB_MEM double t(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return ro(tape + p * ps + off); }
+  ATHB_MEM double lo(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return ro(lout + p * ps + off); }
   ATHB_MEM double& li(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return lin[p * ps + off]; }
   ATHB_MEM double& a(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return adj[p * ps + off]; }
-  ATHB_MEM double av(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return adj[p * ps + off]; }
+  ATHB_MEM double av(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return ro(adj + p * ps + off); }
+
+ private:
+  // What a stage reads through s, t, lo and av it never writes (each stage's
+  // output planes are others than its input planes), so these are read-only
+  // loads, which the compiler may move above the stage's stores: the small
+  // stages are otherwise chains of one memory round trip per plane.
+  ATHB_MEM static double ro(const double* q) {
+#if defined(__CUDA_ARCH__)
+    return __ldg(q);
+#else
+    return *q;
+#endif
+  }
 };
+
+// lin[p[k]] += v[k] at one place, all loads before the first store.
+template <int N>
+ATHB_HD void lin_add(const AdjArgs& a, long long o, const int (&p)[N], const double (&v)[N]) {
+  double x[N];
+#pragma unroll
+  for (int k = 0; k < N; k++) x[k] = a.li(p[k], o);
+#pragma unroll
+  for (int k = 0; k < N; k++) a.li(p[k], o) = x[k] + v[k];
+}
 
 ATHB_HD bool in_range(const GenRange& r, int j, int i) { return j >= r.j0 && j <= r.j1 && i >= r.i0 && i <= r.i1; }
 
-// λ of the conserved vector of a sweep (as loaded by gen_cons) added to lin
-ATHB_HD void lin_add_cons(const AdjArgs& a, long long o, int dir, const Cons1& ub) {
-  a.li(P_D, o) += ub.d;
-  a.li(P_E, o) += ub.e;
+// λ of the conserved vector of a sweep (as loaded by gen_cons) and of its
+// normal field added to lin
+ATHB_HD void lin_add_cons(const AdjArgs& a, long long o, int dir, const Cons1& ub, double bnb) {
+  const double v[8] = {ub.d, ub.e, ub.mx, ub.my, ub.mz, ub.by, ub.bz, bnb};
   if (dir == 0) {
-    a.li(P_M1, o) += ub.mx; a.li(P_M2, o) += ub.my; a.li(P_M3, o) += ub.mz;
-    a.li(P_B2C, o) += ub.by; a.li(P_B3C, o) += ub.bz;
+    const int p[8] = {P_D, P_E, P_M1, P_M2, P_M3, P_B2C, P_B3C, P_B1C};
+    lin_add(a, o, p, v);
   } else {
-    a.li(P_M2, o) += ub.mx; a.li(P_M3, o) += ub.my; a.li(P_M1, o) += ub.mz;
-    a.li(P_B3C, o) += ub.by; a.li(P_B1C, o) += ub.bz;
+    const int p[8] = {P_D, P_E, P_M2, P_M3, P_M1, P_B3C, P_B1C, P_B2C};
+    lin_add(a, o, p, v);
   }
 }
 ATHB_HD Cons1 adj_cons(const AdjArgs& a, int base, long long o) {
@@ -148,14 +171,14 @@ ATHB_HD void corner_k(const AdjArgs& a, int full, int j, int i, double k[8]) {
 // ===========================================================================
 ATHB_HD void adj_update(const AdjArgs& a, int j, int i) {
   const long long o = a.o(j, i), P = a.pitch;
-  double dtb = 0.0;
+  const double dt0 = a.a(A_DT, o);
+  double dtb = 0.0, l1b = 0.0, l2b = 0.0;
   // b1 at x face (j,i), i in [is, ie+1], j in [js, je]
   if (j <= a.je) {
     double lb = a.lo(P_B1I, o);
     if (i <= a.ie) lb += 0.5 * a.lo(P_B1C, o);
     if (i - 1 >= a.is) lb += 0.5 * a.lo(P_B1C, o - 1);
-    a.a(A_LB1, o) = lb;
-    a.li(P_B1I, o) += lb;
+    l1b = lb;
     dtb += -lb * (a.t(G_EMF1, o + P) - a.t(G_EMF1, o)) / a.dx2;
   }
   // b2 at y face (j,i), j in [js, je+1], i in [is, ie]
@@ -163,16 +186,13 @@ ATHB_HD void adj_update(const AdjArgs& a, int j, int i) {
     double lb = a.lo(P_B2I, o);
     if (j <= a.je) lb += 0.5 * a.lo(P_B2C, o);
     if (j - 1 >= a.js) lb += 0.5 * a.lo(P_B2C, o - P);
-    a.a(A_LB2, o) = lb;
-    a.li(P_B2I, o) += lb;
+    l2b = lb;
     dtb += lb * (a.t(G_EMF1, o + 1) - a.t(G_EMF1, o)) / a.dx1;
   }
   // cell planes
   if (i <= a.ie && j <= a.je) {
     const double ld = a.lo(P_D, o), l1 = a.lo(P_M1, o), l2 = a.lo(P_M2, o), l3 = a.lo(P_M3, o), le = a.lo(P_E, o);
     const double lb3 = a.lo(P_B3C, o) + a.lo(P_B3I, o);
-    a.li(P_D, o) += ld; a.li(P_M1, o) += l1; a.li(P_M2, o) += l2; a.li(P_M3, o) += l3; a.li(P_E, o) += le;
-    a.li(P_B3C, o) += lb3;
     // d -= dtodx1 (fx(o+1) - fx(o)) ... ; d -= dtodx2 (fy(o+P) - fy(o)) ...
     double g1 = 0.0, g2 = 0.0;
     g1 += ld * (a.t(G_FX2 + 0, o + 1) - a.t(G_FX2 + 0, o));
@@ -188,8 +208,17 @@ ATHB_HD void adj_update(const AdjArgs& a, int j, int i) {
     g2 += le * (a.t(G_FY2 + 4, o + P) - a.t(G_FY2 + 4, o));
     g2 += lb3 * (a.t(G_FY2 + 5, o + P) - a.t(G_FY2 + 5, o));
     dtb += -g1 / a.dx1 - g2 / a.dx2;
+    const int p[8] = {P_D, P_M1, P_M2, P_M3, P_E, P_B3C, P_B1I, P_B2I};
+    const double v[8] = {ld, l1, l2, l3, le, lb3, l1b, l2b};
+    lin_add(a, o, p, v);
+  } else if (j <= a.je) {
+    a.li(P_B1I, o) += l1b;
+  } else if (i <= a.ie) {
+    a.li(P_B2I, o) += l2b;
   }
-  a.a(A_DT, o) += dtb;
+  if (j <= a.je) a.a(A_LB1, o) = l1b;
+  if (i <= a.ie) a.a(A_LB2, o) = l2b;
+  a.a(A_DT, o) = dt0 + dtb;
 }
 
 // Corner emf of the full step: corners [is, ie+1] x [js, je+1].
@@ -417,6 +446,7 @@ ATHB_HD double correct_y_dtb(const AdjArgs& a, int j, int i, const Cons1& lul, c
 template <int FLUX>
 ATHB_HD void adj_correct_x(const AdjArgs& a, int j, int i) {
   const long long o = a.o(j, i);
+  const double dt0 = a.a(A_DT, o);
   Cons1 ul, ur;
   double b1f;
   correct_x_states(a, j, i, ul, ur, b1f);
@@ -429,15 +459,16 @@ ATHB_HD void adj_correct_x(const AdjArgs& a, int j, int i) {
   riemann_adj<FLUX>(ul, ur, wl, wr, b1f, a.eos, adj_cons(a, A_FX2, o), ulb, urb, wlb, wrb, b1fb);
   cons_to_prim_adj(ul, b1f, a.eos, wlb, ulb, b1fb);
   cons_to_prim_adj(ur, b1f, a.eos, wrb, urb, b1fb);
+  a.a(A_DT, o) = dt0 + correct_x_dtb(a, j, i, ulb, urb);
   adj_put_cons(a, A_ULX, o, ulb);
   adj_put_cons(a, A_URX, o, urb);
   a.a(A_B1F, o) = b1fb;
-  a.a(A_DT, o) += correct_x_dtb(a, j, i, ulb, urb);
 }
 
 template <int FLUX>
 ATHB_HD void adj_correct_y(const AdjArgs& a, int j, int i) {
   const long long o = a.o(j, i);
+  const double dt0 = a.a(A_DT, o);
   Cons1 ul, ur;
   double b2f;
   correct_y_states(a, j, i, ul, ur, b2f);
@@ -450,10 +481,10 @@ ATHB_HD void adj_correct_y(const AdjArgs& a, int j, int i) {
   riemann_adj<FLUX>(ul, ur, wl, wr, b2f, a.eos, adj_cons(a, A_FY2, o), ulb, urb, wlb, wrb, b2fb);
   cons_to_prim_adj(ul, b2f, a.eos, wlb, ulb, b2fb);
   cons_to_prim_adj(ur, b2f, a.eos, wrb, urb, b2fb);
+  a.a(A_DT, o) = dt0 + correct_y_dtb(a, j, i, ulb, urb);
   adj_put_cons(a, A_ULY, o, ulb);
   adj_put_cons(a, A_URY, o, urb);
   a.a(A_B2F, o) = b2fb;
-  a.a(A_DT, o) += correct_y_dtb(a, j, i, ulb, urb);
 }
 
 // step 7 reversed: cells [is-1, ie+1] x [js-1, je+1]
@@ -474,17 +505,18 @@ ATHB_HD void adj_correct_e(const AdjArgs& a, int j, int i) {
   const double B2c = 0.5 * (b2f_c + b2f_n);
   const double e = (B1c * M2 - B2c * M1) / d;
   const double lam = a.av(A_ECC1, o);
+  const double dt0 = a.a(A_DT, o);
   const double ld = -lam * e / d, lM1 = -lam * B2c / d, lM2 = lam * B1c / d;
+  const int p[3] = {P_D, P_M1, P_M2};
+  const double v[3] = {ld, lM1, lM2};
+  lin_add(a, o, p, v);
   a.a(A_HALF + 0, o) = ld;
   a.a(A_HALF + 1, o) = lM1;
   a.a(A_HALF + 2, o) = lM2;
   a.a(A_HALF + 3, o) = lam * M2 / d;
   a.a(A_HALF + 4, o) = -lam * M1 / d;
-  a.li(P_D, o) += ld;
-  a.li(P_M1, o) += lM1;
-  a.li(P_M2, o) += lM2;
-  a.a(A_DT, o) += 0.5 * (-(ld * dfx0 + lM1 * dfx1 + lM2 * dfx2)) / a.dx1 +
-                  0.5 * (-(ld * dfy0 + lM1 * dfy3 + lM2 * dfy1)) / a.dx2;
+  a.a(A_DT, o) = dt0 + (0.5 * (-(ld * dfx0 + lM1 * dfx1 + lM2 * dfx2)) / a.dx1 +
+                        0.5 * (-(ld * dfy0 + lM1 * dfy3 + lM2 * dfy1)) / a.dx2);
 }
 
 // Every consumer of the half-step face fields: x faces [is-1, ie+2] x
@@ -493,26 +525,29 @@ ATHB_HD void adj_correct_e(const AdjArgs& a, int j, int i) {
 ATHB_HD void adj_half_faces(const AdjArgs& a, int j, int i) {
   const long long o = a.o(j, i), P = a.pitch;
   const GenRange E = range_correct_e(a.is, a.ie, a.js, a.je);
+  const bool xface = j <= a.je + 1, yface = i <= a.ie + 1;
+  const double dt0 = a.a(A_DT, o);
+  const double b10 = xface ? a.li(P_B1I, o) : 0.0, b20 = yface ? a.li(P_B2I, o) : 0.0;
   double dtb = 0.0;
-  if (j <= a.je + 1) {  // x face
+  if (xface) {
     double lb = 0.0;
     if (in_range(range_correct_x(a.is, a.ie, a.js, a.je), j, i)) lb += a.av(A_B1F, o);
     if (in_range(E, j, i)) lb += 0.5 * a.av(A_HALF + 3, o);
     if (in_range(E, j, i - 1)) lb += 0.5 * a.av(A_HALF + 3, o - 1);
     a.a(A_LB1F, o) = lb;
-    a.li(P_B1I, o) += lb;
+    a.li(P_B1I, o) = b10 + lb;
     dtb += -lb * (a.t(G_EMF0, o + P) - a.t(G_EMF0, o)) * 0.5 / a.dx2;
   }
-  if (i <= a.ie + 1) {  // y face
+  if (yface) {
     double lb = 0.0;
     if (in_range(range_correct_y(a.is, a.ie, a.js, a.je), j, i)) lb += a.av(A_B2F, o);
     if (in_range(E, j, i)) lb += 0.5 * a.av(A_HALF + 4, o);
     if (in_range(E, j - 1, i)) lb += 0.5 * a.av(A_HALF + 4, o - P);
     a.a(A_LB2F, o) = lb;
-    a.li(P_B2I, o) += lb;
+    a.li(P_B2I, o) = b20 + lb;
     dtb += lb * (a.t(G_EMF0, o + 1) - a.t(G_EMF0, o)) * 0.5 / a.dx1;
   }
-  a.a(A_DT, o) += dtb;
+  a.a(A_DT, o) = dt0 + dtb;
 }
 
 // Half-step corner emf: corners [is-1, ie+2] x [js-1, je+2].
@@ -591,11 +626,9 @@ ATHB_HD void adj_flux1(const AdjArgs& a, int j, int i) {
     if (v != 0.0) {
       const double d = a.s(P_D, o), M1 = a.s(P_M1, o), M2 = a.s(P_M2, o), B1 = a.s(P_B1C, o), B2 = a.s(P_B2C, o);
       const double e = (B1 * M2 - B2 * M1) / d;
-      a.li(P_B1C, o) += v * M2 / d;
-      a.li(P_M2, o) += v * B1 / d;
-      a.li(P_B2C, o) -= v * M1 / d;
-      a.li(P_M1, o) -= v * B2 / d;
-      a.li(P_D, o) -= v * e / d;
+      const int p[5] = {P_B1C, P_M2, P_B2C, P_M1, P_D};
+      const double w[5] = {v * M2 / d, v * B1 / d, -(v * M1 / d), -(v * B2 / d), -(v * e / d)};
+      lin_add(a, o, p, w);
     }
   }
 }
@@ -668,11 +701,9 @@ ATHB_HD void adj_sources(const AdjArgs& a, int j, int i) {
       lB3 += h2 * dby * (a.av(A_URY + 2, o) + V3 * a.av(A_URY + 4, o));
       lV3 += h2 * dby * (a.av(A_URY + 5, o) + B3 * a.av(A_URY + 4, o));
     }
-    a.li(P_B1C, o) += lB1;
-    a.li(P_B2C, o) += lB2;
-    a.li(P_B3C, o) += lB3;
-    a.li(P_M3, o) += lV3 / d;
-    a.li(P_D, o) -= lV3 * V3 / d;
+    const int p[5] = {P_B1C, P_B2C, P_B3C, P_M3, P_D};
+    const double v[5] = {lB1, lB2, lB3, lV3 / d, -(lV3 * V3 / d)};
+    lin_add(a, o, p, v);
   }
   // x face (j,i): B1i through dbx of ul/ur of x faces i, i+1, i-1
   if (j <= a.je + 1 && j >= a.js - 1 && i >= a.is - 1 && i <= a.ie + 2)
@@ -731,9 +762,7 @@ ATHB_HD void adj_plm(const AdjArgs& a, int dir, int j, int i) {
   const double src = (mt / d) * db / dxs;
   const double lsrc = a.c.hdt * lsum;
   double dtb = 0.5 * src * lsum;
-  a.a(dir == 0 ? A_SRCX : A_SRCY, o) = lsrc;
-  a.li(dir == 0 ? P_M2 : P_M1, o) += lsrc * db / dxs / d;
-  a.li(P_D, o) -= lsrc * (mt / d / d) * db / dxs;
+  const double dt0 = a.a(A_DT, o);
   // PLM
   const Cons1 um = state_cons(a, o - step, dir), u0 = state_cons(a, o, dir), up = state_cons(a, o + step, dir);
   const int bxp = dir == 0 ? P_B1C : P_B2C;
@@ -745,12 +774,15 @@ ATHB_HD void adj_plm(const AdjArgs& a, int dir, int j, int i) {
   double bxcb = 0.0, dtodxb = 0.0;
   plm_cell_adj(wm, w0, wp, a.s(bxp, o), dir == 0 ? a.c.dtodx1 : a.c.dtodx2, a.eos, lwl, lwr, wmb, w0b, wpb, bxcb,
                dtodxb);
+  const int p[3] = {dir == 0 ? P_M2 : P_M1, P_D, bxp};
+  const double v[3] = {lsrc * db / dxs / d, -(lsrc * (mt / d / d) * db / dxs), bxcb};
+  lin_add(a, o, p, v);
+  a.a(dir == 0 ? A_SRCX : A_SRCY, o) = lsrc;
   adj_put_prim(a, dir == 0 ? A_WXM : A_WYM, o, wmb);
   adj_put_prim(a, dir == 0 ? A_WX0 : A_WY0, o, w0b);
   adj_put_prim(a, dir == 0 ? A_WXP : A_WYP, o, wpb);
-  a.li(bxp, o) += bxcb;
   dtb += dtodxb / dxs;
-  a.a(A_DT, o) += dtb;
+  a.a(A_DT, o) = dt0 + dtb;
 }
 
 // Primitive-variable adjoints of cell (j,i) gathered from the PLM of cells
@@ -775,8 +807,7 @@ ATHB_HD void adj_prim_gather(const AdjArgs& a, int dir, int j, int i) {
     zero(ub);
     double bxb = 0.0;
     cons_to_prim_adj(state_cons(a, o, dir), a.s(bxp, o), a.eos, lw, ub, bxb);
-    lin_add_cons(a, o, dir, ub);
-    a.li(bxp, o) += bxb;
+    lin_add_cons(a, o, dir, ub, bxb);
   }
   // normal face field at face (j,i)
   const GenRange F = dir == 0 ? range_riemann_x(a.is, a.ie, a.js, a.je) : range_riemann_y(a.is, a.ie, a.js, a.je);
@@ -849,63 +880,51 @@ ATHB_HD void gen_ghost(const Planes<T>& s, long long ps, int pitch, const GhostG
   (void)gxa; (void)gya;
 }
 
-// Adjoint, pass 1 (x2): rows [js, je(+1 for B2i)], every column: add the
-// adjoints of the ghost rows that copy this row.
-ATHB_HD void fold_x2(double* l, long long ps, int pitch, const GhostGeom& g, int j, int i) {
-  for (int kind = 0; kind < 3; kind++) {
-    const int je_int = g.je + (kind == 2 ? 1 : 0);
-    if (j < g.js || j > je_int) continue;
-    const long long o = (long long)j * pitch + i;
-    for (int gq = 0; gq < 2 * kNghostA; gq++) {   // the ghost rows: js-4..js-1, je_int+1..je_int+4
-      const int jj = gq < kNghostA ? g.js - kNghostA + gq : je_int + 1 + (gq - kNghostA);
-      if (jj < 0 || jj >= g.sy) continue;
-      bool f = false;
-      if (ghost_map1(jj, g.js, g.je, kind == 2, g.bc[2], g.bc[3], f) != j) continue;
-      const long long q = (long long)jj * pitch + i;
-      if (kind == 0) {
-        for (int p = 0; p < 8; p++) l[p * ps + o] += (p == P_M2 && f) ? -l[p * ps + q] : l[p * ps + q];
-        l[P_B3I * ps + o] += l[P_B3I * ps + q];
-      } else {
-        const int p = kind == 1 ? P_B1I : P_B2I;
-        l[p * ps + o] += l[p * ps + q];
-      }
-    }
-  }
-}
-// Adjoint, pass 2 (x1): interior cells add the adjoints of the ghost
-// columns of their row that copy them.
-ATHB_HD void fold_x1(double* l, long long ps, int pitch, const GhostGeom& g, int j, int i) {
-  for (int kind = 0; kind < 3; kind++) {
-    const int ie_int = g.ie + (kind == 1 ? 1 : 0), je_int = g.je + (kind == 2 ? 1 : 0);
-    if (j < g.js || j > je_int || i < g.is || i > ie_int) continue;
-    const long long o = (long long)j * pitch + i;
-    for (int gq = 0; gq < 2 * kNghostA; gq++) {   // the ghost columns: is-4..is-1, ie_int+1..ie_int+4
-      const int ii = gq < kNghostA ? g.is - kNghostA + gq : ie_int + 1 + (gq - kNghostA);
-      if (ii < 0 || ii >= g.sx) continue;
-      bool f = false;
-      if (ghost_map1(ii, g.is, g.ie, kind == 1, g.bc[0], g.bc[1], f) != i) continue;
-      const long long q = (long long)j * pitch + ii;
-      if (kind == 0) {
-        for (int p = 0; p < 8; p++) l[p * ps + o] += (p == P_M1 && f) ? -l[p * ps + q] : l[p * ps + q];
-        l[P_B3I * ps + o] += l[P_B3I * ps + q];
-      } else {
-        const int p = kind == 1 ? P_B1I : P_B2I;
-        l[p * ps + o] += l[p * ps + q];
-      }
-    }
-  }
-}
-// Zero every entry that is not a cell the step writes (ghosts after the
-// fold), so the folded adjoint is exactly the interior one.
-ATHB_HD void clear_frame(double* l, long long ps, int pitch, const GhostGeom& g, int j, int i) {
+// The kind of a plane at the boundaries: 1 for B1i, 2 for B2i, else 0.
+ATHB_HD int plane_kind(int p) { return p == P_B1I ? 1 : p == P_B2I ? 2 : 0; }
+
+// Adjoint, pass 1 (x2) of plane p: rows [js, je(+1 for B2i)], every column: add
+// the adjoints of the ghost rows that copy this row.  One item per plane and
+// place (11 times the threads, none with a chain of 11 planes).
+ATHB_HD void fold_x2(double* l, long long ps, int pitch, const GhostGeom& g, int p, int j, int i) {
+  const int kind = plane_kind(p), je_int = g.je + (kind == 2 ? 1 : 0);
+  if (j < g.js || j > je_int) return;
+  double* q = l + p * ps;
   const long long o = (long long)j * pitch + i;
-  const bool cell_int = j >= g.js && j <= g.je && i >= g.is && i <= g.ie;
-  for (int p = 0; p < NSTATE; p++) {
-    bool keep = cell_int;
-    if (p == P_B1I) keep = j >= g.js && j <= g.je && i >= g.is && i <= g.ie + 1;
-    if (p == P_B2I) keep = j >= g.js && j <= g.je + 1 && i >= g.is && i <= g.ie;
-    if (!keep) l[p * ps + o] = 0.0;
+  double v = q[o];
+#pragma unroll
+  for (int gq = 0; gq < 2 * kNghostA; gq++) {   // the ghost rows: js-4..js-1, je_int+1..je_int+4
+    const int jj = gq < kNghostA ? g.js - kNghostA + gq : je_int + 1 + (gq - kNghostA);
+    bool f = false;
+    if (jj < 0 || jj >= g.sy || ghost_map1(jj, g.js, g.je, kind == 2, g.bc[2], g.bc[3], f) != j) continue;
+    const double x = q[(long long)jj * pitch + i];
+    v += (p == P_M2 && f) ? -x : x;
   }
+  q[o] = v;
+}
+// Adjoint, pass 2 (x1) of plane p: interior cells add the adjoints of the
+// ghost columns of their row that copy them.
+ATHB_HD void fold_x1(double* l, long long ps, int pitch, const GhostGeom& g, int p, int j, int i) {
+  const int kind = plane_kind(p), ie_int = g.ie + (kind == 1 ? 1 : 0), je_int = g.je + (kind == 2 ? 1 : 0);
+  if (j < g.js || j > je_int || i < g.is || i > ie_int) return;
+  double* q = l + p * ps + (long long)j * pitch;
+  double v = q[i];
+#pragma unroll
+  for (int gq = 0; gq < 2 * kNghostA; gq++) {   // the ghost columns: is-4..is-1, ie_int+1..ie_int+4
+    const int ii = gq < kNghostA ? g.is - kNghostA + gq : ie_int + 1 + (gq - kNghostA);
+    bool f = false;
+    if (ii < 0 || ii >= g.sx || ghost_map1(ii, g.is, g.ie, kind == 1, g.bc[0], g.bc[1], f) != i) continue;
+    const double x = q[ii];
+    v += (p == P_M1 && f) ? -x : x;
+  }
+  q[i] = v;
+}
+// Zero plane p at a place that is not one the step writes (ghosts after the
+// fold), so the folded adjoint is exactly the interior one.
+ATHB_HD void clear_frame(double* l, long long ps, int pitch, const GhostGeom& g, int p, int j, int i) {
+  const int kind = plane_kind(p);
+  const bool keep = j >= g.js && j <= g.je + (kind == 2 ? 1 : 0) && i >= g.is && i <= g.ie + (kind == 1 ? 1 : 0);
+  if (!keep) l[p * ps + (long long)j * pitch + i] = 0.0;
 }
 
 }  // namespace athb
