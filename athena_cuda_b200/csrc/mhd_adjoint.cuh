@@ -21,7 +21,7 @@
 //   src/flux_hlle.c:60-199       flux_hlle
 #pragma once
 
-#include "mhd_physics.cuh"
+#include "mhd_fast.cuh"
 
 namespace athb {
 
@@ -531,6 +531,378 @@ ATHB_HD void plm_cell_adj(const Prim1& wm, const Prim1& w0, const Prim1& wp, dou
   prim_add_arr(wmb, Wmb);
   prim_add_arr(w0b, W0b);
   prim_add_arr(wpb, Wpb);
+}
+
+// ---------------------------------------------------------------------------
+// The same adjoint in the fast form of mhd_fast.cuh: the forward values (and so
+// every branch) are plm_cell_fast's, bit for bit; the reverse uses the pairs
+// the eigenvectors come in (waves n and 6-n share all entries up to sign, so
+// each entry is visited once per pair), fused multiply-adds, and the
+// reciprocals and 1/(2 root) the forward has at hand, and divides nowhere.
+// A third of the FP64 instructions of plm_cell_adj, no branch around them.
+// ---------------------------------------------------------------------------
+ATHB_HD double mad(double a, double b, double c) { return fma_n(a, b, c); }
+// x, as a value the compiler takes for a new one: what is formed from it is
+// formed again instead of kept in a register (or a spill) since the first time.
+ATHB_HD double anew(double x) {
+#if defined(__CUDA_ARCH__)
+  asm volatile("" : "+d"(x));
+#endif
+  return x;
+}
+
+// Adjoint of esys_prim_fast: Eb holds the adjoints of the entries (signs as in
+// PrimEigT); db, v1b, .. are set.
+ATHB_HD void esys_prim_reverse(const EsysKeep& K, const PrimLeft& L, double d, double p, double di, double b1,
+                               double b2, double b3, const Eos& eos, const PrimEig& Eb, double& db, double& v1b,
+                               double& pb, double& b1b, double& b2b, double& b3b) {
+  const double af = K.af, as = K.as, cf = K.cf, cs = K.cs, na = K.na, s = K.sgn, a = K.a, sq = K.sqrtd;
+  const double bet2 = K.bet2, bet3 = K.bet3, asq = K.asq;
+  const double qf = cf * af * s, qs = cs * as * s, AF = a * af * sq, AS = a * as * sq;
+  const double qf2 = na * qf, qs2 = na * qs, AFP = na * AF * di, ASP = na * AS * di;
+  const double rs = K.h_d + K.h_d;   // 1/sqrt(d)
+  // products of rows and columns with the transverse direction
+  const double aspb = mad(Eb.L05, bet2, Eb.L06 * bet3), afpb = -mad(Eb.L25, bet2, Eb.L26 * bet3);
+  const double qs2b = mad(Eb.L02, bet2, Eb.L03 * bet3), qf2b = -mad(Eb.L22, bet2, Eb.L23 * bet3);
+  const double ASb0 = mad(Eb.R50, bet2, Eb.R60 * bet3), AFb0 = -mad(Eb.R52, bet2, Eb.R62 * bet3);
+  const double qsb0 = mad(Eb.R20, bet2, Eb.R30 * bet3), qfb0 = -mad(Eb.R22, bet2, Eb.R32 * bet3);
+  const double hrs = 0.5 * s * rs, ssq = s * sq;
+  double bet2b = mad(Eb.L05, ASP, mad(-Eb.L25, AFP, mad(Eb.L02, qs2, -Eb.L22 * qf2)));
+  bet2b = mad(Eb.L16, hrs, mad(0.5, Eb.L13, bet2b));
+  bet2b += mad(Eb.R61, ssq, mad(Eb.R50, AS, mad(-Eb.R52, AF, mad(Eb.R20, qs, mad(-Eb.R22, qf, Eb.R31)))));
+  double bet3b = mad(Eb.L06, ASP, mad(-Eb.L26, AFP, mad(Eb.L03, qs2, -Eb.L23 * qf2)));
+  bet3b = mad(-Eb.L15, hrs, mad(-0.5, Eb.L12, bet3b));
+  bet3b += mad(-Eb.R51, ssq, mad(Eb.R60, AS, mad(-Eb.R62, AF, mad(Eb.R30, qs, mad(-Eb.R32, qf, -Eb.R21)))));
+  double sqrtdb = rs * mad(Eb.L15, L.l15, -Eb.L16 * L.l16);
+  sqrtdb = mad(s, mad(Eb.R61, bet2, -Eb.R51 * bet3), sqrtdb);
+  // scalars of the left rows
+  double nab = di * mad(Eb.L24, as, Eb.L04 * af);
+  nab = mad(-Eb.L21, cs * as, mad(-Eb.L01, cf * af, nab));
+  nab = mad(di, mad(aspb, AS, afpb * AF), mad(qs2b, qs, mad(qf2b, qf, nab)));
+  double asb_ = mad(Eb.L24, na * di, -Eb.L21 * (na * cs)), afb_ = mad(Eb.L04, na * di, -Eb.L01 * (na * cf));
+  double dib = na * mad(Eb.L24, as, mad(Eb.L04, af, mad(aspb, AS, afpb * AF)));
+  double csb = -Eb.L21 * (na * as), cfb = -Eb.L01 * (na * af);
+  double asqb = L.l34 * mad(Eb.L34, L.l34, -nab * na);
+  const double ASb = mad(aspb, na * di, ASb0), AFb = mad(afpb, na * di, AFb0);
+  const double qsb = mad(qs2b, na, qsb0), qfb = mad(qf2b, na, qfb0);
+  // right columns
+  const double dasq = d * asq;
+  db = mad(asq, mad(Eb.R42, as, Eb.R40 * af), mad(Eb.R02, as, Eb.R00 * af));
+  asqb = mad(d, mad(Eb.R42, as, Eb.R40 * af), asqb);
+  asb_ = mad(Eb.R42, dasq, mad(-Eb.R12, cs, mad(Eb.R02, d, asb_)));
+  afb_ = mad(Eb.R40, dasq, mad(-Eb.R10, cf, mad(Eb.R00, d, afb_)));
+  csb = mad(-Eb.R12, as, csb);
+  cfb = mad(-Eb.R10, af, cfb);
+  // eigenvalues
+  v1b = Eb.ev[0] + Eb.ev[1] + Eb.ev[2] + Eb.ev[3] + Eb.ev[4] + Eb.ev[5] + Eb.ev[6];
+  cfb += Eb.ev[6] - Eb.ev[0];
+  const double vaxb = Eb.ev[5] - Eb.ev[1];
+  csb += Eb.ev[4] - Eb.ev[2];
+  double vaxsqb = K.vax > 0.0 ? vaxb * K.h_vax : 0.0;
+  const double ab = sq * mad(ASb, as, AFb * af);
+  asb_ = mad(ASb * a, sq, mad(qsb * cs, s, asb_));
+  afb_ = mad(AFb * a, sq, mad(qfb * cf, s, afb_));
+  sqrtdb = mad(a, mad(ASb, as, AFb * af), sqrtdb);
+  csb = mad(qsb * as, s, csb);
+  cfb = mad(qfb * af, s, cfb);
+  asqb = mad(ab, K.h_a, asqb);
+  db = mad(sqrtdb, K.h_d, db);
+  double cssqb = 0.0, cfsqb = 0.0, c2b = 0.0;
+  if (K.general) {
+    // alpha_f^2 = (asq - cssq)/c2, alpha_s^2 = (cfsq - asq)/c2.  Where a weight is
+    // small these terms are large and cancel later, so each is rounded once
+    // and used as it is.
+    const double Afr = afb_ * K.h_af * K.r_c2, Asr = asb_ * K.h_as * K.r_c2;
+    asqb = (asqb + Afr) - Asr;
+    cssqb = -Afr;
+    cfsqb = Asr;
+    c2b = -mad(Afr, af * af, Asr * (as * as));
+  }
+  double btsqb = 0.0;
+  b2b = 0.0;
+  b3b = 0.0;
+  if (K.btsq != 0.0 && !(K.btsq < kBetaFreeze * (b1 * b1 + d * asq))) {   // freeze_beta
+    // r_bt is 1/|b_t| here: a field whose square is small enough to be scaled is frozen
+    const double btb = -K.r_bt * mad(bet2b, bet2, bet3b * bet3);
+    b2b = bet2b * K.r_bt;
+    b3b = bet3b * K.r_bt;
+    btsqb = 0.5 * btb * K.r_bt;
+  }
+  if (cs > 0.0) cssqb = mad(csb, K.h_cs, cssqb);
+  const double cr = cssqb * K.r_cfsq;
+  asqb = mad(cr, K.vaxsq, asqb);
+  vaxsqb = mad(cr, asq, vaxsqb);
+  cfsqb = mad(-cr, K.cssq, cfsqb);
+  cfsqb = mad(cfb, K.h_cf, cfsqb);
+  const double tsumb = 0.5 * cfsqb;
+  c2b += tsumb;
+  const double Xb = K.c2 > 0.0 ? c2b * K.h_c2 : 0.0;
+  const double tdifb = 2.0 * K.tdif * Xb;
+  const double plus = tdifb + tsumb;
+  asqb = mad(4.0 * K.ct2, Xb, asqb) + (tsumb - tdifb);
+  const double ct2b = mad(4.0 * asq, Xb, plus);
+  vaxsqb += plus;
+  btsqb = mad(ct2b, di, btsqb);
+  pb = asqb * eos.gamma * di;
+  dib = mad(ct2b, K.btsq, mad(asqb * eos.gamma, p, mad(vaxsqb * b1, b1, dib)));
+  b1b = 2.0 * vaxsqb * b1 * di;
+  b2b = mad(2.0 * b2, btsqb, b2b);
+  b3b = mad(2.0 * b3, btsqb, b3b);
+  db = mad(-di * di, dib, db);
+}
+
+// plm_cell_adj for three cells that pass cell_outside (di = 1/w0.d, hdtodx =
+// 0.5 dtodx); the outputs are set, not accumulated.  false: outside the ranges,
+// the outputs are not valid.
+ATHB_HD bool plm_cell_adj_fast(const Prim1& wm, const Prim1& w0, const Prim1& wp, double di, double bxc,
+                               double hdtodx, const Eos& eos, const Prim1& wlb, const Prim1& wrb, Prim1& wmb,
+                               Prim1& w0b, Prim1& wpb, double& bxcb, double& dtodxb) {
+  bool bad = false;
+  PrimLeft L;
+  PrimRight R;
+  EsysKeep K;
+  esys_prim_fast(w0, di, bxc, eos, L, R, K, bad);
+  bad |= K.tiny_waves;   // their derivatives count where their values do not
+  double Wm[7], W0[7], Wp[7], Pl[7], Pr[7];
+  prim_arr(wm, Wm); prim_arr(w0, W0); prim_arr(wp, Wp);
+  prim_arr(wlb, Pl); prim_arr(wrb, Pr);
+  PlmSlopes S;
+  limited_slopes(Wm, W0, Wp, L, R, S, bad);
+  // which slope each limited wave took, and the sign its adjoint passes with
+  unsigned took_l = 0, took_r = 0, took_c = 0, took_g = 0, neg = 0;
+#pragma unroll
+  for (int n = 0; n < 7; n++) {
+    const double x = fabs(S.al[n]), y = fabs(S.ar[n]), c = 0.5 * fabs(S.ac[n]), v = fabs(S.ag[n]);
+    const bool on = S.al[n] * S.ar[n] > 0.0;
+    const bool one_sided = 2.0 * rmin(x, y) < rmin(c, v), left = x < y, centred = c < v;
+    const bool minus = S.ac[n] < 0.0;
+    took_l |= (unsigned)(on && one_sided && left) << n;
+    took_r |= (unsigned)(on && one_sided && !left) << n;
+    took_c |= (unsigned)(on && !one_sided && centred) << n;
+    took_g |= (unsigned)(on && !one_sided && !centred) << n;
+    const bool other = one_sided ? (left ? S.al[n] < 0.0 : S.ar[n] < 0.0) : centred ? minus : S.ag[n] < 0.0;
+    neg |= (unsigned)(minus != other) << n;
+  }
+  double dW[7];
+  unsigned own_l = 0, own_r = 0, cen_l = 0, cen_r = 0;   // bit n: own value kept; clipped at the centre cell's
+#pragma unroll
+  for (int n = 0; n < 7; n++) {
+    const double half = 0.5 * S.dWm[n];
+    double l = W0[n] - half, r = W0[n] + half;
+    const bool cm = W0[n] < Wm[n], cp = W0[n] < Wp[n];
+    const double lo = cm ? W0[n] : Wm[n], hi = cm ? Wm[n] : W0[n];
+    const bool l1 = lo > l;
+    l = l1 ? lo : l;
+    const bool l2 = hi < l;
+    l = l2 ? hi : l;
+    const double lor = cp ? W0[n] : Wp[n], hir = cp ? Wp[n] : W0[n];
+    const bool r1 = lor > r;
+    r = r1 ? lor : r;
+    const bool r2 = hir < r;
+    r = r2 ? hir : r;
+    own_l |= (unsigned)(!l1 && !l2) << n;
+    own_r |= (unsigned)(!r1 && !r2) << n;
+    // the second clip, where both hold, decides
+    cen_l |= (unsigned)(l2 ? W0[n] > Wm[n] : l1 && cm) << n;
+    cen_r |= (unsigned)(r2 ? W0[n] > Wp[n] : r1 && cp) << n;
+    dW[n] = r - l;
+  }
+
+  // ---- reverse of steps 9 and 8 ----
+  PrimEig Eb;
+  const double H = hdtodx;
+  double dWb[7];
+  dtodxb = 0.0;
+  double e0b = 0.0, e6b = 0.0;
+  // wave n: strength w, q1 (q0) = its column times the adjoint of pWl (pWr).
+  // Returns the coefficient of w, and A (B), the weight of pWl's (pWr's) adjoint
+  // in the adjoint of the column.
+  auto wave = [&](int n, double w, double q1, double q0, double& A, double& B) {
+    const bool on1 = n != 6 && R.ev[n] != 0.0, on0 = n != 0 && R.ev[n] < 0.0;
+    const double d1 = on1 ? R.ev[6] - R.ev[n] : 0.0, d0 = on0 ? R.ev[0] - R.ev[n] : 0.0;
+    q1 = on1 ? q1 : 0.0;
+    q0 = on0 ? q0 : 0.0;
+    const double t = mad(q1, d1, q0 * d0), Hw = H * w;
+    A = Hw * d1;
+    B = Hw * d0;
+    e6b = mad(q1, Hw, e6b);
+    e0b = mad(q0, Hw, e0b);
+    Eb.ev[n] = -(q1 + q0) * Hw;
+    dtodxb = mad(0.5 * w, t, dtodxb);
+    return H * t;
+  };
+  {  // waves 0 and 6
+    const double t = mad(L.l01, dW[1], mad(L.l02, dW[2], L.l03 * dW[3]));
+    const double u = mad(L.l04, dW[4], mad(L.l05, dW[5], L.l06 * dW[6]));
+    const double x1 = mad(R.R00, Pl[0], mad(R.R40, Pl[4], mad(R.R50, Pl[5], R.R60 * Pl[6])));
+    const double y1 = mad(R.R10, Pl[1], mad(R.R20, Pl[2], R.R30 * Pl[3]));
+    const double x0 = mad(R.R00, Pr[0], mad(R.R40, Pr[4], mad(R.R50, Pr[5], R.R60 * Pr[6])));
+    const double y0 = mad(R.R10, Pr[1], mad(R.R20, Pr[2], R.R30 * Pr[3]));
+    double A0, B0, A6, B6;
+    const double c0 = wave(0, u + t, x1 + y1, 0.0, A0, B0), c6 = wave(6, u - t, 0.0, x0 - y0, A6, B6);
+    const double Ap = A0 + A6, Am = A0 - A6, Bp = B0 + B6, Bm = B0 - B6, cp = c0 + c6, cm = c0 - c6;
+    Eb.R00 = mad(Ap, Pl[0], Bp * Pr[0]); Eb.R40 = mad(Ap, Pl[4], Bp * Pr[4]);
+    Eb.R50 = mad(Ap, Pl[5], Bp * Pr[5]); Eb.R60 = mad(Ap, Pl[6], Bp * Pr[6]);
+    Eb.R10 = mad(Am, Pl[1], Bm * Pr[1]); Eb.R20 = mad(Am, Pl[2], Bm * Pr[2]); Eb.R30 = mad(Am, Pl[3], Bm * Pr[3]);
+    Eb.L01 = cm * dW[1]; Eb.L02 = cm * dW[2]; Eb.L03 = cm * dW[3];
+    Eb.L04 = cp * dW[4]; Eb.L05 = cp * dW[5]; Eb.L06 = cp * dW[6];
+    dWb[1] = cm * L.l01; dWb[2] = cm * L.l02; dWb[3] = cm * L.l03;
+    dWb[4] = cp * L.l04; dWb[5] = cp * L.l05; dWb[6] = cp * L.l06;
+  }
+  {  // waves 1 and 5
+    const double t = mad(L.b2, dW[3], -L.b3 * dW[2]), u = mad(L.l16, dW[6], -L.l15 * dW[5]);
+    const double x1 = mad(R.R51, Pl[5], R.R61 * Pl[6]), y1 = mad(R.R21, Pl[2], R.R31 * Pl[3]);
+    const double x0 = mad(R.R51, Pr[5], R.R61 * Pr[6]), y0 = mad(R.R21, Pr[2], R.R31 * Pr[3]);
+    double A1, B1, A5, B5;
+    const double c1 = wave(1, u + t, x1 + y1, x0 + y0, A1, B1), c5 = wave(5, u - t, x1 - y1, x0 - y0, A5, B5);
+    const double Ap = A1 + A5, Am = A1 - A5, Bp = B1 + B5, Bm = B1 - B5, cp = c1 + c5, cm = c1 - c5;
+    Eb.R21 = mad(Am, Pl[2], Bm * Pr[2]); Eb.R31 = mad(Am, Pl[3], Bm * Pr[3]);
+    Eb.R51 = mad(Ap, Pl[5], Bp * Pr[5]); Eb.R61 = mad(Ap, Pl[6], Bp * Pr[6]);
+    Eb.L12 = cm * dW[2]; Eb.L13 = cm * dW[3]; Eb.L15 = cp * dW[5]; Eb.L16 = cp * dW[6];
+    dWb[2] = mad(-cm, L.b3, dWb[2]); dWb[3] = mad(cm, L.b2, dWb[3]);
+    dWb[5] = mad(-cp, L.l15, dWb[5]); dWb[6] = mad(cp, L.l16, dWb[6]);
+  }
+  {  // waves 2 and 4
+    const double t = mad(L.l21, dW[1], -mad(L.l22, dW[2], L.l23 * dW[3]));
+    const double u = mad(L.l24, dW[4], -mad(L.l25, dW[5], L.l26 * dW[6]));
+    const double x1 = mad(R.R02, Pl[0], mad(R.R42, Pl[4], mad(R.R52, Pl[5], R.R62 * Pl[6])));
+    const double y1 = mad(R.R12, Pl[1], mad(R.R22, Pl[2], R.R32 * Pl[3]));
+    const double x0 = mad(R.R02, Pr[0], mad(R.R42, Pr[4], mad(R.R52, Pr[5], R.R62 * Pr[6])));
+    const double y0 = mad(R.R12, Pr[1], mad(R.R22, Pr[2], R.R32 * Pr[3]));
+    double A2, B2, A4, B4;
+    const double c2 = wave(2, u + t, x1 + y1, x0 + y0, A2, B2), c4 = wave(4, u - t, x1 - y1, x0 - y0, A4, B4);
+    const double Ap = A2 + A4, Am = A2 - A4, Bp = B2 + B4, Bm = B2 - B4, cp = c2 + c4, cm = c2 - c4;
+    Eb.R02 = mad(Ap, Pl[0], Bp * Pr[0]); Eb.R42 = mad(Ap, Pl[4], Bp * Pr[4]);
+    Eb.R52 = mad(Ap, Pl[5], Bp * Pr[5]); Eb.R62 = mad(Ap, Pl[6], Bp * Pr[6]);
+    Eb.R12 = mad(Am, Pl[1], Bm * Pr[1]); Eb.R22 = mad(Am, Pl[2], Bm * Pr[2]); Eb.R32 = mad(Am, Pl[3], Bm * Pr[3]);
+    Eb.L21 = cm * dW[1]; Eb.L22 = cm * dW[2]; Eb.L23 = cm * dW[3];
+    Eb.L24 = cp * dW[4]; Eb.L25 = cp * dW[5]; Eb.L26 = cp * dW[6];
+    dWb[1] = mad(cm, L.l21, dWb[1]); dWb[2] = mad(-cm, L.l22, dWb[2]); dWb[3] = mad(-cm, L.l23, dWb[3]);
+    dWb[4] = mad(cp, L.l24, dWb[4]); dWb[5] = mad(-cp, L.l25, dWb[5]); dWb[6] = mad(-cp, L.l26, dWb[6]);
+  }
+  {  // wave 3
+    double A3, B3;
+    const double c3 = wave(3, mad(-L.l34, dW[4], dW[0]), Pl[0], Pr[0], A3, B3);
+    Eb.L34 = c3 * dW[4];
+    dWb[0] = c3;
+    dWb[4] = mad(-c3, L.l34, dWb[4]);
+  }
+  {  // step 8: pWl = r - qx dW, pWr = l - qy dW
+    const double m6 = rmax(R.ev[6], 0.0), m0 = rmin(R.ev[0], 0.0), qx = m6 * H, qy = m0 * H;
+    double qxb = 0.0, qyb = 0.0;
+#pragma unroll
+    for (int n = 0; n < 7; n++) {
+      qxb = mad(-Pl[n], dW[n], qxb);
+      qyb = mad(-Pr[n], dW[n], qyb);
+      dWb[n] = mad(-qx, Pl[n], mad(-qy, Pr[n], dWb[n]));
+    }
+    if (R.ev[6] > 0.0) e6b = mad(qxb, H, e6b);
+    if (R.ev[0] < 0.0) e0b = mad(qyb, H, e0b);
+    dtodxb = mad(0.5 * m6, qxb, mad(0.5 * m0, qyb, dtodxb));
+  }
+  Eb.ev[0] += e0b;
+  Eb.ev[6] += e6b;
+  // step 7: dW = r - l, and the clips
+  double Wmb[7], W0b[7], Wpb[7], g[7];
+#pragma unroll
+  for (int n = 0; n < 7; n++) {
+    const double lr = Pl[n] + dWb[n], ll = Pr[n] - dWb[n];
+    const bool ol = (own_l >> n) & 1u, orr = (own_r >> n) & 1u, cl = (cen_l >> n) & 1u, cr = (cen_r >> n) & 1u;
+    g[n] = 0.5 * ((orr ? lr : 0.0) - (ol ? ll : 0.0));
+    W0b[n] = (ol || cl ? ll : 0.0) + (orr || cr ? lr : 0.0);
+    Wmb[n] = ol || cl ? 0.0 : ll;
+    Wpb[n] = orr || cr ? 0.0 : lr;
+  }
+  // step 5: dWm = R da
+  double dab[7];
+  {
+    const double x0 = mad(g[0], R.R00, mad(g[4], R.R40, mad(g[5], R.R50, g[6] * R.R60)));
+    const double y0 = mad(g[1], R.R10, mad(g[2], R.R20, g[3] * R.R30));
+    const double x1 = mad(g[5], R.R51, g[6] * R.R61), y1 = mad(g[2], R.R21, g[3] * R.R31);
+    const double x2 = mad(g[0], R.R02, mad(g[4], R.R42, mad(g[5], R.R52, g[6] * R.R62)));
+    const double y2 = mad(g[1], R.R12, mad(g[2], R.R22, g[3] * R.R32));
+    dab[0] = x0 + y0; dab[6] = x0 - y0;
+    dab[1] = x1 + y1; dab[5] = x1 - y1;
+    dab[2] = x2 + y2; dab[4] = x2 - y2;
+    dab[3] = g[0];
+    const double* da = S.da;
+    const double p0 = da[0] + da[6], m0 = da[0] - da[6], p1 = da[1] + da[5], m1 = da[1] - da[5], p2 = da[2] + da[4],
+                 m2 = da[2] - da[4];
+    Eb.R00 = mad(g[0], p0, Eb.R00); Eb.R02 = mad(g[0], p2, Eb.R02);
+    Eb.R10 = mad(g[1], m0, Eb.R10); Eb.R12 = mad(g[1], m2, Eb.R12);
+    Eb.R20 = mad(g[2], m0, Eb.R20); Eb.R21 = mad(g[2], m1, Eb.R21); Eb.R22 = mad(g[2], m2, Eb.R22);
+    Eb.R30 = mad(g[3], m0, Eb.R30); Eb.R31 = mad(g[3], m1, Eb.R31); Eb.R32 = mad(g[3], m2, Eb.R32);
+    Eb.R40 = mad(g[4], p0, Eb.R40); Eb.R42 = mad(g[4], p2, Eb.R42);
+    Eb.R50 = mad(g[5], p0, Eb.R50); Eb.R51 = mad(g[5], p1, Eb.R51); Eb.R52 = mad(g[5], p2, Eb.R52);
+    Eb.R60 = mad(g[6], p0, Eb.R60); Eb.R61 = mad(g[6], p1, Eb.R61); Eb.R62 = mad(g[6], p2, Eb.R62);
+  }
+  // step 4: each limited wave passes its adjoint to the one slope it took
+  auto passed = [&](unsigned took, double factor, double ab[7]) {
+#pragma unroll
+    for (int n = 0; n < 7; n++) {
+      const double v = factor * dab[n];
+      ab[n] = (took >> n) & 1u ? ((neg >> n) & 1u ? -v : v) : 0.0;
+    }
+  };
+  // the differences again (not kept live through the reverse of the waves)
+#pragma unroll
+  for (int n = 0; n < 7; n++) W0[n] = anew(W0[n]);
+  // step 3: projections a = L v of the four differences
+  auto project_adj = [&](const double v[7], const double ab[7], double vb[7]) {
+    const double s06 = ab[0] - ab[6], t06 = ab[0] + ab[6];
+    const double s15 = ab[1] - ab[5], t15 = ab[1] + ab[5];
+    const double s24 = ab[2] - ab[4], t24 = ab[2] + ab[4];
+    vb[0] = ab[3];
+    vb[1] = mad(L.l01, s06, L.l21 * s24);
+    vb[2] = mad(L.l02, s06, -mad(L.b3, s15, L.l22 * s24));
+    vb[3] = mad(L.l03, s06, mad(L.b2, s15, -L.l23 * s24));
+    vb[4] = mad(L.l04, t06, mad(L.l24, t24, -L.l34 * ab[3]));
+    vb[5] = mad(L.l05, t06, -mad(L.l15, t15, L.l25 * t24));
+    vb[6] = mad(L.l06, t06, mad(L.l16, t15, -L.l26 * t24));
+    Eb.L01 = mad(v[1], s06, Eb.L01); Eb.L02 = mad(v[2], s06, Eb.L02); Eb.L03 = mad(v[3], s06, Eb.L03);
+    Eb.L04 = mad(v[4], t06, Eb.L04); Eb.L05 = mad(v[5], t06, Eb.L05); Eb.L06 = mad(v[6], t06, Eb.L06);
+    Eb.L12 = mad(v[2], s15, Eb.L12); Eb.L13 = mad(v[3], s15, Eb.L13);
+    Eb.L15 = mad(v[5], t15, Eb.L15); Eb.L16 = mad(v[6], t15, Eb.L16);
+    Eb.L21 = mad(v[1], s24, Eb.L21); Eb.L22 = mad(v[2], s24, Eb.L22); Eb.L23 = mad(v[3], s24, Eb.L23);
+    Eb.L24 = mad(v[4], t24, Eb.L24); Eb.L25 = mad(v[5], t24, Eb.L25); Eb.L26 = mad(v[6], t24, Eb.L26);
+    Eb.L34 = mad(v[4], ab[3], Eb.L34);
+  };
+  double vb[7], ab[7], dif[7];
+#pragma unroll
+  for (int n = 0; n < 7; n++) dif[n] = anew(Wp[n]) - Wm[n];
+  passed(took_c, 0.5, ab);
+  project_adj(dif, ab, vb);
+#pragma unroll
+  for (int n = 0; n < 7; n++) { Wpb[n] += vb[n]; Wmb[n] -= vb[n]; dif[n] = W0[n] - Wm[n]; }
+  passed(took_l, 2.0, ab);
+  project_adj(dif, ab, vb);
+#pragma unroll
+  for (int n = 0; n < 7; n++) { W0b[n] += vb[n]; Wmb[n] -= vb[n]; dif[n] = Wp[n] - W0[n]; }
+  passed(took_r, 2.0, ab);
+  project_adj(dif, ab, vb);
+#pragma unroll
+  for (int n = 0; n < 7; n++) { Wpb[n] += vb[n]; W0b[n] -= vb[n]; }
+  passed(took_g, 1.0, ab);
+  project_adj(S.dg, ab, vb);
+  // step 2: the van Leer mean
+#pragma unroll
+  for (int n = 0; n < 7; n++) {
+    const double dl = W0[n] - Wm[n], dr = Wp[n] - W0[n], r = recip(fabs(dl + dr));
+    const bool on = dl * dr > 0.0;
+    const double ql = dl * r, qr = dr * r, t = vb[n] + vb[n];
+    const double lb = on ? t * qr * qr : 0.0, rb = on ? t * ql * ql : 0.0;
+    Wpb[n] += rb;
+    Wmb[n] -= lb;
+    W0b[n] += lb - rb;
+  }
+  double db, v1b, pb, b2b, b3b;
+  esys_prim_reverse(K, L, w0.d, w0.p, di, bxc, w0.by, w0.bz, eos, Eb, db, v1b, pb, bxcb, b2b, b3b);
+  W0b[0] += db; W0b[1] += v1b; W0b[4] += pb; W0b[5] += b2b; W0b[6] += b3b;
+  zero(wmb); zero(w0b); zero(wpb);
+  prim_add_arr(wmb, Wmb);
+  prim_add_arr(w0b, W0b);
+  prim_add_arr(wpb, Wpb);
+  return !bad;
 }
 
 // ---------------------------------------------------------------------------

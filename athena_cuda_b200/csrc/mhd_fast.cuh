@@ -241,24 +241,28 @@ ATHB_HD Cons1 cons_of(const Prim1& w, double bx, const Eos& eos, double r_gamma_
   return u;
 }
 
-// Direction of the transverse field: (1, 0) where it vanishes.
-ATHB_HD void field_direction(double b2, double b3, double btsq, double& bet2, double& bet3, bool& bad) {
+// Direction of the transverse field: (1, 0) where it vanishes.  r_bt: 1/|b_t| of
+// the field scaled as small_root scales its square.
+ATHB_HD void field_direction(double b2, double b3, double btsq, double& bet2, double& bet3, double& r_bt,
+                             bool& bad) {
   double g, scale, h;
   (void)small_root(btsq, g, scale, h);
   const bool none = g == 0.0;
-  const double r = recip_of_root(g, h);
-  bet2 = none ? 1.0 : quot(b2 * scale, g, r);
-  bet3 = none ? 0.0 : quot(b3 * scale, g, r);
+  r_bt = recip_of_root(g, h);
+  bet2 = none ? 1.0 : quot(b2 * scale, g, r_bt);
+  bet3 = none ? 0.0 : quot(b3 * scale, g, r_bt);
   bad |= above<400>(btsq) | outside0<-200, 1>(bet2) | outside0<-200, 1>(bet3);
 }
-// alpha_f, alpha_s (src/esystem_prim.c:76-91): roots of gap / span
-ATHB_HD void wave_weights(double span, double slow_gap, double fast_gap, double& af, double& as) {
-  const double r = recip(span);
-  const bool special = span == 0.0 || slow_gap <= 0.0 || fast_gap <= 0.0;
+// alpha_f, alpha_s (src/esystem_prim.c:76-91): roots of gap / span (general), or
+// 0 and 1; r = 1/span, h_f = 1/(2 alpha_f), h_s = 1/(2 alpha_s)
+ATHB_HD void wave_weights(double span, double slow_gap, double fast_gap, double& af, double& as, bool& general,
+                          double& r, double& h_f, double& h_s) {
+  r = recip(span);
+  general = !(span == 0.0 || slow_gap <= 0.0 || fast_gap <= 0.0);
   const bool all_slow = span != 0.0 && slow_gap <= 0.0;
-  const double f = root(quot(slow_gap, span, r)), s = root(quot(fast_gap, span, r));
-  af = special ? (all_slow ? 0.0 : 1.0) : f;
-  as = special ? (all_slow ? 1.0 : 0.0) : s;
+  const double f = root(quot(slow_gap, span, r), h_f), s = root(quot(fast_gap, span, r), h_s);
+  af = general ? f : (all_slow ? 0.0 : 1.0);
+  as = general ? s : (all_slow ? 1.0 : 0.0);
 }
 
 // ---------------------------------------------------------------------------
@@ -295,121 +299,140 @@ ATHB_HD void project(const PrimLeft& L, const double v[7], double a[7]) {
   a[3] = v[0] - L.l34 * v[4];
 }
 
+// Right eigenvectors and eigenvalues of a cell (names as PrimEigT).
+struct PrimRight {
+  double ev[7], R00, R02, R10, R12, R20, R21, R22, R30, R31, R32, R40, R42, R50, R51, R52, R60, R61, R62;
+};
+// Scalars on the way there and 1/(2 root) of each root taken, for the adjoint.
+struct EsysKeep {
+  double btsq, vaxsq, asq, ct2, tdif, c2, cfsq, cf, cssq, cs, vax, bet2, bet3, af, as, sqrtd, sgn, a, na, r_cfsq, r_c2;
+  double h_c2, h_cf, h_cs, h_vax, h_d, h_a, h_af, h_as, r_bt;
+  bool general;      // alpha_f, alpha_s are the roots (no special case)
+  bool tiny_waves;   // slow or Alfven speeds below 2^-480 and not zero
+};
+ATHB_HD void esys_prim_fast(const Prim1& w0, double di, double bxc, const Eos& eos, PrimLeft& L, PrimRight& R,
+                            EsysKeep& K, bool& bad) {
+  const double d = w0.d, v1 = w0.vx, b2 = w0.by, b3 = w0.bz;
+  const double btsq = b2 * b2 + b3 * b3;
+  const double vaxsq = bxc * bxc * di;
+  const double asq = eos.gamma * w0.p * di;
+  const double ct2 = btsq * di;
+  const double tsum = vaxsq + ct2 + asq;
+  const double tdif = vaxsq + ct2 - asq;
+  const double cf2_cs2 = root(tdif * tdif + 4.0 * asq * ct2, K.h_c2);
+  const double cfsq = 0.5 * (tsum + cf2_cs2);
+  const double cf = root(cfsq, K.h_cf);
+  const double csnum = asq * vaxsq;
+  K.r_cfsq = recip_from(cfsq, 4.0 * (K.h_cf * K.h_cf));
+  const double cssq = quot(csnum, cfsq, K.r_cfsq);
+  const double cs = root(cssq, K.h_cs);
+  const double vax = root(vaxsq, K.h_vax);
+  K.tiny_waves = outside0<-960, 500>(csnum) | outside0<-960, 500>(vaxsq) | outside0<-960, 500>(cssq);
+  double bet2, bet3, alpha_f, alpha_s;
+  field_direction(b2, b3, btsq, bet2, bet3, K.r_bt, bad);
+  wave_weights(cf2_cs2, asq - cssq, cfsq - asq, alpha_f, alpha_s, K.general, K.r_c2, K.h_af, K.h_as);
+  // slow and Alfven speeds below 2^-480 that do not show beside v1, nor in
+  // a slow wave of weight 0, need no exact value
+  bad |= K.tiny_waves && !(alpha_s == 0.0 && above<-300>(v1) && !above<400>(vaxsq));
+  const double sqrtd = root(d, K.h_d);
+  const double a = root(asq, K.h_a);
+  const unsigned s = bxc < 0. ? 0x80000000u : 0u;
+  const double qf = flip(cf * alpha_f, s), qs = flip(cs * alpha_s, s);
+  const double af = a * alpha_f * sqrtd, as = a * alpha_s * sqrtd;
+  R.ev[0] = v1 - cf; R.ev[1] = v1 - vax; R.ev[2] = v1 - cs; R.ev[3] = v1;
+  R.ev[4] = v1 + cs; R.ev[5] = v1 + vax; R.ev[6] = v1 + cf;
+  R.R00 = d * alpha_f;        R.R02 = d * alpha_s;
+  R.R10 = -cf * alpha_f;      R.R12 = -cs * alpha_s;
+  R.R20 = qs * bet2;          R.R21 = -bet3;      R.R22 = -qf * bet2;
+  R.R30 = qs * bet3;          R.R31 = bet2;       R.R32 = -qf * bet3;
+  const double dasq = d * asq;
+  R.R40 = dasq * alpha_f;     R.R42 = dasq * alpha_s;
+  const double bet2s = flip(bet2, s), bet3s = flip(bet3, s);
+  R.R50 = as * bet2;          R.R51 = -bet3s * sqrtd;  R.R52 = -af * bet2;
+  R.R60 = as * bet3;          R.R61 = bet2s * sqrtd;   R.R62 = -af * bet3;
+  L.l34 = recip_from(asq, 4.0 * (K.h_a * K.h_a));
+  const double na = 0.5 * L.l34;
+  const double nqf = na * qf, nqs = na * qs;
+  const double afp = na * af * di, asp = na * as * di;
+  const double rs = recip_of_root(sqrtd, K.h_d);
+  L.l01 = -na * cf * alpha_f; L.l02 = nqs * bet2; L.l03 = nqs * bet3;
+  L.l04 = na * alpha_f * di;  L.l05 = asp * bet2; L.l06 = asp * bet3;
+  L.b2 = 0.5 * bet2; L.b3 = 0.5 * bet3;
+  L.l15 = quot(0.5 * bet3s, sqrtd, rs); L.l16 = quot(0.5 * bet2s, sqrtd, rs);
+  L.l21 = -na * cs * alpha_s; L.l22 = nqf * bet2; L.l23 = nqf * bet3;
+  L.l24 = na * alpha_s * di;  L.l25 = afp * bet2; L.l26 = afp * bet3;
+  K.btsq = btsq; K.vaxsq = vaxsq; K.asq = asq; K.ct2 = ct2; K.tdif = tdif; K.c2 = cf2_cs2;
+  K.cfsq = cfsq; K.cf = cf; K.cssq = cssq; K.cs = cs; K.vax = vax; K.bet2 = bet2; K.bet3 = bet3;
+  K.af = alpha_f; K.as = alpha_s; K.sqrtd = sqrtd; K.sgn = bxc < 0. ? -1.0 : 1.0; K.a = a; K.na = na;
+}
+
+// Steps 2-5: differences, their projections, the limited wave slopes da and
+// the primitive slopes dWm.
+struct PlmSlopes {
+  double dl[7], dr[7], dc[7], dg[7], al[7], ar[7], ac[7], ag[7], da[7], dWm[7];
+};
+ATHB_HD void limited_slopes(const double Wm[7], const double W0[7], const double Wp[7], const PrimLeft& L,
+                            const PrimRight& R, PlmSlopes& S, bool& bad) {
+#pragma unroll
+  for (int n = 0; n < 7; n++) {
+    const double dl = W0[n] - Wm[n], dr = Wp[n] - W0[n];
+    S.dl[n] = dl;
+    S.dr[n] = dr;
+    S.dc[n] = Wp[n] - Wm[n];
+    const double prod = dl * dr, sum = dl + dr, size = fabs(sum);
+    if (n < 5) {
+      // 2 dl dr / (dl + dr) as 2 (dl dr / (dl + dr)): with the product zero or
+      // at least 2^-960 the halves are exact
+      const double g = with_sign(quot(prod, size, recip(size)), sum);
+      S.dg[n] = (int)hi_word(prod) > 0 ? g + g : 0.0;
+      bad |= outside0<-960, 500>(prod);
+    } else {
+      const double num = 2.0 * dl * dr;
+      const bool small = !above<-960>(num);
+      const double g = with_sign(quot(small ? num * 0x1p+200 : num, size, recip(size)), sum);
+      S.dg[n] = prod > 0.0 ? (small ? g * 0x1p-200 : g) : 0.0;
+      bad |= above<500>(prod);
+    }
+  }
+  project(L, S.dl, S.al);
+  project(L, S.dr, S.ar);
+  project(L, S.dc, S.ac);
+  project(L, S.dg, S.ag);
+  double* da = S.da;
+#pragma unroll
+  for (int n = 0; n < 7; n++) {
+    const double x = 2.0 * rmin(fabs(S.al[n]), fabs(S.ar[n]));
+    const double y = rmin(0.5 * fabs(S.ac[n]), fabs(S.ag[n]));
+    da[n] = S.al[n] * S.ar[n] > 0.0 ? with_sign(rmin(x, y), S.ac[n]) : 0.0;
+  }
+  S.dWm[0] = da[0] * R.R00 + da[2] * R.R02 + da[3] + da[4] * R.R02 + da[6] * R.R00;
+  S.dWm[1] = da[0] * R.R10 + da[2] * R.R12 - da[4] * R.R12 - da[6] * R.R10;
+  S.dWm[2] = da[0] * R.R20 + da[1] * R.R21 + da[2] * R.R22 - da[4] * R.R22 - da[5] * R.R21 - da[6] * R.R20;
+  S.dWm[3] = da[0] * R.R30 + da[1] * R.R31 + da[2] * R.R32 - da[4] * R.R32 - da[5] * R.R31 - da[6] * R.R30;
+  S.dWm[4] = da[0] * R.R40 + da[2] * R.R42 + da[4] * R.R42 + da[6] * R.R40;
+  S.dWm[5] = da[0] * R.R50 + da[1] * R.R51 + da[2] * R.R52 + da[4] * R.R52 + da[5] * R.R51 + da[6] * R.R50;
+  S.dWm[6] = da[0] * R.R60 + da[1] * R.R61 + da[2] * R.R62 + da[4] * R.R62 + da[5] * R.R61 + da[6] * R.R60;
+}
+
 ATHB_HD bool plm_cell_fast(const Prim1& wm, const Prim1& w0, const Prim1& wp, double di, double bxc, double hdtodx,
                            const Eos& eos, Prim1& wl_next, Prim1& wr_this) {
   bool bad = false;
-  // eigensystem of the cell
   PrimLeft L;
-  double ev[7], R00, R02, R10, R12, R20, R21, R22, R30, R31, R32, R40, R42, R50, R51, R52, R60, R61, R62;
-  {
-    const double d = w0.d, v1 = w0.vx, b2 = w0.by, b3 = w0.bz;
-    const double btsq = b2 * b2 + b3 * b3;
-    const double vaxsq = bxc * bxc * di;
-    const double asq = eos.gamma * w0.p * di;
-    const double ct2 = btsq * di;
-    const double tsum = vaxsq + ct2 + asq;
-    const double tdif = vaxsq + ct2 - asq;
-    const double cf2_cs2 = root(tdif * tdif + 4.0 * asq * ct2);
-    const double cfsq = 0.5 * (tsum + cf2_cs2);
-    double hcf, ha, hd;
-    const double cf = root(cfsq, hcf);
-    const double csnum = asq * vaxsq;
-    const double cssq = quot(csnum, cfsq, recip_from(cfsq, 4.0 * (hcf * hcf)));
-    const double cs = root(cssq);
-    const double vax = root(vaxsq);
-    const bool tiny_waves = outside0<-960, 500>(csnum) | outside0<-960, 500>(vaxsq) | outside0<-960, 500>(cssq);
-    double bet2, bet3, alpha_f, alpha_s;
-    field_direction(b2, b3, btsq, bet2, bet3, bad);
-    wave_weights(cf2_cs2, asq - cssq, cfsq - asq, alpha_f, alpha_s);
-    // slow and Alfven speeds below 2^-480 that do not show beside v1, nor in
-    // a slow wave of weight 0, need no exact value
-    bad |= tiny_waves && !(alpha_s == 0.0 && above<-300>(v1) && !above<400>(vaxsq));
-    const double sqrtd = root(d, hd);
-    const double a = root(asq, ha);
-    const unsigned s = bxc < 0. ? 0x80000000u : 0u;
-    const double qf = flip(cf * alpha_f, s), qs = flip(cs * alpha_s, s);
-    const double af = a * alpha_f * sqrtd, as = a * alpha_s * sqrtd;
-    ev[0] = v1 - cf; ev[1] = v1 - vax; ev[2] = v1 - cs; ev[3] = v1;
-    ev[4] = v1 + cs; ev[5] = v1 + vax; ev[6] = v1 + cf;
-    R00 = d * alpha_f;        R02 = d * alpha_s;
-    R10 = -cf * alpha_f;      R12 = -cs * alpha_s;
-    R20 = qs * bet2;          R21 = -bet3;      R22 = -qf * bet2;
-    R30 = qs * bet3;          R31 = bet2;       R32 = -qf * bet3;
-    const double dasq = d * asq;
-    R40 = dasq * alpha_f;     R42 = dasq * alpha_s;
-    const double bet2s = flip(bet2, s), bet3s = flip(bet3, s);
-    R50 = as * bet2;          R51 = -bet3s * sqrtd;  R52 = -af * bet2;
-    R60 = as * bet3;          R61 = bet2s * sqrtd;   R62 = -af * bet3;
-    L.l34 = recip_from(asq, 4.0 * (ha * ha));
-    const double na = 0.5 * L.l34;
-    const double nqf = na * qf, nqs = na * qs;
-    const double afp = na * af * di, asp = na * as * di;
-    const double rs = recip_of_root(sqrtd, hd);
-    L.l01 = -na * cf * alpha_f; L.l02 = nqs * bet2; L.l03 = nqs * bet3;
-    L.l04 = na * alpha_f * di;  L.l05 = asp * bet2; L.l06 = asp * bet3;
-    L.b2 = 0.5 * bet2; L.b3 = 0.5 * bet3;
-    L.l15 = quot(0.5 * bet3s, sqrtd, rs); L.l16 = quot(0.5 * bet2s, sqrtd, rs);
-    L.l21 = -na * cs * alpha_s; L.l22 = nqf * bet2; L.l23 = nqf * bet3;
-    L.l24 = na * alpha_s * di;  L.l25 = afp * bet2; L.l26 = afp * bet3;
-  }
-
+  PrimRight R;
+  EsysKeep K;
+  esys_prim_fast(w0, di, bxc, eos, L, R, K, bad);
   const double Wm[7] = {wm.d, wm.vx, wm.vy, wm.vz, wm.p, wm.by, wm.bz};
   const double W0[7] = {w0.d, w0.vx, w0.vy, w0.vz, w0.p, w0.by, w0.bz};
   const double Wp[7] = {wp.d, wp.vx, wp.vy, wp.vz, wp.p, wp.by, wp.bz};
-
-  // Steps 2-4.
-  double da[7];
-  {
-    double dl[7], dr[7], dc[7], dg[7];
-#pragma unroll
-    for (int n = 0; n < 7; n++) {
-      dl[n] = W0[n] - Wm[n];
-      dr[n] = Wp[n] - W0[n];
-      dc[n] = Wp[n] - Wm[n];
-      const double prod = dl[n] * dr[n], sum = dl[n] + dr[n], size = fabs(sum);
-      if (n < 5) {
-        // 2 dl dr / (dl + dr) as 2 (dl dr / (dl + dr)): with the product zero or
-        // at least 2^-960 the halves are exact
-        const double g = with_sign(quot(prod, size, recip(size)), sum);
-        dg[n] = (int)hi_word(prod) > 0 ? g + g : 0.0;
-        bad |= outside0<-960, 500>(prod);
-      } else {
-        const double num = 2.0 * dl[n] * dr[n];
-        const bool small = !above<-960>(num);
-        const double g = with_sign(quot(small ? num * 0x1p+200 : num, size, recip(size)), sum);
-        dg[n] = prod > 0.0 ? (small ? g * 0x1p-200 : g) : 0.0;
-        bad |= above<500>(prod);
-      }
-    }
-    double al[7], ar[7], ac[7], ag[7];
-    project(L, dl, al);
-    project(L, dr, ar);
-    project(L, dc, ac);
-    project(L, dg, ag);
-#pragma unroll
-    for (int n = 0; n < 7; n++) {
-      const double x = 2.0 * rmin(fabs(al[n]), fabs(ar[n]));
-      const double y = rmin(0.5 * fabs(ac[n]), fabs(ag[n]));
-      da[n] = al[n] * ar[n] > 0.0 ? with_sign(rmin(x, y), ac[n]) : 0.0;
-    }
-  }
-
-  // Step 5: primitive slopes.
-  double dWm[7];
-  dWm[0] = da[0] * R00 + da[2] * R02 + da[3] + da[4] * R02 + da[6] * R00;
-  dWm[1] = da[0] * R10 + da[2] * R12 - da[4] * R12 - da[6] * R10;
-  dWm[2] = da[0] * R20 + da[1] * R21 + da[2] * R22 - da[4] * R22 - da[5] * R21 - da[6] * R20;
-  dWm[3] = da[0] * R30 + da[1] * R31 + da[2] * R32 - da[4] * R32 - da[5] * R31 - da[6] * R30;
-  dWm[4] = da[0] * R40 + da[2] * R42 + da[4] * R42 + da[6] * R40;
-  dWm[5] = da[0] * R50 + da[1] * R51 + da[2] * R52 + da[4] * R52 + da[5] * R51 + da[6] * R50;
-  dWm[6] = da[0] * R60 + da[1] * R61 + da[2] * R62 + da[4] * R62 + da[5] * R61 + da[6] * R60;
+  PlmSlopes S;
+  limited_slopes(Wm, W0, Wp, L, R, S, bad);
 
   // Steps 7 and 8.
   double dW[7], pWl[7], pWr[7];
-  const double qx = rmax(ev[6], 0.0) * hdtodx, qy = rmin(ev[0], 0.0) * hdtodx;
+  const double qx = rmax(R.ev[6], 0.0) * hdtodx, qy = rmin(R.ev[0], 0.0) * hdtodx;
 #pragma unroll
   for (int n = 0; n < 7; n++) {
-    const double half = 0.5 * dWm[n];
+    const double half = 0.5 * S.dWm[n];
     double l = W0[n] - half, r = W0[n] + half;
     const bool cm = W0[n] < Wm[n], cp = W0[n] < Wp[n];
     l = rmax(cm ? W0[n] : Wm[n], l);
@@ -450,25 +473,25 @@ ATHB_HD bool plm_cell_fast(const Prim1& wm, const Prim1& w0, const Prim1& wp, do
   auto add = [&](int n, double qa, double p[7]) {
     const double sg = n > 3 ? -qa : qa;   // columns n and 6-n share rows up to sign
     if (n == 0 || n == 6) {
-      p[0] += qa * R00; p[1] += sg * R10; p[2] += sg * R20; p[3] += sg * R30;
-      p[4] += qa * R40; p[5] += qa * R50; p[6] += qa * R60;
+      p[0] += qa * R.R00; p[1] += sg * R.R10; p[2] += sg * R.R20; p[3] += sg * R.R30;
+      p[4] += qa * R.R40; p[5] += qa * R.R50; p[6] += qa * R.R60;
     } else if (n == 1 || n == 5) {
-      p[2] += sg * R21; p[3] += sg * R31; p[5] += qa * R51; p[6] += qa * R61;
+      p[2] += sg * R.R21; p[3] += sg * R.R31; p[5] += qa * R.R51; p[6] += qa * R.R61;
     } else if (n == 2 || n == 4) {
-      p[0] += qa * R02; p[1] += sg * R12; p[2] += sg * R22; p[3] += sg * R32;
-      p[4] += qa * R42; p[5] += qa * R52; p[6] += qa * R62;
+      p[0] += qa * R.R02; p[1] += sg * R.R12; p[2] += sg * R.R22; p[3] += sg * R.R32;
+      p[4] += qa * R.R42; p[5] += qa * R.R52; p[6] += qa * R.R62;
     } else {
       p[0] += qa;
     }
   };
 #pragma unroll
   for (int n = 0; n < 6; n++)
-    if (ev[n] > 0.) add(n, strength(n, ev[6] - ev[n]), pWl);
+    if (R.ev[n] > 0.) add(n, strength(n, R.ev[6] - R.ev[n]), pWl);
 #pragma unroll
   for (int n = 0; n < 7; n++)
-    if (ev[n] < 0.) {
-      if (n != 0) add(n, strength(n, ev[0] - ev[n]), pWr);
-      add(n, -strength(n, ev[n] - ev[6]), pWl);
+    if (R.ev[n] < 0.) {
+      if (n != 0) add(n, strength(n, R.ev[0] - R.ev[n]), pWr);
+      add(n, -strength(n, R.ev[n] - R.ev[6]), pWl);
     }
 
   wl_next.d = pWl[0]; wl_next.vx = pWl[1]; wl_next.vy = pWl[2]; wl_next.vz = pWl[3];
@@ -606,7 +629,9 @@ ATHB_HD bool flux_roe_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
   const double v1 = r.v1, v2 = r.v2, v3 = r.v3, b2 = r.b2, b3 = r.b3, d = r.droe;
   const double cf = s.cf, cs = s.cs, vsq = s.vsq, hp = s.hp;
   double bet2, bet3, hg, hd, ha, af, as;
-  field_direction(b2, b3, s.btsq, bet2, bet3, bad);
+  double u0_, u1_, u2_, u3_;
+  bool u4_;
+  field_direction(b2, b3, s.btsq, bet2, bet3, u0_, bad);
   double g_, scale_, h_;
   const double bt_star = small_root(s.bt_starsq, g_, scale_, h_);
   const double sg = root(s.gfac, hg);
@@ -614,7 +639,7 @@ ATHB_HD bool flux_roe_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
   const double bet2s = quot(bet2, sg, rsg), bet3s = quot(bet3, sg, rsg);
   const double bet_starsq = bet2s * bet2s + bet3s * bet3s;
   const double vbet = v2 * bet2s + v3 * bet3s;
-  wave_weights(s.cfsq - s.cssq, s.twid_asq - s.cssq, s.cfsq - s.twid_asq, af, as);
+  wave_weights(s.cfsq - s.cssq, s.twid_asq - s.cssq, s.cfsq - s.twid_asq, af, as, u4_, u1_, u2_, u3_);
   bad |= f.tiny_waves && !(as == 0.0 && above<-300>(v1));
   const double sqrtd = root(d, hd);
   const double isqrtd = recip_of_root(sqrtd, hd);

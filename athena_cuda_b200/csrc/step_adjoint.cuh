@@ -66,6 +66,7 @@ struct AdjArgs {
   int pitch;
   int is, ie, js, je;
   double dx1, dx2;
+  double rdx1, rdx2;    // 1/dx1, 1/dx2
   Eos eos;
   ATHB_MEM long long o(int j, int i) const { return (long long)j * pitch + i; }
   ATHB_MEM double s(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return ro(in + p * ps + off); }
@@ -743,6 +744,21 @@ ATHB_HD void adj_riemann(const AdjArgs& a, int dir, int j, int i) {
   a.a(dir == 0 ? A_BNX : A_BNY, o) = bnb;
 }
 
+// plm_cell_adj out of line, from the conserved states: cells outside the ranges
+// of the fast form.
+ATHB_COLD void plm_adj_general(Cons1 um, Cons1 u0, Cons1 up, double bxm, double bx0, double bxp, double dtodx, Eos eos,
+                               Prim1 wlb, Prim1 wrb, Prim1* wmb, Prim1* w0b, Prim1* wpb, double* bxcb,
+                               double* dtodxb) {
+  Prim1 x, y, z;
+  zero(x); zero(y); zero(z);
+  double bb = 0.0, tb = 0.0;
+  plm_cell_adj(cons_to_prim(um, bxm, eos), cons_to_prim(u0, bx0, eos), cons_to_prim(up, bxp, eos), bx0, dtodx, eos, wlb,
+               wrb, x, y, z, bb, tb);
+  *wmb = x; *w0b = y; *wpb = z;
+  *bxcb = bb;
+  *dtodxb = tb;
+}
+
 // PLM + source term of cell (j,i) of sweep dir: cells of range_plm.
 ATHB_HD void adj_plm(const AdjArgs& a, int dir, int j, int i) {
   const long long o = a.o(j, i);
@@ -755,33 +771,44 @@ ATHB_HD void adj_plm(const AdjArgs& a, int dir, int j, int i) {
   if (in_range(F, j, i)) lwr = adj_prim(a, dir == 0 ? A_WRTX : A_WRTY, o); else zero(lwr);
   // source term: wln.(by|bz) += hdt*src, wrt.(by|bz) += hdt*src
   const double lsum = dir == 0 ? (lwl.by + lwr.by) : (lwl.bz + lwr.bz);
-  const double d = a.s(P_D, o), mt = a.s(dir == 0 ? P_M2 : P_M1, o);
-  const int bnp = dir == 0 ? P_B1I : P_B2I;
-  const double db = a.s(bnp, o + step) - a.s(bnp, o);
-  const double dxs = dir == 0 ? a.dx1 : a.dx2;
-  const double src = (mt / d) * db / dxs;
-  const double lsrc = a.c.hdt * lsum;
-  double dtb = 0.5 * src * lsum;
+  const double mt = a.s(dir == 0 ? P_M2 : P_M1, o);
+  const int bnp = dir == 0 ? P_B1I : P_B2I, bxp = dir == 0 ? P_B1C : P_B2C;
+  const double rdx = dir == 0 ? a.rdx1 : a.rdx2;
+  const double db = (a.s(bnp, o + step) - a.s(bnp, o)) * rdx;
+  const Cons1 um = state_cons(a, o - step, dir), u0 = state_cons(a, o, dir), up = state_cons(a, o + step, dir);
+  const double bxm = a.s(bxp, o - step), bx0 = a.s(bxp, o), bxq = a.s(bxp, o + step);
   const double dt0 = a.a(A_DT, o);
   // PLM
-  const Cons1 um = state_cons(a, o - step, dir), u0 = state_cons(a, o, dir), up = state_cons(a, o + step, dir);
-  const int bxp = dir == 0 ? P_B1C : P_B2C;
-  const Prim1 wm = cons_to_prim(um, a.s(bxp, o - step), a.eos);
-  const Prim1 w0 = cons_to_prim(u0, a.s(bxp, o), a.eos);
-  const Prim1 wp = cons_to_prim(up, a.s(bxp, o + step), a.eos);
+  const double hdtodx = dir == 0 ? a.c.hdtodx1 : a.c.hdtodx2;
+  double di = recip(u0.d);
+  const Prim1 wm = prim_of(um, bxm, recip(um.d), a.eos), w0 = prim_of(u0, bx0, di, a.eos),
+              wp = prim_of(up, bxq, recip(up.d), a.eos);
   Prim1 wmb, w0b, wpb;
-  zero(wmb); zero(w0b); zero(wpb);
-  double bxcb = 0.0, dtodxb = 0.0;
-  plm_cell_adj(wm, w0, wp, a.s(bxp, o), dir == 0 ? a.c.dtodx1 : a.c.dtodx2, a.eos, lwl, lwr, wmb, w0b, wpb, bxcb,
-               dtodxb);
+  double bxcb, dtodxb;
+  bool fast = !(outside<-100, 100>(hdtodx) | cell_outside(um, bxm, wm.p) | cell_outside(u0, bx0, w0.p) |
+                cell_outside(up, bxq, wp.p));
+  if (fast) fast = plm_cell_adj_fast(wm, w0, wp, di, bx0, hdtodx, a.eos, lwl, lwr, wmb, w0b, wpb, bxcb, dtodxb);
+  if (!fast) {
+    Prim1 x, y, z;
+    double bb, tb;
+    plm_adj_general(um, u0, up, bxm, bx0, bxq, dir == 0 ? a.c.dtodx1 : a.c.dtodx2, a.eos, lwl, lwr, &x, &y, &z, &bb,
+                    &tb);
+    wmb = x; w0b = y; wpb = z;
+    bxcb = bb;
+    dtodxb = tb;
+    di = 1.0 / u0.d;
+  }
+  // source term: src = (mt / d) db, d(B)/dx in db
+  const double v0 = mt * di, lsrc = a.c.hdt * lsum;
+  double dtb = 0.5 * v0 * db * lsum;
   const int p[3] = {dir == 0 ? P_M2 : P_M1, P_D, bxp};
-  const double v[3] = {lsrc * db / dxs / d, -(lsrc * (mt / d / d) * db / dxs), bxcb};
+  const double v[3] = {lsrc * db * di, -(lsrc * v0 * di * db), bxcb};
   lin_add(a, o, p, v);
   a.a(dir == 0 ? A_SRCX : A_SRCY, o) = lsrc;
   adj_put_prim(a, dir == 0 ? A_WXM : A_WYM, o, wmb);
   adj_put_prim(a, dir == 0 ? A_WX0 : A_WY0, o, w0b);
   adj_put_prim(a, dir == 0 ? A_WXP : A_WYP, o, wpb);
-  dtb += dtodxb / dxs;
+  dtb += dtodxb * rdx;
   a.a(A_DT, o) = dt0 + dtb;
 }
 

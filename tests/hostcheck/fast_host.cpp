@@ -3,7 +3,7 @@
 // outputs.
 #include <cmath>
 
-#include "mhd_fast.cuh"
+#include "mhd_adjoint.cuh"
 
 using namespace athb;
 
@@ -58,6 +58,30 @@ void fast_plm(int n, const double* w, const double* bx, const double* dtodx, dou
     took[k] = !bad && done;
     put(l, fast + 14 * k);
     put(r, fast + 14 * k + 7);
+  }
+}
+
+// Adjoints of n cells as fast_plm's, lam = adjoints of the left and right
+// states; out: 23 values of each form (m, 0, p states, normal field, dtodx).
+void fast_plm_adj(int n, const double* w, const double* bx, const double* dtodx, const double* lam, double gamma,
+                  int* took, double* fast, double* plain) {
+  const Eos eos{gamma, gamma - 1.0, gamma - 2.0};
+  for (int k = 0; k < n; k++) {
+    Prim1 p[3];
+    for (int c = 0; c < 3; c++) p[c] = prim(w + 21 * k + 7 * c);
+    const Prim1 ll = prim(lam + 14 * k), lr = prim(lam + 14 * k + 7);
+    Prim1 m, z, q;
+    double b = 0.0, t = 0.0;
+    zero(m); zero(z); zero(q);
+    plm_cell_adj(p[0], p[1], p[2], bx[3 * k + 1], dtodx[k], eos, ll, lr, m, z, q, b, t);
+    double* o = plain + 23 * k;
+    put(m, o); put(z, o + 7); put(q, o + 14);
+    o[21] = b; o[22] = t;
+    took[k] = plm_cell_adj_fast(p[0], p[1], p[2], recip(p[1].d), bx[3 * k + 1], 0.5 * dtodx[k], eos, ll, lr, m, z, q,
+                                b, t);
+    o = fast + 23 * k;
+    put(m, o); put(z, o + 7); put(q, o + 14);
+    o[21] = b; o[22] = t;
   }
 }
 

@@ -198,3 +198,25 @@ def test_flux_identical(fast, kind, gamma, hlle):
     ok = took.astype(bool)
     assert ok.mean() >= {"smooth": 0.99, "zeros": 0.9, "jumps": 0.5, "still": 0.7}.get(kind, 0.0)
     np.testing.assert_array_equal(f[ok], g[ok])
+
+
+@pytest.mark.parametrize("kind", ["smooth", "jumps", "zeros"])
+def test_plm_adjoint_agrees(fast, kind):
+    """The adjoint's reverse is regrouped (fused multiply-adds, shared factors),
+    so it agrees to rounding, not in bits: 23 outputs of ~1000 operations on
+    terms up to 1/alpha times the result (alpha the smaller wave weight; 1e-3
+    or more for all but 1 cell in 1000 here), hence 1000 eps / 1e-3 of the
+    largest output, and no branch taken otherwise."""
+    n = 20000
+    rng = np.random.default_rng(20)
+    w0, b0 = _states(rng, 3 * n, kind)
+    w, bx = np.ascontiguousarray(w0.reshape(n, 3, 7)), np.ascontiguousarray(b0.reshape(n, 3))
+    w[rng.random(n) < 0.3, :, 1] += rng.choice([-8.0, 8.0])
+    dtodx, lam = rng.uniform(0.05, 0.4, n), rng.normal(size=(n, 14))
+    took = np.zeros(n, dtype=np.int32)
+    f, g = np.empty((n, 23)), np.empty((n, 23))
+    fast.fast_plm_adj(n, _p(w), _p(bx), _p(dtodx), _p(lam), C.c_double(5.0 / 3.0), _p(took), _p(f), _p(g))
+    ok = took.astype(bool)
+    assert ok.mean() > 0.95
+    err = np.abs(f - g)[ok].max(axis=1) / np.abs(g)[ok].max(axis=1)
+    assert np.quantile(err, 0.999) <= 1000 * 2.0 ** -52 / 1e-3
