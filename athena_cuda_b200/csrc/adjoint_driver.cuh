@@ -103,28 +103,22 @@ template <class T> struct GhostFn {
   }
 };
 
-enum AdjStage { R_UPD, R_EMF1, R_FLUX2, R_CORX, R_CORY, R_CORE, R_HALF, R_EMF0, R_FLUX1, R_SRC, R_RIEX, R_RIEY,
-                R_PLMX, R_PLMY, R_PRIMX, R_PRIMY };
+enum AdjStage { R_UPD, R_CORX, R_CORY, R_CORE, R_HALF, R_FLUX1, R_RIEX, R_RIEY, R_PLMX, R_PLMY, R_PRIM };
 
 template <int STAGE, int FLUX> struct AdjFn {
   AdjArgs a;
   ATHB_MEM void operator()(int j, int i) const {
     if (STAGE == R_UPD) adj_update(a, j, i);
-    else if (STAGE == R_EMF1) adj_emf1(a, j, i);
-    else if (STAGE == R_FLUX2) adj_flux2(a, j, i);
     else if (STAGE == R_CORX) adj_correct_x<FLUX>(a, j, i);
     else if (STAGE == R_CORY) adj_correct_y<FLUX>(a, j, i);
     else if (STAGE == R_CORE) adj_correct_e(a, j, i);
     else if (STAGE == R_HALF) adj_half_faces(a, j, i);
-    else if (STAGE == R_EMF0) adj_emf0(a, j, i);
-    else if (STAGE == R_FLUX1) adj_flux1(a, j, i);
-    else if (STAGE == R_SRC) adj_sources(a, j, i);
+    else if (STAGE == R_FLUX1) adj_flux1_sources(a, j, i);
     else if (STAGE == R_RIEX) adj_riemann<FLUX>(a, 0, j, i);
     else if (STAGE == R_RIEY) adj_riemann<FLUX>(a, 1, j, i);
     else if (STAGE == R_PLMX) adj_plm(a, 0, j, i);
     else if (STAGE == R_PLMY) adj_plm(a, 1, j, i);
-    else if (STAGE == R_PRIMX) adj_prim_gather(a, 0, j, i);
-    else adj_prim_gather(a, 1, j, i);
+    else adj_prim(a, j, i);
   }
 };
 
@@ -308,6 +302,7 @@ struct DtStepAdjFn {
   const StepRec* rec;
   int n;      // step reversed
   int last;   // n == N-1 (dt_rule^{n+1} is not used)
+  DtRuleAdjFn rule;   // dt_rule^n, at S^n
   ATHB_MEM void operator()() const {
     double ldt = sc->dtsum + sc->ltime;   // time^{n+1} = time^n + dt^n
     if (!last && rec[n + 1].cap) ldt += 2.0 * sc->lrule;
@@ -320,8 +315,52 @@ struct DtStepAdjFn {
     sc->ltime = ltime;
     sc->lrule = lrule;
     if (!(ldt == ldt) || !(ltime == ltime)) sc->nonfinite = 1;
+    rule();
   }
 };
+
+// Launches that an executor may run together; one without the call runs the
+// parts in turn.  The parts of one items2/items3 call read nothing that another
+// part writes, so their items may run in any order or at the same time.
+//   items2(ra, fa, rb, fb) / items3(...)   f over r for each pair
+//   argmax_then(plane, range, pitch, out, f), sum_then(...)   the reduction,
+//     then f() with its result in place
+template <class X, class FA, class FB>
+auto run_items2(X& x, int, const GenRange& ra, const FA& fa, const GenRange& rb, const FB& fb)
+    -> decltype(x.items2(ra, fa, rb, fb)) { return x.items2(ra, fa, rb, fb); }
+template <class X, class FA, class FB>
+void run_items2(X& x, long, const GenRange& ra, const FA& fa, const GenRange& rb, const FB& fb) {
+  x.items(ra, fa);
+  x.items(rb, fb);
+}
+template <class X, class FA, class FB, class FC>
+auto run_items3(X& x, int, const GenRange& ra, const FA& fa, const GenRange& rb, const FB& fb, const GenRange& rc,
+                const FC& fc) -> decltype(x.items3(ra, fa, rb, fb, rc, fc)) {
+  return x.items3(ra, fa, rb, fb, rc, fc);
+}
+template <class X, class FA, class FB, class FC>
+void run_items3(X& x, long, const GenRange& ra, const FA& fa, const GenRange& rb, const FB& fb, const GenRange& rc,
+                const FC& fc) {
+  x.items(ra, fa);
+  x.items(rb, fb);
+  x.items(rc, fc);
+}
+template <class X, class F>
+auto run_argmax(X& x, int, const double* p, const GenRange& r, int pitch, MaxLoc* out, const F& f)
+    -> decltype(x.argmax_then(p, r, pitch, out, f)) { return x.argmax_then(p, r, pitch, out, f); }
+template <class X, class F>
+void run_argmax(X& x, long, const double* p, const GenRange& r, int pitch, MaxLoc* out, const F& f) {
+  x.argmax(p, r, pitch, out);
+  x.single(f);
+}
+template <class X, class F>
+auto run_sum(X& x, int, const double* p, const GenRange& r, int pitch, double* out, const F& f)
+    -> decltype(x.sum_then(p, r, pitch, out, f)) { return x.sum_then(p, r, pitch, out, f); }
+template <class X, class F>
+void run_sum(X& x, long, const double* p, const GenRange& r, int pitch, double* out, const F& f) {
+  x.sum(p, r, pitch, out);
+  x.single(f);
+}
 
 // ---------------------------------------------------------------------------
 // the driver
@@ -386,7 +425,7 @@ template <class Exec> struct AdjointDriver {
   double* tape0 = nullptr;                // the working tape
   StepRec* rec = nullptr;
   AdjScal* sc = nullptr;
-  MaxLoc* ml = nullptr;
+  MaxLoc* ml = nullptr;                   // max CFL rate of S^n and its cell (TLM: the current one)
   StepCoef<double>* cf = nullptr;
   StepCoef<Dual>* cfd = nullptr;
   double* timev = nullptr;
@@ -415,7 +454,7 @@ template <class Exec> struct AdjointDriver {
     tape = x.alloc((size_t)NTAPE * G.ps);
     tape0 = tape;
     sc = (AdjScal*)x.alloc_bytes(sizeof(AdjScal));
-    ml = (MaxLoc*)x.alloc_bytes(sizeof(MaxLoc));
+    ml = (MaxLoc*)x.alloc_bytes(sizeof(MaxLoc) * (size_t)nrec);
     cf = (StepCoef<double>*)x.alloc_bytes(sizeof(StepCoef<double>));
     timev = x.alloc(1);
     rec = (StepRec*)x.alloc_bytes(sizeof(StepRec) * (size_t)nrec);
@@ -504,6 +543,9 @@ template <class Exec> struct AdjointDriver {
   template <int FLUX> void fwd_step_double(int cur, bool taped = false) {
     x.template forward_step<FLUX>(*this, cur, taped);
   }
+  // The CFL rates are read in the first sweep alone (the maxima are kept):
+  // false in the reverse sweep, whose steps an executor may run without them.
+  bool rates = true;
   template <int FLUX> void generic_step_double(int cur) {
     step<FLUX, double>(pd(S[cur]), pd(S[cur ^ 1]), pd(tape), cf);
   }
@@ -516,14 +558,14 @@ template <class Exec> struct AdjointDriver {
     Planes<Dual> s0 = pdual(S[0], dS[0]);
     x.items(full(), GhostFn<Dual>{s0, G.ps, G.pitch, ghost_geom()});
     cfl(s0, pdual(tape + (long long)G_DTI * G.ps, dtape + (long long)G_DTI * G.ps));
-    x.argmax(tape + (long long)G_DTI * G.ps, interior(), G.pitch, ml);
-    x.single(Dt0Fn<Dual>{cfd, timed, ml, dtape + (long long)G_DTI * G.ps, nullptr, G.cour, G.tlim, G.dx1, G.dx2});
+    run_argmax(x, 0, tape + (long long)G_DTI * G.ps, interior(), G.pitch, ml,
+               Dt0Fn<Dual>{cfd, timed, ml, dtape + (long long)G_DTI * G.ps, nullptr, G.cour, G.tlim, G.dx1, G.dx2});
     for (int n = 0; n < N; n++) {
       step<FLUX, Dual>(pdual(S[cur], dS[cur]), pdual(S[cur ^ 1], dS[cur ^ 1]), pdual(tape, dtape), cfd);
       cur ^= 1;
-      x.argmax(tape + (long long)G_DTI * G.ps, interior(), G.pitch, ml);
-      x.single(DtNextFn<Dual>{cfd, timed, ml, dtape + (long long)G_DTI * G.ps, nullptr, n + 1, G.cour, G.tlim,
-                              G.dx1, G.dx2});
+      run_argmax(x, 0, tape + (long long)G_DTI * G.ps, interior(), G.pitch, ml,
+                 DtNextFn<Dual>{cfd, timed, ml, dtape + (long long)G_DTI * G.ps, nullptr, n + 1, G.cour, G.tlim,
+                                G.dx1, G.dx2});
     }
     objective(S[cur], dS[cur]);
     return x.ok() ? 0 : -1;
@@ -596,50 +638,41 @@ template <class Exec> struct AdjointDriver {
   // (folded); on return lam[lc^1] holds that of S^n (folded), lc flipped.
   template <int FLUX> void reverse_step(int cur, int n, int N, int& lc, const std::vector<StepRec>& hrec) {
     const double* Sn;
-    const double* Sn1;
-    if (tapes) {   // tape mode: S^n, S^{n+1} in the slots, the tape of step n recorded by the first sweep
+    if (tapes) {   // tape mode: S^n in its slot, the tape of step n recorded by the first sweep
       tape = tape_of(n);
       Sn = slot_ptr(n);
-      Sn1 = n + 1 < N ? slot_ptr(n + 1) : nullptr;
-    } else {       // recorded forward step n: S^n -> S^{n+1}, tape, CFL rates of S^{n+1}
+    } else {       // recorded forward step n: S^n -> S^{n+1}, tape
       x.single(CoefFromRecFn{cf, rec, n, G.dx1, G.dx2});
       fwd_step_double<FLUX>(cur, true);
       taped++;
       Sn = S[cur];
-      Sn1 = S[cur ^ 1];
-    }
-    // dt_rule^{n+1} = CourNo / m(S^{n+1}): its adjoint into lam[lc]
-    if (n + 1 < N) {
-      x.argmax(tape + (long long)G_DTI * G.ps, interior(), G.pitch, ml);
-      x.single(DtRuleAdjFn{Sn1, lam[lc], ml, sc, rec, n + 1, G.ps, G.cour, G.dx1, G.dx2, G.eos});
     }
     double* lin = lam[lc ^ 1];
-    x.zero(lin, state_doubles());
-    x.zero(adj + (long long)A_DT * G.ps, plane());
     AdjArgs a = adj_args(Sn, lam[lc], lin);
     a.c = make_coef(hrec[n].dt, G.dx1, G.dx2);
     const int is = G.is, ie = G.ie, js = G.js, je = G.je;
-    x.items(GenRange{is, ie + 1, js, je + 1}, AdjFn<R_UPD, FLUX>{a});
-    x.items(range_emf1(is, ie, js, je), AdjFn<R_EMF1, FLUX>{a});
-    x.items(GenRange{is - 1, ie + 1, js - 1, je + 1}, AdjFn<R_FLUX2, FLUX>{a});
-    x.items(range_correct_x(is, ie, js, je), AdjFn<R_CORX, FLUX>{a});
-    x.items(range_correct_y(is, ie, js, je), AdjFn<R_CORY, FLUX>{a});
-    x.items(range_correct_e(is, ie, js, je), AdjFn<R_CORE, FLUX>{a});
+    // 7 launches where a stage each would make 16: the two sweeps of a stage
+    // run side by side (a small grid's stage leaves most SMs idle), and a
+    // gather too small for a launch is formed by its reader.  With the dt rule
+    // in the sum's launch and nothing cleared beforehand a step of the gradient
+    // makes 21 launches instead of 40: 266 -> 189 us at 64 x 48, 504 -> 440 us
+    // at 256 x 256, 176 us at 16 x 16, where the launches' latency is all
+    x.items(full(), AdjFn<R_UPD, FLUX>{a});
+    run_items3(x, 0, range_correct_x(is, ie, js, je), AdjFn<R_CORX, FLUX>{a}, range_correct_y(is, ie, js, je),
+               AdjFn<R_CORY, FLUX>{a}, range_correct_e(is, ie, js, je), AdjFn<R_CORE, FLUX>{a});
     x.items(GenRange{is - 1, ie + 2, js - 1, je + 2}, AdjFn<R_HALF, FLUX>{a});
-    x.items(range_emf0(is, ie, js, je), AdjFn<R_EMF0, FLUX>{a});
     x.items(GenRange{is - 2, ie + 2, js - 2, je + 2}, AdjFn<R_FLUX1, FLUX>{a});
-    x.items(GenRange{is - 1, ie + 2, js - 1, je + 2}, AdjFn<R_SRC, FLUX>{a});
-    x.items(range_riemann_x(is, ie, js, je), AdjFn<R_RIEX, FLUX>{a});
-    x.items(range_riemann_y(is, ie, js, je), AdjFn<R_RIEY, FLUX>{a});
-    x.items(range_plm(is, ie, js, je), AdjFn<R_PLMX, FLUX>{a});
-    x.items(range_plm(is, ie, js, je), AdjFn<R_PLMY, FLUX>{a});
-    x.items(GenRange{is - 3, ie + 3, js - 2, je + 2}, AdjFn<R_PRIMX, FLUX>{a});
-    x.items(GenRange{is - 2, ie + 2, js - 3, je + 3}, AdjFn<R_PRIMY, FLUX>{a});
+    run_items2(x, 0, range_riemann_x(is, ie, js, je), AdjFn<R_RIEX, FLUX>{a}, range_riemann_y(is, ie, js, je),
+               AdjFn<R_RIEY, FLUX>{a});
+    run_items2(x, 0, range_plm(is, ie, js, je), AdjFn<R_PLMX, FLUX>{a}, range_plm(is, ie, js, je),
+               AdjFn<R_PLMY, FLUX>{a});
+    x.items(GenRange{is - 3, ie + 3, js - 3, je + 3}, AdjFn<R_PRIM, FLUX>{a});
     // the ghost fill of S^n, reversed: x2 rows, then x1 columns, then clear
     fold_ghosts(lin);
-    // dt^n
-    x.sum(adj + (long long)A_DT * G.ps, GenRange{is - 3, ie + 3, js - 3, je + 3}, G.pitch, &sc->dtsum);
-    x.single(DtStepAdjFn{sc, rec, n, n + 1 == N ? 1 : 0});
+    // dt^n, then dt_rule^n = CourNo / m(S^n), whose cell and rate the first sweep kept, into lin
+    run_sum(x, 0, adj + (long long)A_DT * G.ps, GenRange{is - 3, ie + 3, js - 3, je + 3}, G.pitch, &sc->dtsum,
+            DtStepAdjFn{sc, rec, n, n + 1 == N ? 1 : 0,
+                        DtRuleAdjFn{Sn, lin, ml + n, sc, rec, n, G.ps, G.cour, G.dx1, G.dx2, G.eos}});
     lc ^= 1;
   }
 
@@ -687,8 +720,8 @@ template <class Exec> struct AdjointDriver {
   void entry() {
     x.items(full(), GhostFn<double>{pd(S[0]), G.ps, G.pitch, ghost_geom()});
     cfl(pd(S[0]), pd(tape + (long long)G_DTI * G.ps));
-    x.argmax(tape + (long long)G_DTI * G.ps, interior(), G.pitch, ml);
-    x.single(Dt0Fn<double>{cf, timev, ml, nullptr, rec, G.cour, G.tlim, G.dx1, G.dx2});
+    run_argmax(x, 0, tape + (long long)G_DTI * G.ps, interior(), G.pitch, ml,
+               Dt0Fn<double>{cf, timev, ml, nullptr, rec, G.cour, G.tlim, G.dx1, G.dx2});
   }
 
   template <int FLUX> int adjoint(int N, int& lc, int& steps_done) {
@@ -717,8 +750,8 @@ template <class Exec> struct AdjointDriver {
       fwd_step_double<FLUX>(cur, tapes != nullptr);
       cur ^= 1;
       if (tapes) taped++; else advances++;
-      x.argmax(tape + (long long)G_DTI * G.ps, interior(), G.pitch, ml);
-      x.single(DtNextFn<double>{cf, timev, ml, nullptr, rec, n + 1, G.cour, G.tlim, G.dx1, G.dx2});
+      run_argmax(x, 0, tape + (long long)G_DTI * G.ps, interior(), G.pitch, ml + n + 1,
+                 DtNextFn<double>{cf, timev, ml + n + 1, nullptr, rec, n + 1, G.cour, G.tlim, G.dx1, G.dx2});
       if (tapes) {
         if (n + 1 < N) x.copy(slot_ptr(n + 1), S[cur], state_doubles());
       } else if (n + 1 < N && spine[n + 1] >= 0) {
@@ -727,6 +760,7 @@ template <class Exec> struct AdjointDriver {
     }
     tape = tape0;
     objective(S[cur], nullptr);
+    rates = false;
     std::vector<StepRec> hrec(N + 1);
     x.to_host(hrec.data(), rec, sizeof(StepRec) * (size_t)(N + 1));
     // stop at tlim as the main loop does
@@ -764,11 +798,6 @@ template <class Exec> struct AdjointDriver {
     } else if (M > 0) {
       reverse<FLUX>(0, M, 0, fr, M, lc, hrec, spine);
     }
-    // dt_rule^0 = CourNo / m(S^0)
-    x.copy(S[0], slot_ptr(0), state_doubles());
-    cfl(pd(S[0]), pd(tape + (long long)G_DTI * G.ps));
-    x.argmax(tape + (long long)G_DTI * G.ps, interior(), G.pitch, ml);
-    x.single(DtRuleAdjFn{S[0], lam[lc], ml, sc, rec, 0, G.ps, G.cour, G.dx1, G.dx2, G.eos});
     return x.ok() ? 0 : -1;
   }
 };

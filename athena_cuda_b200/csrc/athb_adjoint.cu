@@ -2,11 +2,12 @@
 // loop on the GPU: the sm_100a executor of adjoint_driver.cuh and the C ABI
 // (athb_tlm_run, athb_adjoint_gradient).
 //
-// Every stage is one launch of a per-item kernel over its range on the
-// context's stream; reductions (the CFL max with the cell that attains it,
-// the adjoint of dt, the objective) are two-pass and deterministic: a fixed
-// assignment of items to blocks, a fixed tree inside a block, blocks summed
-// in order by one thread.
+// Every stage, or group of stages that are independent of each other, is one
+// launch of a per-item kernel on the context's stream; reductions (the CFL max
+// with the cell that attains it, the adjoint of dt, the objective) are one
+// launch too and deterministic: a fixed assignment of items to blocks, a fixed
+// tree inside a block, the partials folded by a fixed tree in the block that
+// finishes last.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -54,19 +55,85 @@ template <int STAGE, int FLUX> struct ItemMinBlocks<AdjFn<STAGE, FLUX>> {
                                                                       : 1;
 };
 
+// A range cut into blocks of items.
+struct Part {
+  GenRange r;
+  unsigned n;   // items: 32 bits, a 64-bit division costs a small stage dearly
+  int blocks;
+};
+
 template <class F>
-__global__ void __launch_bounds__(kItemThreads, ItemMinBlocks<F>::value) k_items(GenRange r, unsigned n, F f) {
-  const unsigned t = blockIdx.x * kItemThreads + threadIdx.x;   // 32 bits: a 64-bit division costs a small stage dearly
-  if (t >= n) return;
-  const unsigned w = (unsigned)(r.i1 - r.i0 + 1);
-  f(r.j0 + (int)(t / w), r.i0 + (int)(t % w));
+__device__ __forceinline__ void run_item(const Part& p, unsigned block, const F& f) {
+  const unsigned t = block * kItemThreads + threadIdx.x;
+  if (t >= p.n) return;
+  const unsigned w = (unsigned)(p.r.i1 - p.r.i0 + 1);
+  f(p.r.j0 + (int)(t / w), p.r.i0 + (int)(t % w));
+}
+
+template <class F>
+__global__ void __launch_bounds__(kItemThreads, ItemMinBlocks<F>::value) k_items(Part p, F f) {
+  run_item(p, blockIdx.x, f);
+}
+
+// Stages that read nothing of each other in one launch.  The parts' blocks
+// come one part after the other, so that an SM holds one code at a time but
+// for the seam: the sweeps' codes together do not fit its instruction cache.
+template <class FA, class FB>
+__global__ void __launch_bounds__(kItemThreads, ItemMinBlocks<FA>::value) k_items2(Part pa, FA fa, Part pb, FB fb) {
+  if (blockIdx.x < pa.blocks) run_item(pa, blockIdx.x, fa);
+  else run_item(pb, blockIdx.x - pa.blocks, fb);
+}
+template <class FA, class FB, class FC>
+__global__ void __launch_bounds__(kItemThreads, ItemMinBlocks<FA>::value)
+    k_items3(Part pa, FA fa, Part pb, FB fb, Part pc, FC fc) {
+  if (blockIdx.x < pa.blocks) run_item(pa, blockIdx.x, fa);
+  else if (blockIdx.x < pa.blocks + pb.blocks) run_item(pb, blockIdx.x - pa.blocks, fb);
+  else run_item(pc, blockIdx.x - pa.blocks - pb.blocks, fc);
 }
 
 template <class F>
 __global__ void k_single(F f) { f(); }
 
-__global__ void __launch_bounds__(kRedThreads) k_argmax_part(const double* p, GenRange r, int pitch, long long n,
-                                                             MaxLoc* part) {
+// The reductions: every block folds its share to one partial, and the block
+// that finishes last folds the partials by a fixed tree, stores the result and
+// runs f() on it (one thread).  Which block that is does not change the result.
+// ticket counts the blocks and is back at zero at the end.
+
+// true in the last block of the grid to come here, once its threads may read
+// what every block's thread 0 stored before coming
+__device__ __forceinline__ bool last_block(unsigned* ticket) {
+  __shared__ int last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (last) *ticket = 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  return last;
+}
+
+// maximum, the lowest index among equals, to element 0
+__device__ __forceinline__ void fold_max(double m, long long arg, double* sm, long long* sa) {
+  sm[threadIdx.x] = m;
+  sa[threadIdx.x] = arg;
+  __syncthreads();
+  for (int s = kRedThreads / 2; s > 0; s >>= 1) {
+    if (threadIdx.x < s) {
+      const double m2 = sm[threadIdx.x + s];
+      const long long a2 = sa[threadIdx.x + s];
+      if (m2 > sm[threadIdx.x] || (m2 == sm[threadIdx.x] && a2 < sa[threadIdx.x])) {
+        sm[threadIdx.x] = m2;
+        sa[threadIdx.x] = a2;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <class F>
+__global__ void __launch_bounds__(kRedThreads) k_argmax(const double* p, GenRange r, int pitch, long long n,
+                                                        MaxLoc* part, unsigned* ticket, MaxLoc* out, F f) {
   __shared__ double sm[kRedThreads];
   __shared__ long long sa[kRedThreads];
   double m = -INFINITY;
@@ -78,54 +145,37 @@ __global__ void __launch_bounds__(kRedThreads) k_argmax_part(const double* p, Ge
     const double v = p[o];
     if (v > m || (v == m && o < arg)) { m = v; arg = o; }
   }
-  sm[threadIdx.x] = m;
-  sa[threadIdx.x] = arg;
-  __syncthreads();
-  for (int s = kRedThreads / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      const double m2 = sm[threadIdx.x + s];
-      const long long a2 = sa[threadIdx.x + s];
-      if (m2 > sm[threadIdx.x] || (m2 == sm[threadIdx.x] && a2 < sa[threadIdx.x])) {
-        sm[threadIdx.x] = m2;
-        sa[threadIdx.x] = a2;
-      }
-    }
-    __syncthreads();
-  }
+  fold_max(m, arg, sm, sa);
   if (threadIdx.x == 0) { part[blockIdx.x].m = sm[0]; part[blockIdx.x].arg = sa[0]; }
-}
-
-// one block: the partials folded by a fixed tree (max, then lowest index)
-__global__ void __launch_bounds__(kRedThreads) k_argmax_final(const MaxLoc* part, int nb, long long first,
-                                                              MaxLoc* out) {
-  __shared__ double sm[kRedThreads];
-  __shared__ long long sa[kRedThreads];
-  double m = -INFINITY;
-  long long arg = LLONG_MAX;
-  for (int b = threadIdx.x; b < nb; b += kRedThreads)
-    if (part[b].m > m || (part[b].m == m && part[b].arg < arg)) { m = part[b].m; arg = part[b].arg; }
-  sm[threadIdx.x] = m;
-  sa[threadIdx.x] = arg;
-  __syncthreads();
-  for (int s = kRedThreads / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      const double m2 = sm[threadIdx.x + s];
-      const long long a2 = sa[threadIdx.x + s];
-      if (m2 > sm[threadIdx.x] || (m2 == sm[threadIdx.x] && a2 < sa[threadIdx.x])) {
-        sm[threadIdx.x] = m2;
-        sa[threadIdx.x] = a2;
-      }
-    }
-    __syncthreads();
+  if (!last_block(ticket)) return;
+  m = -INFINITY;
+  arg = LLONG_MAX;
+  for (int b = threadIdx.x; b < gridDim.x; b += kRedThreads) {
+    const double v = __ldcg(&part[b].m);
+    const long long o = __ldcg(&part[b].arg);
+    if (v > m || (v == m && o < arg)) { m = v; arg = o; }
   }
+  fold_max(m, arg, sm, sa);
   if (threadIdx.x == 0) {
     out->m = sm[0];
-    out->arg = sa[0] == LLONG_MAX ? first : sa[0];   // no comparable value (NaN everywhere): keep the index valid
+    // no comparable value (NaN everywhere): keep the index valid
+    out->arg = sa[0] == LLONG_MAX ? (long long)r.j0 * pitch + r.i0 : sa[0];
+    f();
   }
 }
 
-__global__ void __launch_bounds__(kRedThreads) k_sum_part(const double* p, GenRange r, int pitch, long long n,
-                                                          double* part) {
+__device__ __forceinline__ void fold_sum(double s, double* sm) {
+  sm[threadIdx.x] = s;
+  __syncthreads();
+  for (int k = kRedThreads / 2; k > 0; k >>= 1) {
+    if (threadIdx.x < k) sm[threadIdx.x] += sm[threadIdx.x + k];
+    __syncthreads();
+  }
+}
+
+template <class F>
+__global__ void __launch_bounds__(kRedThreads) k_sum(const double* p, GenRange r, int pitch, long long n,
+                                                     double* part, unsigned* ticket, double* out, F f) {
   __shared__ double sm[kRedThreads];
   double s = 0.0;
   for (long long t = (long long)blockIdx.x * kRedThreads + threadIdx.x; t < n; t += (long long)gridDim.x * kRedThreads) {
@@ -133,28 +183,21 @@ __global__ void __launch_bounds__(kRedThreads) k_sum_part(const double* p, GenRa
     range_item(r, t, j, i);
     s += p[(long long)j * pitch + i];
   }
-  sm[threadIdx.x] = s;
-  __syncthreads();
-  for (int k = kRedThreads / 2; k > 0; k >>= 1) {
-    if (threadIdx.x < k) sm[threadIdx.x] += sm[threadIdx.x + k];
-    __syncthreads();
-  }
+  fold_sum(s, sm);
   if (threadIdx.x == 0) part[blockIdx.x] = sm[0];
+  if (!last_block(ticket)) return;
+  s = 0.0;
+  for (int b = threadIdx.x; b < gridDim.x; b += kRedThreads) s += __ldcg(&part[b]);
+  fold_sum(s, sm);
+  if (threadIdx.x == 0) {
+    *out = sm[0];
+    f();
+  }
 }
 
-// one block: the partials summed by a fixed tree
-__global__ void __launch_bounds__(kRedThreads) k_sum_final(const double* part, int nb, double* out) {
-  __shared__ double sm[kRedThreads];
-  double s = 0.0;
-  for (int b = threadIdx.x; b < nb; b += kRedThreads) s += part[b];
-  sm[threadIdx.x] = s;
-  __syncthreads();
-  for (int k = kRedThreads / 2; k > 0; k >>= 1) {
-    if (threadIdx.x < k) sm[threadIdx.x] += sm[threadIdx.x + k];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *out = sm[0];
-}
+struct Nothing {
+  __device__ void operator()() const {}
+};
 
 // StepState of the fast kernels from the step's factors
 struct SetStFn {
@@ -166,6 +209,15 @@ struct SetStFn {
     st->hdtodx1 = cf->hdtodx1; st->hdtodx2 = cf->hdtodx2; st->hdt = cf->hdt;
     st->done = 0;
     st->max_dti_bits = 0ull;
+  }
+};
+// f, which forms the factors, and then that
+template <class F> struct AndSetSt {
+  F f;
+  SetStFn set;
+  __device__ void operator()() const {
+    f();
+    set();
   }
 };
 
@@ -208,6 +260,7 @@ struct GpuExec {
   cudaError_t err = cudaSuccess;
   double* red = nullptr;       // reduction partials
   MaxLoc* redm = nullptr;
+  unsigned* ticket = nullptr;  // blocks of the reduction in flight
   std::vector<std::pair<void*, size_t>> owned;
   size_t bytes = 0;
 
@@ -216,39 +269,78 @@ struct GpuExec {
     note(cudaGetLastError());
     return err == cudaSuccess;
   }
+  // the executor's own blocks; the plain step's factors are the driver's, see with_st
+  void setup() {
+    red = alloc(kRedBlocks);
+    redm = (MaxLoc*)alloc_bytes(sizeof(MaxLoc) * (kRedBlocks + 1));   // the last one holds the ticket
+    ticket = (unsigned*)(redm + kRedBlocks);
+    st = (StepState*)alloc_bytes(sizeof(StepState));
+    if (ok()) zero_bytes(ticket, sizeof *ticket);
+  }
   static int blocks(long long n, int threads) { return (int)((n + threads - 1) / threads); }
 
-  template <class F> void items(const GenRange& r, const F& f) {
+  // false: an empty range (nothing to launch) or one no grid has (2^30 cells at most)
+  bool part(const GenRange& r, Part& p) {
     const long long n = range_count(r);
-    if (n <= 0 || err != cudaSuccess) return;
-    if (n > INT_MAX) { note(cudaErrorInvalidValue); return; }   // grids hold at most 2^30 cells
-    k_items<F><<<blocks(n, kItemThreads), kItemThreads, 0, s>>>(r, (unsigned)n, f);
+    if (n > INT_MAX) { note(cudaErrorInvalidValue); return false; }
+    p.r = r;
+    p.n = (unsigned)std::max(n, 0LL);
+    p.blocks = blocks(p.n, kItemThreads);
+    return true;
   }
+  template <class F> void items(const GenRange& r, const F& f) {
+    Part p;
+    if (err != cudaSuccess || !part(r, p) || !p.blocks) return;
+    k_items<F><<<p.blocks, kItemThreads, 0, s>>>(p, f);
+  }
+  template <class FA, class FB>
+  void items2(const GenRange& ra, const FA& fa, const GenRange& rb, const FB& fb) {
+    Part a, b;
+    if (err != cudaSuccess || !part(ra, a) || !part(rb, b) || !(a.blocks + b.blocks)) return;
+    k_items2<<<a.blocks + b.blocks, kItemThreads, 0, s>>>(a, fa, b, fb);
+  }
+  template <class FA, class FB, class FC>
+  void items3(const GenRange& ra, const FA& fa, const GenRange& rb, const FB& fb, const GenRange& rc, const FC& fc) {
+    Part a, b, c;
+    if (err != cudaSuccess || !part(ra, a) || !part(rb, b) || !part(rc, c) || !(a.blocks + b.blocks + c.blocks)) return;
+    k_items3<<<a.blocks + b.blocks + c.blocks, kItemThreads, 0, s>>>(a, fa, b, fb, c, fc);
+  }
+  // The factors of the next plain step (driver.cf) formed by f; the step
+  // kernels' own copy of them is made in the same launch, and st_set says so.
+  bool st_set = false;
+  StepCoef<double>* cf = nullptr;   // driver.cf
+  template <class F> AndSetSt<F> with_st(const F& f) {
+    st_set = true;
+    return AndSetSt<F>{f, SetStFn{st, cf}};
+  }
+  AndSetSt<CoefFromRecFn> after(const CoefFromRecFn& f) { return with_st(f); }
+  AndSetSt<Dt0Fn<double>> after(const Dt0Fn<double>& f) { return with_st(f); }
+  AndSetSt<DtNextFn<double>> after(const DtNextFn<double>& f) { return with_st(f); }
+  template <class F> const F& after(const F& f) { return f; }
+
   template <class F> void single(const F& f) {
     if (err != cudaSuccess) return;
-    k_single<F><<<1, 1, 0, s>>>(f);
+    k_single<<<1, 1, 0, s>>>(after(f));
   }
   int red_blocks(long long n) const { return (int)std::max(1LL, std::min((long long)kRedBlocks, (n + kRedThreads - 1) / kRedThreads)); }
-  void argmax(const double* p, const GenRange& r, int pitch, MaxLoc* out) {
+  template <class F> void argmax_then(const double* p, const GenRange& r, int pitch, MaxLoc* out, const F& f) {
     const long long n = range_count(r);
     if (err != cudaSuccess) return;
-    const int nb = red_blocks(n);
-    k_argmax_part<<<nb, kRedThreads, 0, s>>>(p, r, pitch, n, redm);
-    k_argmax_final<<<1, kRedThreads, 0, s>>>(redm, nb, (long long)r.j0 * pitch + r.i0, out);
+    k_argmax<<<red_blocks(n), kRedThreads, 0, s>>>(p, r, pitch, n, redm, ticket, out, after(f));
   }
-  void sum(const double* p, const GenRange& r, int pitch, double* out) {
+  template <class F> void sum_then(const double* p, const GenRange& r, int pitch, double* out, const F& f) {
     const long long n = range_count(r);
     if (err != cudaSuccess) return;
-    const int nb = red_blocks(n);
-    k_sum_part<<<nb, kRedThreads, 0, s>>>(p, r, pitch, n, red);
-    k_sum_final<<<1, kRedThreads, 0, s>>>(red, nb, out);
+    k_sum<<<red_blocks(n), kRedThreads, 0, s>>>(p, r, pitch, n, red, ticket, out, f);
   }
+  void sum(const double* p, const GenRange& r, int pitch, double* out) { sum_then(p, r, pitch, out, Nothing{}); }
   // One plain step on the fast kernels (step_kernels.cuh); taped: the
   // predictor also keeps its face states and the half-step emf is saved.
   template <int FLUX, class D> void forward_step(D& d, int cur, bool taped) {
     if (err != cudaSuccess) return;
     const LoopGeom& G = d.G;
-    single(SetStFn{st, d.cf});
+    if (!st_set) single(SetStFn{st, d.cf});
+    st_set = false;
     GridArgs g;
     g.in = d.S[cur];
     g.out = d.S[cur ^ 1];
@@ -279,7 +371,7 @@ struct GpuExec {
     GridArgs gg = g;
     gg.in = d.S[cur ^ 1];
     k_ghost<<<blocks(nframe, kThreads), kThreads, 0, s>>>(gg, G.sx, G.sy, nframe, 3, 3);
-    d.cfl(d.pd(d.S[cur ^ 1]), d.pd(d.tape + (size_t)G_DTI * G.ps));
+    if (d.rates) d.cfl(d.pd(d.S[cur ^ 1]), d.pd(d.tape + (size_t)G_DTI * G.ps));
   }
 
   // With a cache (athb_adjoint_keep_workspace on) a block of the same size
@@ -389,10 +481,9 @@ extern "C" int athb_tlm_run(athb_ctx* ctx, int nsteps, const double* dstate0, do
   x.s = ctx->stream;
   x.cache = ctx->adj_keep ? ctx->adj_cache : nullptr;
   AdjointDriver<GpuExec> d(x, geom_of(ctx));
-  x.red = x.alloc(kRedBlocks);
-  x.redm = (MaxLoc*)x.alloc_bytes(sizeof(MaxLoc) * kRedBlocks);
-  x.st = (StepState*)x.alloc_bytes(sizeof(StepState));
+  x.setup();
   if (d.setup(nsteps, true)) return finish(x, "athb_tlm_run: allocation");
+  x.cf = d.cf;
   std::vector<double> h((size_t)NSTATE * ctx->sy * ctx->sx);
   std::copy(dstate0, dstate0 + h.size(), h.begin());
   interior_only(ctx, h);
@@ -424,10 +515,9 @@ int adjoint_impl(athb_ctx* ctx, int nsteps, long long snapshot_bytes, const doub
   x.s = ctx->stream;
   x.cache = ctx->adj_keep ? ctx->adj_cache : nullptr;
   AdjointDriver<GpuExec> d(x, geom_of(ctx));
-  x.red = x.alloc(kRedBlocks);
-  x.redm = (MaxLoc*)x.alloc_bytes(sizeof(MaxLoc) * kRedBlocks);
-  x.st = (StepState*)x.alloc_bytes(sizeof(StepState));
+  x.setup();
   if (d.setup(nsteps, false)) return finish(x, "athb_adjoint_gradient: workspace");
+  x.cf = d.cf;
   if (seed_host) {   // the cotangent of S^N, on the entries a step writes
     std::vector<double> h((size_t)NSTATE * ctx->sy * ctx->sx);
     std::copy(seed_host, seed_host + h.size(), h.begin());

@@ -30,9 +30,9 @@ namespace athb {
 
 // Adjoint workspace planes.
 enum AdjPlane {
-  A_LB1 = 0,     // full-step face field b1 at x faces (update)
-  A_LB2 = 1,     // ... b2 at y faces
-  A_EMF1 = 2,    // corner emf of the full step
+  A_DTY = 0,     // dt terms of the corrector's y faces, then of the PLM in y
+  A_DTC = 1,     // ... of the corrector's cells
+  A_PLMYD = 2,   // the density's share of the PLM source term in y
   A_FX2 = 3,     // corrector x flux (7)
   A_FY2 = 10,    // corrector y flux (7)
   A_ECC1 = 17,   // cell emf3 at t^{n+1/2}
@@ -43,7 +43,6 @@ enum AdjPlane {
   A_HALF = 48,   // half-step d, M1, M2, B1c, B2c of a cell (correct_e)
   A_LB1F = 53,   // half-step b1: every consumer
   A_LB2F = 54,
-  A_EMF0 = 55,   // corner emf of the half step
   A_FX = 56, A_FY = 63,     // predictor fluxes (7 each)
   A_WLNX = 70, A_WRTX = 77, A_WLNY = 84, A_WRTY = 91,  // PLM outputs (7 each)
   A_BNX = 98, A_BNY = 99,   // normal face field at predictor faces
@@ -59,7 +58,7 @@ struct AdjArgs {
   const double* in;     // S^n, ghosts filled
   const double* tape;   // GenPlane planes of the recorded step
   const double* lout;   // adjoint of S^{n+1} (cells the step writes)
-  double* lin;          // adjoint of S^n (accumulated; zeroed before the step)
+  double* lin;          // adjoint of S^n (adj_update writes it, later stages add)
   double* adj;          // AdjPlane planes
   StepCoef<double> c;   // dt^n and its factors, exactly as the forward formed them
   long long ps;
@@ -102,18 +101,6 @@ ATHB_HD void lin_add(const AdjArgs& a, long long o, const int (&p)[N], const dou
 
 ATHB_HD bool in_range(const GenRange& r, int j, int i) { return j >= r.j0 && j <= r.j1 && i >= r.i0 && i <= r.i1; }
 
-// λ of the conserved vector of a sweep (as loaded by gen_cons) and of its
-// normal field added to lin
-ATHB_HD void lin_add_cons(const AdjArgs& a, long long o, int dir, const Cons1& ub, double bnb) {
-  const double v[8] = {ub.d, ub.e, ub.mx, ub.my, ub.mz, ub.by, ub.bz, bnb};
-  if (dir == 0) {
-    const int p[8] = {P_D, P_E, P_M1, P_M2, P_M3, P_B2C, P_B3C, P_B1C};
-    lin_add(a, o, p, v);
-  } else {
-    const int p[8] = {P_D, P_E, P_M2, P_M3, P_M1, P_B3C, P_B1C, P_B2C};
-    lin_add(a, o, p, v);
-  }
-}
 ATHB_HD Cons1 adj_cons(const AdjArgs& a, int base, long long o) {
   Cons1 u;
   u.d = a.av(base + 0, o); u.mx = a.av(base + 1, o); u.my = a.av(base + 2, o); u.mz = a.av(base + 3, o);
@@ -166,32 +153,84 @@ ATHB_HD void corner_k(const AdjArgs& a, int full, int j, int i, double k[8]) {
   corner_emf_coeffs(a.t(fx, o - a.pitch), a.t(fx, o), a.t(fy, o - 1), a.t(fy, o), k);
 }
 
+// The corner emf reversed at place (j,i): t[m] is the adjoint of corner input m
+// of the one corner where this place is that input (corners (j,i), (j,i+1),
+// (j+1,i) and (j+1,i+1)).  lb1 and lb2 give the adjoints of the face fields
+// that CT forms from the emf, zero where there is no such face; the emf's own
+// adjoint is formed here from six faces of each kind, which are in L1, instead
+// of in a launch and a plane of its own.
+template <class B1, class B2>
+ATHB_HD void corner_terms(const AdjArgs& a, int full, const GenRange& K, double w1, double w2, int j, int i,
+                          const B1& lb1, const B2& lb2, double t[8]) {
+  double b1[3][2], b2[2][3];
+#pragma unroll
+  for (int r = 0; r < 3; r++)
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      b1[r][c] = lb1(j - 1 + r, i + c);
+      b2[c][r] = lb2(j + c, i - 1 + r);
+    }
+#pragma unroll
+  for (int m = 0; m < 8; m++) t[m] = 0.0;
+#pragma unroll
+  for (int r = 0; r < 2; r++)
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      if (!in_range(K, j + r, i + c)) continue;
+      const double e = w1 * (b1[r + 1][c] - b1[r][c]) + w2 * (b2[r][c] - b2[r][c + 1]);
+      double k[8];
+      corner_k(a, full, j + r, i + c, k);
+      if (r == 0 && c == 0) { t[1] = k[1] * e; t[3] = k[3] * e; t[7] = k[7] * e; }
+      else if (r == 0) { t[2] = k[2] * e; t[6] = k[6] * e; }
+      else if (c == 0) { t[0] = k[0] * e; t[5] = k[5] * e; }
+      else t[4] = k[4] * e;
+    }
+}
+
 // ===========================================================================
-// Reverse of step 9/11/13 (update): face fields b1, b2 and the cell planes.
-// Items over [is, ie+1] x [js, je+1].
+// Reverse of step 9/11/13 (update): the cell planes, the face fields b1, b2,
+// the corner emf of the full step, and what they leave to the corrector's
+// fluxes and to the half-step cell emf.  One item per place of the whole
+// array: it writes every plane of lin and A_DT (zero where the update adds
+// nothing), so neither is cleared before.  Fluxes and cell emf are gathered
+// over [is-1, ie+1] x [js-1, je+1].
 // ===========================================================================
 ATHB_HD void adj_update(const AdjArgs& a, int j, int i) {
   const long long o = a.o(j, i), P = a.pitch;
-  const double dt0 = a.a(A_DT, o);
-  double dtb = 0.0, l1b = 0.0, l2b = 0.0;
-  // b1 at x face (j,i), i in [is, ie+1], j in [js, je]
-  if (j <= a.je) {
-    double lb = a.lo(P_B1I, o);
-    if (i <= a.ie) lb += 0.5 * a.lo(P_B1C, o);
-    if (i - 1 >= a.is) lb += 0.5 * a.lo(P_B1C, o - 1);
-    l1b = lb;
-    dtb += -lb * (a.t(G_EMF1, o + P) - a.t(G_EMF1, o)) / a.dx2;
+  // b1 at x face (jj,ii), ii in [is, ie+1], jj in [js, je]
+  auto lb1 = [&](int jj, int ii) {
+    if (!(jj >= a.js && jj <= a.je && ii >= a.is && ii <= a.ie + 1)) return 0.0;
+    const long long q = a.o(jj, ii);
+    double lb = a.lo(P_B1I, q);
+    if (ii <= a.ie) lb += 0.5 * a.lo(P_B1C, q);
+    if (ii - 1 >= a.is) lb += 0.5 * a.lo(P_B1C, q - 1);
+    return lb;
+  };
+  // b2 at y face (jj,ii), jj in [js, je+1], ii in [is, ie]
+  auto lb2 = [&](int jj, int ii) {
+    if (!(jj >= a.js && jj <= a.je + 1 && ii >= a.is && ii <= a.ie)) return 0.0;
+    const long long q = a.o(jj, ii);
+    double lb = a.lo(P_B2I, q);
+    if (jj <= a.je) lb += 0.5 * a.lo(P_B2C, q);
+    if (jj - 1 >= a.js) lb += 0.5 * a.lo(P_B2C, q - P);
+    return lb;
+  };
+  double v[NSTATE], dtb = 0.0;
+#pragma unroll
+  for (int p = 0; p < NSTATE; p++) v[p] = 0.0;
+  const GenRange corners = range_emf1(a.is, a.ie, a.js, a.je);
+  const GenRange interior = range_interior(a.is, a.ie, a.js, a.je);
+  if (in_range(corners, j, i)) {
+    if (j <= a.je) {
+      v[P_B1I] = lb1(j, i);
+      dtb += -v[P_B1I] * (a.t(G_EMF1, o + P) - a.t(G_EMF1, o)) / a.dx2;
+    }
+    if (i <= a.ie) {
+      v[P_B2I] = lb2(j, i);
+      dtb += v[P_B2I] * (a.t(G_EMF1, o + 1) - a.t(G_EMF1, o)) / a.dx1;
+    }
   }
-  // b2 at y face (j,i), j in [js, je+1], i in [is, ie]
-  if (i <= a.ie) {
-    double lb = a.lo(P_B2I, o);
-    if (j <= a.je) lb += 0.5 * a.lo(P_B2C, o);
-    if (j - 1 >= a.js) lb += 0.5 * a.lo(P_B2C, o - P);
-    l2b = lb;
-    dtb += lb * (a.t(G_EMF1, o + 1) - a.t(G_EMF1, o)) / a.dx1;
-  }
-  // cell planes
-  if (i <= a.ie && j <= a.je) {
+  if (in_range(interior, j, i)) {
     const double ld = a.lo(P_D, o), l1 = a.lo(P_M1, o), l2 = a.lo(P_M2, o), l3 = a.lo(P_M3, o), le = a.lo(P_E, o);
     const double lb3 = a.lo(P_B3C, o) + a.lo(P_B3I, o);
     // d -= dtodx1 (fx(o+1) - fx(o)) ... ; d -= dtodx2 (fy(o+P) - fy(o)) ...
@@ -209,77 +248,37 @@ ATHB_HD void adj_update(const AdjArgs& a, int j, int i) {
     g2 += le * (a.t(G_FY2 + 4, o + P) - a.t(G_FY2 + 4, o));
     g2 += lb3 * (a.t(G_FY2 + 5, o + P) - a.t(G_FY2 + 5, o));
     dtb += -g1 / a.dx1 - g2 / a.dx2;
-    const int p[8] = {P_D, P_M1, P_M2, P_M3, P_E, P_B3C, P_B1I, P_B2I};
-    const double v[8] = {ld, l1, l2, l3, le, lb3, l1b, l2b};
-    lin_add(a, o, p, v);
-  } else if (j <= a.je) {
-    a.li(P_B1I, o) += l1b;
-  } else if (i <= a.ie) {
-    a.li(P_B2I, o) += l2b;
+    v[P_D] = ld; v[P_M1] = l1; v[P_M2] = l2; v[P_M3] = l3; v[P_E] = le; v[P_B3C] = lb3;
   }
-  if (j <= a.je) a.a(A_LB1, o) = l1b;
-  if (i <= a.ie) a.a(A_LB2, o) = l2b;
-  a.a(A_DT, o) = dt0 + dtb;
-}
+#pragma unroll
+  for (int p = 0; p < NSTATE; p++) a.li(p, o) = v[p];
+  a.a(A_DT, o) = dtb;
 
-// Corner emf of the full step: corners [is, ie+1] x [js, je+1].
-ATHB_HD void adj_emf1(const AdjArgs& a, int j, int i) {
-  const long long o = a.o(j, i), P = a.pitch;
-  auto lb1 = [&](int jj, int ii) { return (jj >= a.js && jj <= a.je && ii >= a.is && ii <= a.ie + 1) ? a.av(A_LB1, a.o(jj, ii)) : 0.0; };
-  auto lb2 = [&](int jj, int ii) { return (jj >= a.js && jj <= a.je + 1 && ii >= a.is && ii <= a.ie) ? a.av(A_LB2, a.o(jj, ii)) : 0.0; };
-  (void)P;
-  a.a(A_EMF1, o) = a.c.dtodx2 * (lb1(j, i) - lb1(j - 1, i)) + a.c.dtodx1 * (lb2(j, i - 1) - lb2(j, i));
-}
-
-// Corrector fluxes and the half-step cell emf: gathers over
-// [is-1, ie+1] x [js-1, je+1].
-ATHB_HD void adj_flux2(const AdjArgs& a, int j, int i) {
-  const long long o = a.o(j, i), P = a.pitch;
-  const GenRange corners = range_emf1(a.is, a.ie, a.js, a.je);
-  const GenRange interior = range_interior(a.is, a.ie, a.js, a.je);
-  auto le = [&](int jj, int ii) { return in_range(corners, jj, ii) ? a.av(A_EMF1, a.o(jj, ii)) : 0.0; };
+  if (j < a.js - 1 || j > a.je + 1 || i < a.is - 1 || i > a.ie + 1) return;
+  double t[8];
+  corner_terms(a, 1, corners, a.c.dtodx2, a.c.dtodx1, j, i, lb1, lb2, t);
   auto lcell = [&](int p, int jj, int ii) {
     if (!in_range(interior, jj, ii)) return 0.0;
     const long long q = a.o(jj, ii);
     return p == P_B3C ? a.lo(P_B3C, q) + a.lo(P_B3I, q) : a.lo(p, q);
   };
-  double k[8];
   // x face (j,i) in the corrector range
   if (in_range(range_correct_x(a.is, a.ie, a.js, a.je), j, i)) {
-    static const int map[7] = {P_D, P_M1, P_M2, P_M3, P_E, -1, P_B3C};
-    for (int c = 0; c < 7; c++) {
-      double v = 0.0;
-      if (map[c] >= 0) v = a.c.dtodx1 * (lcell(map[c], j, i) - lcell(map[c], j, i - 1));
-      a.a(A_FX2 + c, o) = v;
-    }
-    double by = 0.0;
-    if (in_range(corners, j, i)) { corner_k(a, 1, j, i, k); by += k[1] * le(j, i); }
-    if (in_range(corners, j + 1, i)) { corner_k(a, 1, j + 1, i, k); by += k[0] * le(j + 1, i); }
-    a.a(A_FX2 + 5, o) = by;
+    constexpr int map[7] = {P_D, P_M1, P_M2, P_M3, P_E, -1, P_B3C};
+#pragma unroll
+    for (int c = 0; c < 7; c++)
+      if (map[c] >= 0) a.a(A_FX2 + c, o) = a.c.dtodx1 * (lcell(map[c], j, i) - lcell(map[c], j, i - 1));
+    a.a(A_FX2 + 5, o) = t[1] + t[0];
   }
   // y face (j,i)
   if (in_range(range_correct_y(a.is, a.ie, a.js, a.je), j, i)) {
-    static const int map[7] = {P_D, P_M2, P_M3, P_M1, P_E, P_B3C, -1};
-    for (int c = 0; c < 7; c++) {
-      double v = 0.0;
-      if (map[c] >= 0) v = a.c.dtodx2 * (lcell(map[c], j, i) - lcell(map[c], j - 1, i));
-      a.a(A_FY2 + c, o) = v;
-    }
-    double bz = 0.0;
-    if (in_range(corners, j, i)) { corner_k(a, 1, j, i, k); bz += k[3] * le(j, i); }
-    if (in_range(corners, j, i + 1)) { corner_k(a, 1, j, i + 1, k); bz += k[2] * le(j, i + 1); }
-    a.a(A_FY2 + 6, o) = bz;
+    constexpr int map[7] = {P_D, P_M2, P_M3, P_M1, P_E, P_B3C, -1};
+#pragma unroll
+    for (int c = 0; c < 7; c++)
+      if (map[c] >= 0) a.a(A_FY2 + c, o) = a.c.dtodx2 * (lcell(map[c], j, i) - lcell(map[c], j - 1, i));
+    a.a(A_FY2 + 6, o) = t[3] + t[2];
   }
-  // cell (j,i): e_c of corner (j,i), e_w of (j,i+1), e_s of (j+1,i), e_sw of (j+1,i+1)
-  {
-    double v = 0.0;
-    if (in_range(corners, j, i)) { corner_k(a, 1, j, i, k); v += k[7] * le(j, i); }
-    if (in_range(corners, j, i + 1)) { corner_k(a, 1, j, i + 1, k); v += k[6] * le(j, i + 1); }
-    if (in_range(corners, j + 1, i)) { corner_k(a, 1, j + 1, i, k); v += k[5] * le(j + 1, i); }
-    if (in_range(corners, j + 1, i + 1)) { corner_k(a, 1, j + 1, i + 1, k); v += k[4] * le(j + 1, i + 1); }
-    a.a(A_ECC1, o) = v;
-  }
-  (void)P;
+  a.a(A_ECC1, o) = t[7] + t[6] + t[5] + t[4];
 }
 
 // ===========================================================================
@@ -469,7 +468,6 @@ ATHB_HD void adj_correct_x(const AdjArgs& a, int j, int i) {
 template <int FLUX>
 ATHB_HD void adj_correct_y(const AdjArgs& a, int j, int i) {
   const long long o = a.o(j, i);
-  const double dt0 = a.a(A_DT, o);
   Cons1 ul, ur;
   double b2f;
   correct_y_states(a, j, i, ul, ur, b2f);
@@ -482,7 +480,7 @@ ATHB_HD void adj_correct_y(const AdjArgs& a, int j, int i) {
   riemann_adj<FLUX>(ul, ur, wl, wr, b2f, a.eos, adj_cons(a, A_FY2, o), ulb, urb, wlb, wrb, b2fb);
   cons_to_prim_adj(ul, b2f, a.eos, wlb, ulb, b2fb);
   cons_to_prim_adj(ur, b2f, a.eos, wrb, urb, b2fb);
-  a.a(A_DT, o) = dt0 + correct_y_dtb(a, j, i, ulb, urb);
+  a.a(A_DTY, o) = correct_y_dtb(a, j, i, ulb, urb);
   adj_put_cons(a, A_ULY, o, ulb);
   adj_put_cons(a, A_URY, o, urb);
   a.a(A_B2F, o) = b2fb;
@@ -506,7 +504,6 @@ ATHB_HD void adj_correct_e(const AdjArgs& a, int j, int i) {
   const double B2c = 0.5 * (b2f_c + b2f_n);
   const double e = (B1c * M2 - B2c * M1) / d;
   const double lam = a.av(A_ECC1, o);
-  const double dt0 = a.a(A_DT, o);
   const double ld = -lam * e / d, lM1 = -lam * B2c / d, lM2 = lam * B1c / d;
   const int p[3] = {P_D, P_M1, P_M2};
   const double v[3] = {ld, lM1, lM2};
@@ -516,18 +513,21 @@ ATHB_HD void adj_correct_e(const AdjArgs& a, int j, int i) {
   a.a(A_HALF + 2, o) = lM2;
   a.a(A_HALF + 3, o) = lam * M2 / d;
   a.a(A_HALF + 4, o) = -lam * M1 / d;
-  a.a(A_DT, o) = dt0 + (0.5 * (-(ld * dfx0 + lM1 * dfx1 + lM2 * dfx2)) / a.dx1 +
-                        0.5 * (-(ld * dfy0 + lM1 * dfy3 + lM2 * dfy1)) / a.dx2);
+  a.a(A_DTC, o) = 0.5 * (-(ld * dfx0 + lM1 * dfx1 + lM2 * dfx2)) / a.dx1 +
+                  0.5 * (-(ld * dfy0 + lM1 * dfy3 + lM2 * dfy1)) / a.dx2;
 }
 
 // Every consumer of the half-step face fields: x faces [is-1, ie+2] x
 // [js-1, je+1] and y faces [is-1, ie+1] x [js-1, je+2]; items over
-// [is-1, ie+2] x [js-1, je+2].
+// [is-1, ie+2] x [js-1, je+2].  The dt terms of the corrector's y faces and
+// cells join A_DT here, in the order x faces, y faces, cells.
 ATHB_HD void adj_half_faces(const AdjArgs& a, int j, int i) {
   const long long o = a.o(j, i), P = a.pitch;
   const GenRange E = range_correct_e(a.is, a.ie, a.js, a.je);
   const bool xface = j <= a.je + 1, yface = i <= a.ie + 1;
-  const double dt0 = a.a(A_DT, o);
+  double dt0 = a.a(A_DT, o);
+  if (in_range(range_correct_y(a.is, a.ie, a.js, a.je), j, i)) dt0 += a.av(A_DTY, o);
+  if (in_range(E, j, i)) dt0 += a.av(A_DTC, o);
   const double b10 = xface ? a.li(P_B1I, o) : 0.0, b20 = yface ? a.li(P_B2I, o) : 0.0;
   double dtb = 0.0;
   if (xface) {
@@ -551,26 +551,19 @@ ATHB_HD void adj_half_faces(const AdjArgs& a, int j, int i) {
   a.a(A_DT, o) = dt0 + dtb;
 }
 
-// Half-step corner emf: corners [is-1, ie+2] x [js-1, je+2].
-ATHB_HD void adj_emf0(const AdjArgs& a, int j, int i) {
-  const GenRange fx(range_correct_x(a.is, a.ie, a.js, a.je));
-  auto lb1 = [&](int jj, int ii) { return (jj >= a.js - 1 && jj <= a.je + 1 && ii >= a.is - 1 && ii <= a.ie + 2) ? a.av(A_LB1F, a.o(jj, ii)) : 0.0; };
-  auto lb2 = [&](int jj, int ii) { return (jj >= a.js - 1 && jj <= a.je + 2 && ii >= a.is - 1 && ii <= a.ie + 1) ? a.av(A_LB2F, a.o(jj, ii)) : 0.0; };
-  (void)fx;
-  a.a(A_EMF0, a.o(j, i)) = a.c.hdtodx2 * (lb1(j, i) - lb1(j - 1, i)) + a.c.hdtodx1 * (lb2(j, i - 1) - lb2(j, i));
-}
-
 // The predictor fluxes and the t^n cell emf, gathered from the corrector
-// (transverse terms), correct_e and the half-step corner emf; items over
-// [is-2, ie+2] x [js-2, je+2].
+// (transverse terms), correct_e and the half-step corner emf (reversed here
+// from the half-step face fields): [is-2, ie+2] x [js-2, je+2].
 ATHB_HD void adj_flux1(const AdjArgs& a, int j, int i) {
   const long long o = a.o(j, i);
   const StepCoef<double>& c = a.c;
   const GenRange CX = range_correct_x(a.is, a.ie, a.js, a.je), CY = range_correct_y(a.is, a.ie, a.js, a.je);
   const GenRange E = range_correct_e(a.is, a.ie, a.js, a.je), K = range_emf0(a.is, a.ie, a.js, a.je);
-  auto le = [&](int jj, int ii) { return in_range(K, jj, ii) ? a.av(A_EMF0, a.o(jj, ii)) : 0.0; };
+  auto lb1 = [&](int jj, int ii) { return (jj >= a.js - 1 && jj <= a.je + 1 && ii >= a.is - 1 && ii <= a.ie + 2) ? a.av(A_LB1F, a.o(jj, ii)) : 0.0; };
+  auto lb2 = [&](int jj, int ii) { return (jj >= a.js - 1 && jj <= a.je + 2 && ii >= a.is - 1 && ii <= a.ie + 1) ? a.av(A_LB2F, a.o(jj, ii)) : 0.0; };
   auto half = [&](int q, int jj, int ii) { return in_range(E, jj, ii) ? a.av(A_HALF + q, a.o(jj, ii)) : 0.0; };
-  double k[8];
+  double t[8];
+  corner_terms(a, 0, K, c.hdtodx2, c.hdtodx1, j, i, lb1, lb2, t);
   // x face (j,i) of the predictor
   if (in_range(range_riemann_x(a.is, a.ie, a.js, a.je), j, i)) {
     double f[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -590,8 +583,7 @@ ATHB_HD void adj_flux1(const AdjArgs& a, int j, int i) {
     f[1] += c.hdtodx1 * (half(1, j, i) - half(1, j, i - 1));
     f[2] += c.hdtodx1 * (half(2, j, i) - half(2, j, i - 1));
     // half-step corner emf: fx_by of corner (j,i), fx_by_s of corner (j+1,i)
-    if (in_range(K, j, i)) { corner_k(a, 0, j, i, k); f[5] += k[1] * le(j, i); }
-    if (in_range(K, j + 1, i)) { corner_k(a, 0, j + 1, i, k); f[5] += k[0] * le(j + 1, i); }
+    f[5] = t[1] + t[0];
     for (int q = 0; q < 7; q++) a.a(A_FX + q, o) = f[q];
   }
   // y face (j,i)
@@ -613,17 +605,12 @@ ATHB_HD void adj_flux1(const AdjArgs& a, int j, int i) {
     f[3] += c.hdtodx2 * (half(1, j, i) - half(1, j - 1, i));
     f[1] += c.hdtodx2 * (half(2, j, i) - half(2, j - 1, i));
     // corner emf: fy_bz of corner (j,i), fy_bz_w of corner (j,i+1)
-    if (in_range(K, j, i)) { corner_k(a, 0, j, i, k); f[6] += k[3] * le(j, i); }
-    if (in_range(K, j, i + 1)) { corner_k(a, 0, j, i + 1, k); f[6] += k[2] * le(j, i + 1); }
+    f[6] = t[3] + t[2];
     for (int q = 0; q < 7; q++) a.a(A_FY + q, o) = f[q];
   }
   // t^n cell emf of cell (j,i) -> the state
   {
-    double v = 0.0;
-    if (in_range(K, j, i)) { corner_k(a, 0, j, i, k); v += k[7] * le(j, i); }
-    if (in_range(K, j, i + 1)) { corner_k(a, 0, j, i + 1, k); v += k[6] * le(j, i + 1); }
-    if (in_range(K, j + 1, i)) { corner_k(a, 0, j + 1, i, k); v += k[5] * le(j + 1, i); }
-    if (in_range(K, j + 1, i + 1)) { corner_k(a, 0, j + 1, i + 1, k); v += k[4] * le(j + 1, i + 1); }
+    const double v = t[7] + t[6] + t[5] + t[4];
     if (v != 0.0) {
       const double d = a.s(P_D, o), M1 = a.s(P_M1, o), M2 = a.s(P_M2, o), B1 = a.s(P_B1C, o), B2 = a.s(P_B2C, o);
       const double e = (B1 * M2 - B2 * M1) / d;
@@ -636,8 +623,7 @@ ATHB_HD void adj_flux1(const AdjArgs& a, int j, int i) {
 
 // The corrector's MHD source terms (steps 5b, 6b) back to the state: cells
 // [is-1, ie+1] x [js-1, je+1] and the face fields of x faces [is-1, ie+2] x
-// [js-1, je+1], y faces [is-1, ie+1] x [js-1, je+2]; items over
-// [is-1, ie+2] x [js-1, je+2].
+// [js-1, je+1], y faces [is-1, ie+1] x [js-1, je+2].
 ATHB_HD void adj_sources(const AdjArgs& a, int j, int i) {
   const long long o = a.o(j, i), P = a.pitch;
   const double h1 = a.c.hdtodx1, h2 = a.c.hdtodx2;
@@ -714,6 +700,13 @@ ATHB_HD void adj_sources(const AdjArgs& a, int j, int i) {
     a.li(P_B2I, o) += dby_l(j, i) - dby_l(j + 1, i) - dby_r(j, i) + dby_r(j - 1, i);
 }
 
+// Both, items over [is-2, ie+2] x [js-2, je+2]: they read the same corrector
+// adjoints, and neither reads what the other writes.
+ATHB_HD void adj_flux1_sources(const AdjArgs& a, int j, int i) {
+  adj_flux1(a, j, i);
+  if (i >= a.is - 1 && j >= a.js - 1) adj_sources(a, j, i);
+}
+
 // ===========================================================================
 // Reverse of the predictor.
 // ===========================================================================
@@ -759,7 +752,9 @@ ATHB_COLD void plm_adj_general(Cons1 um, Cons1 u0, Cons1 up, double bxm, double 
   *dtodxb = tb;
 }
 
-// PLM + source term of cell (j,i) of sweep dir: cells of range_plm.
+// PLM + source term of cell (j,i) of sweep dir: cells of range_plm.  Both
+// sweeps run in one launch: the y sweep's shares of the density and of dt,
+// which the x sweep adds to as well, go to planes that adj_prim adds.
 ATHB_HD void adj_plm(const AdjArgs& a, int dir, int j, int i) {
   const long long o = a.o(j, i);
   const long long step = dir == 0 ? 1 : a.pitch;
@@ -777,7 +772,7 @@ ATHB_HD void adj_plm(const AdjArgs& a, int dir, int j, int i) {
   const double db = (a.s(bnp, o + step) - a.s(bnp, o)) * rdx;
   const Cons1 um = state_cons(a, o - step, dir), u0 = state_cons(a, o, dir), up = state_cons(a, o + step, dir);
   const double bxm = a.s(bxp, o - step), bx0 = a.s(bxp, o), bxq = a.s(bxp, o + step);
-  const double dt0 = a.a(A_DT, o);
+  const double dt0 = dir == 0 ? a.a(A_DT, o) : 0.0;
   // PLM
   const double hdtodx = dir == 0 ? a.c.hdtodx1 : a.c.hdtodx2;
   double di = recip(u0.d);
@@ -801,22 +796,31 @@ ATHB_HD void adj_plm(const AdjArgs& a, int dir, int j, int i) {
   // source term: src = (mt / d) db, d(B)/dx in db
   const double v0 = mt * di, lsrc = a.c.hdt * lsum;
   double dtb = 0.5 * v0 * db * lsum;
-  const int p[3] = {dir == 0 ? P_M2 : P_M1, P_D, bxp};
-  const double v[3] = {lsrc * db * di, -(lsrc * v0 * di * db), bxcb};
-  lin_add(a, o, p, v);
+  const double ld = -(lsrc * v0 * di * db);
+  if (dir == 0) {
+    const int p[3] = {P_M2, P_D, P_B1C};
+    const double v[3] = {lsrc * db * di, ld, bxcb};
+    lin_add(a, o, p, v);
+  } else {
+    const int p[2] = {P_M1, P_B2C};
+    const double v[2] = {lsrc * db * di, bxcb};
+    lin_add(a, o, p, v);
+    a.a(A_PLMYD, o) = ld;
+  }
   a.a(dir == 0 ? A_SRCX : A_SRCY, o) = lsrc;
   adj_put_prim(a, dir == 0 ? A_WXM : A_WYM, o, wmb);
   adj_put_prim(a, dir == 0 ? A_WX0 : A_WY0, o, w0b);
   adj_put_prim(a, dir == 0 ? A_WXP : A_WYP, o, wpb);
   dtb += dtodxb * rdx;
-  a.a(A_DT, o) = dt0 + dtb;
+  if (dir == 0) a.a(A_DT, o) = dt0 + dtb;
+  else a.a(A_DTY, o) = dtb;
 }
 
-// Primitive-variable adjoints of cell (j,i) gathered from the PLM of cells
-// c-1, c, c+1, back through cons -> prim; and the normal face field of face
-// (j,i) (Riemann states, source terms).  Items over the PLM range widened by
-// one cell along the sweep.
-ATHB_HD void adj_prim_gather(const AdjArgs& a, int dir, int j, int i) {
+// Primitive-variable adjoints of cell (j,i) of sweep dir gathered from the PLM
+// of cells c-1, c, c+1, back through cons -> prim, and the adjoint of the
+// normal face field of face (j,i) (Riemann states, source terms), returned.
+// Cells of the PLM range widened by one along the sweep.
+ATHB_HD double adj_prim_gather(const AdjArgs& a, int dir, int j, int i, Cons1& ub, double& bxb) {
   const long long o = a.o(j, i);
   const long long step = dir == 0 ? 1 : a.pitch;
   const GenRange L = range_plm(a.is, a.ie, a.js, a.je);
@@ -824,21 +828,12 @@ ATHB_HD void adj_prim_gather(const AdjArgs& a, int dir, int j, int i) {
   const int jp = dir == 0 ? j : j + 1, ip = dir == 0 ? i + 1 : i;   // next cell
   Prim1 lw;
   zero(lw);
-  bool any = false;
-  if (in_range(L, j, i)) { addto(lw, adj_prim(a, dir == 0 ? A_WX0 : A_WY0, o)); any = true; }
-  if (in_range(L, jm, im)) { addto(lw, adj_prim(a, dir == 0 ? A_WXP : A_WYP, o - step)); any = true; }
-  if (in_range(L, jp, ip)) { addto(lw, adj_prim(a, dir == 0 ? A_WXM : A_WYM, o + step)); any = true; }
-  if (any) {
-    const int bxp = dir == 0 ? P_B1C : P_B2C;
-    Cons1 ub;
-    zero(ub);
-    double bxb = 0.0;
-    cons_to_prim_adj(state_cons(a, o, dir), a.s(bxp, o), a.eos, lw, ub, bxb);
-    lin_add_cons(a, o, dir, ub, bxb);
-  }
+  if (in_range(L, j, i)) addto(lw, adj_prim(a, dir == 0 ? A_WX0 : A_WY0, o));
+  if (in_range(L, jm, im)) addto(lw, adj_prim(a, dir == 0 ? A_WXP : A_WYP, o - step));
+  if (in_range(L, jp, ip)) addto(lw, adj_prim(a, dir == 0 ? A_WXM : A_WYM, o + step));
+  cons_to_prim_adj(state_cons(a, o, dir), a.s(dir == 0 ? P_B1C : P_B2C, o), a.eos, lw, ub, bxb);
   // normal face field at face (j,i)
   const GenRange F = dir == 0 ? range_riemann_x(a.is, a.ie, a.js, a.je) : range_riemann_y(a.is, a.ie, a.js, a.je);
-  const int bnp = dir == 0 ? P_B1I : P_B2I;
   const int mtp = dir == 0 ? P_M2 : P_M1;
   const double dxs = dir == 0 ? a.dx1 : a.dx2;
   double lb = 0.0;
@@ -847,7 +842,42 @@ ATHB_HD void adj_prim_gather(const AdjArgs& a, int dir, int j, int i) {
   if (in_range(L, j, i)) lb -= a.av(dir == 0 ? A_SRCX : A_SRCY, o) * (a.s(mtp, o) / a.s(P_D, o)) / dxs;
   if (in_range(L, jm, im))
     lb += a.av(dir == 0 ? A_SRCX : A_SRCY, o - step) * (a.s(mtp, o - step) / a.s(P_D, o - step)) / dxs;
-  a.li(bnp, o) += lb;
+  return lb;
+}
+
+// Both sweeps of cell (j,i) onto lin, one read and one write of each plane;
+// items over [is-3, ie+3] x [js-3, je+3].
+ATHB_HD void adj_prim(const AdjArgs& a, int j, int i) {
+  const long long o = a.o(j, i);
+  const bool gx = j >= a.js - 2 && j <= a.je + 2, gy = i >= a.is - 2 && i <= a.ie + 2;
+  if (!gx && !gy) return;
+  const bool plm = gx && gy;   // range_plm
+  const int p[10] = {P_D, P_E, P_M1, P_M2, P_M3, P_B1C, P_B2C, P_B3C, P_B1I, P_B2I};
+  double v[10];
+#pragma unroll
+  for (int k = 0; k < 10; k++) v[k] = a.li(p[k], o);
+  if (plm) {
+    a.a(A_DT, o) += a.av(A_DTY, o);
+    v[0] += a.av(A_PLMYD, o);
+  }
+  if (gx) {
+    Cons1 ub;
+    zero(ub);
+    double bxb = 0.0;
+    v[8] += adj_prim_gather(a, 0, j, i, ub, bxb);
+    v[0] += ub.d; v[1] += ub.e; v[2] += ub.mx; v[3] += ub.my; v[4] += ub.mz;
+    v[6] += ub.by; v[7] += ub.bz; v[5] += bxb;
+  }
+  if (gy) {
+    Cons1 ub;
+    zero(ub);
+    double bxb = 0.0;
+    v[9] += adj_prim_gather(a, 1, j, i, ub, bxb);
+    v[0] += ub.d; v[1] += ub.e; v[3] += ub.mx; v[4] += ub.my; v[2] += ub.mz;
+    v[7] += ub.by; v[5] += ub.bz; v[6] += bxb;
+  }
+#pragma unroll
+  for (int k = 0; k < 10; k++) a.li(p[k], o) = v[k];
 }
 
 // ===========================================================================
