@@ -606,7 +606,7 @@ template <class Exec> struct AdjointDriver {
     a.ps = G.ps; a.pitch = G.pitch;
     a.is = G.is; a.ie = G.ie; a.js = G.js; a.je = G.je;
     a.dx1 = G.dx1; a.dx2 = G.dx2; a.eos = G.eos;
-    a.rdx1 = 1.0 / G.dx1; a.rdx2 = 1.0 / G.dx2;
+    a.fe = make_fast_eos(G.eos, G.dx1, G.dx2);
     return a;
   }
 

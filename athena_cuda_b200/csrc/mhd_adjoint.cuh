@@ -40,8 +40,9 @@ ATHB_HD void addto(Prim1& a, const Prim1& b) {
 }
 
 // --- src/convert_var.c:37-55 -------------------------------------------------
-ATHB_HD void cons_to_prim_adj(const Cons1& u, double bx, const Eos& eos, const Prim1& wb, Cons1& ub, double& bxb) {
-  const double di = 1.0 / u.d;
+// di = 1/u.d
+ATHB_HD void cons_to_prim_adj(const Cons1& u, double bx, const Eos& eos, double di, const Prim1& wb, Cons1& ub,
+                              double& bxb) {
   const double K = u.mx * u.mx + u.my * u.my + u.mz * u.mz;
   const double p2 = (u.e - 0.5 * K * di - 0.5 * (bx * bx + u.by * u.by + u.bz * u.bz)) * eos.gamma_1;
   double dib = 0.0;
@@ -66,18 +67,26 @@ ATHB_HD void cons_to_prim_adj(const Cons1& u, double bx, const Eos& eos, const P
   dib += wb.vx * u.mx + wb.vy * u.my + wb.vz * u.mz;
   ub.d += -di * di * dib;
 }
+ATHB_HD void cons_to_prim_adj(const Cons1& u, double bx, const Eos& eos, const Prim1& wb, Cons1& ub, double& bxb) {
+  cons_to_prim_adj(u, bx, eos, 1.0 / u.d, wb, ub, bxb);
+}
 
 // --- src/convert_var.c:64-92 -------------------------------------------------
-ATHB_HD void prim_to_cons_adj(const Prim1& w, double bx, const Eos& eos, const Cons1& ub, Prim1& wb, double& bxb) {
+// r_gamma_1 = 1/(gamma - 1)
+ATHB_HD void prim_to_cons_adj(const Prim1& w, double bx, double r_gamma_1, const Cons1& ub, Prim1& wb, double& bxb) {
   const double V2 = w.vx * w.vx + w.vy * w.vy + w.vz * w.vz;
   wb.d += ub.d + ub.mx * w.vx + ub.my * w.vy + ub.mz * w.vz + ub.e * 0.5 * V2;
   wb.vx += ub.mx * w.d + ub.e * w.d * w.vx;
   wb.vy += ub.my * w.d + ub.e * w.d * w.vy;
   wb.vz += ub.mz * w.d + ub.e * w.d * w.vz;
-  wb.p += ub.e / eos.gamma_1;
+  wb.p += ub.e * r_gamma_1;
   bxb += ub.e * bx;
   wb.by += ub.by + ub.e * w.by;
   wb.bz += ub.bz + ub.e * w.bz;
+}
+
+ATHB_HD void prim_to_cons_adj(const Prim1& w, double bx, const Eos& eos, const Cons1& ub, Prim1& wb, double& bxb) {
+  prim_to_cons_adj(w, bx, 1.0 / eos.gamma_1, ub, wb, bxb);
 }
 
 // --- src/esystem_prim.c:36-235 -------------------------------------------------
@@ -1559,6 +1568,430 @@ ATHB_HD void flux_roe_adj(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, con
   sb.cs += evb[4] - evb[2];
   roe_speeds_adj(r, Bxi, eos, s, sb, rb, Bxib);
   roe_average_adj(Ul, Ur, Wl, Wr, Bxi, rb, Ulb, Urb, Wlb, Wrb, Bxib);
+}
+
+// ---------------------------------------------------------------------------
+// flux_roe_adj in the fast form: forward values and branches are those of
+// flux_roe_fast, bit for bit (the same operations in the same order), the
+// reverse goes over the pairs of waves n and 6-n and divides nowhere.
+// The general form is bound by its chains of divisions and roots with branches
+// around them (255 registers, 8 warps an SM): at 256 x 256 the corrector's
+// launch took 82 us and the predictor's 69 us with it, 42 and 25 us with this.
+// Error against 80-bit arithmetic: mean 2.4e-16 of the largest output (general:
+// 2.6e-16).
+// ---------------------------------------------------------------------------
+
+// Adjoints of the face's averages, speeds and their inputs, set by the parts below.
+struct RoeBars {
+  RoeAvg r;      // v1, v2, v3, b2, b3, x, droe, pbl, pbr
+  double vsq, hp, cf, cs, vax, gfac, btsq, bt_starsq, twid_asq, cfsq, cssq;
+};
+
+// side_flux_adj; the outputs are set (weight w on Fb).
+ATHB_HD void side_flux_reverse(const Cons1& U, const Prim1& W, double Bxi, double pb, const Cons1& Fb, double w,
+                               Cons1& Ub, Prim1& Wb, double& Bxib, double& pbb) {
+  const double fd = w * Fb.d, fx = w * Fb.mx, fy = w * Fb.my, fz = w * Fb.mz, fe = w * Fb.e, f5 = w * Fb.by,
+               f6 = w * Fb.bz;
+  const double eB = fe * Bxi;
+  Ub.d = 0.0; Ub.my = 0.0; Ub.mz = 0.0; Ub.by = 0.0; Ub.bz = 0.0;
+  Ub.mx = mad(fx, W.vx, mad(fy, W.vy, mad(fz, W.vz, fd)));
+  Ub.e = fe * W.vx;
+  Wb.d = 0.0;
+  Wb.vx = mad(fx, U.mx, mad(fe, (U.e + W.p) + (pb - Bxi * Bxi), mad(f5, W.by, f6 * W.bz)));
+  Wb.vy = mad(fy, U.mx, mad(-eB, W.by, -f5 * Bxi));
+  Wb.vz = mad(fz, U.mx, mad(-eB, W.bz, -f6 * Bxi));
+  Wb.p = mad(fe, W.vx, fx);
+  Wb.by = mad(fx, W.by, mad(-fy, Bxi, mad(-eB, W.vy, f5 * W.vx)));
+  Wb.bz = mad(fx, W.bz, mad(-fz, Bxi, mad(-eB, W.vz, f6 * W.vx)));
+  Bxib = -mad(fx, Bxi, mad(fy, W.by, mad(fz, W.bz, mad(f5, W.vy, f6 * W.vz))));
+  Bxib = mad(-fe, mad(2.0 * Bxi, W.vx, mad(W.by, W.vy, W.bz * W.vz)), Bxib);
+  pbb = fe * W.vx;
+}
+
+// Adjoint of face_averages' speeds (src/esystem_roe.c:68-144), then of its
+// averages (src/flux_roe.c:91-114): onto the two sides.
+ATHB_HD void face_averages_reverse(const Prim1& Wl, const Prim1& Wr, double Bxi, const Eos& eos, const RoeAvg& r,
+                                   const RoeSpeeds& s, const FaceRoots& f, RoeBars& B, Cons1& Ulb, Cons1& Urb,
+                                   Prim1& Wlb, Prim1& Wrb, double& Bxib) {
+  double vaxsqb = s.vax > 0.0 ? B.vax * f.h_vax : 0.0;
+  if (s.cs > 0.0) B.cssq = mad(B.cs, f.h_cs, B.cssq);
+  const double cr = B.cssq * f.r_cfsq;
+  double tab = mad(cr, s.vaxsq, B.twid_asq);
+  vaxsqb = mad(cr, s.twid_asq, vaxsqb);
+  double cfsqb = mad(-cr, s.cssq, B.cfsq);
+  cfsqb = mad(B.cf, f.h_cf, cfsqb);
+  const double tsumb = 0.5 * cfsqb;
+  const double Xb = f.c2 > 0.0 ? tsumb * f.h_c2 : 0.0;
+  const double tdifb = 2.0 * f.tdif * Xb;
+  const double plus = tdifb + tsumb;
+  tab = mad(4.0 * f.ct2, Xb, tab) + (tsumb - tdifb);
+  const double ct2b = mad(4.0 * s.twid_asq, Xb, plus);
+  vaxsqb += plus;
+  double bssb = mad(ct2b, f.rd, B.bt_starsq);
+  double dib = ct2b * s.bt_starsq;
+  double hpb = B.hp, vsqb = B.vsq, xb = B.r.x;
+  if (eos.gamma_1 * (s.hp - 0.5 * s.vsq) - eos.gamma_2 * r.x > kTiny) {
+    hpb = mad(eos.gamma_1, tab, hpb);
+    vsqb = mad(-0.5 * eos.gamma_1, tab, vsqb);
+    xb = mad(-eos.gamma_2, tab, xb);
+  }
+  vaxsqb -= hpb;
+  double btsqb = mad(-hpb, f.rd, B.btsq);
+  dib = mad(-hpb, s.btsq, dib);
+  double bb = 2.0 * vaxsqb * Bxi * f.rd;
+  dib = mad(vaxsqb * Bxi, Bxi, dib);
+  const double gb = mad(bssb, s.btsq, B.gfac);
+  btsqb = mad(bssb, s.gfac, btsqb);
+  const double yb = -eos.gamma_2 * gb;
+  const double b2b = mad(2.0 * r.b2, btsqb, B.r.b2), b3b = mad(2.0 * r.b3, btsqb, B.r.b3);
+  const double v1b = mad(2.0 * r.v1, vsqb, B.r.v1), v2b = mad(2.0 * r.v2, vsqb, B.r.v2),
+               v3b = mad(2.0 * r.v3, vsqb, B.r.v3);
+  double droeb = mad(-f.rd * f.rd, dib, B.r.droe);
+
+  // averages: h = (el / sqrtdl + er / sqrtdr) isd, the others weighted sums times isd
+  const double sl = r.sqrtdl, sr = r.sqrtdr, isd = r.isdlpdr;
+  const double Qb = hpb * isd, Ab = Qb * f.rl, Bb = Qb * f.rr;
+  const double Al = f.el * f.rl, Ar = f.er * f.rr;
+  double slb = -Ab * Al, srb = -Bb * Ar;
+  double isdb = hpb * (Al + Ar);
+  const double pbl = B.r.pbl + Ab, pbr = B.r.pbr + Bb;
+  Ulb.e += Ab; Wlb.p += Ab;
+  Urb.e += Bb; Wrb.p += Bb;
+  Bxib += mad(pbl + pbr, Bxi, bb);
+  // y = 0.5 (dl + dr) / droe
+  const double yd = 0.5 * yb * f.rd;
+  droeb = mad(-yb * r.y, f.rd, droeb);
+  // x = 0.5 (dby^2 + dbz^2) / (sl + sr)^2
+  const double xs = xb * isd * isd;
+  const double dby = Wl.by - Wr.by, dbz = Wl.bz - Wr.bz;
+  const double ssb = -2.0 * xb * r.x * isd;
+  // fields (crossed weights) and velocities
+  const double n2b = b2b * isd, n3b = b3b * isd, m1b = v1b * isd, m2b = v2b * isd, m3b = v3b * isd;
+  Wlb.by += mad(n2b, sr, mad(xs, dby, pbl * Wl.by));
+  Wrb.by += mad(n2b, sl, mad(-xs, dby, pbr * Wr.by));
+  Wlb.bz += mad(n3b, sr, mad(xs, dbz, pbl * Wl.bz));
+  Wrb.bz += mad(n3b, sl, mad(-xs, dbz, pbr * Wr.bz));
+  Wlb.vx = mad(m1b, sl, Wlb.vx); Wlb.vy = mad(m2b, sl, Wlb.vy); Wlb.vz = mad(m3b, sl, Wlb.vz);
+  Wrb.vx = mad(m1b, sr, Wrb.vx); Wrb.vy = mad(m2b, sr, Wrb.vy); Wrb.vz = mad(m3b, sr, Wrb.vz);
+  // isd b: b2 * n2 with n2 = r.b2 / isd and so on
+  isdb = mad(mad(b2b, r.b2, mad(b3b, r.b3, mad(v1b, r.v1, mad(v2b, r.v2, v3b * r.v3)))), sl + sr, isdb);
+  slb += mad(n2b, Wr.by, mad(n3b, Wr.bz, mad(m1b, Wl.vx, mad(m2b, Wl.vy, m3b * Wl.vz))));
+  srb += mad(n2b, Wl.by, mad(n3b, Wl.bz, mad(m1b, Wr.vx, mad(m2b, Wr.vy, m3b * Wr.vz))));
+  const double common = mad(-isdb * isd, isd, ssb);
+  slb = mad(droeb, sr, slb) + common;
+  srb = mad(droeb, sl, srb) + common;
+  Wlb.d += mad(slb, f.hl, yd);
+  Wrb.d += mad(srb, f.hr, yd);
+}
+
+// The outputs are set.  false: outside the ranges, or a face whose
+// intermediate states may send it to HLLE: the outputs are not valid.
+ATHB_HD bool flux_roe_adj_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, const Prim1& Wr, double Bxi,
+                               const Eos& eos, double r_gamma_1, const Cons1& Fb, Cons1& Ulb, Cons1& Urb,
+                               Prim1& Wlb, Prim1& Wrb, double& Bxib) {
+  bool bad = false;
+  RoeAvg r;
+  RoeSpeeds s;
+  FaceRoots f;
+  face_averages(Ul, Ur, Wl, Wr, Bxi, eos, r, s, f, bad);
+  const double v1 = r.v1, v2 = r.v2, v3 = r.v3, b2 = r.b2, b3 = r.b3, d = r.droe;
+  const double cf = s.cf, cs = s.cs, vsq = s.vsq, hp = s.hp;
+  const double ev0 = v1 - cf, ev6 = v1 + cf;
+  RoeBars B;
+  if (ev0 >= 0.0 || ev6 <= 0.0) {   // supersonic: the upwind side's flux, and through its field pressure the averages
+    const bool left = ev0 >= 0.0;
+    double pbb, bxb;
+    Cons1 ub;
+    Prim1 wb;
+    side_flux_reverse(left ? Ul : Ur, left ? Wl : Wr, Bxi, left ? r.pbl : r.pbr, Fb, 1.0, ub, wb, bxb, pbb);
+    // pb = 0.5 |B|^2 of the side: all that is left of the averages
+    wb.by = mad(pbb, left ? Wl.by : Wr.by, wb.by);
+    wb.bz = mad(pbb, left ? Wl.bz : Wr.bz, wb.bz);
+    Bxib = mad(pbb, Bxi, bxb);
+    Cons1 uz;
+    Prim1 wz;
+    zero(uz);
+    zero(wz);
+    Ulb = left ? ub : uz; Wlb = left ? wb : wz;
+    Urb = left ? uz : ub; Wrb = left ? wz : wb;
+    return !bad;
+  }
+
+  // Eigenvector scalars, as flux_roe_fast.
+  double bet2, bet3, hg, hd, ha, af, as, r_bt, r_span, h_af, h_as, g_, scale, h_bs;
+  bool general;
+  field_direction(b2, b3, s.btsq, bet2, bet3, r_bt, bad);
+  const double bt_star = small_root(s.bt_starsq, g_, scale, h_bs);
+  const double sg = root(s.gfac, hg);
+  const double rsg = recip_of_root(sg, hg);
+  const double bet2s = quot(bet2, sg, rsg), bet3s = quot(bet3, sg, rsg);
+  const double bsq = bet2s * bet2s + bet3s * bet3s;
+  const double vbet = v2 * bet2s + v3 * bet3s;
+  wave_weights(s.cfsq - s.cssq, s.twid_asq - s.cssq, s.cfsq - s.twid_asq, af, as, general, r_span, h_af, h_as);
+  bad |= f.tiny_waves && !(as == 0.0 && above<-300>(v1));
+  const double sqrtd = root(d, hd);
+  const double isd = recip_of_root(sqrtd, hd);
+  const unsigned sgn = Bxi < 0. ? 0x80000000u : 0u;
+  const double twid_a = root(s.twid_asq, ha);
+  const double qf = flip(cf * af, sgn), qs = flip(cs * as, sgn);
+  const double afp = twid_a * af * isd, asp = twid_a * as * isd;
+  const double afpbb = afp * bt_star * bsq, aspbb = asp * bt_star * bsq;
+  const double g2x = eos.gamma_2 * r.x;
+  bad |= above<400>(g2x);
+  const double gx = quot(g2x, eos.gamma_1, r_gamma_1);
+  const double norm = 0.5 * recip_from(s.twid_asq, 4.0 * (ha * ha));
+  const double cff = norm * af * cf, css = norm * as * cs;
+  const double qfn = qf * norm, qsn = qs * norm;
+  const double Afn = norm * afp * d, Asn = norm * asp * d;
+  const double afpb = norm * afp * bt_star, aspb = norm * asp * bt_star;
+  const double norm1 = norm * eos.gamma_1;
+  const double afn = af * norm1, asn = as * norm1, norm2 = norm1 * 2.0;
+  const double r_bsq = recip(bsq);
+  const double q2s = quot(bet2s, bsq, r_bsq), q3s = quot(bet3s, bsq, r_bsq);
+  const double vqstr = v2 * q2s + v3 * q3s;
+  const double vh = vsq - hp;
+  const double ds = flip(isd, sgn), hs = flip(0.5 * sqrtd, sgn);
+  const double cross = v2 * bet3 - v3 * bet2;
+
+  // wave strengths
+  const double u0 = Ur.d - Ul.d, u1 = Ur.mx - Ul.mx, u2 = Ur.my - Ul.my, u3 = Ur.mz - Ul.mz, u4 = Ur.e - Ul.e,
+               u5 = Ur.by - Ul.by, u6 = Ur.bz - Ul.bz;
+  double a[7];
+  {
+    const double p4 = afn * u4;
+    const double p5 = (Asn * q2s - afn * b2) * u5, p6 = (Asn * q3s - afn * b3) * u6;
+    const double t0 = afn * vh, tq = qsn * vqstr, t1 = afn * v1, t2 = afn * v2, t3 = afn * v3;
+    const double k2 = qsn * q2s, k3 = qsn * q3s;
+    a[0] = (t0 + cff * (cf + v1) - tq - aspb) * u0 - (t1 + cff) * u1 + (k2 - t2) * u2 + (k3 - t3) * u3 + p4 + p5 + p6;
+    a[6] = (t0 + cff * (cf - v1) + tq - aspb) * u0 + (cff - t1) * u1 - (t2 + k2) * u2 - (t3 + k3) * u3 + p4 + p5 + p6;
+  }
+  {
+    const double p0 = (0.5 * cross) * u0;
+    const double p5 = hs * bet3 * u5, p6 = hs * bet2 * u6;
+    const double t = p0 - (0.5 * bet3) * u2 + (0.5 * bet2) * u3;
+    a[1] = t - p5 + p6;
+    a[5] = p6 - (t + p5);
+  }
+  {
+    const double p4 = asn * u4;
+    const double p5 = (Afn * q2s + asn * b2) * u5, p6 = (Afn * q3s + asn * b3) * u6;
+    const double t0 = asn * vh, tq = qfn * vqstr, t1 = asn * v1, t2 = asn * v2, t3 = asn * v3;
+    const double k2 = qfn * q2s, k3 = qfn * q3s;
+    a[2] = (t0 + css * (cs + v1) + tq + afpb) * u0 - (t1 + css) * u1 - (t2 + k2) * u2 - (t3 + k3) * u3 + p4 - p5 - p6;
+    a[4] = (t0 + css * (cs - v1) - tq + afpb) * u0 + (css - t1) * u1 + (k2 - t2) * u2 + (k3 - t3) * u3 + p4 - p5 - p6;
+  }
+  a[3] = (1.0 - norm2 * (0.5 * vsq - gx)) * u0 + (norm2 * v1) * u1 + (norm2 * v2) * u2 + (norm2 * v3) * u3 -
+         norm2 * u4 + (norm2 * b2) * u5 + (norm2 * b3) * u6;
+
+  // the positivity test of flux_roe_fast (step 7), on the states themselves
+  {
+    const double c1a = af * v2, c1b = qs * bet2s, c2a = af * v3, c2b = qs * bet3s, e0 = qs * vbet;
+    const double s1a = as * v2, s1b = qf * bet2s, s2a = as * v3, s2b = qf * bet3s, e2 = qf * vbet;
+    const double vcf = v1 * cf, vcs = v1 * cs;
+    const double fb2 = asp * bet2s, fb3 = asp * bet3s, sb2 = -afp * bet2s, sb3 = -afp * bet3s;
+    const double C[6][7] = {
+        {af, af * ev0, c1a + c1b, c2a + c2b, af * (hp - vcf) + e0 + aspbb, fb2, fb3},
+        {0.0, 0.0, -bet3, bet2, -cross, -bet3 * ds, bet2 * ds},
+        {as, as * (v1 - cs), s1a - s1b, s2a - s2b, as * (hp - vcs) - e2 - afpbb, sb2, sb3},
+        {1.0, v1, v2, v3, 0.5 * vsq + gx, 0.0, 0.0},
+        {as, as * (v1 + cs), s1a + s1b, s2a + s2b, as * (hp + vcs) + e2 - afpbb, sb2, sb3},
+        {0.0, 0.0, bet3, -bet2, cross, -bet3 * ds, bet2 * ds}};
+    double u[7] = {Ul.d, Ul.mx, Ul.my, Ul.mz, Ul.e, Ul.by, Ul.bz};
+#pragma unroll
+    for (int n = 0; n < 6; n++) {
+#pragma unroll
+      for (int m = 0; m < 7; m++)
+        if ((roe_right_mask(n) >> m) & 1) u[m] = mad(a[n], C[n][m], u[m]);
+      const double k = 0.5 * (u[5] * u[5] + u[6] * u[6] + Bxi * Bxi);
+      const double m2 = 0.5 * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]);
+      bad |= !(u[0] > 0.0) || !((u[4] - k) * u[0] - m2 > 1.0e-12 * (u[4] * u[0]));
+    }
+  }
+
+  // ---- reverse.  F = 0.5 (Fl + Fr) - sum_n 0.5 |ev_n| a_n c_n: q_n is the
+  // adjoint of column n over Fb, ab_n that of a_n, eb_n that of ev_n.
+  const double f0 = Fb.d, f1 = Fb.mx, f2 = Fb.my, f3 = Fb.mz, f4 = Fb.e, f5 = Fb.by, f6 = Fb.bz;
+  const double pb = mad(f2, bet2s, mad(f3, bet3s, f4 * vbet)), tb = mad(f5, bet2s, f6 * bet3s);
+  const double g = mad(f4, v1, f1);
+  const double base = mad(f1, v1, mad(f2, v2, mad(f3, v3, mad(f4, hp, f0))));
+  const double ev[7] = {ev0, v1 - s.vax, v1 - cs, v1, v1 + cs, v1 + s.vax, ev6};
+  double q[7], ab[7], eb[7];
+  {
+    double k[7];   // minus the product of Fb and column n
+    const double cg = cf * g, fs = mad(f4, aspbb, asp * tb), qp = qs * pb;
+    k[0] = -(mad(af, base - cg, qp) + fs);
+    k[6] = -(mad(af, base + cg, -qp) + fs);
+    const double sgm = cs * g, ss = -mad(f4, afpbb, afp * tb), qq = qf * pb;
+    k[2] = -(mad(as, base - sgm, -qq) + ss);
+    k[4] = -(mad(as, base + sgm, qq) + ss);
+    const double X = mad(-f4, cross, mad(f3, bet2, -f2 * bet3)), Y = ds * mad(f6, bet2, -f5 * bet3);
+    k[1] = -(X + Y);
+    k[5] = X - Y;
+    k[3] = -mad(f4, mad(0.5, vsq, gx), mad(f1, v1, mad(f2, v2, mad(f3, v3, f0))));
+#pragma unroll
+    for (int n = 0; n < 7; n++) {
+      const double h = 0.5 * fabs(ev[n]);
+      q[n] = -h * a[n];
+      ab[n] = h * k[n];
+      eb[n] = ev[n] == 0.0 ? 0.0 : flip(0.5 * a[n] * k[n], hi_word(ev[n]));
+    }
+  }
+  const double Q0 = q[0] + q[6], D0 = q[0] - q[6], Q2 = q[2] + q[4], D2 = q[4] - q[2], Q1 = q[1] + q[5],
+               D1 = q[1] - q[5], q3 = q[3];
+  eb[0] = mad(q[0] * f1, af, eb[0]);
+  eb[6] = mad(q[6] * f1, af, eb[6]);
+  eb[2] = mad(q[2] * f1, as, eb[2]);
+  eb[4] = mad(q[4] * f1, as, eb[4]);
+  // the columns' scalars
+  double afb = mad(Q0, base, -D0 * (cf * g)), asb = mad(Q2, base, D2 * (cs * g));
+  const double A = mad(Q0, af, Q2 * as);            // weight of f2, f3, f4 on v2, v3, hp
+  const double M = mad(D2 * as, cs, -D0 * af * cf); // ... of f4 on v1
+  double v1b = mad(f4, M, q3 * f1);
+  double v2b = mad(f2, A, q3 * f2), v3b = mad(f3, A, q3 * f3);
+  double hpb = f4 * A;
+  double cfb = -D0 * af * (f4 * v1), csb = D2 * as * (f4 * v1);
+  double qsb = D0 * pb, qfb = D2 * pb;
+  const double Rq = mad(D0, qs, D2 * qf), Rp = mad(Q0, asp, -Q2 * afp);
+  double bet2sb = mad(f2, Rq, f5 * Rp), bet3sb = mad(f3, Rq, f6 * Rp);
+  const double vbetb = f4 * Rq;
+  const double aspbbb = f4 * Q0, afpbbb = -f4 * Q2;
+  double aspb_ = Q0 * tb, afpb_ = -Q2 * tb;
+  double bet3b = -mad(D1, mad(f4, v2, f2), Q1 * f5 * ds), bet2b = mad(D1, mad(f4, v3, f3), Q1 * f6 * ds);
+  v2b = mad(-D1 * f4, bet3, v2b);
+  v3b = mad(D1 * f4, bet2, v3b);
+  double isdb = flip(Q1, sgn) * mad(f6, bet2, -f5 * bet3);
+  double vsqb = 0.5 * q3 * f4, gxb = q3 * f4;
+
+  // a = L (Ur - Ul)
+  const double t = ab[0] + ab[6], dd = ab[0] - ab[6], t2 = ab[2] + ab[4], d2 = ab[2] - ab[4], t1 = ab[1] + ab[5],
+               d1 = ab[1] - ab[5], a3 = ab[3], m = norm2 * a3;
+  const double vu = mad(v1, u1, mad(v2, u2, mad(v3, u3, mad(b2, u5, mad(b3, u6, -u4)))));
+  const double W = mad(vh, u0, -vu);
+  const double Z = mad(q2s, u5, q3s * u6);
+  const double Yq = mad(q2s, u2, mad(q3s, u3, -vqstr * u0));
+  const double E0 = mad(afn, t, asn * t2), E = E0 - m;
+  const double H = mad(qsn, dd, -qfn * d2), Kn = mad(Asn, t, -Afn * t2);
+  const double Cd = mad(cff, dd, css * d2);
+  const double l0 = mad(cf, t, v1 * dd), l2 = mad(cs, t2, v1 * d2);
+  Cons1 du;
+  du.d = mad(E0, vh, mad(-H, vqstr, mad(cff, l0, mad(css, l2, mad(-aspb, t, afpb * t2)))));
+  du.d = mad(0.5 * cross, d1, du.d) + mad(-m, mad(0.5, vsq, -gx), a3);
+  du.mx = -mad(E, v1, Cd);
+  du.my = mad(-E, v2, mad(H, q2s, -0.5 * bet3 * d1));
+  du.mz = mad(-E, v3, mad(H, q3s, 0.5 * bet2 * d1));
+  du.e = E;
+  du.by = mad(-E, b2, mad(Kn, q2s, -hs * bet3 * t1));
+  du.bz = mad(-E, b3, mad(Kn, q3s, hs * bet2 * t1));
+  const double afnb = W * t, asnb = W * t2, Asnb = Z * t, Afnb = -Z * t2, qsnb = Yq * dd, qfnb = -Yq * d2;
+  const double cffb = mad(u0, l0, -u1 * dd), cssb = mad(u0, l2, -u1 * d2);
+  cfb = mad(cff * u0, t, cfb);
+  csb = mad(css * u0, t2, csb);
+  v1b = mad(Cd, u0, mad(-E, u1, v1b));
+  const double hd1 = 0.5 * d1;
+  v2b = mad(-E, u2, mad(hd1 * bet3, u0, v2b));
+  v3b = mad(-E, u3, mad(-hd1 * bet2, u0, v3b));
+  double b2b = -E * u5, b3b = -E * u6;
+  const double vqstrb = -H * u0, aspbn = -u0 * t, afpbn = u0 * t2;
+  double q2sb = mad(H, u2, Kn * u5), q3sb = mad(H, u3, Kn * u6);
+  bet3b = mad(hd1, mad(v2, u0, -u2), mad(-hs * u5, t1, bet3b));
+  bet2b = mad(hd1, mad(-v3, u0, u3), mad(hs * u6, t1, bet2b));
+  double sqrtdb = flip(0.5 * t1, sgn) * mad(bet2, u6, -bet3 * u5);
+  const double norm2b = a3 * mad(gx - 0.5 * vsq, u0, vu);
+  vsqb = mad(-0.5 * m, u0, mad(u0, E0, vsqb));
+  hpb = mad(-u0, E0, hpb);
+  gxb = mad(m, u0, gxb);
+
+  // the scalars back to speeds and averages
+  v2b = mad(vqstrb, q2s, v2b);
+  v3b = mad(vqstrb, q3s, v3b);
+  q2sb = mad(vqstrb, v2, q2sb);
+  q3sb = mad(vqstrb, v3, q3sb);
+  double bsqb = -r_bsq * mad(q2sb, q2s, q3sb * q3s);
+  bet2sb = mad(q2sb, r_bsq, bet2sb);
+  bet3sb = mad(q3sb, r_bsq, bet3sb);
+  afb = mad(afnb, norm1, afb);
+  asb = mad(asnb, norm1, asb);
+  double normb = eos.gamma_1 * mad(afnb, af, mad(asnb, as, 2.0 * norm2b));
+  normb = mad(bt_star, mad(aspbn, asp, afpbn * afp), normb);
+  normb = mad(d, mad(Asnb, asp, Afnb * afp), normb);
+  normb = mad(qsnb, qs, mad(qfnb, qf, mad(cssb * as, cs, mad(cffb * af, cf, normb))));
+  const double nb = norm * bt_star, nd = norm * d, bb = bt_star * bsq;
+  aspb_ = mad(aspbn, nb, mad(Asnb, nd, mad(aspbbb, bb, aspb_)));
+  afpb_ = mad(afpbn, nb, mad(Afnb, nd, mad(afpbbb, bb, afpb_)));
+  const double pp = mad(aspbbb, asp, afpbbb * afp);
+  const double btsb = mad(norm, mad(aspbn, asp, afpbn * afp), bsq * pp);
+  bsqb = mad(bt_star, pp, bsqb);
+  double db = norm * mad(Asnb, asp, Afnb * afp);
+  qsb = mad(qsnb, norm, qsb);
+  qfb = mad(qfnb, norm, qfb);
+  asb = mad(cssb * norm, cs, asb);
+  afb = mad(cffb * norm, cf, afb);
+  csb = mad(cssb * norm, as, csb);
+  cfb = mad(cffb * norm, af, cfb);
+  double twb = -2.0 * normb * norm * norm;   // norm = 0.5 / twid_asq
+  const double wp = mad(aspb_, as, afpb_ * af);
+  twb = mad(wp * isd, ha, twb);
+  const double ti = twid_a * isd;
+  asb = mad(aspb_, ti, asb);
+  afb = mad(afpb_, ti, afb);
+  isdb = mad(wp, twid_a, isdb);
+  const double qsf = flip(qsb, sgn), qff = flip(qfb, sgn);
+  csb = mad(qsf, as, csb);
+  asb = mad(qsf, cs, asb);
+  cfb = mad(qff, af, cfb);
+  afb = mad(qff, cf, afb);
+  sqrtdb = mad(-isdb * isd, isd, sqrtdb);
+  db = mad(sqrtdb, hd, db);
+  B.cfsq = 0.0;
+  B.cssq = 0.0;
+  if (general) {
+    // alpha_f^2 = (twid_asq - cssq)/span, alpha_s^2 = (cfsq - twid_asq)/span: each
+    // term is rounded once and used as it is (they cancel where a weight is small)
+    const double Afr = afb * h_af * r_span, Asr = asb * h_as * r_span;
+    const double Db = mad(Afr, af * af, Asr * (as * as));
+    twb = (twb + Afr) - Asr;
+    B.cssq = Db - Afr;
+    B.cfsq = Asr - Db;
+  }
+  v2b = mad(vbetb, bet2s, v2b);
+  v3b = mad(vbetb, bet3s, v3b);
+  bet2sb = mad(2.0 * bet2s, bsqb, mad(vbetb, v2, bet2sb));
+  bet3sb = mad(2.0 * bet3s, bsqb, mad(vbetb, v3, bet3sb));
+  bet2b = mad(bet2sb, rsg, bet2b);
+  bet3b = mad(bet3sb, rsg, bet3b);
+  B.gfac = -rsg * mad(bet2sb, bet2s, bet3sb * bet3s) * hg;
+  B.btsq = 0.0;
+  if (s.btsq != 0.0 && !(s.btsq < kBetaFreeze * (Bxi * Bxi + d * s.twid_asq))) {   // freeze_beta
+    // r_bt is 1/|b_t| here: a field whose square is small enough to be scaled is frozen
+    const double btb = -r_bt * mad(bet2b, bet2, bet3b * bet3);
+    b2b = mad(bet2b, r_bt, b2b);
+    b3b = mad(bet3b, r_bt, b3b);
+    B.btsq = 0.5 * btb * r_bt;
+  }
+  B.bt_starsq = bt_star > 0.0 ? btsb * (h_bs * scale) : 0.0;
+  B.r.x = gxb * eos.gamma_2 * r_gamma_1;
+  B.r.v1 = v1b + (((eb[0] + eb[6]) + (eb[1] + eb[5])) + ((eb[2] + eb[4]) + eb[3]));
+  B.r.v2 = v2b;
+  B.r.v3 = v3b;
+  B.r.b2 = b2b;
+  B.r.b3 = b3b;
+  B.r.droe = db;
+  B.vsq = vsqb;
+  B.hp = hpb;
+  B.cf = cfb + (eb[6] - eb[0]);
+  B.cs = csb + (eb[4] - eb[2]);
+  B.vax = eb[5] - eb[1];
+  B.twid_asq = twb;
+
+  // the sides' own fluxes, the jump, the averages
+  double bl, br;
+  side_flux_reverse(Ul, Wl, Bxi, r.pbl, Fb, 0.5, Ulb, Wlb, bl, B.r.pbl);
+  side_flux_reverse(Ur, Wr, Bxi, r.pbr, Fb, 0.5, Urb, Wrb, br, B.r.pbr);
+  Bxib = bl + br;
+  Ulb.d -= du.d; Ulb.mx -= du.mx; Ulb.my -= du.my; Ulb.mz -= du.mz; Ulb.e -= du.e; Ulb.by -= du.by; Ulb.bz -= du.bz;
+  addto(Urb, du);
+  face_averages_reverse(Wl, Wr, Bxi, eos, r, s, f, B, Ulb, Urb, Wlb, Wrb, Bxib);
+  return !bad;
 }
 
 template <int FLUX>

@@ -509,13 +509,15 @@ ATHB_HD bool plm_cell_fast(const Prim1& wm, const Prim1& w0, const Prim1& wp, do
 struct FaceRoots {
   double rd;         // 1/droe
   bool tiny_waves;   // slow or Alfven speeds below 2^-480 and not zero
+  // for the adjoint: 1/sqrt(d) and 1/(2 sqrt(d)) of the sides, energies over
+  // them, the discriminant's terms, 1/(2 root) of the speeds' roots, 1/cfsq
+  double rl, rr, hl, hr, el, er, ct2, tdif, c2, h_c2, h_cf, h_cs, h_vax, r_cfsq;
 };
 ATHB_HD void face_averages(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, const Prim1& Wr, double Bxi,
                            const Eos& eos, RoeAvg& r, RoeSpeeds& s, FaceRoots& f, bool& bad) {
   bad |= outside<-100, 100>(Wl.d) | outside<-100, 100>(Wr.d) | above<100>(Bxi);
-  double hl, hr;
-  r.sqrtdl = root(Wl.d, hl);
-  r.sqrtdr = root(Wr.d, hr);
+  r.sqrtdl = root(Wl.d, f.hl);
+  r.sqrtdr = root(Wr.d, f.hr);
   const double ss = r.sqrtdl + r.sqrtdr;
   r.isdlpdr = recip(ss);
   r.droe = r.sqrtdl * r.sqrtdr;
@@ -536,8 +538,11 @@ ATHB_HD void face_averages(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
   r.pbr = 0.5 * (bx2 + Wr.by * Wr.by + Wr.bz * Wr.bz);
   const double el = Ul.e + Wl.p + r.pbl, er = Ur.e + Wr.p + r.pbr;
   bad |= outside0<-700, 400>(el) | outside0<-700, 400>(er);
-  r.h = (quot(el, r.sqrtdl, recip_of_root(r.sqrtdl, hl)) + quot(er, r.sqrtdr, recip_of_root(r.sqrtdr, hr))) *
-        r.isdlpdr;
+  f.rl = recip_of_root(r.sqrtdl, f.hl);
+  f.rr = recip_of_root(r.sqrtdr, f.hr);
+  f.el = el;
+  f.er = er;
+  r.h = (quot(el, r.sqrtdl, f.rl) + quot(er, r.sqrtdr, f.rr)) * r.isdlpdr;
   s.di = f.rd;
   s.vsq = r.v1 * r.v1 + r.v2 * r.v2 + r.v3 * r.v3;
   s.btsq = r.b2 * r.b2 + r.b3 * r.b3;
@@ -550,14 +555,16 @@ ATHB_HD void face_averages(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
   const double tsum = s.vaxsq + ct2 + s.twid_asq;
   const double tdif = s.vaxsq + ct2 - s.twid_asq;
   bad |= outside<-100, 200>(s.gfac) | outside<-100, 200>(s.twid_asq) | outside<-150, 300>(tsum);
-  const double cf2_cs2 = root(tdif * tdif + 4.0 * s.twid_asq * ct2);
-  s.cfsq = 0.5 * (tsum + cf2_cs2);
-  double hf;
-  s.cf = root(s.cfsq, hf);
+  f.c2 = root(tdif * tdif + 4.0 * s.twid_asq * ct2, f.h_c2);
+  s.cfsq = 0.5 * (tsum + f.c2);
+  s.cf = root(s.cfsq, f.h_cf);
   const double csnum = s.twid_asq * s.vaxsq;
-  s.cssq = quot(csnum, s.cfsq, recip_from(s.cfsq, 4.0 * (hf * hf)));
-  s.cs = root(s.cssq);
-  s.vax = root(s.vaxsq);
+  f.r_cfsq = recip_from(s.cfsq, 4.0 * (f.h_cf * f.h_cf));
+  s.cssq = quot(csnum, s.cfsq, f.r_cfsq);
+  s.cs = root(s.cssq, f.h_cs);
+  s.vax = root(s.vaxsq, f.h_vax);
+  f.ct2 = ct2;
+  f.tdif = tdif;
   f.tiny_waves = outside0<-960, 500>(csnum) | outside0<-960, 500>(s.vaxsq) | outside0<-960, 500>(s.cssq);
   // x below 2^-700 does not show beside the squared velocity, nor in the
   // sound speed

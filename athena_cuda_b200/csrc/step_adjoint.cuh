@@ -65,8 +65,8 @@ struct AdjArgs {
   int pitch;
   int is, ie, js, je;
   double dx1, dx2;
-  double rdx1, rdx2;    // 1/dx1, 1/dx2
   Eos eos;
+  FastEos fe;           // constants of the fast forms
   ATHB_MEM long long o(int j, int i) const { return (long long)j * pitch + i; }
   ATHB_MEM double s(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return ro(in + p * ps + off); }
   ATHB_MEM double t(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return ro(tape + p * ps + off); }
@@ -443,6 +443,41 @@ ATHB_HD double correct_y_dtb(const AdjArgs& a, int j, int i, const Cons1& lul, c
   return 0.5 * g1 / a.dx1 + 0.5 * g2 / a.dx2;
 }
 
+// The adjoint of the face flux: the fast form where it applies, else the
+// general one, out of line.  The outputs are set.
+template <int FLUX>
+ATHB_COLD void face_adj_general(const Cons1* ul, const Cons1* ur, const Prim1* wl, const Prim1* wr, double bn,
+                                const Eos* eos, const Cons1* fb, Cons1* ulb, Cons1* urb, Prim1* wlb, Prim1* wrb,
+                                double* bnb) {
+  zero(*ulb); zero(*urb); zero(*wlb); zero(*wrb);
+  *bnb = 0.0;
+  riemann_adj<FLUX>(*ul, *ur, *wl, *wr, bn, *eos, *fb, *ulb, *urb, *wlb, *wrb, *bnb);
+}
+template <int FLUX>
+ATHB_HD void face_adj(const AdjArgs& a, const Cons1& ul, const Cons1& ur, const Prim1& wl, const Prim1& wr, double bn,
+                      const Cons1& fb, Cons1& ulb, Cons1& urb, Prim1& wlb, Prim1& wrb, double& bnb) {
+  if (FLUX == kFluxHlle) {
+    zero(ulb); zero(urb); zero(wlb); zero(wrb);
+    bnb = 0.0;
+    flux_hlle_adj(ul, ur, wl, wr, bn, a.eos, fb, ulb, urb, wlb, wrb, bnb);
+    return;
+  }
+  if (flux_roe_adj_fast(ul, ur, wl, wr, bn, a.eos, a.fe.r_gamma_1, fb, ulb, urb, wlb, wrb, bnb) && a.fe.ok) return;
+  const Cons1 u = ul, v = ur, f = fb;
+  const Prim1 w = wl, x = wr;
+  const Eos eos = a.eos;
+  Cons1 ub, vb;
+  Prim1 wb, xb;
+  double bb;
+  face_adj_general<FLUX>(&u, &v, &w, &x, bn, &eos, &f, &ub, &vb, &wb, &xb, &bb);
+  ulb = ub; urb = vb; wlb = wb; wrb = xb;
+  bnb = bb;
+}
+// prim_to_cons with the launch's 1/(gamma - 1)
+ATHB_HD Cons1 face_cons(const AdjArgs& a, const Prim1& w, double bn) {
+  return a.fe.ok ? cons_of(w, bn, a.eos, a.fe.r_gamma_1) : prim_to_cons(w, bn, a.eos);
+}
+
 template <int FLUX>
 ATHB_HD void adj_correct_x(const AdjArgs& a, int j, int i) {
   const long long o = a.o(j, i);
@@ -450,15 +485,14 @@ ATHB_HD void adj_correct_x(const AdjArgs& a, int j, int i) {
   Cons1 ul, ur;
   double b1f;
   correct_x_states(a, j, i, ul, ur, b1f);
-  const Prim1 wl = cons_to_prim(ul, b1f, a.eos);
-  const Prim1 wr = cons_to_prim(ur, b1f, a.eos);
+  const double dil = any_recip(ul.d), dir = any_recip(ur.d);
+  const Prim1 wl = prim_of(ul, b1f, dil, a.eos), wr = prim_of(ur, b1f, dir, a.eos);
   Cons1 ulb, urb;
   Prim1 wlb, wrb;
-  zero(ulb); zero(urb); zero(wlb); zero(wrb);
-  double b1fb = 0.0;
-  riemann_adj<FLUX>(ul, ur, wl, wr, b1f, a.eos, adj_cons(a, A_FX2, o), ulb, urb, wlb, wrb, b1fb);
-  cons_to_prim_adj(ul, b1f, a.eos, wlb, ulb, b1fb);
-  cons_to_prim_adj(ur, b1f, a.eos, wrb, urb, b1fb);
+  double b1fb;
+  face_adj<FLUX>(a, ul, ur, wl, wr, b1f, adj_cons(a, A_FX2, o), ulb, urb, wlb, wrb, b1fb);
+  cons_to_prim_adj(ul, b1f, a.eos, dil, wlb, ulb, b1fb);
+  cons_to_prim_adj(ur, b1f, a.eos, dir, wrb, urb, b1fb);
   a.a(A_DT, o) = dt0 + correct_x_dtb(a, j, i, ulb, urb);
   adj_put_cons(a, A_ULX, o, ulb);
   adj_put_cons(a, A_URX, o, urb);
@@ -471,15 +505,14 @@ ATHB_HD void adj_correct_y(const AdjArgs& a, int j, int i) {
   Cons1 ul, ur;
   double b2f;
   correct_y_states(a, j, i, ul, ur, b2f);
-  const Prim1 wl = cons_to_prim(ul, b2f, a.eos);
-  const Prim1 wr = cons_to_prim(ur, b2f, a.eos);
+  const double dil = any_recip(ul.d), dir = any_recip(ur.d);
+  const Prim1 wl = prim_of(ul, b2f, dil, a.eos), wr = prim_of(ur, b2f, dir, a.eos);
   Cons1 ulb, urb;
   Prim1 wlb, wrb;
-  zero(ulb); zero(urb); zero(wlb); zero(wrb);
-  double b2fb = 0.0;
-  riemann_adj<FLUX>(ul, ur, wl, wr, b2f, a.eos, adj_cons(a, A_FY2, o), ulb, urb, wlb, wrb, b2fb);
-  cons_to_prim_adj(ul, b2f, a.eos, wlb, ulb, b2fb);
-  cons_to_prim_adj(ur, b2f, a.eos, wrb, urb, b2fb);
+  double b2fb;
+  face_adj<FLUX>(a, ul, ur, wl, wr, b2f, adj_cons(a, A_FY2, o), ulb, urb, wlb, wrb, b2fb);
+  cons_to_prim_adj(ul, b2f, a.eos, dil, wlb, ulb, b2fb);
+  cons_to_prim_adj(ur, b2f, a.eos, dir, wrb, urb, b2fb);
   a.a(A_DTY, o) = correct_y_dtb(a, j, i, ulb, urb);
   adj_put_cons(a, A_ULY, o, ulb);
   adj_put_cons(a, A_URY, o, urb);
@@ -718,20 +751,18 @@ ATHB_HD void adj_riemann(const AdjArgs& a, int dir, int j, int i) {
   const Prim1 wl = tape_prim(a, dir == 0 ? G_WLNX : G_WLNY, o - step);
   const Prim1 wr = tape_prim(a, dir == 0 ? G_WRTX : G_WRTY, o);
   const double bn = a.s(dir == 0 ? P_B1I : P_B2I, o);
-  const Cons1 ul = prim_to_cons(wl, bn, a.eos);
-  const Cons1 ur = prim_to_cons(wr, bn, a.eos);
+  const Cons1 ul = face_cons(a, wl, bn), ur = face_cons(a, wr, bn);
   Cons1 ulb, urb;
   Prim1 wlb, wrb;
-  zero(ulb); zero(urb); zero(wlb); zero(wrb);
-  double bnb = 0.0;
-  riemann_adj<FLUX>(ul, ur, wl, wr, bn, a.eos, adj_cons(a, dir == 0 ? A_FX : A_FY, o), ulb, urb, wlb, wrb, bnb);
+  double bnb;
+  face_adj<FLUX>(a, ul, ur, wl, wr, bn, adj_cons(a, dir == 0 ? A_FX : A_FY, o), ulb, urb, wlb, wrb, bnb);
   const GenRange C = dir == 0 ? range_correct_x(a.is, a.ie, a.js, a.je) : range_correct_y(a.is, a.ie, a.js, a.je);
   if (in_range(C, j, i)) {
     addto(ulb, adj_cons(a, dir == 0 ? A_ULX : A_ULY, o));
     addto(urb, adj_cons(a, dir == 0 ? A_URX : A_URY, o));
   }
-  prim_to_cons_adj(wl, bn, a.eos, ulb, wlb, bnb);
-  prim_to_cons_adj(wr, bn, a.eos, urb, wrb, bnb);
+  prim_to_cons_adj(wl, bn, a.fe.r_gamma_1, ulb, wlb, bnb);
+  prim_to_cons_adj(wr, bn, a.fe.r_gamma_1, urb, wrb, bnb);
   adj_put_prim(a, dir == 0 ? A_WLNX : A_WLNY, o - step, wlb);
   adj_put_prim(a, dir == 0 ? A_WRTX : A_WRTY, o, wrb);
   a.a(dir == 0 ? A_BNX : A_BNY, o) = bnb;
@@ -768,7 +799,7 @@ ATHB_HD void adj_plm(const AdjArgs& a, int dir, int j, int i) {
   const double lsum = dir == 0 ? (lwl.by + lwr.by) : (lwl.bz + lwr.bz);
   const double mt = a.s(dir == 0 ? P_M2 : P_M1, o);
   const int bnp = dir == 0 ? P_B1I : P_B2I, bxp = dir == 0 ? P_B1C : P_B2C;
-  const double rdx = dir == 0 ? a.rdx1 : a.rdx2;
+  const double rdx = dir == 0 ? a.fe.r_dx1 : a.fe.r_dx2;
   const double db = (a.s(bnp, o + step) - a.s(bnp, o)) * rdx;
   const Cons1 um = state_cons(a, o - step, dir), u0 = state_cons(a, o, dir), up = state_cons(a, o + step, dir);
   const double bxm = a.s(bxp, o - step), bx0 = a.s(bxp, o), bxq = a.s(bxp, o + step);

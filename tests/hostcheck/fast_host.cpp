@@ -85,6 +85,29 @@ void fast_plm_adj(int n, const double* w, const double* bx, const double* dtodx,
   }
 }
 
+// n faces: w = left and right primitive states, bx the normal field, lam the
+// adjoint of the flux; out: the adjoints of Ul, Ur, Wl, Wr and of the field.
+void fast_roe_adj(int n, const double* w, const double* bx, const double* lam, double gamma, int* took, double* fast,
+                  double* plain) {
+  const Eos eos{gamma, gamma - 1.0, gamma - 2.0};
+  for (int k = 0; k < n; k++) {
+    const Prim1 wl = prim(w + 14 * k), wr = prim(w + 14 * k + 7), l = prim(lam + 7 * k);
+    const Cons1 ul = prim_to_cons(wl, bx[k], eos), ur = prim_to_cons(wr, bx[k], eos);
+    const Cons1 fb{l.d, l.vx, l.vy, l.vz, l.p, l.by, l.bz};
+    for (int form = 0; form < 2; form++) {
+      Cons1 a, b;
+      Prim1 c, d;
+      double t = 0.0;
+      zero(a); zero(b); zero(c); zero(d);
+      if (form) flux_roe_adj(ul, ur, wl, wr, bx[k], eos, fb, a, b, c, d, t);
+      else took[k] = flux_roe_adj_fast(ul, ur, wl, wr, bx[k], eos, 1.0 / eos.gamma_1, fb, a, b, c, d, t);
+      double* o = (form ? plain : fast) + 29 * k;
+      put(a, o); put(b, o + 7); put(c, o + 14); put(d, o + 21);
+      o[28] = t;
+    }
+  }
+}
+
 // n faces: w = left and right primitive states, bx the normal field.
 void fast_flux(int hlle, int n, const double* w, const double* bx, double gamma, int* took, double* fast,
                double* plain) {

@@ -220,3 +220,27 @@ def test_plm_adjoint_agrees(fast, kind):
     assert ok.mean() > 0.95
     err = np.abs(f - g)[ok].max(axis=1) / np.abs(g)[ok].max(axis=1)
     assert np.quantile(err, 0.999) <= 1000 * 2.0 ** -52 / 1e-3
+
+
+@pytest.mark.parametrize("kind", ["smooth", "jumps", "zeros"])
+def test_roe_adjoint_agrees(fast, kind):
+    """The adjoint of the Roe flux, to rounding as above: ~1000 operations on
+    terms up to 1/alpha (1e-3 or more for all but 1 face in 1000) times the
+    largest output; subsonic faces of both signs, supersonic ones (the shift).
+    It takes every face the fast flux takes (the others are the HLLE ones)."""
+    n = 20000
+    rng = np.random.default_rng(21)
+    w0, b0 = _states(rng, 2 * n, kind)
+    w, bx = np.ascontiguousarray(w0.reshape(n, 2, 7)), np.ascontiguousarray(b0[:n])
+    w[rng.random(n) < 0.3, :, 1] += rng.choice([-8.0, 8.0])
+    lam = rng.normal(size=(n, 7))
+    took = np.zeros(n, dtype=np.int32)
+    f, g = np.empty((n, 29)), np.empty((n, 29))
+    fast.fast_roe_adj(n, _p(w), _p(bx), _p(lam), C.c_double(5.0 / 3.0), _p(took), _p(f), _p(g))
+    ok = took.astype(bool)
+    flux = np.zeros(n, dtype=np.int32)
+    F, G = np.empty((n, 7)), np.empty((n, 7))
+    fast.fast_flux(0, n, _p(w), _p(bx), C.c_double(5.0 / 3.0), _p(flux), _p(F), _p(G))
+    assert ok.sum() > n // 4 and np.all(ok[flux.astype(bool)])
+    err = np.abs(f - g)[ok].max(axis=1) / np.abs(g)[ok].max(axis=1)
+    assert np.quantile(err, 0.999) <= 1000 * 2.0 ** -52 / 1e-3
