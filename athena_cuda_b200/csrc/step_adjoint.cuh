@@ -74,6 +74,16 @@ struct AdjArgs {
   ATHB_MEM double& li(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return lin[p * ps + off]; }
   ATHB_MEM double& a(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return adj[p * ps + off]; }
   ATHB_MEM double av(int p, long long off) const { ATHB_CHECK_OFF(off, ps); return ro(adj + p * ps + off); }
+  // av (lo) at off where in holds, else 0, without a branch before the load: a
+  // gather's loads then all start at once.  safe: a place of the array.
+  ATHB_MEM double av_if(bool in, int p, long long off, long long safe) const {
+    const double x = av(p, in ? off : safe);
+    return in ? x : 0.0;
+  }
+  ATHB_MEM double lo_if(bool in, int p, long long off, long long safe) const {
+    const double x = lo(p, in ? off : safe);
+    return in ? x : 0.0;
+  }
 
  private:
   // What a stage reads through s, t, lo and av it never writes (each stage's
@@ -98,6 +108,10 @@ ATHB_HD void lin_add(const AdjArgs& a, long long o, const int (&p)[N], const dou
 #pragma unroll
   for (int k = 0; k < N; k++) a.li(p[k], o) = x[k] + v[k];
 }
+
+// x / dx1, x / dx2 with the launch's reciprocals (the same bits)
+ATHB_HD double per_dx1(const AdjArgs& a, double x) { return any_quot(x, a.dx1, a.fe.r_dx1); }
+ATHB_HD double per_dx2(const AdjArgs& a, double x) { return any_quot(x, a.dx2, a.fe.r_dx2); }
 
 ATHB_HD bool in_range(const GenRange& r, int j, int i) { return j >= r.j0 && j <= r.j1 && i >= r.i0 && i <= r.i1; }
 
@@ -176,10 +190,10 @@ ATHB_HD void corner_terms(const AdjArgs& a, int full, const GenRange& K, double 
   for (int r = 0; r < 2; r++)
 #pragma unroll
     for (int c = 0; c < 2; c++) {
-      if (!in_range(K, j + r, i + c)) continue;
-      const double e = w1 * (b1[r + 1][c] - b1[r][c]) + w2 * (b2[r][c] - b2[r][c + 1]);
+      const bool in = in_range(K, j + r, i + c);
+      const double e = in ? w1 * (b1[r + 1][c] - b1[r][c]) + w2 * (b2[r][c] - b2[r][c + 1]) : 0.0;
       double k[8];
-      corner_k(a, full, j + r, i + c, k);
+      corner_k(a, full, in ? j + r : K.j0, in ? i + c : K.i0, k);
       if (r == 0 && c == 0) { t[1] = k[1] * e; t[3] = k[3] * e; t[7] = k[7] * e; }
       else if (r == 0) { t[2] = k[2] * e; t[6] = k[6] * e; }
       else if (c == 0) { t[0] = k[0] * e; t[5] = k[5] * e; }
@@ -199,21 +213,17 @@ ATHB_HD void adj_update(const AdjArgs& a, int j, int i) {
   const long long o = a.o(j, i), P = a.pitch;
   // b1 at x face (jj,ii), ii in [is, ie+1], jj in [js, je]
   auto lb1 = [&](int jj, int ii) {
-    if (!(jj >= a.js && jj <= a.je && ii >= a.is && ii <= a.ie + 1)) return 0.0;
+    const bool in = jj >= a.js && jj <= a.je && ii >= a.is && ii <= a.ie + 1;
     const long long q = a.o(jj, ii);
-    double lb = a.lo(P_B1I, q);
-    if (ii <= a.ie) lb += 0.5 * a.lo(P_B1C, q);
-    if (ii - 1 >= a.is) lb += 0.5 * a.lo(P_B1C, q - 1);
-    return lb;
+    return (a.lo_if(in, P_B1I, q, o) + 0.5 * a.lo_if(in && ii <= a.ie, P_B1C, q, o)) +
+           0.5 * a.lo_if(in && ii - 1 >= a.is, P_B1C, q - 1, o);
   };
   // b2 at y face (jj,ii), jj in [js, je+1], ii in [is, ie]
   auto lb2 = [&](int jj, int ii) {
-    if (!(jj >= a.js && jj <= a.je + 1 && ii >= a.is && ii <= a.ie)) return 0.0;
+    const bool in = jj >= a.js && jj <= a.je + 1 && ii >= a.is && ii <= a.ie;
     const long long q = a.o(jj, ii);
-    double lb = a.lo(P_B2I, q);
-    if (jj <= a.je) lb += 0.5 * a.lo(P_B2C, q);
-    if (jj - 1 >= a.js) lb += 0.5 * a.lo(P_B2C, q - P);
-    return lb;
+    return (a.lo_if(in, P_B2I, q, o) + 0.5 * a.lo_if(in && jj <= a.je, P_B2C, q, o)) +
+           0.5 * a.lo_if(in && jj - 1 >= a.js, P_B2C, q - P, o);
   };
   double v[NSTATE], dtb = 0.0;
 #pragma unroll
@@ -223,11 +233,11 @@ ATHB_HD void adj_update(const AdjArgs& a, int j, int i) {
   if (in_range(corners, j, i)) {
     if (j <= a.je) {
       v[P_B1I] = lb1(j, i);
-      dtb += -v[P_B1I] * (a.t(G_EMF1, o + P) - a.t(G_EMF1, o)) / a.dx2;
+      dtb += per_dx2(a, -v[P_B1I] * (a.t(G_EMF1, o + P) - a.t(G_EMF1, o)));
     }
     if (i <= a.ie) {
       v[P_B2I] = lb2(j, i);
-      dtb += v[P_B2I] * (a.t(G_EMF1, o + 1) - a.t(G_EMF1, o)) / a.dx1;
+      dtb += per_dx1(a, v[P_B2I] * (a.t(G_EMF1, o + 1) - a.t(G_EMF1, o)));
     }
   }
   if (in_range(interior, j, i)) {
@@ -247,7 +257,7 @@ ATHB_HD void adj_update(const AdjArgs& a, int j, int i) {
     g2 += l1 * (a.t(G_FY2 + 3, o + P) - a.t(G_FY2 + 3, o));
     g2 += le * (a.t(G_FY2 + 4, o + P) - a.t(G_FY2 + 4, o));
     g2 += lb3 * (a.t(G_FY2 + 5, o + P) - a.t(G_FY2 + 5, o));
-    dtb += -g1 / a.dx1 - g2 / a.dx2;
+    dtb += per_dx1(a, -g1) - per_dx2(a, g2);
     v[P_D] = ld; v[P_M1] = l1; v[P_M2] = l2; v[P_M3] = l3; v[P_E] = le; v[P_B3C] = lb3;
   }
 #pragma unroll
@@ -258,9 +268,9 @@ ATHB_HD void adj_update(const AdjArgs& a, int j, int i) {
   double t[8];
   corner_terms(a, 1, corners, a.c.dtodx2, a.c.dtodx1, j, i, lb1, lb2, t);
   auto lcell = [&](int p, int jj, int ii) {
-    if (!in_range(interior, jj, ii)) return 0.0;
+    const bool in = in_range(interior, jj, ii);
     const long long q = a.o(jj, ii);
-    return p == P_B3C ? a.lo(P_B3C, q) + a.lo(P_B3I, q) : a.lo(p, q);
+    return p == P_B3C ? a.lo_if(in, P_B3C, q, o) + a.lo_if(in, P_B3I, q, o) : a.lo_if(in, p, q, o);
   };
   // x face (j,i) in the corrector range
   if (in_range(range_correct_x(a.is, a.ie, a.js, a.je), j, i)) {
@@ -313,7 +323,7 @@ ATHB_HD void correct_x_states(const AdjArgs& a, int j, int i, Cons1& ul, Cons1& 
     const long long ow = o - 1;
     const double dbx = a.s(P_B1I, o) - a.s(P_B1I, ow);
     const double B1 = a.s(P_B1C, ow), B2 = a.s(P_B2C, ow), B3 = a.s(P_B3C, ow);
-    const double V3 = a.s(P_M3, ow) / a.s(P_D, ow);
+    const double V3 = ratio(a.s(P_M3, ow), a.s(P_D, ow));
     ul.mx += c.hdtodx1 * B1 * dbx;
     ul.my += c.hdtodx1 * B2 * dbx;
     ul.mz += c.hdtodx1 * B3 * dbx;
@@ -323,7 +333,7 @@ ATHB_HD void correct_x_states(const AdjArgs& a, int j, int i, Cons1& ul, Cons1& 
   {
     const double dbx = a.s(P_B1I, o + 1) - a.s(P_B1I, o);
     const double B1 = a.s(P_B1C, o), B2 = a.s(P_B2C, o), B3 = a.s(P_B3C, o);
-    const double V3 = a.s(P_M3, o) / a.s(P_D, o);
+    const double V3 = ratio(a.s(P_M3, o), a.s(P_D, o));
     ur.mx += c.hdtodx1 * B1 * dbx;
     ur.my += c.hdtodx1 * B2 * dbx;
     ur.mz += c.hdtodx1 * B3 * dbx;
@@ -360,7 +370,7 @@ ATHB_HD void correct_y_states(const AdjArgs& a, int j, int i, Cons1& ul, Cons1& 
     const long long osn = o - P;
     const double dby = a.s(P_B2I, o) - a.s(P_B2I, osn);
     const double B1 = a.s(P_B1C, osn), B2 = a.s(P_B2C, osn), B3 = a.s(P_B3C, osn);
-    const double V3 = a.s(P_M3, osn) / a.s(P_D, osn);
+    const double V3 = ratio(a.s(P_M3, osn), a.s(P_D, osn));
     ul.mz += c.hdtodx2 * B1 * dby;
     ul.mx += c.hdtodx2 * B2 * dby;
     ul.my += c.hdtodx2 * B3 * dby;
@@ -370,7 +380,7 @@ ATHB_HD void correct_y_states(const AdjArgs& a, int j, int i, Cons1& ul, Cons1& 
   {
     const double dby = a.s(P_B2I, o + P) - a.s(P_B2I, o);
     const double B1 = a.s(P_B1C, o), B2 = a.s(P_B2C, o), B3 = a.s(P_B3C, o);
-    const double V3 = a.s(P_M3, o) / a.s(P_D, o);
+    const double V3 = ratio(a.s(P_M3, o), a.s(P_D, o));
     ur.mz += c.hdtodx2 * B1 * dby;
     ur.mx += c.hdtodx2 * B2 * dby;
     ur.my += c.hdtodx2 * B3 * dby;
@@ -401,16 +411,16 @@ ATHB_HD double correct_x_dtb(const AdjArgs& a, int j, int i, const Cons1& lul, c
     const long long ow = o - 1;
     const double dbx = a.s(P_B1I, o) - a.s(P_B1I, ow);
     const double B1 = a.s(P_B1C, ow), B2 = a.s(P_B2C, ow), B3 = a.s(P_B3C, ow);
-    const double V3 = a.s(P_M3, ow) / a.s(P_D, ow);
+    const double V3 = ratio(a.s(P_M3, ow), a.s(P_D, ow));
     g1 += dbx * (B1 * lul.mx + B2 * lul.my + B3 * lul.mz + V3 * lul.bz + B3 * V3 * lul.e);
   }
   {
     const double dbx = a.s(P_B1I, o + 1) - a.s(P_B1I, o);
     const double B1 = a.s(P_B1C, o), B2 = a.s(P_B2C, o), B3 = a.s(P_B3C, o);
-    const double V3 = a.s(P_M3, o) / a.s(P_D, o);
+    const double V3 = ratio(a.s(P_M3, o), a.s(P_D, o));
     g1 += dbx * (B1 * lur.mx + B2 * lur.my + B3 * lur.mz + V3 * lur.bz + B3 * V3 * lur.e);
   }
-  return 0.5 * g1 / a.dx1 + 0.5 * g2 / a.dx2;
+  return per_dx1(a, 0.5 * g1) + per_dx2(a, 0.5 * g2);
 }
 ATHB_HD double correct_y_dtb(const AdjArgs& a, int j, int i, const Cons1& lul, const Cons1& lur) {
   const long long o = a.o(j, i), P = a.pitch;
@@ -431,16 +441,16 @@ ATHB_HD double correct_y_dtb(const AdjArgs& a, int j, int i, const Cons1& lul, c
     const long long osn = o - P;
     const double dby = a.s(P_B2I, o) - a.s(P_B2I, osn);
     const double B1 = a.s(P_B1C, osn), B2 = a.s(P_B2C, osn), B3 = a.s(P_B3C, osn);
-    const double V3 = a.s(P_M3, osn) / a.s(P_D, osn);
+    const double V3 = ratio(a.s(P_M3, osn), a.s(P_D, osn));
     g2 += dby * (B1 * lul.mz + B2 * lul.mx + B3 * lul.my + V3 * lul.by + B3 * V3 * lul.e);
   }
   {
     const double dby = a.s(P_B2I, o + P) - a.s(P_B2I, o);
     const double B1 = a.s(P_B1C, o), B2 = a.s(P_B2C, o), B3 = a.s(P_B3C, o);
-    const double V3 = a.s(P_M3, o) / a.s(P_D, o);
+    const double V3 = ratio(a.s(P_M3, o), a.s(P_D, o));
     g2 += dby * (B1 * lur.mz + B2 * lur.mx + B3 * lur.my + V3 * lur.by + B3 * V3 * lur.e);
   }
-  return 0.5 * g1 / a.dx1 + 0.5 * g2 / a.dx2;
+  return per_dx1(a, 0.5 * g1) + per_dx2(a, 0.5 * g2);
 }
 
 // The adjoint of the face flux: the fast form where it applies, else the
@@ -535,19 +545,20 @@ ATHB_HD void adj_correct_e(const AdjArgs& a, int j, int i) {
   const double b2f_n = a.s(P_B2I, o + P) + c.hdtodx1 * (a.t(G_EMF0, o + P + 1) - a.t(G_EMF0, o + P));
   const double B1c = 0.5 * (b1f_c + b1f_e);
   const double B2c = 0.5 * (b2f_c + b2f_n);
-  const double e = (B1c * M2 - B2c * M1) / d;
+  const double rd = any_recip(d);
+  const double e = any_quot(B1c * M2 - B2c * M1, d, rd);
   const double lam = a.av(A_ECC1, o);
-  const double ld = -lam * e / d, lM1 = -lam * B2c / d, lM2 = lam * B1c / d;
+  const double ld = any_quot(-lam * e, d, rd), lM1 = any_quot(-lam * B2c, d, rd), lM2 = any_quot(lam * B1c, d, rd);
   const int p[3] = {P_D, P_M1, P_M2};
   const double v[3] = {ld, lM1, lM2};
   lin_add(a, o, p, v);
   a.a(A_HALF + 0, o) = ld;
   a.a(A_HALF + 1, o) = lM1;
   a.a(A_HALF + 2, o) = lM2;
-  a.a(A_HALF + 3, o) = lam * M2 / d;
-  a.a(A_HALF + 4, o) = -lam * M1 / d;
-  a.a(A_DTC, o) = 0.5 * (-(ld * dfx0 + lM1 * dfx1 + lM2 * dfx2)) / a.dx1 +
-                  0.5 * (-(ld * dfy0 + lM1 * dfy3 + lM2 * dfy1)) / a.dx2;
+  a.a(A_HALF + 3, o) = any_quot(lam * M2, d, rd);
+  a.a(A_HALF + 4, o) = any_quot(-lam * M1, d, rd);
+  a.a(A_DTC, o) = per_dx1(a, 0.5 * (-(ld * dfx0 + lM1 * dfx1 + lM2 * dfx2))) +
+                  per_dx2(a, 0.5 * (-(ld * dfy0 + lM1 * dfy3 + lM2 * dfy1)));
 }
 
 // Every consumer of the half-step face fields: x faces [is-1, ie+2] x
@@ -558,28 +569,23 @@ ATHB_HD void adj_half_faces(const AdjArgs& a, int j, int i) {
   const long long o = a.o(j, i), P = a.pitch;
   const GenRange E = range_correct_e(a.is, a.ie, a.js, a.je);
   const bool xface = j <= a.je + 1, yface = i <= a.ie + 1;
-  double dt0 = a.a(A_DT, o);
-  if (in_range(range_correct_y(a.is, a.ie, a.js, a.je), j, i)) dt0 += a.av(A_DTY, o);
-  if (in_range(E, j, i)) dt0 += a.av(A_DTC, o);
+  const GenRange CX = range_correct_x(a.is, a.ie, a.js, a.je), CY = range_correct_y(a.is, a.ie, a.js, a.je);
+  const double dt0 = (a.a(A_DT, o) + a.av_if(in_range(CY, j, i), A_DTY, o, o)) + a.av_if(in_range(E, j, i), A_DTC, o, o);
   const double b10 = xface ? a.li(P_B1I, o) : 0.0, b20 = yface ? a.li(P_B2I, o) : 0.0;
   double dtb = 0.0;
   if (xface) {
-    double lb = 0.0;
-    if (in_range(range_correct_x(a.is, a.ie, a.js, a.je), j, i)) lb += a.av(A_B1F, o);
-    if (in_range(E, j, i)) lb += 0.5 * a.av(A_HALF + 3, o);
-    if (in_range(E, j, i - 1)) lb += 0.5 * a.av(A_HALF + 3, o - 1);
+    const double lb = (a.av_if(in_range(CX, j, i), A_B1F, o, o) + 0.5 * a.av_if(in_range(E, j, i), A_HALF + 3, o, o)) +
+                      0.5 * a.av_if(in_range(E, j, i - 1), A_HALF + 3, o - 1, o);
     a.a(A_LB1F, o) = lb;
     a.li(P_B1I, o) = b10 + lb;
-    dtb += -lb * (a.t(G_EMF0, o + P) - a.t(G_EMF0, o)) * 0.5 / a.dx2;
+    dtb += per_dx2(a, -lb * (a.t(G_EMF0, o + P) - a.t(G_EMF0, o)) * 0.5);
   }
   if (yface) {
-    double lb = 0.0;
-    if (in_range(range_correct_y(a.is, a.ie, a.js, a.je), j, i)) lb += a.av(A_B2F, o);
-    if (in_range(E, j, i)) lb += 0.5 * a.av(A_HALF + 4, o);
-    if (in_range(E, j - 1, i)) lb += 0.5 * a.av(A_HALF + 4, o - P);
+    const double lb = (a.av_if(in_range(CY, j, i), A_B2F, o, o) + 0.5 * a.av_if(in_range(E, j, i), A_HALF + 4, o, o)) +
+                      0.5 * a.av_if(in_range(E, j - 1, i), A_HALF + 4, o - P, o);
     a.a(A_LB2F, o) = lb;
     a.li(P_B2I, o) = b20 + lb;
-    dtb += lb * (a.t(G_EMF0, o + 1) - a.t(G_EMF0, o)) * 0.5 / a.dx1;
+    dtb += per_dx1(a, lb * (a.t(G_EMF0, o + 1) - a.t(G_EMF0, o)) * 0.5);
   }
   a.a(A_DT, o) = dt0 + dtb;
 }
@@ -592,9 +598,9 @@ ATHB_HD void adj_flux1(const AdjArgs& a, int j, int i) {
   const StepCoef<double>& c = a.c;
   const GenRange CX = range_correct_x(a.is, a.ie, a.js, a.je), CY = range_correct_y(a.is, a.ie, a.js, a.je);
   const GenRange E = range_correct_e(a.is, a.ie, a.js, a.je), K = range_emf0(a.is, a.ie, a.js, a.je);
-  auto lb1 = [&](int jj, int ii) { return (jj >= a.js - 1 && jj <= a.je + 1 && ii >= a.is - 1 && ii <= a.ie + 2) ? a.av(A_LB1F, a.o(jj, ii)) : 0.0; };
-  auto lb2 = [&](int jj, int ii) { return (jj >= a.js - 1 && jj <= a.je + 2 && ii >= a.is - 1 && ii <= a.ie + 1) ? a.av(A_LB2F, a.o(jj, ii)) : 0.0; };
-  auto half = [&](int q, int jj, int ii) { return in_range(E, jj, ii) ? a.av(A_HALF + q, a.o(jj, ii)) : 0.0; };
+  auto lb1 = [&](int jj, int ii) { return a.av_if(jj >= a.js - 1 && jj <= a.je + 1 && ii >= a.is - 1 && ii <= a.ie + 2, A_LB1F, a.o(jj, ii), o); };
+  auto lb2 = [&](int jj, int ii) { return a.av_if(jj >= a.js - 1 && jj <= a.je + 2 && ii >= a.is - 1 && ii <= a.ie + 1, A_LB2F, a.o(jj, ii), o); };
+  auto half = [&](int q, int jj, int ii) { return a.av_if(in_range(E, jj, ii), A_HALF + q, a.o(jj, ii), o); };
   double t[8];
   corner_terms(a, 0, K, c.hdtodx2, c.hdtodx1, j, i, lb1, lb2, t);
   // x face (j,i) of the predictor
@@ -602,10 +608,11 @@ ATHB_HD void adj_flux1(const AdjArgs& a, int j, int i) {
     double f[7] = {0, 0, 0, 0, 0, 0, 0};
     // correct_y transverse terms: (u.d, u.mx, u.my, u.mz, u.e, u.by) <- fx (0, 2, 3, 1, 4, 6)
     auto addy = [&](int base, int jj, int ii, double w) {
-      if (!in_range(CY, jj, ii)) return;
+      const bool in = in_range(CY, jj, ii);
       const long long q = a.o(jj, ii);
-      f[0] += w * a.av(base + 0, q); f[2] += w * a.av(base + 1, q); f[3] += w * a.av(base + 2, q);
-      f[1] += w * a.av(base + 3, q); f[4] += w * a.av(base + 4, q); f[6] += w * a.av(base + 5, q);
+      f[0] += w * a.av_if(in, base + 0, q, o); f[2] += w * a.av_if(in, base + 1, q, o);
+      f[3] += w * a.av_if(in, base + 2, q, o); f[1] += w * a.av_if(in, base + 3, q, o);
+      f[4] += w * a.av_if(in, base + 4, q, o); f[6] += w * a.av_if(in, base + 5, q, o);
     };
     addy(A_ULY, j + 1, i - 1, -c.hdtodx1);
     addy(A_ULY, j + 1, i, c.hdtodx1);
@@ -624,10 +631,11 @@ ATHB_HD void adj_flux1(const AdjArgs& a, int j, int i) {
     double f[7] = {0, 0, 0, 0, 0, 0, 0};
     // correct_x transverse terms: (u.d, u.mx, u.my, u.mz, u.e, u.bz) <- fy (0, 3, 1, 2, 4, 5)
     auto addx = [&](int base, int jj, int ii, double w) {
-      if (!in_range(CX, jj, ii)) return;
+      const bool in = in_range(CX, jj, ii);
       const long long q = a.o(jj, ii);
-      f[0] += w * a.av(base + 0, q); f[3] += w * a.av(base + 1, q); f[1] += w * a.av(base + 2, q);
-      f[2] += w * a.av(base + 3, q); f[4] += w * a.av(base + 4, q); f[5] += w * a.av(base + 6, q);
+      f[0] += w * a.av_if(in, base + 0, q, o); f[3] += w * a.av_if(in, base + 1, q, o);
+      f[1] += w * a.av_if(in, base + 2, q, o); f[2] += w * a.av_if(in, base + 3, q, o);
+      f[4] += w * a.av_if(in, base + 4, q, o); f[5] += w * a.av_if(in, base + 6, q, o);
     };
     addx(A_ULX, j - 1, i + 1, -c.hdtodx2);
     addx(A_ULX, j, i + 1, c.hdtodx2);
@@ -646,9 +654,10 @@ ATHB_HD void adj_flux1(const AdjArgs& a, int j, int i) {
     const double v = t[7] + t[6] + t[5] + t[4];
     if (v != 0.0) {
       const double d = a.s(P_D, o), M1 = a.s(P_M1, o), M2 = a.s(P_M2, o), B1 = a.s(P_B1C, o), B2 = a.s(P_B2C, o);
-      const double e = (B1 * M2 - B2 * M1) / d;
+      const double rd = any_recip(d), e = any_quot(B1 * M2 - B2 * M1, d, rd);
       const int p[5] = {P_B1C, P_M2, P_B2C, P_M1, P_D};
-      const double w[5] = {v * M2 / d, v * B1 / d, -(v * M1 / d), -(v * B2 / d), -(v * e / d)};
+      const double w[5] = {any_quot(v * M2, d, rd), any_quot(v * B1, d, rd), -any_quot(v * M1, d, rd),
+                           -any_quot(v * B2, d, rd), -any_quot(v * e, d, rd)};
       lin_add(a, o, p, w);
     }
   }
@@ -661,76 +670,53 @@ ATHB_HD void adj_sources(const AdjArgs& a, int j, int i) {
   const long long o = a.o(j, i), P = a.pitch;
   const double h1 = a.c.hdtodx1, h2 = a.c.hdtodx2;
   const GenRange CX = range_correct_x(a.is, a.ie, a.js, a.je), CY = range_correct_y(a.is, a.ie, a.js, a.je);
+  // v3 of the three cells whose source terms reach the faces of (j,i)
+  const double rdc = any_recip(a.s(P_D, o)), V3c = any_quot(a.s(P_M3, o), a.s(P_D, o), rdc);
+  const double V3w = ratio(a.s(P_M3, o - 1), a.s(P_D, o - 1)), V3s = ratio(a.s(P_M3, o - P), a.s(P_D, o - P));
   // λ of dbx of face (jj,ii)'s left (ul) or right (ur) state, with its cell
-  auto dbx_l = [&](int jj, int ii) {   // ul of x face (jj,ii): cell (jj, ii-1)
-    if (!in_range(CX, jj, ii)) return 0.0;
-    const long long q = a.o(jj, ii), w = q - 1;
-    const double B1 = a.s(P_B1C, w), B2 = a.s(P_B2C, w), B3 = a.s(P_B3C, w), V3 = a.s(P_M3, w) / a.s(P_D, w);
-    return h1 * (B1 * a.av(A_ULX + 1, q) + B2 * a.av(A_ULX + 2, q) + B3 * a.av(A_ULX + 3, q) +
-                 V3 * a.av(A_ULX + 6, q) + B3 * V3 * a.av(A_ULX + 4, q));
-  };
-  auto dbx_r = [&](int jj, int ii) {   // ur of x face (jj,ii): cell (jj, ii)
-    if (!in_range(CX, jj, ii)) return 0.0;
+  auto dbx = [&](int base, int jj, int ii, long long cell, double V3) {
+    const bool in = in_range(CX, jj, ii);
     const long long q = a.o(jj, ii);
-    const double B1 = a.s(P_B1C, q), B2 = a.s(P_B2C, q), B3 = a.s(P_B3C, q), V3 = a.s(P_M3, q) / a.s(P_D, q);
-    return h1 * (B1 * a.av(A_URX + 1, q) + B2 * a.av(A_URX + 2, q) + B3 * a.av(A_URX + 3, q) +
-                 V3 * a.av(A_URX + 6, q) + B3 * V3 * a.av(A_URX + 4, q));
+    const double B1 = a.s(P_B1C, cell), B2 = a.s(P_B2C, cell), B3 = a.s(P_B3C, cell);
+    return h1 * (B1 * a.av_if(in, base + 1, q, o) + B2 * a.av_if(in, base + 2, q, o) + B3 * a.av_if(in, base + 3, q, o) +
+                 V3 * a.av_if(in, base + 6, q, o) + B3 * V3 * a.av_if(in, base + 4, q, o));
   };
-  auto dby_l = [&](int jj, int ii) {   // ul of y face (jj,ii): cell (jj-1, ii)
-    if (!in_range(CY, jj, ii)) return 0.0;
-    const long long q = a.o(jj, ii), s = q - P;
-    const double B1 = a.s(P_B1C, s), B2 = a.s(P_B2C, s), B3 = a.s(P_B3C, s), V3 = a.s(P_M3, s) / a.s(P_D, s);
-    return h2 * (B1 * a.av(A_ULY + 3, q) + B2 * a.av(A_ULY + 1, q) + B3 * a.av(A_ULY + 2, q) +
-                 V3 * a.av(A_ULY + 5, q) + B3 * V3 * a.av(A_ULY + 4, q));
-  };
-  auto dby_r = [&](int jj, int ii) {   // ur of y face (jj,ii): cell (jj, ii)
-    if (!in_range(CY, jj, ii)) return 0.0;
+  auto dby = [&](int base, int jj, int ii, long long cell, double V3) {
+    const bool in = in_range(CY, jj, ii);
     const long long q = a.o(jj, ii);
-    const double B1 = a.s(P_B1C, q), B2 = a.s(P_B2C, q), B3 = a.s(P_B3C, q), V3 = a.s(P_M3, q) / a.s(P_D, q);
-    return h2 * (B1 * a.av(A_URY + 3, q) + B2 * a.av(A_URY + 1, q) + B3 * a.av(A_URY + 2, q) +
-                 V3 * a.av(A_URY + 5, q) + B3 * V3 * a.av(A_URY + 4, q));
+    const double B1 = a.s(P_B1C, cell), B2 = a.s(P_B2C, cell), B3 = a.s(P_B3C, cell);
+    return h2 * (B1 * a.av_if(in, base + 3, q, o) + B2 * a.av_if(in, base + 1, q, o) + B3 * a.av_if(in, base + 2, q, o) +
+                 V3 * a.av_if(in, base + 5, q, o) + B3 * V3 * a.av_if(in, base + 4, q, o));
   };
   // cell (j,i)
   if (in_range(range_correct_e(a.is, a.ie, a.js, a.je), j, i)) {
     const double B3 = a.s(P_B3C, o);
-    const double d = a.s(P_D, o), V3 = a.s(P_M3, o) / d;
+    const double d = a.s(P_D, o), V3 = V3c;
     double lB1 = 0, lB2 = 0, lB3 = 0, lV3 = 0;
-    if (in_range(CX, j, i + 1)) {  // ul of x face (j,i+1)
-      const long long q = o + 1;
-      const double dbx = a.s(P_B1I, q) - a.s(P_B1I, o);
-      lB1 += h1 * dbx * a.av(A_ULX + 1, q); lB2 += h1 * dbx * a.av(A_ULX + 2, q);
-      lB3 += h1 * dbx * (a.av(A_ULX + 3, q) + V3 * a.av(A_ULX + 4, q));
-      lV3 += h1 * dbx * (a.av(A_ULX + 6, q) + B3 * a.av(A_ULX + 4, q));
-    }
-    if (in_range(CX, j, i)) {      // ur of x face (j,i)
-      const double dbx = a.s(P_B1I, o + 1) - a.s(P_B1I, o);
-      lB1 += h1 * dbx * a.av(A_URX + 1, o); lB2 += h1 * dbx * a.av(A_URX + 2, o);
-      lB3 += h1 * dbx * (a.av(A_URX + 3, o) + V3 * a.av(A_URX + 4, o));
-      lV3 += h1 * dbx * (a.av(A_URX + 6, o) + B3 * a.av(A_URX + 4, o));
-    }
-    if (in_range(CY, j + 1, i)) {  // ul of y face (j+1,i): mz<-B1, mx<-B2, my<-B3, by<-V3
-      const long long q = o + P;
-      const double dby = a.s(P_B2I, q) - a.s(P_B2I, o);
-      lB1 += h2 * dby * a.av(A_ULY + 3, q); lB2 += h2 * dby * a.av(A_ULY + 1, q);
-      lB3 += h2 * dby * (a.av(A_ULY + 2, q) + V3 * a.av(A_ULY + 4, q));
-      lV3 += h2 * dby * (a.av(A_ULY + 5, q) + B3 * a.av(A_ULY + 4, q));
-    }
-    if (in_range(CY, j, i)) {      // ur of y face (j,i)
-      const double dby = a.s(P_B2I, o + P) - a.s(P_B2I, o);
-      lB1 += h2 * dby * a.av(A_URY + 3, o); lB2 += h2 * dby * a.av(A_URY + 1, o);
-      lB3 += h2 * dby * (a.av(A_URY + 2, o) + V3 * a.av(A_URY + 4, o));
-      lV3 += h2 * dby * (a.av(A_URY + 5, o) + B3 * a.av(A_URY + 4, o));
-    }
+    auto add = [&](bool in, double w, int base, long long q, int m1, int m2, int m3, int mv) {
+      const double l4 = a.av_if(in, base + 4, q, o);
+      lB1 += w * a.av_if(in, base + m1, q, o);
+      lB2 += w * a.av_if(in, base + m2, q, o);
+      lB3 += w * (a.av_if(in, base + m3, q, o) + V3 * l4);
+      lV3 += w * (a.av_if(in, base + mv, q, o) + B3 * l4);
+    };
+    const double dx = a.s(P_B1I, o + 1) - a.s(P_B1I, o), dy = a.s(P_B2I, o + P) - a.s(P_B2I, o);
+    add(in_range(CX, j, i + 1), h1 * dx, A_ULX, o + 1, 1, 2, 3, 6);   // ul of x face (j,i+1)
+    add(in_range(CX, j, i), h1 * dx, A_URX, o, 1, 2, 3, 6);           // ur of x face (j,i)
+    add(in_range(CY, j + 1, i), h2 * dy, A_ULY, o + P, 3, 1, 2, 5);   // ul of y face (j+1,i): mz<-B1, mx<-B2, my<-B3, by<-V3
+    add(in_range(CY, j, i), h2 * dy, A_URY, o, 3, 1, 2, 5);           // ur of y face (j,i)
     const int p[5] = {P_B1C, P_B2C, P_B3C, P_M3, P_D};
-    const double v[5] = {lB1, lB2, lB3, lV3 / d, -(lV3 * V3 / d)};
+    const double v[5] = {lB1, lB2, lB3, any_quot(lV3, d, rdc), -any_quot(lV3 * V3, d, rdc)};
     lin_add(a, o, p, v);
   }
   // x face (j,i): B1i through dbx of ul/ur of x faces i, i+1, i-1
   if (j <= a.je + 1 && j >= a.js - 1 && i >= a.is - 1 && i <= a.ie + 2)
-    a.li(P_B1I, o) += dbx_l(j, i) - dbx_l(j, i + 1) - dbx_r(j, i) + dbx_r(j, i - 1);
+    a.li(P_B1I, o) += dbx(A_ULX, j, i, o - 1, V3w) - dbx(A_ULX, j, i + 1, o, V3c) - dbx(A_URX, j, i, o, V3c) +
+                      dbx(A_URX, j, i - 1, o - 1, V3w);
   // y face (j,i)
   if (i <= a.ie + 1 && i >= a.is - 1 && j >= a.js - 1 && j <= a.je + 2)
-    a.li(P_B2I, o) += dby_l(j, i) - dby_l(j + 1, i) - dby_r(j, i) + dby_r(j - 1, i);
+    a.li(P_B2I, o) += dby(A_ULY, j, i, o - P, V3s) - dby(A_ULY, j + 1, i, o, V3c) - dby(A_URY, j, i, o, V3c) +
+                      dby(A_URY, j - 1, i, o - P, V3s);
 }
 
 // Both, items over [is-2, ie+2] x [js-2, je+2]: they read the same corrector
@@ -851,29 +837,29 @@ ATHB_HD void adj_plm(const AdjArgs& a, int dir, int j, int i) {
 // of cells c-1, c, c+1, back through cons -> prim, and the adjoint of the
 // normal face field of face (j,i) (Riemann states, source terms), returned.
 // Cells of the PLM range widened by one along the sweep.
-ATHB_HD double adj_prim_gather(const AdjArgs& a, int dir, int j, int i, Cons1& ub, double& bxb) {
+ATHB_HD double adj_prim_gather(const AdjArgs& a, int dir, int j, int i, double di, Cons1& ub, double& bxb) {
   const long long o = a.o(j, i);
   const long long step = dir == 0 ? 1 : a.pitch;
   const GenRange L = range_plm(a.is, a.ie, a.js, a.je);
   const int jm = dir == 0 ? j : j - 1, im = dir == 0 ? i - 1 : i;   // previous cell along the sweep
   const int jp = dir == 0 ? j : j + 1, ip = dir == 0 ? i + 1 : i;   // next cell
-  Prim1 lw;
-  zero(lw);
-  if (in_range(L, j, i)) addto(lw, adj_prim(a, dir == 0 ? A_WX0 : A_WY0, o));
-  if (in_range(L, jm, im)) addto(lw, adj_prim(a, dir == 0 ? A_WXP : A_WYP, o - step));
-  if (in_range(L, jp, ip)) addto(lw, adj_prim(a, dir == 0 ? A_WXM : A_WYM, o + step));
-  cons_to_prim_adj(state_cons(a, o, dir), a.s(dir == 0 ? P_B1C : P_B2C, o), a.eos, lw, ub, bxb);
+  const bool in0 = in_range(L, j, i), inm = in_range(L, jm, im), inp = in_range(L, jp, ip);
+  auto sum = [&](int k) {
+    return (a.av_if(in0, (dir == 0 ? A_WX0 : A_WY0) + k, o, o) + a.av_if(inm, (dir == 0 ? A_WXP : A_WYP) + k, o - step, o)) +
+           a.av_if(inp, (dir == 0 ? A_WXM : A_WYM) + k, o + step, o);
+  };
+  const Prim1 lw{sum(0), sum(1), sum(2), sum(3), sum(4), sum(5), sum(6)};
+  cons_to_prim_adj(state_cons(a, o, dir), a.s(dir == 0 ? P_B1C : P_B2C, o), a.eos, di, lw, ub, bxb);
   // normal face field at face (j,i)
   const GenRange F = dir == 0 ? range_riemann_x(a.is, a.ie, a.js, a.je) : range_riemann_y(a.is, a.ie, a.js, a.je);
   const int mtp = dir == 0 ? P_M2 : P_M1;
-  const double dxs = dir == 0 ? a.dx1 : a.dx2;
-  double lb = 0.0;
-  if (in_range(F, j, i)) lb += a.av(dir == 0 ? A_BNX : A_BNY, o);
+  const int src = dir == 0 ? A_SRCX : A_SRCY;
+  const double bn = a.av_if(in_range(F, j, i), dir == 0 ? A_BNX : A_BNY, o, o);
   // src(c) = (Mt/d)(c) (B(c+1) - B(c)) / dx: face (j,i) is B(c) of cell (j,i) and B(c+1) of the previous cell
-  if (in_range(L, j, i)) lb -= a.av(dir == 0 ? A_SRCX : A_SRCY, o) * (a.s(mtp, o) / a.s(P_D, o)) / dxs;
-  if (in_range(L, jm, im))
-    lb += a.av(dir == 0 ? A_SRCX : A_SRCY, o - step) * (a.s(mtp, o - step) / a.s(P_D, o - step)) / dxs;
-  return lb;
+  const long long om = inm ? o - step : o;
+  const double s0 = a.av_if(in0, src, o, o) * any_quot(a.s(mtp, o), a.s(P_D, o), di);
+  const double sm = a.av_if(inm, src, om, o) * ratio(a.s(mtp, om), a.s(P_D, om));
+  return dir == 0 ? (bn - per_dx1(a, s0)) + per_dx1(a, sm) : (bn - per_dx2(a, s0)) + per_dx2(a, sm);
 }
 
 // Both sweeps of cell (j,i) onto lin, one read and one write of each plane;
@@ -883,6 +869,7 @@ ATHB_HD void adj_prim(const AdjArgs& a, int j, int i) {
   const bool gx = j >= a.js - 2 && j <= a.je + 2, gy = i >= a.is - 2 && i <= a.ie + 2;
   if (!gx && !gy) return;
   const bool plm = gx && gy;   // range_plm
+  const double di = any_recip(a.s(P_D, o));
   const int p[10] = {P_D, P_E, P_M1, P_M2, P_M3, P_B1C, P_B2C, P_B3C, P_B1I, P_B2I};
   double v[10];
 #pragma unroll
@@ -895,7 +882,7 @@ ATHB_HD void adj_prim(const AdjArgs& a, int j, int i) {
     Cons1 ub;
     zero(ub);
     double bxb = 0.0;
-    v[8] += adj_prim_gather(a, 0, j, i, ub, bxb);
+    v[8] += adj_prim_gather(a, 0, j, i, di, ub, bxb);
     v[0] += ub.d; v[1] += ub.e; v[2] += ub.mx; v[3] += ub.my; v[4] += ub.mz;
     v[6] += ub.by; v[7] += ub.bz; v[5] += bxb;
   }
@@ -903,7 +890,7 @@ ATHB_HD void adj_prim(const AdjArgs& a, int j, int i) {
     Cons1 ub;
     zero(ub);
     double bxb = 0.0;
-    v[9] += adj_prim_gather(a, 1, j, i, ub, bxb);
+    v[9] += adj_prim_gather(a, 1, j, i, di, ub, bxb);
     v[0] += ub.d; v[1] += ub.e; v[3] += ub.mx; v[4] += ub.my; v[2] += ub.mz;
     v[7] += ub.by; v[5] += ub.bz; v[6] += bxb;
   }
