@@ -122,9 +122,9 @@ template <int STAGE, int FLUX> struct AdjFn {
   }
 };
 
-// One pass of the ghost fold over bands of places, all planes in one launch:
-// item (k, m) is plane k / n1 and place (k % n1, m) of the bands.  A band pair
-// is the first nlo places from lo and the rest up to hi.
+// The ghost fold over bands of places, all planes in one launch: item (k, m)
+// is plane k / rows.n at place (k % rows.n, m) of the bands.  A band pair is
+// the first nlo places from lo and the rest up to hi.
 struct Bands {
   int n, nlo, lo, hi;
   ATHB_MEM int at(int k) const { return k < nlo ? lo + k : hi + 1 - n + k; }
@@ -134,29 +134,32 @@ struct FoldFn {
   long long ps;
   int pitch;
   GhostGeom g;
-  int pass;      // 2: x2 rows, 1: x1 columns, 0: clear the frame
-  Bands rows;    // rows visited (pass 0: unused)
-  Bands cols;
+  Bands rows, cols;
   ATHB_MEM void operator()(int k, int m) const {
-    if (pass == 0) {   // m runs over the frame: whole rows below and above, then the columns beside the rows between
-      const int nrows = g.js + g.sy - g.je - 1, ncols = g.is + g.sx - g.ie - 1;
-      const int u = m - nrows * g.sx;
-      int j, i;
-      if (u < 0) {
-        j = m / g.sx;
-        i = m % g.sx;
-        if (j >= g.js) j += g.je + 1 - g.js;
-      } else {
-        j = g.js + u / ncols;
-        i = u % ncols;
-        if (i >= g.is) i += g.ie + 1 - g.is;
-      }
-      clear_frame(l, ps, pitch, g, k, j, i);
-      return;
+    fold_ghost(l, ps, pitch, g, k / rows.n, rows.at(k % rows.n), cols.at(m));
+  }
+};
+// The frame of plane k cleared; m runs over whole rows below and above, then
+// the columns beside the rows between.
+struct ClearFrameFn {
+  double* l;
+  long long ps;
+  int pitch;
+  GhostGeom g;
+  ATHB_MEM void operator()(int k, int m) const {
+    const int nrows = g.js + g.sy - g.je - 1, ncols = g.is + g.sx - g.ie - 1;
+    const int u = m - nrows * g.sx;
+    int j, i;
+    if (u < 0) {
+      j = m / g.sx;
+      i = m % g.sx;
+      if (j >= g.js) j += g.je + 1 - g.js;
+    } else {
+      j = g.js + u / ncols;
+      i = u % ncols;
+      if (i >= g.is) i += g.ie + 1 - g.is;
     }
-    const int p = k / rows.n, j = rows.at(k % rows.n), i = cols.at(m);
-    if (pass == 2) fold_x2(l, ps, pitch, g, p, j, i);
-    else fold_x1(l, ps, pitch, g, p, j, i);
+    clear_frame(l, ps, pitch, g, k, j, i);
   }
 };
 
@@ -610,12 +613,12 @@ template <class Exec> struct AdjointDriver {
     return a;
   }
 
-  // The ghost fill of a state, reversed on its adjoint l: the ghost rows'
-  // adjoints added onto the rows they copy (x2), then the ghost columns'
-  // onto the columns they copy (x1), then the frame cleared.  Only rows and
+  // The ghost fill of a state, reversed on its adjoint l.  Only rows and
   // columns within kBand of an edge are copied by a ghost (periodic wraps
-  // reach 4 cells in, reflection 4, outflow 1), so the passes visit those
-  // bands alone; every target cell adds the same terms in the same order.
+  // reach 4 cells in, reflection 4, outflow 1), so those bands alone are
+  // visited: the rows next to the edges, then the columns of the rows between.
+  // The frame keeps what it held: no reader of l looks there (adj_update reads
+  // the places a step writes), and clear_ghosts empties it at the end.
   void fold_ghosts(double* l) {
     const GhostGeom gg = ghost_geom();
     constexpr int kBand = kNghostA + 2;
@@ -626,12 +629,16 @@ template <class Exec> struct AdjointDriver {
       return 2 * kBand >= n ? Bands{n, n, lo, hi} : Bands{2 * kBand, kBand, lo, hi};
     };
     const Bands rows = bands(js, je + 1), cols = bands(is, ie + 1);
-    const Bands all_rows{je + 2 - js, je + 2 - js, js, je + 1}, all_cols{G.sx, G.sx, 0, G.sx - 1};
-    x.items(GenRange{0, all_cols.n - 1, 0, NSTATE * rows.n - 1}, FoldFn{l, G.ps, G.pitch, gg, 2, rows, all_cols});
-    x.items(GenRange{0, cols.n - 1, 0, NSTATE * all_rows.n - 1}, FoldFn{l, G.ps, G.pitch, gg, 1, all_rows, cols});
-    // the frame (B2i's row je+1 and B1i's column ie+1 are kept by the functor)
-    const int frame = (js + G.sy - je - 1) * G.sx + (is + G.sx - ie - 1) * (je + 1 - js);
-    x.items(GenRange{0, frame - 1, 0, NSTATE - 1}, FoldFn{l, G.ps, G.pitch, gg, 0, rows, cols});
+    const Bands all_cols{ie + 2 - is, ie + 2 - is, is, ie + 1};
+    const int mid = je + 2 - js - rows.n;
+    const Bands mid_rows{mid, mid, js + kBand, js + kBand + mid - 1};
+    run_items2(x, 0, GenRange{0, all_cols.n - 1, 0, NSTATE * rows.n - 1}, FoldFn{l, G.ps, G.pitch, gg, rows, all_cols},
+               GenRange{0, cols.n - 1, 0, NSTATE * mid - 1}, FoldFn{l, G.ps, G.pitch, gg, mid_rows, cols});
+  }
+  // the frame (B2i's row je+1 and B1i's column ie+1 are kept by the functor)
+  void clear_ghosts(double* l) {
+    const int frame = (G.js + G.sy - G.je - 1) * G.sx + (G.is + G.sx - G.ie - 1) * (G.je + 1 - G.js);
+    x.items(GenRange{0, frame - 1, 0, NSTATE - 1}, ClearFrameFn{l, G.ps, G.pitch, ghost_geom()});
   }
 
   // Reverse step n: S^n in S[cur].  lam[lc] holds the adjoint of S^{n+1}
@@ -655,8 +662,9 @@ template <class Exec> struct AdjointDriver {
     // run side by side (a small grid's stage leaves most SMs idle), and a
     // gather too small for a launch is formed by its reader.  With the dt rule
     // in the sum's launch and nothing cleared beforehand a step of the gradient
-    // makes 21 launches instead of 40: 266 -> 189 us at 64 x 48, 504 -> 440 us
-    // at 256 x 256, 176 us at 16 x 16, where the launches' latency is all
+    // makes 19 launches where it made 40: 21 of them took 266 -> 189 us at
+    // 64 x 48 and 504 -> 440 us at 256 x 256 before the stages themselves
+    // became faster
     x.items(full(), AdjFn<R_UPD, FLUX>{a});
     run_items3(x, 0, range_correct_x(is, ie, js, je), AdjFn<R_CORX, FLUX>{a}, range_correct_y(is, ie, js, je),
                AdjFn<R_CORY, FLUX>{a}, range_correct_e(is, ie, js, je), AdjFn<R_CORE, FLUX>{a});
@@ -667,7 +675,7 @@ template <class Exec> struct AdjointDriver {
     run_items2(x, 0, range_plm(is, ie, js, je), AdjFn<R_PLMX, FLUX>{a}, range_plm(is, ie, js, je),
                AdjFn<R_PLMY, FLUX>{a});
     x.items(GenRange{is - 3, ie + 3, js - 3, je + 3}, AdjFn<R_PRIM, FLUX>{a});
-    // the ghost fill of S^n, reversed: x2 rows, then x1 columns, then clear
+    // the ghost fill of S^n, reversed
     fold_ghosts(lin);
     // dt^n, then dt_rule^n = CourNo / m(S^n), whose cell and rate the first sweep kept, into lin
     run_sum(x, 0, adj + (long long)A_DT * G.ps, GenRange{is - 3, ie + 3, js - 3, je + 3}, G.pitch, &sc->dtsum,
@@ -798,6 +806,7 @@ template <class Exec> struct AdjointDriver {
     } else if (M > 0) {
       reverse<FLUX>(0, M, 0, fr, M, lc, hrec, spine);
     }
+    clear_ghosts(lam[lc]);
     return x.ok() ? 0 : -1;
   }
 };

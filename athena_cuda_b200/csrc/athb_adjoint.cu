@@ -113,22 +113,29 @@ __device__ __forceinline__ bool last_block(unsigned* ticket) {
   return last;
 }
 
-// maximum, the lowest index among equals, to element 0
-__device__ __forceinline__ void fold_max(double m, long long arg, double* sm, long long* sa) {
+// maximum, the lowest index among equals, to thread 0: across warps through
+// shared memory, the last warp by shuffles (the same pairs, five barriers fewer)
+__device__ __forceinline__ void keep_max(double& m, long long& arg, double m2, long long a2) {
+  if (m2 > m || (m2 == m && a2 < arg)) { m = m2; arg = a2; }
+}
+__device__ __forceinline__ void fold_max(double& m, long long& arg, double* sm, long long* sa) {
   sm[threadIdx.x] = m;
   sa[threadIdx.x] = arg;
   __syncthreads();
-  for (int s = kRedThreads / 2; s > 0; s >>= 1) {
+  for (int s = kRedThreads / 2; s >= 32; s >>= 1) {
     if (threadIdx.x < s) {
-      const double m2 = sm[threadIdx.x + s];
-      const long long a2 = sa[threadIdx.x + s];
-      if (m2 > sm[threadIdx.x] || (m2 == sm[threadIdx.x] && a2 < sa[threadIdx.x])) {
-        sm[threadIdx.x] = m2;
-        sa[threadIdx.x] = a2;
-      }
+      keep_max(m, arg, sm[threadIdx.x + s], sa[threadIdx.x + s]);
+      sm[threadIdx.x] = m;
+      sa[threadIdx.x] = arg;
     }
     __syncthreads();
   }
+  if (threadIdx.x < 32)
+    for (int s = 16; s > 0; s >>= 1) {
+      const double m2 = __shfl_down_sync(0xffffffffu, m, s);
+      const long long a2 = __shfl_down_sync(0xffffffffu, arg, s);
+      keep_max(m, arg, m2, a2);
+    }
 }
 
 template <class F>
@@ -146,7 +153,7 @@ __global__ void __launch_bounds__(kRedThreads) k_argmax(const double* p, GenRang
     if (v > m || (v == m && o < arg)) { m = v; arg = o; }
   }
   fold_max(m, arg, sm, sa);
-  if (threadIdx.x == 0) { part[blockIdx.x].m = sm[0]; part[blockIdx.x].arg = sa[0]; }
+  if (threadIdx.x == 0) { part[blockIdx.x].m = m; part[blockIdx.x].arg = arg; }
   if (!last_block(ticket)) return;
   m = -INFINITY;
   arg = LLONG_MAX;
@@ -157,20 +164,25 @@ __global__ void __launch_bounds__(kRedThreads) k_argmax(const double* p, GenRang
   }
   fold_max(m, arg, sm, sa);
   if (threadIdx.x == 0) {
-    out->m = sm[0];
+    out->m = m;
     // no comparable value (NaN everywhere): keep the index valid
-    out->arg = sa[0] == LLONG_MAX ? (long long)r.j0 * pitch + r.i0 : sa[0];
+    out->arg = arg == LLONG_MAX ? (long long)r.j0 * pitch + r.i0 : arg;
     f();
   }
 }
 
-__device__ __forceinline__ void fold_sum(double s, double* sm) {
+__device__ __forceinline__ void fold_sum(double& s, double* sm) {
   sm[threadIdx.x] = s;
   __syncthreads();
-  for (int k = kRedThreads / 2; k > 0; k >>= 1) {
-    if (threadIdx.x < k) sm[threadIdx.x] += sm[threadIdx.x + k];
+  for (int k = kRedThreads / 2; k >= 32; k >>= 1) {
+    if (threadIdx.x < k) {
+      s += sm[threadIdx.x + k];
+      sm[threadIdx.x] = s;
+    }
     __syncthreads();
   }
+  if (threadIdx.x < 32)
+    for (int k = 16; k > 0; k >>= 1) s += __shfl_down_sync(0xffffffffu, s, k);
 }
 
 template <class F>
@@ -184,13 +196,13 @@ __global__ void __launch_bounds__(kRedThreads) k_sum(const double* p, GenRange r
     s += p[(long long)j * pitch + i];
   }
   fold_sum(s, sm);
-  if (threadIdx.x == 0) part[blockIdx.x] = sm[0];
+  if (threadIdx.x == 0) part[blockIdx.x] = s;
   if (!last_block(ticket)) return;
   s = 0.0;
   for (int b = threadIdx.x; b < gridDim.x; b += kRedThreads) s += __ldcg(&part[b]);
   fold_sum(s, sm);
   if (threadIdx.x == 0) {
-    *out = sm[0];
+    *out = s;
     f();
   }
 }

@@ -958,41 +958,46 @@ ATHB_HD void gen_ghost(const Planes<T>& s, long long ps, int pitch, const GhostG
 // The kind of a plane at the boundaries: 1 for B1i, 2 for B2i, else 0.
 ATHB_HD int plane_kind(int p) { return p == P_B1I ? 1 : p == P_B2I ? 2 : 0; }
 
-// Adjoint, pass 1 (x2) of plane p: rows [js, je(+1 for B2i)], every column: add
-// the adjoints of the ghost rows that copy this row.  One item per plane and
-// place (11 times the threads, none with a chain of 11 planes).
-ATHB_HD void fold_x2(double* l, long long ps, int pitch, const GhostGeom& g, int p, int j, int i) {
-  const int kind = plane_kind(p), je_int = g.je + (kind == 2 ? 1 : 0);
-  if (j < g.js || j > je_int) return;
-  double* q = l + p * ps;
-  const long long o = (long long)j * pitch + i;
-  double v = q[o];
-#pragma unroll
-  for (int gq = 0; gq < 2 * kNghostA; gq++) {   // the ghost rows: js-4..js-1, je_int+1..je_int+4
-    const int jj = gq < kNghostA ? g.js - kNghostA + gq : je_int + 1 + (gq - kNghostA);
-    bool f = false;
-    if (jj < 0 || jj >= g.sy || ghost_map1(jj, g.js, g.je, kind == 2, g.bc[2], g.bc[3], f) != j) continue;
-    const double x = q[(long long)jj * pitch + i];
-    v += (p == P_M2 && f) ? -x : x;
-  }
-  q[o] = v;
-}
-// Adjoint, pass 2 (x1) of plane p: interior cells add the adjoints of the
-// ghost columns of their row that copy them.
-ATHB_HD void fold_x1(double* l, long long ps, int pitch, const GhostGeom& g, int p, int j, int i) {
+// The fill reversed on plane p at place (j,i), one the step writes: the ghost
+// rows that copy row j added (x2), in every column, then the ghost columns
+// that copy column i, each with its ghost rows added first (x1): the order of
+// the fill backwards.  Ghosts are read and never written, so one pass does it.
+// One item per plane and place (11 times the threads, none with a chain of 11
+// planes).
+ATHB_HD void fold_ghost(double* l, long long ps, int pitch, const GhostGeom& g, int p, int j, int i) {
   const int kind = plane_kind(p), ie_int = g.ie + (kind == 1 ? 1 : 0), je_int = g.je + (kind == 2 ? 1 : 0);
   if (j < g.js || j > je_int || i < g.is || i > ie_int) return;
-  double* q = l + p * ps + (long long)j * pitch;
-  double v = q[i];
+  double* q = l + p * ps;
+  int row[2 * kNghostA];   // 0, or the ghost row's sign: rows js-4..js-1, je_int+1..je_int+4
 #pragma unroll
-  for (int gq = 0; gq < 2 * kNghostA; gq++) {   // the ghost columns: is-4..is-1, ie_int+1..ie_int+4
-    const int ii = gq < kNghostA ? g.is - kNghostA + gq : ie_int + 1 + (gq - kNghostA);
+  for (int k = 0; k < 2 * kNghostA; k++) {
+    const int jj = k < kNghostA ? g.js - kNghostA + k : je_int + 1 + (k - kNghostA);
+    bool f = false;
+    row[k] = jj < 0 || jj >= g.sy || ghost_map1(jj, g.js, g.je, kind == 2, g.bc[2], g.bc[3], f) != j ? 0
+             : p == P_M2 && f                                                                        ? -1
+                                                                                                     : 1;
+  }
+  auto column = [&](int ii) {
+    double v = q[(long long)j * pitch + ii];
+#pragma unroll
+    for (int k = 0; k < 2 * kNghostA; k++) {
+      if (row[k] == 0) continue;
+      const int jj = k < kNghostA ? g.js - kNghostA + k : je_int + 1 + (k - kNghostA);
+      const double x = q[(long long)jj * pitch + ii];
+      v += row[k] < 0 ? -x : x;
+    }
+    return v;
+  };
+  double v = column(i);
+#pragma unroll
+  for (int k = 0; k < 2 * kNghostA; k++) {   // the ghost columns: is-4..is-1, ie_int+1..ie_int+4
+    const int ii = k < kNghostA ? g.is - kNghostA + k : ie_int + 1 + (k - kNghostA);
     bool f = false;
     if (ii < 0 || ii >= g.sx || ghost_map1(ii, g.is, g.ie, kind == 1, g.bc[0], g.bc[1], f) != i) continue;
-    const double x = q[ii];
+    const double x = column(ii);
     v += (p == P_M1 && f) ? -x : x;
   }
-  q[i] = v;
+  q[(long long)j * pitch + i] = v;
 }
 // Zero plane p at a place that is not one the step writes (ghosts after the
 // fold), so the folded adjoint is exactly the interior one.
