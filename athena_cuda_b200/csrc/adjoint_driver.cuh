@@ -516,15 +516,14 @@ template <class Exec> struct AdjointDriver {
     dti.v += (long long)G_DTI * G.ps;
     offset_tangent(dti);
     const int is = G.is, ie = G.ie, js = G.js, je = G.je;
-    x.items(range_plm(is, ie, js, je), FwdFn<F_PLMX, FLUX, T>{a, dti});
-    x.items(range_plm(is, ie, js, je), FwdFn<F_PLMY, FLUX, T>{a, dti});
-    x.items(range_riemann_x(is, ie, js, je), FwdFn<F_RIEX, FLUX, T>{a, dti});
-    x.items(range_riemann_y(is, ie, js, je), FwdFn<F_RIEY, FLUX, T>{a, dti});
-    x.items(range_plm(is, ie, js, je), FwdFn<F_ECC0, FLUX, T>{a, dti});
+    // the stages that do not read each other side by side, as in reverse_step
+    run_items2(x, 0, range_plm(is, ie, js, je), FwdFn<F_PLMX, FLUX, T>{a, dti}, range_plm(is, ie, js, je),
+               FwdFn<F_PLMY, FLUX, T>{a, dti});
+    run_items3(x, 0, range_riemann_x(is, ie, js, je), FwdFn<F_RIEX, FLUX, T>{a, dti}, range_riemann_y(is, ie, js, je),
+               FwdFn<F_RIEY, FLUX, T>{a, dti}, range_plm(is, ie, js, je), FwdFn<F_ECC0, FLUX, T>{a, dti});
     x.items(range_emf0(is, ie, js, je), FwdFn<F_EMF0, FLUX, T>{a, dti});
-    x.items(range_correct_x(is, ie, js, je), FwdFn<F_CORX, FLUX, T>{a, dti});
-    x.items(range_correct_y(is, ie, js, je), FwdFn<F_CORY, FLUX, T>{a, dti});
-    x.items(range_correct_e(is, ie, js, je), FwdFn<F_CORE, FLUX, T>{a, dti});
+    run_items3(x, 0, range_correct_x(is, ie, js, je), FwdFn<F_CORX, FLUX, T>{a, dti}, range_correct_y(is, ie, js, je),
+               FwdFn<F_CORY, FLUX, T>{a, dti}, range_correct_e(is, ie, js, je), FwdFn<F_CORE, FLUX, T>{a, dti});
     x.items(range_emf1(is, ie, js, je), FwdFn<F_EMF1, FLUX, T>{a, dti});
     x.items(interior(), FwdFn<F_UPD, FLUX, T>{a, dti});
     x.items(full(), GhostFn<T>{out, G.ps, G.pitch, ghost_geom()});
