@@ -58,7 +58,7 @@ OPS_STEP = sum(OPS_PER_ZC.values())
 # (profiles/k_predict_field_loop_1024.md, k_correct_k_update_field_loop_1024.md),
 # scaled to 2048x2048 by the cell ratio 4.  Applies to the 2048x2048 default
 # workload.
-TRAFFIC_1024 = {"predict": 508.49e6, "correct": 725.48e6, "update_cfl": 244.51e6}
+TRAFFIC_1024 = {"predict": 469.49e6, "correct": 702.56e6, "update_cfl": 241.91e6}
 
 
 def parse():
