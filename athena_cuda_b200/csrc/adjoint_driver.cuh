@@ -92,6 +92,18 @@ template <class T> struct CflFn {
   }
 };
 
+// the same rate of a double state as a value
+struct RateVal {
+  const double* s;
+  long long ps;
+  double dx1, dx2;
+  Eos eos;
+  ATHB_MEM double operator()(long long o) const {
+    return gen_cell_dti(s[P_D * ps + o], s[P_M1 * ps + o], s[P_M2 * ps + o], s[P_M3 * ps + o], s[P_E * ps + o], eos,
+                        dx1, dx2);
+  }
+};
+
 template <class T> struct GhostFn {
   Planes<T> s;
   long long ps;
@@ -275,27 +287,41 @@ struct DtRuleAdjFn {
   const double* s;       // S^k
   double* l;             // adjoint of S^k
   const MaxLoc* ml;
-  AdjScal* sc;
   const StepRec* rec;
   int k;                 // which dt_rule
   long long ps;
   double cour, dx1, dx2;
   Eos eos;
-  ATHB_MEM void operator()() const {
-    const double lr = sc->lrule;
+  // What it reads, loaded by the caller before it stores anything: one thread
+  // runs this, and its round trips to memory are its time.
+  struct In {
+    double m, u[5], l[5];
+    long long o;
+    int cap;
+  };
+  ATHB_MEM In load() const {
+    In a;
+    a.m = ml->m;
+    a.o = ml->arg;
+    a.cap = rec[k].cap;
+    const long long p[5] = {P_D * ps, P_M1 * ps, P_M2 * ps, P_M3 * ps, P_E * ps};
+    for (int q = 0; q < 5; q++) {
+      a.u[q] = s[p[q] + a.o];
+      a.l[q] = l[p[q] + a.o];
+    }
+    return a;
+  }
+  ATHB_MEM void apply(const In& a, double lr) const {
     if (lr == 0.0) return;
-    if (k >= 1 && rec[k].cap) return;  // the 2 dt branch: carried by the caller
-    const double m = ml->m;
-    const double lm = -cour / (m * m) * lr;
-    const long long o = ml->arg;
+    if (k >= 1 && a.cap) return;  // the 2 dt branch: carried by the caller
+    const double lm = -cour / (a.m * a.m) * lr;
     double g[5];
-    cell_dti_adj(s[P_D * ps + o], s[P_M1 * ps + o], s[P_M2 * ps + o], s[P_M3 * ps + o], s[P_E * ps + o], eos, dx1,
-                 dx2, lm, g);
-    l[P_D * ps + o] += g[0];
-    l[P_M1 * ps + o] += g[1];
-    l[P_M2 * ps + o] += g[2];
-    l[P_M3 * ps + o] += g[3];
-    l[P_E * ps + o] += g[4];
+    cell_dti_adj(a.u[0], a.u[1], a.u[2], a.u[3], a.u[4], eos, dx1, dx2, lm, g);
+    l[P_D * ps + a.o] = a.l[0] + g[0];
+    l[P_M1 * ps + a.o] = a.l[1] + g[1];
+    l[P_M2 * ps + a.o] = a.l[2] + g[2];
+    l[P_M3 * ps + a.o] = a.l[3] + g[3];
+    l[P_E * ps + a.o] = a.l[4] + g[4];
   }
 };
 
@@ -307,18 +333,20 @@ struct DtStepAdjFn {
   int last;   // n == N-1 (dt_rule^{n+1} is not used)
   DtRuleAdjFn rule;   // dt_rule^n, at S^n
   ATHB_MEM void operator()() const {
-    double ldt = sc->dtsum + sc->ltime;   // time^{n+1} = time^n + dt^n
-    if (!last && rec[n + 1].cap) ldt += 2.0 * sc->lrule;
+    const DtRuleAdjFn::In in = rule.load();
+    const int cap = last ? 0 : rec[n + 1].cap, clamped = rec[n].clamped;
     double ltime = sc->ltime;
+    double ldt = sc->dtsum + ltime;       // time^{n+1} = time^n + dt^n
+    if (cap) ldt += 2.0 * sc->lrule;
     double lrule = ldt;
-    if (rec[n].clamped) {                 // dt^n = tlim - time^n
+    if (clamped) {                        // dt^n = tlim - time^n
       ltime -= ldt;
       lrule = 0.0;
     }
     sc->ltime = ltime;
     sc->lrule = lrule;
     if (!(ldt == ldt) || !(ltime == ltime)) sc->nonfinite = 1;
-    rule();
+    rule.apply(in, lrule);
   }
 };
 
@@ -328,6 +356,8 @@ struct DtStepAdjFn {
 //   items2(ra, fa, rb, fb) / items3(...)   f over r for each pair
 //   argmax_then(plane, range, pitch, out, f), sum_then(...)   the reduction,
 //     then f() with its result in place
+//   argmax_of(value, range, pitch, out, f)   argmax_then of value(place); for an
+//     executor without it (in host memory) the values go to a plane first
 template <class X, class FA, class FB>
 auto run_items2(X& x, int, const GenRange& ra, const FA& fa, const GenRange& rb, const FB& fb)
     -> decltype(x.items2(ra, fa, rb, fb)) { return x.items2(ra, fa, rb, fb); }
@@ -353,6 +383,16 @@ auto run_argmax(X& x, int, const double* p, const GenRange& r, int pitch, MaxLoc
     -> decltype(x.argmax_then(p, r, pitch, out, f)) { return x.argmax_then(p, r, pitch, out, f); }
 template <class X, class F>
 void run_argmax(X& x, long, const double* p, const GenRange& r, int pitch, MaxLoc* out, const F& f) {
+  x.argmax(p, r, pitch, out);
+  x.single(f);
+}
+template <class X, class V, class F>
+auto run_argmax_of(X& x, int, const V& v, const double*, const GenRange& r, int pitch, MaxLoc* out, const F& f)
+    -> decltype(x.argmax_of(v, r, pitch, out, f)) { return x.argmax_of(v, r, pitch, out, f); }
+template <class X, class V, class F>
+void run_argmax_of(X& x, long, const V& v, double* p, const GenRange& r, int pitch, MaxLoc* out, const F& f) {
+  for (int j = r.j0; j <= r.j1; j++)
+    for (int i = r.i0; i <= r.i1; i++) p[(long long)j * pitch + i] = v((long long)j * pitch + i);
   x.argmax(p, r, pitch, out);
   x.single(f);
 }
@@ -538,16 +578,18 @@ template <class Exec> struct AdjointDriver {
     x.items(interior(), CflFn<T>{s, dti, G.ps, G.pitch, G.dx1, G.dx2, G.eos});
   }
 
-  // One plain step S[cur] -> S[cur^1] with the factors in cf, ghosts filled,
-  // the CFL rates of the result in the G_DTI tape plane; taped: every
-  // intermediate the adjoint reads is kept in the tape.  The executor runs it
+  // One plain step S[cur] -> S[cur^1] with the factors in cf, ghosts filled;
+  // taped: every intermediate the adjoint reads is kept in the tape.  The executor runs it
   // (the GPU with the fast kernels, the host with the generic step).
   template <int FLUX> void fwd_step_double(int cur, bool taped = false) {
     x.template forward_step<FLUX>(*this, cur, taped);
   }
-  // The CFL rates are read in the first sweep alone (the maxima are kept):
-  // false in the reverse sweep, whose steps an executor may run without them.
-  bool rates = true;
+  // The CFL maximum of a state, kept at m, then f: the rates are formed where
+  // they are compared, without a plane and a launch of their own.
+  template <class F> void max_rate(double* state, MaxLoc* m, const F& f) {
+    run_argmax_of(x, 0, RateVal{state, G.ps, G.dx1, G.dx2, G.eos}, tape + (long long)G_DTI * G.ps, interior(), G.pitch,
+                  m, f);
+  }
   template <int FLUX> void generic_step_double(int cur) {
     step<FLUX, double>(pd(S[cur]), pd(S[cur ^ 1]), pd(tape), cf);
   }
@@ -661,7 +703,7 @@ template <class Exec> struct AdjointDriver {
     // run side by side (a small grid's stage leaves most SMs idle), and a
     // gather too small for a launch is formed by its reader.  With the dt rule
     // in the sum's launch and nothing cleared beforehand a step of the gradient
-    // makes 19 launches where it made 40: 21 of them took 266 -> 189 us at
+    // makes 18 launches where it made 40: 21 of them took 266 -> 189 us at
     // 64 x 48 and 504 -> 440 us at 256 x 256 before the stages themselves
     // became faster
     x.items(full(), AdjFn<R_UPD, FLUX>{a});
@@ -679,7 +721,7 @@ template <class Exec> struct AdjointDriver {
     // dt^n, then dt_rule^n = CourNo / m(S^n), whose cell and rate the first sweep kept, into lin
     run_sum(x, 0, adj + (long long)A_DT * G.ps, GenRange{is - 3, ie + 3, js - 3, je + 3}, G.pitch, &sc->dtsum,
             DtStepAdjFn{sc, rec, n, n + 1 == N ? 1 : 0,
-                        DtRuleAdjFn{Sn, lin, ml + n, sc, rec, n, G.ps, G.cour, G.dx1, G.dx2, G.eos}});
+                        DtRuleAdjFn{Sn, lin, ml + n, rec, n, G.ps, G.cour, G.dx1, G.dx2, G.eos}});
     lc ^= 1;
   }
 
@@ -726,9 +768,7 @@ template <class Exec> struct AdjointDriver {
   // Loop entry on S[0] (src/main.c:139-149): set_bvals, then dt^0 from new_dt.
   void entry() {
     x.items(full(), GhostFn<double>{pd(S[0]), G.ps, G.pitch, ghost_geom()});
-    cfl(pd(S[0]), pd(tape + (long long)G_DTI * G.ps));
-    run_argmax(x, 0, tape + (long long)G_DTI * G.ps, interior(), G.pitch, ml,
-               Dt0Fn<double>{cf, timev, ml, nullptr, rec, G.cour, G.tlim, G.dx1, G.dx2});
+    max_rate(S[0], ml, Dt0Fn<double>{cf, timev, ml, nullptr, rec, G.cour, G.tlim, G.dx1, G.dx2});
   }
 
   template <int FLUX> int adjoint(int N, int& lc, int& steps_done) {
@@ -757,8 +797,8 @@ template <class Exec> struct AdjointDriver {
       fwd_step_double<FLUX>(cur, tapes != nullptr);
       cur ^= 1;
       if (tapes) taped++; else advances++;
-      run_argmax(x, 0, tape + (long long)G_DTI * G.ps, interior(), G.pitch, ml + n + 1,
-                 DtNextFn<double>{cf, timev, ml + n + 1, nullptr, rec, n + 1, G.cour, G.tlim, G.dx1, G.dx2});
+      max_rate(S[cur], ml + n + 1,
+               DtNextFn<double>{cf, timev, ml + n + 1, nullptr, rec, n + 1, G.cour, G.tlim, G.dx1, G.dx2});
       if (tapes) {
         if (n + 1 < N) x.copy(slot_ptr(n + 1), S[cur], state_doubles());
       } else if (n + 1 < N && spine[n + 1] >= 0) {
@@ -767,7 +807,6 @@ template <class Exec> struct AdjointDriver {
     }
     tape = tape0;
     objective(S[cur], nullptr);
-    rates = false;
     std::vector<StepRec> hrec(N + 1);
     x.to_host(hrec.data(), rec, sizeof(StepRec) * (size_t)(N + 1));
     // stop at tlim as the main loop does

@@ -138,8 +138,12 @@ __device__ __forceinline__ void fold_max(double& m, long long& arg, double* sm, 
     }
 }
 
-template <class F>
-__global__ void __launch_bounds__(kRedThreads) k_argmax(const double* p, GenRange r, int pitch, long long n,
+struct PlaneVal {
+  const double* p;
+  __device__ double operator()(long long o) const { return p[o]; }
+};
+template <class V, class F>
+__global__ void __launch_bounds__(kRedThreads) k_argmax(V p, GenRange r, int pitch, long long n,
                                                         MaxLoc* part, unsigned* ticket, MaxLoc* out, F f) {
   __shared__ double sm[kRedThreads];
   __shared__ long long sa[kRedThreads];
@@ -149,7 +153,7 @@ __global__ void __launch_bounds__(kRedThreads) k_argmax(const double* p, GenRang
     int j, i;
     range_item(r, t, j, i);
     const long long o = (long long)j * pitch + i;
-    const double v = p[o];
+    const double v = p(o);
     if (v > m || (v == m && o < arg)) { m = v; arg = o; }
   }
   fold_max(m, arg, sm, sa);
@@ -336,6 +340,9 @@ struct GpuExec {
   }
   int red_blocks(long long n) const { return (int)std::max(1LL, std::min((long long)kRedBlocks, (n + kRedThreads - 1) / kRedThreads)); }
   template <class F> void argmax_then(const double* p, const GenRange& r, int pitch, MaxLoc* out, const F& f) {
+    argmax_of(PlaneVal{p}, r, pitch, out, f);
+  }
+  template <class V, class F> void argmax_of(const V& p, const GenRange& r, int pitch, MaxLoc* out, const F& f) {
     const long long n = range_count(r);
     if (err != cudaSuccess) return;
     k_argmax<<<red_blocks(n), kRedThreads, 0, s>>>(p, r, pitch, n, redm, ticket, out, after(f));
@@ -383,7 +390,6 @@ struct GpuExec {
     GridArgs gg = g;
     gg.in = d.S[cur ^ 1];
     k_ghost<<<blocks(nframe, kThreads), kThreads, 0, s>>>(gg, G.sx, G.sy, nframe, 3, 3);
-    if (d.rates) d.cfl(d.pd(d.S[cur ^ 1]), d.pd(d.tape + (size_t)G_DTI * G.ps));
   }
 
   // With a cache (athb_adjoint_keep_workspace on) a block of the same size
