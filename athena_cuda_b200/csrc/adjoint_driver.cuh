@@ -489,6 +489,16 @@ template <class Exec> struct AdjointDriver {
     return g;
   }
 
+  // Bytes of the blocks that setup allocates, each rounded up to kBlockAlign.
+  static constexpr size_t kBlockAlign = 512;
+  size_t setup_bytes(int nsteps, bool tlm) const {
+    auto up = [](size_t b) { return (b + kBlockAlign - 1) / kBlockAlign * kBlockAlign; };
+    const size_t state = up(state_doubles() * sizeof(double)), planes = sizeof(double) * (size_t)G.ps;
+    return 4 * state + up(NTAPE * planes) + up((tlm ? (size_t)NTAPE : (size_t)NADJ) * planes) +
+           up(sizeof(StepRec) * ((size_t)nsteps + 1)) + up(sizeof(MaxLoc) * ((size_t)nsteps + 1)) +
+           up(sizeof(AdjScal)) + up(sizeof(StepCoef<double>)) + up(sizeof(StepCoef<Dual>)) + 2 * kBlockAlign;
+  }
+
   // Allocate everything but the snapshots; nsteps bounds the records.
   int setup(int nsteps, bool tlm) {
     nrec = nsteps + 1;
