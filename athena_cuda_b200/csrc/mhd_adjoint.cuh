@@ -1728,7 +1728,7 @@ ATHB_HD bool flux_roe_adj_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl
   const double bsq = bet2s * bet2s + bet3s * bet3s;
   const double vbet = v2 * bet2s + v3 * bet3s;
   wave_weights(s.cfsq - s.cssq, s.twid_asq - s.cssq, s.cfsq - s.twid_asq, af, as, general, r_span, h_af, h_as);
-  bad |= f.tiny_waves && !(as == 0.0 && above<-300>(v1));
+  bad |= f.tiny_waves;   // their derivatives count where their values do not
   const double sqrtd = root(d, hd);
   const double isd = recip_of_root(sqrtd, hd);
   const unsigned sgn = Bxi < 0. ? 0x80000000u : 0u;

@@ -244,3 +244,72 @@ def test_roe_adjoint_agrees(fast, kind):
     assert ok.sum() > n // 4 and np.all(ok[flux.astype(bool)])
     err = np.abs(f - g)[ok].max(axis=1) / np.abs(g)[ok].max(axis=1)
     assert np.quantile(err, 0.999) <= 1000 * 2.0 ** -52 / 1e-3
+
+
+def _fading(rng, n, sides, kind):
+    """States where the field fades out (kind "edge" or "still"), every side of
+    its own density, velocity and pressure, so that all jumps count."""
+    w, b = _states(rng, sides * n, kind)
+    w[:, 0] *= np.exp(0.1 * rng.normal(size=sides * n))
+    w[:, 4] *= np.exp(0.1 * rng.normal(size=sides * n))
+    w[:, 1:4] += 0.2 * rng.normal(size=(sides * n, 3))
+    return np.ascontiguousarray(w.reshape(n, sides, 7)), b
+
+
+def _worst(fast_values, general_values):
+    return (np.abs(fast_values - general_values).max(axis=1) / np.abs(general_values).max(axis=1)).max()
+
+
+# Fast and general adjoint of one face or cell where alpha_s = 0 (a field whose
+# square does not show beside the pressure), so that nothing is divided by a small
+# weight: ~1000 operations on terms no larger than the largest output.
+FADING_TOL = 1000 * 2.0 ** -52
+
+
+@pytest.mark.parametrize("kind", ["edge", "still"])
+def test_roe_adjoint_where_fields_fade(fast, kind):
+    """Wave speeds far below the flow speed do not show in the flux, but their
+    derivatives do: every face the adjoint takes agrees with the general form."""
+    n = 40000
+    rng = np.random.default_rng(22)
+    w, b = _fading(rng, n, 2, kind)
+    bx, lam = np.ascontiguousarray(b[:n]), rng.normal(size=(n, 7))
+    took = np.zeros(n, dtype=np.int32)
+    f, g = np.empty((n, 29)), np.empty((n, 29))
+    fast.fast_roe_adj(n, _p(w), _p(bx), _p(lam), C.c_double(5.0 / 3.0), _p(took), _p(f), _p(g))
+    ok = took.astype(bool)
+    assert ok.mean() > 0.5
+    assert _worst(f[ok], g[ok]) <= FADING_TOL
+
+
+def test_roe_adjoint_over_normal_fields(fast):
+    """The normal field of one subsonic face from 1e-100 down to where it is zero."""
+    bx = np.concatenate([10.0 ** np.linspace(-100, -170, 2801), [0.0]])
+    bx = np.ascontiguousarray(np.concatenate([bx, -bx]))
+    n = bx.size
+    rng = np.random.default_rng(23)
+    w = np.tile(np.array([[1.0, 0.5, 0.3, -0.2, 1.0, 0.0, 0.0], [1.1, 0.4, -0.1, 0.25, 0.9, 0.0, 0.0]]), (n, 1, 1))
+    lam = rng.normal(size=(n, 7))
+    took = np.zeros(n, dtype=np.int32)
+    f, g = np.empty((n, 29)), np.empty((n, 29))
+    fast.fast_roe_adj(n, _p(w), _p(bx), _p(lam), C.c_double(5.0 / 3.0), _p(took), _p(f), _p(g))
+    ok = took.astype(bool)
+    assert ok.mean() > 0.5
+    assert _worst(f[ok], g[ok]) <= FADING_TOL
+
+
+@pytest.mark.parametrize("kind", ["edge", "still"])
+def test_plm_adjoint_where_fields_fade(fast, kind):
+    n = 40000
+    rng = np.random.default_rng(24)
+    w, b = _fading(rng, n, 3, kind)
+    bx = np.ascontiguousarray(b.reshape(n, 3))
+    dtodx, lam = rng.uniform(0.05, 0.4, n), rng.normal(size=(n, 14))
+    took = np.zeros(n, dtype=np.int32)
+    f, g = np.empty((n, 23)), np.empty((n, 23))
+    fast.fast_plm_adj(n, _p(w), _p(bx), _p(dtodx), _p(lam), C.c_double(5.0 / 3.0), _p(took), _p(f), _p(g))
+    # the general form forms dl dr / (dl + dr) and has few bits of it where dl dr is denormal
+    prod = np.abs((w[:, 1, 5:] - w[:, 0, 5:]) * (w[:, 2, 5:] - w[:, 1, 5:]))
+    ok = took.astype(bool) & ~((prod > 0) & (prod < np.finfo(float).tiny)).any(axis=1)
+    assert ok.mean() > 0.5
+    assert _worst(f[ok], g[ok]) <= FADING_TOL
