@@ -1571,9 +1571,12 @@ ATHB_HD void flux_roe_adj(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, con
 }
 
 // ---------------------------------------------------------------------------
-// flux_roe_adj in the fast form: forward values and branches are those of
-// flux_roe_fast, bit for bit (the same operations in the same order), the
-// reverse goes over the pairs of waves n and 6-n and divides nowhere.
+// flux_roe_adj in the fast form: the forward values are those of flux_roe_fast,
+// bit for bit (the same operations in the same order), the reverse goes over the
+// pairs of waves n and 6-n and divides nowhere.  It takes only faces that
+// flux_roe_fast takes: of these it leaves the ones with tiny wave speeds, and any
+// that pass the flux's bound on the intermediate states but not the test of the
+// states themselves, to the general form.
 // The general form is bound by its chains of divisions and roots with branches
 // around them (255 registers, 8 warps an SM): at 256 x 256 the corrector's
 // launch took 82 us and the predictor's 69 us with it, 42 and 25 us with this.
@@ -1783,7 +1786,8 @@ ATHB_HD bool flux_roe_adj_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl
   a[3] = (1.0 - norm2 * (0.5 * vsq - gx)) * u0 + (norm2 * v1) * u1 + (norm2 * v2) * u2 + (norm2 * v3) * u3 -
          norm2 * u4 + (norm2 * b2) * u5 + (norm2 * b3) * u6;
 
-  // the positivity test of flux_roe_fast (step 7), on the states themselves
+  // the positivity test of flux_roe_fast (step 7), on the states themselves,
+  // formed as there: a face the flux sends to HLLE must not pass here
   {
     const double c1a = af * v2, c1b = qs * bet2s, c2a = af * v3, c2b = qs * bet3s, e0 = qs * vbet;
     const double s1a = as * v2, s1b = qf * bet2s, s2a = as * v3, s2b = qf * bet3s, e2 = qf * vbet;
@@ -1801,7 +1805,7 @@ ATHB_HD bool flux_roe_adj_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl
     for (int n = 0; n < 6; n++) {
 #pragma unroll
       for (int m = 0; m < 7; m++)
-        if ((roe_right_mask(n) >> m) & 1) u[m] = mad(a[n], C[n][m], u[m]);
+        if ((roe_right_mask(n) >> m) & 1) u[m] += a[n] * C[n][m];
       const double k = 0.5 * (u[5] * u[5] + u[6] * u[6] + Bxi * Bxi);
       const double m2 = 0.5 * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]);
       bad |= !(u[0] > 0.0) || !((u[4] - k) * u[0] - m2 > 1.0e-12 * (u[4] * u[0]));

@@ -313,3 +313,42 @@ def test_plm_adjoint_where_fields_fade(fast, kind):
     ok = took.astype(bool) & ~((prod > 0) & (prod < np.finfo(float).tiny)).any(axis=1)
     assert ok.mean() > 0.5
     assert _worst(f[ok], g[ok]) <= FADING_TOL
+
+
+@pytest.mark.parametrize("spread", [1.0, 3.0, 8.0])
+def test_roe_adjoint_branches_as_the_flux(fast, spread):
+    """Faces on the path from a small jump to one that needs the HLLE fallback,
+    bisected to the last pair of doubles where the flux still takes the fast
+    form: the adjoint never goes on with Roe where the flux does not."""
+    n = 20000
+    rng = np.random.default_rng(int(spread))
+    A = np.empty((n, 2, 7))
+    A[:, :, 0], A[:, :, 4] = np.exp(spread * rng.normal(size=(2, n, 2)))
+    A[:, :, 1:4], A[:, :, 5:] = 2.0 * rng.normal(size=(n, 2, 3)), rng.normal(size=(n, 2, 2))
+    B = A.copy()
+    B[:, 1] = B[:, 0] * (1 + 1e-3)
+    bx, lam = rng.normal(size=n), np.ones((n, 7))
+
+    def taken(t):
+        t = t[:, None]
+        w = (1 - t)[:, :, None] * B + t[:, :, None] * A
+        for c in (0, 4):
+            w[:, :, c] = np.exp((1 - t) * np.log(B[:, :, c]) + t * np.log(A[:, :, c]))
+        w = np.ascontiguousarray(w)
+        flux, adj = np.zeros((2, n), dtype=np.int32)
+        f, g = np.empty((2, n, 29))
+        fast.fast_flux(0, n, _p(w), _p(bx), C.c_double(5.0 / 3.0), _p(flux), _p(f), _p(g))
+        fast.fast_roe_adj(n, _p(w), _p(bx), _p(lam), C.c_double(5.0 / 3.0), _p(adj), _p(f), _p(g))
+        return flux.astype(bool), adj.astype(bool)
+
+    lo, hi = np.zeros(n), np.ones(n)
+    crossing = taken(lo)[0] & ~taken(hi)[0]
+    assert crossing.sum() > n // 10
+    for _ in range(54):
+        mid = 0.5 * (lo + hi)
+        flux, adj = taken(mid)
+        assert not np.any(adj & ~flux)
+        lo, hi = np.where(flux, mid, lo), np.where(flux, hi, mid)
+    for k in range(-8, 9):
+        flux, adj = taken(hi * (1 + k * 2.0 ** -52))
+        assert not np.any(adj & ~flux)
