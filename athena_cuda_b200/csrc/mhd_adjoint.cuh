@@ -1574,9 +1574,9 @@ ATHB_HD void flux_roe_adj(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, con
 // flux_roe_adj in the fast form: the forward values are those of flux_roe_fast,
 // bit for bit (the same operations in the same order), the reverse goes over the
 // pairs of waves n and 6-n and divides nowhere.  It takes only faces that
-// flux_roe_fast takes: of these it leaves the ones with tiny wave speeds, and any
-// that pass the flux's bound on the intermediate states but not the test of the
-// states themselves, to the general form.
+// flux_roe_fast takes: of these it leaves any that pass the flux's bound on the
+// intermediate states but not the test of the states themselves to the general
+// form.
 // The general form is bound by its chains of divisions and roots with branches
 // around them (255 registers, 8 warps an SM): at 256 x 256 the corrector's
 // launch took 82 us and the predictor's 69 us with it, 42 and 25 us with this.
@@ -1731,7 +1731,16 @@ ATHB_HD bool flux_roe_adj_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl
   const double bsq = bet2s * bet2s + bet3s * bet3s;
   const double vbet = v2 * bet2s + v3 * bet3s;
   wave_weights(s.cfsq - s.cssq, s.twid_asq - s.cssq, s.cfsq - s.twid_asq, af, as, general, r_span, h_af, h_as);
-  bad |= f.tiny_waves;   // their derivatives count where their values do not
+  bad |= f.tiny_waves && !(as == 0.0 && above<-300>(v1));
+  if (f.tiny_waves) {
+    // the flow speed absorbs these speeds, but not their derivatives (1 / (2 speed)
+    // times 2 Bxi / d): the operations of the general form, which hold at any size
+    s.cssq = s.twid_asq * s.vaxsq / s.cfsq;
+    s.cs = sqrt(s.cssq);
+    s.vax = sqrt(s.vaxsq);
+    f.h_cs = 0.5 / s.cs;
+    f.h_vax = 0.5 / s.vax;
+  }
   const double sqrtd = root(d, hd);
   const double isd = recip_of_root(sqrtd, hd);
   const unsigned sgn = Bxi < 0. ? 0x80000000u : 0u;
