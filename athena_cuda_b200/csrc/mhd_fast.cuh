@@ -393,6 +393,9 @@ ATHB_HD void limited_slopes(const double Wm[7], const double W0[7], const double
       S.dg[n] = prod > 0.0 ? (small ? g * 0x1p-200 : g) : 0.0;
       bad |= above<500>(prod);
     }
+    // a quotient of denormal size is rounded once in the general form and more
+    // than once here (differences of density and pressure are never that small)
+    if (n != 0 && n != 4) bad |= prod > 0.0 && !above<-1021>(S.dg[n]);
   }
   project(L, S.dl, S.al);
   project(L, S.dr, S.ar);

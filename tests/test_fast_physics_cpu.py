@@ -352,3 +352,28 @@ def test_roe_adjoint_branches_as_the_flux(fast, spread):
     for k in range(-8, 9):
         flux, adj = taken(hi * (1 + k * 2.0 ** -52))
         assert not np.any(adj & ~flux)
+
+
+@pytest.mark.parametrize("component,exponent", [(5, 0), (6, 0), (1, 115), (2, 115), (3, 115)])
+def test_plm_slopes_of_denormal_size(fast, component, exponent):
+    """The limiter's quotient 2 dl dr / (dl + dr) where it is a denormal: a jump of
+    a few denormal ulps beside one of O(1) (of 2^115 where the fast form wants
+    the product of the two above 2^-960), quotients on and next to a tie."""
+    n = 40000
+    rng = np.random.default_rng(30 + component)
+    size = np.ldexp(rng.uniform(0.01, 1.0, n), exponent)
+    size[::2] = np.ldexp(2.0 * rng.integers(1, 64, n // 2) / (rng.integers(1, 200, n // 2) + 0.5), exponent)
+    w = np.zeros((n, 3, 7))
+    w[:, :, 0], w[:, :, 4] = 2.0 ** -30, 1.0
+    w[:, :, 1] = rng.choice([0.3, -0.2, 0.0], n)[:, None]
+    w[:, :, component] = 0.0
+    dl = np.ldexp(rng.integers(1 << 51 if exponent else 1, 1 << 52 if exponent else 2000, n).astype(float), -1074)
+    if exponent == 0:   # such that 2 dl dr is a few denormal ulps
+        dl[::2] = np.ldexp(np.round(rng.integers(1, 64, n // 2) / size[::2]), -1074)
+    w[:, 0, component], w[:, 2, component] = -dl, size
+    bx, dtodx = np.zeros((n, 3)), rng.uniform(0.05, 0.4, n)
+    took = np.zeros(n, dtype=np.int32)
+    f, g = np.empty((n, 14)), np.empty((n, 14))
+    fast.fast_plm(n, _p(w), _p(bx), _p(dtodx), C.c_double(5.0 / 3.0), _p(took), _p(f), _p(g))
+    ok = took.astype(bool)
+    np.testing.assert_array_equal(f[ok], g[ok])
