@@ -389,11 +389,11 @@ struct GpuExec {
     k_emf<<<blocks((long long)(nx1 + 1) * (nx2 + 1), kThreads), kThreads, 0, s>>>(g, G.is, G.js, nx1 + 1, nx2 + 1,
                                                                                    S_FX2, S_FY2);
     const int n = nx1 * nx2;
-    k_update<<<blocks(n, kThreads), kThreads, 0, s>>>(g, nx1, n, 0);
+    k_update<<<blocks(n, kThreads), kThreads, 0, s>>>(g, nx1, n);
     const int nframe = G.js * G.sx + (G.sy - G.je - 1) * G.sx + nx2 * 2 * G.is;
     GridArgs gg = g;
     gg.in = d.S[cur ^ 1];
-    k_ghost<<<blocks(nframe, kThreads), kThreads, 0, s>>>(gg, G.sx, G.sy, nframe, 3, 3);
+    k_ghost<<<blocks(nframe, kThreads), kThreads, 0, s>>>(gg, G.sx, G.sy, nframe, 3, 3, 0);
   }
 
   // With a cache (athb_adjoint_keep_workspace on) a block of the same size

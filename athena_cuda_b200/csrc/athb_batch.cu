@@ -702,7 +702,7 @@ extern "C" int athb_batch_prepare(athb_batch* b) {
     if (cur[k]) { const double* a = g.in; g.in = g.out; g.out = const_cast<double*>(a); }
     GridArgs gg = g;  // ghost fill writes the current buffer
     gg.out = const_cast<double*>(g.in);
-    k_ghost<<<(I.nframe + kThreads - 1) / kThreads, kThreads, 0, b->stream>>>(gg, I.sx, I.sy, I.nframe, 3, 3);
+    k_ghost<<<(I.nframe + kThreads - 1) / kThreads, kThreads, 0, b->stream>>>(gg, I.sx, I.sy, I.nframe, 3, 3, 0);
     const int ncell = I.nx1 * I.nx2;
     k_cfl<<<(ncell + kThreads - 1) / kThreads, kThreads, 0, b->stream>>>(g, I.nx1, ncell);
     k_finalize<<<1, 1, 0, b->stream>>>(b->st + k, g.dx1, g.dx2, 0);

@@ -237,15 +237,19 @@ extern "C" int athb_download(athb_ctx* c, double* planes, double* dt, double* ti
 // ---------------------------------------------------------------------------
 // launch sequences
 // ---------------------------------------------------------------------------
-int athb_launch_ghost_phase(athb_ctx* c, int buf, int mode, int sides) {
+// final: the launch also ends the step (finalize_state, mode 1)
+static int launch_ghost(athb_ctx* c, int buf, int mode, int sides, int final) {
   GridArgs g = grid_args(c, buf ^ 1);  // out = buf
   const int nframe = c->js * c->sx + (c->sy - c->je - 1) * c->sx + c->cfg.nx2 * 2 * c->is;
-  k_ghost<<<blocks_for(nframe), kThreads, 0, c->stream>>>(g, c->sx, c->sy, nframe, mode, sides);
+  k_ghost<<<blocks_for(nframe) + final, kThreads, 0, c->stream>>>(g, c->sx, c->sy, nframe, mode, sides, final);
   CUDA_TRY(cudaGetLastError());
   return ATHB_OK;
 }
 
-int athb_launch_ghost(athb_ctx* c, int buf) { return athb_launch_ghost_phase(c, buf, 3, 3); }
+int athb_launch_ghost_phase(athb_ctx* c, int buf, int mode, int sides) {
+  return launch_ghost(c, buf, mode, sides, 0);
+}
+int athb_launch_ghost(athb_ctx* c, int buf) { return launch_ghost(c, buf, 3, 3, 0); }
 
 int athb_launch_set_dt(athb_ctx* c, double dt) {
   k_set_dt<<<1, 1, 0, c->stream>>>(c->st, dt, c->dx1, c->dx2);
@@ -261,10 +265,9 @@ int athb_launch_cfl(athb_ctx* c, int buf) {
   return ATHB_OK;
 }
 
-// The integrator proper: reads state[from], writes the interior of
-// state[from^1]; final: also ends the step (finalize_state, mode 1).
+// The integrator proper: reads state[from], writes the interior of state[from^1].
 // With ev != nullptr, events ev[0..5] bracket the five kernels.
-static int launch_integrate(athb_ctx* c, int from, int final, cudaEvent_t* ev) {
+static int launch_integrate(athb_ctx* c, int from, cudaEvent_t* ev) {
 #define MARK(k) do { if (ev) CUDA_TRY(cudaEventRecord(ev[k], c->stream)); } while (0)
   GridArgs g = grid_args(c, from);
   const int nx1 = c->cfg.nx1, nx2 = c->cfg.nx2;
@@ -297,18 +300,18 @@ static int launch_integrate(athb_ctx* c, int from, int final, cudaEvent_t* ev) {
 
   MARK(4);
   const int n = nx1 * nx2;
-  k_update<<<blocks_for(n), kThreads, 0, c->stream>>>(g, nx1, n, final);
+  k_update<<<blocks_for(n), kThreads, 0, c->stream>>>(g, nx1, n);
   CUDA_TRY(cudaGetLastError());
   MARK(5);
   return ATHB_OK;
 #undef MARK
 }
 
-int athb_launch_integrate(athb_ctx* c, int from) { return launch_integrate(c, from, 0, nullptr); }
+int athb_launch_integrate(athb_ctx* c, int from) { return launch_integrate(c, from, nullptr); }
 
 // Per-kernel timing of the loop step (CUDA events on the context's stream
 // between consecutive launches): predict, emf(half), correct, emf(full),
-// update, finalize, ghost; the end of the step runs inside the update kernel and
+// update, finalize, ghost; the end of the step runs inside the ghost kernel and
 // reads 0.
 extern "C" int athb_profile_steps(athb_ctx* c, int nsteps, double* ms_out) {
   if (!c || nsteps < 1 || !ms_out) return athb_fail(ATHB_ERR_ARG, "bad arguments");
@@ -321,8 +324,8 @@ extern "C" int athb_profile_steps(athb_ctx* c, int nsteps, double* ms_out) {
   int rc = ATHB_OK;
   for (int s = 0; s < nsteps && rc == ATHB_OK; s++) {
     cudaEvent_t* e = &ev[(size_t)s * (K + 1)];
-    rc = launch_integrate(c, c->cur, 1, e);
-    if (rc == ATHB_OK) rc = athb_launch_ghost(c, c->cur ^ 1);
+    rc = launch_integrate(c, c->cur, e);
+    if (rc == ATHB_OK) rc = launch_ghost(c, c->cur ^ 1, 3, 3, 1);
     if (rc) break;
     CUDA_TRY(cudaEventRecord(e[K], c->stream));
     c->cur ^= 1;
@@ -342,8 +345,8 @@ extern "C" int athb_profile_steps(athb_ctx* c, int nsteps, double* ms_out) {
 
 // One iteration of the reference main loop (src/main.c:229-307) on the device.
 static int launch_loop_step(athb_ctx* c, int from) {
-  const int rc = launch_integrate(c, from, 1, nullptr);
-  return rc ? rc : athb_launch_ghost(c, from ^ 1);
+  const int rc = launch_integrate(c, from, nullptr);
+  return rc ? rc : launch_ghost(c, from ^ 1, 3, 3, 1);
 }
 
 static int build_graph(athb_ctx* c, int from) {

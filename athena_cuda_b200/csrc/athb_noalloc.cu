@@ -52,7 +52,7 @@ std::mutex g_scratch_mutex;
 __global__ void k_noalloc_begin(StepState* st, double dt, double dx1, double dx2) {
   StepState s;
   s.time = 0.0; s.tlim = 0.0; s.cour_no = 0.0;
-  s.nstep = 0; s.nlim = -1; s.done = 0; s.flags = 0; s.arrived = 0u; s.max_dti_bits = 0ull;
+  s.nstep = 0; s.nlim = -1; s.done = 0; s.flags = 0; s.max_dti_bits = 0ull;
   s.tpause = 0.0; s.has_pause = 0;
   s.dt = dt;
   s.dt_new = dt;
@@ -141,7 +141,7 @@ extern "C" int athb_integrate_noalloc(const athb_config* cfg, const double* d_in
   k_emf<<<blocks_of((long long)(nx1 + 1) * (nx2 + 1)), kThreads, 0, s>>>(gs, gs.is, gs.js, nx1 + 1, nx2 + 1, S_FX2,
                                                                            S_FY2);
   const int n = nx1 * nx2;
-  k_update<<<blocks_of(n), kThreads, 0, s>>>(gs, nx1, n, 0);
+  k_update<<<blocks_of(n), kThreads, 0, s>>>(gs, nx1, n);
   e = cudaGetLastError();
   if (e != cudaSuccess) return athb_fail(ATHB_ERR_CUDA, "athb_integrate_noalloc launch: %s", cudaGetErrorString(e));
   return ATHB_OK;

@@ -19,8 +19,7 @@
 //               role E: 7             (cell-centred EMF at t^{n+1/2})
 //   k_emf_full  step 9 corner EMF
 //   k_update    steps 9 (CT), 11a, 11b, 13 + new_dt per cell (src/new_dt.c)
-//               with warp-shuffle / block max and one 64-bit atomicMax; in the
-//               main loop its last block does k_finalize's work
+//               with warp-shuffle / block max and one 64-bit atomicMax
 //   k_finalize  time += dt, nstep++, dt rule (src/new_dt.c:93-97), tlim clamp
 //               (src/main.c:230-232)
 //   k_ghost     set_bvals (src/set_bvals.c:114-1031) for both directions in
@@ -628,13 +627,12 @@ __device__ __forceinline__ void block_max_to(double v, unsigned long long* dst, 
 
 // ---------------------------------------------------------------------------
 // k_update: CT on the face fields, conservative update, cell-centred B and the
-// per-cell CFL rate, one thread per interior cell; in the main loop (final != 0)
-// its last block also ends the step.
+// per-cell CFL rate, one thread per interior cell.
 //
-// On a large grid it streams (2048^2: 4.7 TB/s); on a small one it is latency:
-// every load comes before the first store, as a store to one plane holds back
-// the loads behind it, and the last block to finish advances the clock in place
-// of a launch of its own.
+// On a large grid it streams (2048^2: 193 us, 203 us with each plane stored as
+// soon as it is formed); on a small one it is latency.  Either way every load
+// comes before the first store, as a store to one plane holds back the loads
+// behind it.
 // ---------------------------------------------------------------------------
 // CT, conservative update and cell-centred field of interior cell t; returns
 // the cell's CFL rate (0 for t >= ncell).
@@ -689,9 +687,7 @@ __device__ __forceinline__ double update_cell(const GridArgs& g, int nx1, int nc
   return cell_dti(d, m1, m2, m3, e, g.eos, g.dx1, g.dx2);
 }
 
-__device__ __forceinline__ void finalize_state(StepState& st, double dx1, double dx2, int mode);
-
-static __global__ void __launch_bounds__(kThreads) k_update(GridArgs g, int nx1, int ncell, int final) {
+static __global__ void __launch_bounds__(kThreads) k_update(GridArgs g, int nx1, int ncell) {
   StepState& st = *g.st;
   const int t = blockIdx.x * kThreads + threadIdx.x;
   if (st.done) {
@@ -707,14 +703,6 @@ static __global__ void __launch_bounds__(kThreads) k_update(GridArgs g, int nx1,
     return;
   }
   block_max_to(update_cell(g, nx1, ncell, t), &st.max_dti_bits, &st.flags);
-  if (final && threadIdx.x == 0) {
-    __threadfence();   // this block's maximum before its arrival
-    if (atomicAdd(&st.arrived, 1u) == gridDim.x - 1) {
-      __threadfence();
-      st.arrived = 0u;
-      finalize_state(st, g.dx1, g.dx2, 1);
-    }
-  }
 }
 
 // Standalone CFL reduction over the interior of the step's input buffer
@@ -906,9 +894,15 @@ __device__ __forceinline__ void ghost_item(const GridArgs& g, int sx, int sy, in
   if (on2) s[P_B2I * ps + o] = b2;
 }
 
+// final (main loop, after k_update): the first block, one more than the frame
+// needs, ends the step, which the fill neither reads nor writes.  A launch of its
+// own costs 1 to 2 us more a step; in k_update's last block (a fence and an
+// atomic in each) it cost that kernel 19 us at 2048^2 (212 against 193) and 2 at 200 x 300.
 static __global__ void __launch_bounds__(kThreads) k_ghost(GridArgs g, int sx, int sy, int nframe, int mode,
-                                                   int sides) {
-  ghost_item(g, sx, sy, nframe, mode, sides, blockIdx.x * kThreads + threadIdx.x);
+                                                   int sides, int final) {
+  const int b = blockIdx.x - final;
+  if (b >= 0) ghost_item(g, sx, sy, nframe, mode, sides, b * kThreads + threadIdx.x);
+  else if (threadIdx.x == 0) finalize_state(*g.st, g.dx1, g.dx2, 1);
 }
 
 }  // namespace athb

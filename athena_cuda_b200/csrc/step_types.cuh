@@ -50,7 +50,6 @@ struct StepState {
                     // tpause; either way steps are no-ops
   int flags;        // error bits, see kErr*
   int has_pause;
-  unsigned arrived; // blocks of the step's k_update that have finished
   unsigned long long max_dti_bits;  // running max of 1/dt (positive doubles
                                     // order like their bit patterns)
 };

@@ -144,7 +144,7 @@ int athb_run_async(athb_ctx *ctx, int nsteps);
 /* Run nsteps loop iterations with CUDA events between the kernels and return
  * the mean time per step of each kernel in ms_out[7]: predict, emf (half
  * step), correct, emf (full step), update (+CFL), finalize, ghost.  The end of
- * the step runs inside update, so finalize is 0.                            */
+ * the step runs inside ghost, so finalize is 0.                             */
 int athb_profile_steps(athb_ctx *ctx, int nsteps, double *ms_out);
 /* Tuning knob: rows per y-sweep march segment (work decomposition only; the
  * results do not depend on it).                                             */
