@@ -105,6 +105,7 @@ def lib() -> C.CDLL:
             "athb_batch_synchronize": (I, [P]),
             "athb_batch_stream": (P, [P]),
             "athb_batch_set_ly": (I, [P, I, I]),
+            "athb_batch_ly": (I, [P, I]),
             "athb_batch_commit": (I, [P]),
             "athb_batch_set_grid": (I, [P, I]),
             "athb_batch_set_threads": (I, [P, I]),
@@ -489,6 +490,9 @@ class Batch:
 
     def set_ly(self, k: int, ly: int) -> None:
         _check(lib().athb_batch_set_ly(self._h, k, ly))
+
+    def ly(self, k: int) -> int:
+        return lib().athb_batch_ly(self._h, k)
 
     def commit(self) -> None:
         _check(lib().athb_batch_commit(self._h))

@@ -340,6 +340,7 @@ struct athb_batch {
   std::vector<athb_config> cfg;
   std::vector<InstGeom> geom;  // host copy
   std::vector<int> ly;         // y-march segment length per instance
+  std::vector<char> ly_given;  // ... set by athb_batch_set_ly
   double* pool = nullptr;
   StepState* st = nullptr;
   int* cur = nullptr;
@@ -396,6 +397,14 @@ static InstGeom make_geom(const athb_config& c, int ly, int nt, double* state0, 
   I.nx1 = nx1; I.nx2 = nx2; I.sx = sx; I.sy = sy;
   I.nframe = g.js * sx + (sy - g.je - 1) * sx + nx2 * 2 * g.is;
   return I;
+}
+
+static long long role_y_faces(const athb_config& c) { return (long long)(c.nx1 + 4) * (c.nx2 + 3); }
+
+// Instance k's geometry from its march length and the batch's threads per unit.
+static void rebuild_geom(athb_batch* b, int k) {
+  const InstGeom& I = b->geom[k];
+  b->geom[k] = make_geom(b->cfg[k], b->ly[k], b->nt, const_cast<double*>(I.g.in), I.g.out, I.g.scr, I.g.st);
 }
 
 static int host_chunks(const InstGeom& I, int seg) {
@@ -483,6 +492,44 @@ static int upload_tables(athb_batch* b) {
   return upload_work(b);
 }
 
+// Work tables of a changed active set.  Its instances share the GPU, so the
+// march lengths that were not given by hand follow the rule of a single grid on
+// all of them together: lengths for the full batch would leave the last
+// instances of an ensemble with a few long marches on a few SMs (23 blasts of
+// 256 x 256 for 11 steps and one of 384 x 512 for 109: 40.6 ms with them, 22.5 ms
+// without; 24 uneven ones to one end time: 102.6 and 82.4).  The lengths are
+// kept when a longer map they need cannot be had.
+static int upload_active(athb_batch* b) {
+  long long faces = 0;
+  for (int k : b->active) faces += role_y_faces(b->cfg[k]);
+  const int rows = march_rows(faces);
+  const std::vector<int> before = b->ly;
+  for (int k : b->active)
+    if (!b->ly_given[k]) b->ly[k] = rows;
+  if (b->ly != before) {
+    size_t items = 0;
+    for (int k : b->active) {
+      rebuild_geom(b, k);
+      for (int seg = 0; seg < kSegs; seg++) items += (size_t)host_chunks(b->geom[k], seg);
+    }
+    if (items > b->wmap_cap) {
+      WorkItem* w = nullptr;
+      if (cudaMalloc(&w, items * sizeof(WorkItem)) == cudaSuccess) {
+        drop_graph(b);
+        cudaFree(b->wmap);
+        b->wmap = w;
+        b->wmap_cap = items;
+      } else {
+        (void)cudaGetLastError();
+        b->ly = before;
+        for (int k : b->active) rebuild_geom(b, k);
+      }
+    }
+    CUDA_TRY(cudaMemcpyAsync(b->dgeom, b->geom.data(), b->n * sizeof(InstGeom), cudaMemcpyHostToDevice, b->stream));
+  }
+  return upload_work(b);
+}
+
 extern "C" int athb_batch_create(int n, const athb_config* cfgs, athb_batch** out) {
   if (!out || n < 1 || !cfgs) return athb_fail(ATHB_ERR_ARG, "bad arguments");
   *out = nullptr;
@@ -498,10 +545,9 @@ extern "C" int athb_batch_create(int n, const athb_config* cfgs, athb_batch** ou
   b->device = cfgs[0].device;
   b->cfg.assign(cfgs, cfgs + n);
   b->ly.resize(n);
-  // the marches of all instances share the GPU: the rule of a single grid on
-  // all of them together
-  long long faces = 0;
-  for (int k = 0; k < n; k++) faces += (long long)(cfgs[k].nx1 + 4) * (cfgs[k].nx2 + 3);
+  b->ly_given.assign(n, 0);
+  long long faces = 0;   // of all instances together, see upload_active
+  for (int k = 0; k < n; k++) faces += role_y_faces(cfgs[k]);
   for (int k = 0; k < n; k++) b->ly[k] = march_rows(faces);
   // one pool: per instance two state buffers and the scratch planes
   std::vector<size_t> base(n);
@@ -567,11 +613,11 @@ extern "C" int athb_batch_size(const athb_batch* b) { return b ? b->n : 0; }
 extern "C" int athb_batch_set_ly(athb_batch* b, int k, int ly) {
   if (!b || k < 0 || k >= b->n || ly < 1) return athb_fail(ATHB_ERR_ARG, "bad arguments");
   b->ly[k] = ly;
-  InstGeom& I = b->geom[k];
-  const double* s0 = I.g.in;
-  b->geom[k] = make_geom(b->cfg[k], ly, b->nt, const_cast<double*>(s0), I.g.out, I.g.scr, I.g.st);
+  b->ly_given[k] = 1;
+  rebuild_geom(b, k);
   return ATHB_OK;
 }
+extern "C" int athb_batch_ly(const athb_batch* b, int k) { return b && k >= 0 && k < b->n ? b->ly[k] : -1; }
 
 // Threads per work unit of the phased launches (64, 128 or 256), applied to
 // every instance by athb_batch_commit.  The persistent kernel keeps 128.
@@ -587,10 +633,7 @@ extern "C" int athb_batch_set_threads(athb_batch* b, int nt) {
                                   kRing256Bytes));
   }
   b->nt = nt;
-  for (int k = 0; k < b->n; k++) {
-    InstGeom& I = b->geom[k];
-    b->geom[k] = make_geom(b->cfg[k], b->ly[k], nt, const_cast<double*>(I.g.in), I.g.out, I.g.scr, I.g.st);
-  }
+  for (int k = 0; k < b->n; k++) rebuild_geom(b, k);
   return ATHB_OK;
 }
 extern "C" int athb_batch_threads(const athb_batch* b) { return b ? b->nt : -1; }
@@ -803,7 +846,8 @@ extern "C" int athb_batch_run_async(athb_batch* b, int nsteps) {
 // Run until every instance is done (or max_steps launches).  Launches as
 // many steps as the earliest-finishing active instance still needs, then
 // re-reads the clocks; instances that finished are dropped from the work
-// tables.  Returns the number of launches.
+// tables, and the marches of the others sized anew.  Returns the number of
+// launches.
 extern "C" int athb_batch_run(athb_batch* b, int max_steps, int* launches) {
   if (!b) return athb_fail(ATHB_ERR_ARG, "null batch");
   CUDA_TRY(cudaSetDevice(b->device));
@@ -835,7 +879,7 @@ extern "C" int athb_batch_run(athb_batch* b, int max_steps, int* launches) {
     if (act.empty() || done_launches >= max_steps) break;
     if (act != b->active) {
       b->active = act;
-      int rc = upload_work(b);
+      int rc = upload_active(b);
       if (rc) return rc;
     }
     want = std::min<long long>(want, max_steps - done_launches);

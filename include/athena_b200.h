@@ -326,8 +326,10 @@ int athb_batch_run_async(athb_batch *b, int nsteps);
 int athb_batch_synchronize(athb_batch *b);
 void *athb_batch_stream(athb_batch *b);
 /* tuning: y-march segment length of instance k (applied by _commit) and the
- * number of persistent blocks (at most the co-resident maximum)             */
+ * number of persistent blocks (at most the co-resident maximum).  A length that
+ * was not set follows the instances still running; _ly reads it.            */
 int athb_batch_set_ly(athb_batch *b, int k, int ly);
+int athb_batch_ly(const athb_batch *b, int k);
 int athb_batch_commit(athb_batch *b);
 int athb_batch_set_grid(athb_batch *b, int blocks);
 /* threads per work unit of the phased launches: 64, 128 (default) or 256;

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import refutil
-from athena_cuda_b200 import PLANES, Batch, Grid, configs, ensemble, write_athinput
+from athena_cuda_b200 import PLANES, Batch, Grid, Params, configs, ensemble, problem_state, write_athinput
 
 pytestmark = pytest.mark.gpu
 
@@ -156,4 +156,39 @@ def test_autotuner_picks_threads_and_segments(tmp_path):
     table = autotune.tune_batch(b, sizes, cache=tmp_path / "tune.json")
     assert table["threads"] in autotune.NT_CANDIDATES and b.threads == table["threads"]
     assert set(table["estimated_ms_per_launch_by_threads"]) == {"64", "128", "256"}
+    b.close()
+
+
+@pytest.mark.parametrize("mode", [Batch.PHASED, Batch.PERSISTENT])
+def test_marches_follow_the_instances_left(mode):
+    """Instances that end early leave the GPU to the others: the last one gets
+    the march length of a grid alone (one that was set by hand keeps it), the
+    results stay those of single grids, and a refilled batch starts over."""
+    items = [("blast", configs.blast(256, 192 + 16 * k, tlim=2e-3 if k < 4 else 2e-2)) for k in range(6)]
+    params = [Params.from_blocks(bl) for _, bl in items]
+    grids = [Grid.create(p.config()) for p in params]
+    b = Batch.from_problems(items)
+    b.mode = mode
+    b.set_ly(5, 7)
+    b.commit()
+    full = b.ly(0)
+    assert full == b.ly(4) and full > grids[4].ly
+    for _ in range(2):   # the second time refilled
+        b.run(10_000)
+        assert b.ly(5) == 7 and b.ly(0) == full
+        assert grids[4].ly <= b.ly(4) < full
+        for k, (g, (name, _)) in enumerate(zip(grids, items)):
+            S = problem_state(name, params[k])
+            g.upload(S)
+            g.set_bvals()
+            g.new_dt()
+            g.run(10_000)
+            planes, dt, t, n = b.download(k)
+            ref = g.download()
+            assert refutil.mismatch_report(ref[0], planes, PLANES) == ""
+            assert (dt, t, n) == ref[1:]
+            b.upload(k, S)
+        b.prepare()
+    for g in grids:
+        g.close()
     b.close()
