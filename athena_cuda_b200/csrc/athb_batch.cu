@@ -496,9 +496,9 @@ static int upload_tables(athb_batch* b) {
 // march lengths that were not given by hand follow the rule of a single grid on
 // all of them together: lengths for the full batch would leave the last
 // instances of an ensemble with a few long marches on a few SMs (23 blasts of
-// 256 x 256 for 11 steps and one of 384 x 512 for 109: 40.6 ms with them, 22.5 ms
-// without; 24 uneven ones to one end time: 102.6 and 82.4).  The lengths are
-// kept when a longer map they need cannot be had.
+// 256 x 256 that end early and one of 384 x 512 that runs on for 109 steps in all:
+// 40.6 ms with them, 22.5 without; 24 uneven blasts to one end time: 102.6 and
+// 82.4).  The lengths are kept when a longer map they need cannot be had.
 static int upload_active(athb_batch* b) {
   long long faces = 0;
   for (int k : b->active) faces += role_y_faces(b->cfg[k]);

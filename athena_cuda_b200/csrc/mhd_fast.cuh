@@ -124,8 +124,11 @@ template <int LO, int HI> ATHB_HD bool outside0(double x) {
 }
 
 // ---------------------------------------------------------------------------
-// Correctly rounded operations.  Positive denominators within 2^+-500,
-// numerators 0 or within [2^-900, 2^500), quotients normal; roots of 0 or [2^-950, 2^950).
+// Correctly rounded operations.  Positive denominators from 2^-540 to 2^500,
+// numerators 0 or within [2^-960, 2^500), quotients normal; roots of 0 or
+// [2^-960, 2^950).  The remainders a - d q and x - g^2 are multiples of 2^-105 of
+// the power of two below a and x: 2^-1065 at the least, above the smallest
+// denormal, so the fused multiply-adds that form them are exact.
 // ---------------------------------------------------------------------------
 // 1/d from an approximation y good to 2^-50 or better
 ATHB_HD double recip_from(double d, double y) {

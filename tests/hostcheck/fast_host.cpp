@@ -19,7 +19,8 @@ void put(const Cons1& u, double* o) {
 
 extern "C" {
 
-// op 0: 1/x, 1: sqrt(x), 2: y/x with the reciprocal of x, 3: 1/sqrt(x) from the root's by-product
+// op 0: 1/x, 1: sqrt(x), 2: y/x with the reciprocal of x, 3: 1/sqrt(x) from the root's by-product,
+// 4: the by-product itself, 1/(2 sqrt(x)) to about an ulp
 void fast_ops(int op, int n, const double* x, const double* y, double* fast, double* plain) {
   for (int k = 0; k < n; k++) {
     double h;
@@ -27,6 +28,7 @@ void fast_ops(int op, int n, const double* x, const double* y, double* fast, dou
     case 0: fast[k] = recip(x[k]); plain[k] = 1.0 / x[k]; break;
     case 1: fast[k] = root(x[k]); plain[k] = std::sqrt(x[k]); break;
     case 2: fast[k] = quot(y[k], x[k], recip(x[k])); plain[k] = y[k] / x[k]; break;
+    case 4: root(x[k], fast[k]); plain[k] = 0.5 / std::sqrt(x[k]); break;
     default: {
       const double g = root(x[k], h);
       fast[k] = recip_of_root(g, h);

@@ -377,3 +377,27 @@ def test_plm_slopes_of_denormal_size(fast, component, exponent):
     fast.fast_plm(n, _p(w), _p(bx), _p(dtodx), C.c_double(5.0 / 3.0), _p(took), _p(f), _p(g))
     ok = took.astype(bool)
     np.testing.assert_array_equal(f[ok], g[ok])
+
+
+def test_operations_at_the_ends_of_their_ranges(fast):
+    """Numerators and roots from 2^-960 on (the smallest the physics passes on as
+    they are), denominators from 2^-540 (two jumps of a field whose product is
+    not zero) to 2^500, and the root's by-product 1/(2 sqrt(x)), on which the
+    adjoints rely: seeds of 20 bits and a cubic step leave 2.5 (2^-20)^3, and
+    two roundings, below 2^-50."""
+    rng = np.random.default_rng(40)
+    n = 200000
+    d = np.concatenate([2.0 ** rng.uniform(-540, -480, n), 2.0 ** rng.uniform(440, 500, n), 2.0 ** rng.uniform(-2, 2, n)])
+    f, g = _ops(fast, 0, d)
+    np.testing.assert_array_equal(f, g)
+    a = rng.choice([-1.0, 1.0], 3 * n) * 2.0 ** np.concatenate([rng.uniform(-960, -870, 2 * n), rng.uniform(-960, 400, n)])
+    # the quotient has to be normal
+    ok = np.abs(np.log2(np.abs(a)) - np.log2(d)) < 1000
+    f, g = _ops(fast, 2, d[ok], a[ok])
+    np.testing.assert_array_equal(f, g)
+    x = np.concatenate([2.0 ** rng.uniform(-960, -900, n), 2.0 ** rng.uniform(-60, 60, n), 2.0 ** rng.uniform(440, 950, n)])
+    for op in (1, 3):
+        f, g = _ops(fast, op, x)
+        np.testing.assert_array_equal(f, g)
+    f, g = _ops(fast, 4, x)
+    assert np.max(np.abs(f / g - 1)) <= 2.0 ** -50
