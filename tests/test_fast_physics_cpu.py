@@ -401,3 +401,46 @@ def test_operations_at_the_ends_of_their_ranges(fast):
         np.testing.assert_array_equal(f, g)
     f, g = _ops(fast, 4, x)
     assert np.max(np.abs(f / g - 1)) <= 2.0 ** -50
+
+
+# 29 outputs of a face, 23 of a cell: fast and general adjoint differ by the
+# rounding of ~1000 operations, each no worse than an ulp of some value on the
+# way; what an ulp of the inputs changes in the general form says how much that
+# is for each item, and no item is left out.
+ITEM_TOL = 1000
+
+
+def _every_item_agrees(adjoint, w, bx, lam, rng):
+    took, f, g = adjoint(w, bx, lam)
+    change = np.abs(g).max(axis=1) * 2.0 ** -52
+    for _ in range(6):
+        moved = [a * (1 + rng.choice([-1, 1], a.shape) * 2.0 ** -52) for a in (w, bx, lam)]
+        again = adjoint(*(np.ascontiguousarray(a) for a in moved))[2]
+        change = np.maximum(change, np.abs(again - g).max(axis=1))
+    worst = np.abs(f - g).max(axis=1) / change
+    assert took.mean() > 0.25
+    assert worst[took].max() <= ITEM_TOL
+
+
+@pytest.mark.parametrize("kind", ["smooth", "jumps", "zeros"])
+def test_adjoints_agree_on_every_item(fast, kind):
+    n = 20000
+    rng = np.random.default_rng(50)
+    dtodx, gamma = rng.uniform(0.05, 0.4, n), C.c_double(5.0 / 3.0)
+
+    def roe(w, bx, lam):
+        took, f, g = np.zeros(n, dtype=np.int32), np.empty((n, 29)), np.empty((n, 29))
+        fast.fast_roe_adj(n, _p(w), _p(bx), _p(lam), gamma, _p(took), _p(f), _p(g))
+        return took.astype(bool), f, g
+
+    def plm(w, bx, lam):
+        took, f, g = np.zeros(n, dtype=np.int32), np.empty((n, 23)), np.empty((n, 23))
+        fast.fast_plm_adj(n, _p(w), _p(bx), _p(dtodx), _p(lam), gamma, _p(took), _p(f), _p(g))
+        return took.astype(bool), f, g
+
+    w, b = _states(rng, 2 * n, kind)
+    _every_item_agrees(roe, np.ascontiguousarray(w.reshape(n, 2, 7)), np.ascontiguousarray(b[:n]),
+                       rng.normal(size=(n, 7)), rng)
+    w, b = _states(rng, 3 * n, kind)
+    _every_item_agrees(plm, np.ascontiguousarray(w.reshape(n, 3, 7)), np.ascontiguousarray(b.reshape(n, 3)),
+                       rng.normal(size=(n, 14)), rng)
