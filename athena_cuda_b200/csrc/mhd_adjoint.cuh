@@ -551,15 +551,6 @@ ATHB_HD void plm_cell_adj(const Prim1& wm, const Prim1& w0, const Prim1& wp, dou
 // A third of the FP64 instructions of plm_cell_adj, no branch around them.
 // ---------------------------------------------------------------------------
 ATHB_HD double mad(double a, double b, double c) { return fma_n(a, b, c); }
-// x, as a value the compiler takes for a new one: what is formed from it is
-// formed again instead of kept in a register (or a spill) since the first time.
-ATHB_HD double anew(double x) {
-#if defined(__CUDA_ARCH__)
-  asm volatile("" : "+d"(x));
-#endif
-  return x;
-}
-
 // Adjoint of esys_prim_fast: Eb holds the adjoints of the entries (signs as in
 // PrimEigT); db, v1b, .. are set.
 ATHB_HD void esys_prim_reverse(const EsysKeep& K, const PrimLeft& L, double d, double p, double di, double b1,

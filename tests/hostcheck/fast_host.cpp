@@ -118,14 +118,35 @@ void fast_flux(int hlle, int n, const double* w, const double* bx, double gamma,
     const Prim1 wl = prim(w + 14 * k), wr = prim(w + 14 * k + 7);
     const Cons1 ul = prim_to_cons(wl, bx[k], eos), ur = prim_to_cons(wr, bx[k], eos);
     Cons1 F{};
+    bool fallback;
     if (hlle) {
       took[k] = flux_hlle_fast(ul, ur, wl, wr, bx[k], eos, F);
       put(flux_hlle(ul, ur, wl, wr, bx[k], eos), plain + 7 * k);
     } else {
-      took[k] = flux_roe_fast(ul, ur, wl, wr, bx[k], eos, 1.0 / eos.gamma_1, F);
+      took[k] = flux_roe_fast(ul, ur, wl, wr, bx[k], eos, 1.0 / eos.gamma_1, F, fallback);
       put(flux_roe(ul, ur, wl, wr, bx[k], eos), plain + 7 * k);
     }
     put(F, fast + 7 * k);
+  }
+}
+
+// n faces as fast_flux's through face_flux, and riemann; fallback[k]: the Roe
+// solver knows that the face takes the HLLE flux.
+void fast_face(int hlle, int n, const double* w, const double* bx, double gamma, int* fallback, double* fast,
+               double* plain) {
+  const Eos eos{gamma, gamma - 1.0, gamma - 2.0};
+  const FastEos fe = make_fast_eos(eos, 0.01, 0.01);
+  for (int k = 0; k < n; k++) {
+    const Prim1 wl = prim(w + 14 * k), wr = prim(w + 14 * k + 7);
+    const Cons1 ul = prim_to_cons(wl, bx[k], eos), ur = prim_to_cons(wr, bx[k], eos);
+    Cons1 F;
+    bool known = false;
+    if (!hlle) (void)flux_roe_fast(ul, ur, wl, wr, bx[k], eos, fe.r_gamma_1, F, known);
+    fallback[k] = known;
+    put(hlle ? face_flux<kFluxHlle>(ul, ur, wl, wr, bx[k], eos, fe) : face_flux<kFluxRoe>(ul, ur, wl, wr, bx[k], eos, fe),
+        fast + 7 * k);
+    put(hlle ? riemann<kFluxHlle>(ul, ur, wl, wr, bx[k], eos) : riemann<kFluxRoe>(ul, ur, wl, wr, bx[k], eos),
+        plain + 7 * k);
   }
 }
 

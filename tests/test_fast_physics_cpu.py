@@ -444,3 +444,53 @@ def test_adjoints_agree_on_every_item(fast, kind):
     w, b = _states(rng, 3 * n, kind)
     _every_item_agrees(plm, np.ascontiguousarray(w.reshape(n, 3, 7)), np.ascontiguousarray(b.reshape(n, 3)),
                        rng.normal(size=(n, 14)), rng)
+
+
+def _faces(fast, hlle, w, bx, gamma=5.0 / 3.0):
+    n = bx.size
+    known, f, g = np.zeros(n, dtype=np.int32), np.empty((n, 7)), np.empty((n, 7))
+    fast.fast_face(hlle, n, _p(w), _p(bx), C.c_double(gamma), _p(known), _p(f), _p(g))
+    np.testing.assert_array_equal(f, g)
+    return known.astype(bool)
+
+
+@pytest.mark.parametrize("hlle", [0, 1])
+@pytest.mark.parametrize("kind", KINDS)
+def test_every_face_identical(fast, kind, hlle):
+    """The flux of every face, whichever form it ends up in: fast, the HLLE
+    fallback known to the fast Roe solver, or general."""
+    n = 40000
+    rng = np.random.default_rng(60 + KINDS.index(kind))
+    w, b = _states(rng, 2 * n, kind)
+    w = w.reshape(n, 2, 7)
+    w[rng.random(n) < 0.2, :, 1] += rng.choice([-8.0, 8.0])
+    known = _faces(fast, hlle, np.ascontiguousarray(w), np.ascontiguousarray(b[:n]))
+    assert hlle or kind != "jumps" or known.mean() > 0.1
+
+
+@pytest.mark.parametrize("spread", [1.0, 3.0, 8.0])
+def test_fallback_known_only_where_taken(fast, spread):
+    """Faces bisected to the last pair of doubles where the fallback is known."""
+    n = 20000
+    rng = np.random.default_rng(100 + int(spread))
+    A = np.empty((n, 2, 7))
+    A[:, :, 0], A[:, :, 4] = np.exp(spread * rng.normal(size=(2, n, 2)))
+    A[:, :, 1:4], A[:, :, 5:] = 2.0 * rng.normal(size=(n, 2, 3)), rng.normal(size=(n, 2, 2))
+    B = A.copy()
+    B[:, 1] = B[:, 0] * (1 + 1e-3)
+    bx = rng.normal(size=n)
+
+    def known(t):
+        w = (1 - t)[:, None, None] * B + t[:, None, None] * A
+        for c in (0, 4):
+            w[:, :, c] = np.exp((1 - t)[:, None] * np.log(B[:, :, c]) + t[:, None] * np.log(A[:, :, c]))
+        return _faces(fast, 0, np.ascontiguousarray(w), bx)
+
+    lo, hi = np.zeros(n), np.ones(n)
+    assert (known(hi) & ~known(lo)).sum() > n // 20
+    for _ in range(54):
+        mid = 0.5 * (lo + hi)
+        k = known(mid)
+        lo, hi = np.where(k, lo, mid), np.where(k, mid, hi)
+    for k in range(-8, 9):
+        known(hi * (1 + k * 2.0 ** -52))
