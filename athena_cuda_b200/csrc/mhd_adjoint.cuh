@@ -662,7 +662,9 @@ ATHB_HD bool plm_cell_adj_fast(const Prim1& wm, const Prim1& w0, const Prim1& wp
   PrimRight R;
   EsysKeep K;
   esys_prim_fast(w0, di, bxc, eos, L, R, K, bad);
-  bad |= K.tiny_waves;   // their derivatives count where their values do not
+  // derivatives count where the values of the speeds, or of the root between the
+  // sound and the Alfven speed, are too small to
+  bad |= K.tiny_waves | outside0<-480, 500>(K.c2);
   double Wm[7], W0[7], Wp[7], Pl[7], Pr[7];
   prim_arr(wm, Wm); prim_arr(w0, W0); prim_arr(wp, Wp);
   prim_arr(wlb, Pl); prim_arr(wrb, Pr);
@@ -1722,7 +1724,7 @@ ATHB_HD bool flux_roe_adj_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl
   const double bsq = bet2s * bet2s + bet3s * bet3s;
   const double vbet = v2 * bet2s + v3 * bet3s;
   wave_weights(s.cfsq - s.cssq, s.twid_asq - s.cssq, s.cfsq - s.twid_asq, af, as, general, r_span, h_af, h_as);
-  bad |= f.tiny_waves && !(as == 0.0 && above<-300>(v1));
+  bad |= (f.tiny_waves && !(as == 0.0 && above<-300>(v1))) | outside0<-480, 500>(f.c2);
   if (f.tiny_waves) {
     // the flow speed absorbs these speeds, but not their derivatives (1 / (2 speed)
     // times 2 Bxi / d): the operations of the general form, which hold at any size

@@ -494,3 +494,33 @@ def test_fallback_known_only_where_taken(fast, spread):
         lo, hi = np.where(k, lo, mid), np.where(k, mid, hi)
     for k in range(-8, 9):
         known(hi * (1 + k * 2.0 ** -52))
+
+
+def test_adjoints_where_sound_and_alfven_speed_agree(fast):
+    """The discriminant of the wave speeds is then the transverse field's alone:
+    its root from O(1) down to denormals and zero, against the general forms."""
+    n = 4000
+    rng = np.random.default_rng(70)
+    t = 10.0 ** np.linspace(-100, -170, n)
+    gamma, lam = 1.5, rng.normal(size=(n, 14))
+    w = np.zeros((n, 3, 7))
+    w[:, 0, :5], w[:, 2, :5] = [0.9, 0.2, 0.1, -0.1, 5.5], [1.2, 0.45, -0.2, 0.3, 6.6]
+    w[:, 1, :5] = [1.0, 0.25, 0.05, 0.02, 6.0]                          # a^2 = gamma p / d = 9
+    w[:, :, 5], w[:, :, 6] = t[:, None], 0.5 * t[:, None]
+    bx, dtodx = np.full((n, 3), 3.0), np.full(n, 0.2)                   # v_A^2 = 9
+    took = np.zeros(n, dtype=np.int32)
+    f, g = np.empty((n, 23)), np.empty((n, 23))
+    fast.fast_plm_adj(n, _p(w), _p(bx), _p(dtodx), _p(lam), C.c_double(gamma), _p(took), _p(f), _p(g))
+    ok = took.astype(bool)
+    assert ok.mean() > 0.25
+    assert _worst(f[ok], g[ok]) <= FADING_TOL
+    w = np.zeros((n, 2, 7))
+    w[:, :, :5] = [1.0, 0.25, 0.5, -0.5, 6.0]
+    w[:, 1, 2:4] += [0.25, -0.5]
+    w[:, :, 5], w[:, :, 6] = t[:, None] * [0.8, 1.0], 0.5 * t[:, None] * [1.1, 1.0]
+    bx, lam = np.full(n, 3.0), np.ascontiguousarray(lam[:, :7])
+    f, g = np.empty((n, 29)), np.empty((n, 29))
+    fast.fast_roe_adj(n, _p(w), _p(bx), _p(lam), C.c_double(gamma), _p(took), _p(f), _p(g))
+    ok = took.astype(bool)
+    assert ok.mean() > 0.25
+    assert _worst(f[ok], g[ok]) <= FADING_TOL
