@@ -234,10 +234,12 @@ ATHB_HD Prim1 prim_of(const Cons1& u, double bx, double di, const Eos& eos) {
   w.bz = u.bz;
   return w;
 }
-// Cell outside the fast functions: densities and pressures within 2^+-100,
-// momenta and fields below 2^100.
+// Cell outside the fast functions: densities and pressures within 2^+-120 (8e-37
+// to 1e36; cgs densities of 1e-31 are 2^-103), momenta and fields below 2^100.
+// Nothing formed from these over- or underflows on the way.  A cell outside
+// runs the general functions at 0.6 of the speed the step had with them alone.
 ATHB_HD bool cell_outside(const Cons1& u, double bx, double p) {
-  return outside<-100, 100>(u.d) | outside<-100, 100>(p) | above<100>(u.mx) | above<100>(u.my) | above<100>(u.mz) |
+  return outside<-120, 120>(u.d) | outside<-120, 120>(p) | above<100>(u.mx) | above<100>(u.my) | above<100>(u.mz) |
          above<100>(bx) | above<100>(u.by) | above<100>(u.bz);
 }
 ATHB_HD Cons1 cons_of(const Prim1& w, double bx, const Eos& eos, double r_gamma_1) {
@@ -530,7 +532,7 @@ struct FaceRoots {
 };
 ATHB_HD void face_averages(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, const Prim1& Wr, double Bxi,
                            const Eos& eos, RoeAvg& r, RoeSpeeds& s, FaceRoots& f, bool& bad) {
-  bad |= outside<-100, 100>(Wl.d) | outside<-100, 100>(Wr.d) | above<100>(Bxi);
+  bad |= outside<-120, 120>(Wl.d) | outside<-120, 120>(Wr.d) | above<100>(Bxi);
   r.sqrtdl = root(Wl.d, f.hl);
   r.sqrtdr = root(Wr.d, f.hr);
   const double ss = r.sqrtdl + r.sqrtdr;
@@ -545,7 +547,7 @@ ATHB_HD void face_averages(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
   bad |= above<100>(r.b2) | above<100>(r.b3);
   const double dby = Wl.by - Wr.by, dbz = Wl.bz - Wr.bz;
   const double db2 = 0.5 * (dby * dby + dbz * dbz), ss2 = ss * ss;
-  const bool tiny_jump = outside0<-900, 300>(db2);
+  const bool tiny_jump = outside0<-880, 300>(db2);
   r.x = quot(db2, ss2, recip_from(ss2, r.isdlpdr * r.isdlpdr));
   r.y = quot(0.5 * (Wl.d + Wr.d), r.droe, f.rd);
   const double bx2 = Bxi * Bxi;

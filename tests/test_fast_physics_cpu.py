@@ -524,3 +524,32 @@ def test_adjoints_where_sound_and_alfven_speed_agree(fast):
     ok = took.astype(bool)
     assert ok.mean() > 0.25
     assert _worst(f[ok], g[ok]) <= FADING_TOL
+
+
+@pytest.mark.parametrize("side", [-1, 1])
+def test_identical_at_the_edge_of_the_densities(fast, side):
+    """States in units that put the density at 2^-120 or 2^120, where the fast
+    forms end: what they take is the general forms', and they take most of it."""
+    n = 30000
+    rng = np.random.default_rng(80 + side)
+    d0, p0 = 2.0 ** (side * rng.uniform(100, 122, n)), 2.0 ** rng.uniform(-100, 100, n)
+    v0, b0 = np.sqrt(p0 / d0) * 2.0 ** rng.uniform(-6, 6, n), np.sqrt(p0) * 2.0 ** rng.choice([-400, -60, -3, 0, 3], n)
+
+    def states(sides):
+        r = rng.normal(size=(n, 1, 7)) + 10.0 ** rng.uniform(-12, 0, (n, 1, 1)) * rng.normal(size=(n, sides, 7))
+        w = np.empty((n, sides, 7))
+        w[:, :, 0], w[:, :, 4] = d0[:, None] * np.exp(0.3 * r[:, :, 0]), p0[:, None] * np.exp(0.3 * r[:, :, 4])
+        w[:, :, 1:4], w[:, :, 5:] = v0[:, None, None] * r[:, :, 1:4], b0[:, None, None] * r[:, :, 5:]
+        w[rng.random(n) < 0.2, :, 2] = 0.0
+        return np.ascontiguousarray(w)
+
+    w, bx, dtodx = states(3), b0[:, None] * rng.normal(size=(n, 3)), 2.0 ** rng.uniform(-8, 0, n)
+    took = np.zeros(n, dtype=np.int32)
+    f, g = np.empty((n, 14)), np.empty((n, 14))
+    fast.fast_plm(n, _p(w), _p(bx), _p(dtodx), C.c_double(5.0 / 3.0), _p(took), _p(f), _p(g))
+    ok = took.astype(bool)
+    inside = np.abs(np.log2(w[:, :, 0])).max(axis=1) < 120
+    assert ok[inside].mean() > 0.9 and not ok[np.abs(np.log2(w[:, 1, 0])) > 120.01].any()
+    np.testing.assert_array_equal(f[ok], g[ok])
+    _faces(fast, 0, states(2), np.ascontiguousarray(bx[:, 0]))
+    _faces(fast, 1, states(2), np.ascontiguousarray(bx[:, 0]))

@@ -37,7 +37,7 @@ def _state(kind: str, nx1: int, nx2: int, seed: int) -> np.ndarray:
     elif kind == "fringe":     # fields that fall to denormals beside exact zeros
         A = 1e-3 * np.exp(-(np.hypot(X - 0.5, Y - 0.5) / 0.012) ** 2)
         v[0], v[1], v[2] = 1.0, 0.5, 1e-200 * rng.normal(0, 1, shape)
-    elif kind == "tiny":       # densities and pressures outside the fast ranges
+    elif kind == "tiny":       # densities close to the end of the fast ranges
         rho, p = 1e-35 * np.exp(rng.normal(0, 0.2, shape)), 1e-15 * np.exp(rng.normal(0, 0.2, shape))
         v = 1e9 * rng.normal(0, 1, (3, *shape))
     elif kind == "cgs":        # small but ordinary units
@@ -115,3 +115,20 @@ def test_batch_bit_exact(threads):
     b.synchronize()
     for k, (cfg, S) in enumerate(zip(cfgs, states)):
         _check(_oracle(cfg, S, bc, 0, 3), b.download(k))
+
+
+@pytest.mark.parametrize("flux", [0, 1])
+@pytest.mark.parametrize("unit", [2.0 ** -10, 2.0 ** 235])
+def test_densities_outside_the_ranges_bit_exact(unit, flux):
+    """The density of "tiny" (1e-35, 2^-116) in other units: below 2^-120 and
+    just short of 2^120, on both sides of it."""
+    bc = (4, 4, 4, 4)
+    cfg = _config(72, 50, bc, flux)
+    S = _state("tiny", 72, 50, 7)
+    S[[0, 1, 2, 3, 4]] *= unit
+    g = Grid.create(cfg)
+    g.upload(S)
+    g.set_bvals()
+    g.new_dt()
+    g.run_async(4)
+    _check(_oracle(cfg, S, bc, flux, 4), g.download())
