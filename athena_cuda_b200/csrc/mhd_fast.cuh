@@ -637,11 +637,11 @@ ATHB_HD bool flux_hlle_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, c
 }
 
 // flux_roe (src/flux_roe.c:54-259); false: outside the ranges, or an
-// intermediate state may fail the positivity test: F not set.  hlle: one of them
-// surely fails it, and the flux is flux_hlle's.
+// intermediate state may fail the positivity test: F not set.  fails: bit n set
+// where a refused face inside the ranges has a state n that surely fails it.
 ATHB_HD bool flux_roe_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, const Prim1& Wr, double Bxi,
-                           const Eos& eos, double r_gamma_1, Cons1& F, bool& hlle) {
-  hlle = false;
+                           const Eos& eos, double r_gamma_1, Cons1& F, unsigned& fails) {
+  fails = 0;
   bool bad = false;
   RoeAvg r;
   RoeSpeeds s;
@@ -774,7 +774,6 @@ ATHB_HD bool flux_roe_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
     // multiplied through by the density, decided only outside its rounding
     double u[7] = {Ul.d, Ul.mx, Ul.my, Ul.mz, Ul.e, Ul.by, Ul.bz};
     bool pass = true;
-    unsigned fails = 0;   // bit n: state n surely fails
 #pragma unroll
     for (int n = 0; n < 6; n++) {
 #pragma unroll
@@ -784,18 +783,10 @@ ATHB_HD bool flux_roe_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
       const double m2 = 0.5 * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]);
       const double p = (u[4] - k) * u[0] - m2;
       pass &= u[0] > 0.0 && p > 1.0e-12 * (u[4] * u[0]);
-      fails |= (unsigned)(u[0] <= 0.0 || p < -1.0e-12 * ((fabs(u[4]) + k) * u[0] + m2)) << n;
+      fails |= (unsigned)(u[0] <= 0.0 || p < -1.0e-12 * (k * u[0] + m2)) << n;
     }
-    if (!pass) {
-      // the reference skips states between equal speeds; the speeds are formed
-      // here so that they take no registers while the states do
-      const double w = anew(v1);
-      const double e7[7] = {w - cf, w - s.vax, w - cs, w, w + cs, w + s.vax, w + cf};
-#pragma unroll
-      for (int n = 0; n < 6; n++) hlle |= ((fails >> n) & 1u) && e7[n + 1] > e7[n];
-      hlle = hlle && !bad;
-      return false;
-    }
+    if (bad | pass) fails = 0;
+    bad |= !pass;
   }
   // Step 8 (src/flux_roe.c:252).
   const Cons1 Fl = side_flux(Ul, Wl, Bxi, r.pbl), Fr = side_flux(Ur, Wr, Bxi, r.pbr);
@@ -814,32 +805,41 @@ ATHB_HD bool flux_roe_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
 }
 
 // The faces the fast function refuses, out of line: the HLLE flux in its fast
-// form where the Roe solver is known to fall back to it, else the general
-// function.  A face that falls back costs its warp this call: noise of order one
-// on every cell, where every warp has such faces, takes 62 us in k_correct at
-// 512 x 384, 88 with the general function alone and 64 without any fast form.
+// form where a state between two speeds that differ (the reference skips the
+// others) is known to fail, else the general function.  A face that falls back
+// costs its warp this call: noise of order one on every cell, where every warp
+// has such faces, takes 63 us in k_correct at 512 x 384, 88 with the general
+// function alone and 64 without any fast form.  The speeds are formed again here,
+// so that the fast function keeps no more than a mask for the few.
 template <int FLUX>
 ATHB_COLD void riemann_refused(const Cons1* ul, const Cons1* ur, const Prim1* wl, const Prim1* wr, double bxi,
-                               const Eos* eos, bool hlle, Cons1* F) {
-  if (hlle && flux_hlle_fast(*ul, *ur, *wl, *wr, bxi, *eos, *F)) return;
+                               const Eos* eos, unsigned fails, Cons1* F) {
+  if (fails) {
+    RoeAvg r;
+    RoeSpeeds s;
+    FaceRoots f;
+    bool bad = false;
+    face_averages(*ul, *ur, *wl, *wr, bxi, *eos, r, s, f, bad);
+    const double e[7] = {r.v1 - s.cf, r.v1 - s.vax, r.v1 - s.cs, r.v1, r.v1 + s.cs, r.v1 + s.vax, r.v1 + s.cf};
+    bool hlle = false;
+    for (int n = 0; n < 6; n++) hlle |= ((fails >> n) & 1u) && e[n + 1] > e[n];
+    if (hlle && flux_hlle_fast(*ul, *ur, *wl, *wr, bxi, *eos, *F)) return;
+  }
   *F = riemann<FLUX>(*ul, *ur, *wl, *wr, bxi, *eos);
 }
-
-// Face flux: riemann<FLUX> by the fast functions where they apply (fe.ok: the
-// launch's constants lie in their ranges).
 template <int FLUX>
 ATHB_HD Cons1 face_flux(const Cons1& ul, const Cons1& ur, const Prim1& wl, const Prim1& wr, double bxi,
                         const Eos& eos, const FastEos& fe) {
   Cons1 F;
-  bool hlle = false;
+  unsigned fails = 0;
   const bool done = FLUX == kFluxHlle ? flux_hlle_fast(ul, ur, wl, wr, bxi, eos, F)
-                                      : flux_roe_fast(ul, ur, wl, wr, bxi, eos, fe.r_gamma_1, F, hlle);
+                                      : flux_roe_fast(ul, ur, wl, wr, bxi, eos, fe.r_gamma_1, F, fails);
   if (!done || !fe.ok) {
     const Cons1 a = ul, b = ur;
     const Prim1 c = wl, e = wr;
     const Eos q = eos;
     Cons1 G;
-    riemann_refused<FLUX>(&a, &b, &c, &e, bxi, &q, hlle && fe.ok, &G);
+    riemann_refused<FLUX>(&a, &b, &c, &e, bxi, &q, fe.ok ? fails : 0u, &G);
     return G;
   }
   return F;

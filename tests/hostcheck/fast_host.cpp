@@ -118,12 +118,12 @@ void fast_flux(int hlle, int n, const double* w, const double* bx, double gamma,
     const Prim1 wl = prim(w + 14 * k), wr = prim(w + 14 * k + 7);
     const Cons1 ul = prim_to_cons(wl, bx[k], eos), ur = prim_to_cons(wr, bx[k], eos);
     Cons1 F{};
-    bool fallback;
+    unsigned fails;
     if (hlle) {
       took[k] = flux_hlle_fast(ul, ur, wl, wr, bx[k], eos, F);
       put(flux_hlle(ul, ur, wl, wr, bx[k], eos), plain + 7 * k);
     } else {
-      took[k] = flux_roe_fast(ul, ur, wl, wr, bx[k], eos, 1.0 / eos.gamma_1, F, fallback);
+      took[k] = flux_roe_fast(ul, ur, wl, wr, bx[k], eos, 1.0 / eos.gamma_1, F, fails);
       put(flux_roe(ul, ur, wl, wr, bx[k], eos), plain + 7 * k);
     }
     put(F, fast + 7 * k);
@@ -131,7 +131,7 @@ void fast_flux(int hlle, int n, const double* w, const double* bx, double gamma,
 }
 
 // n faces as fast_flux's through face_flux, and riemann; fallback[k]: the Roe
-// solver knows that the face takes the HLLE flux.
+// solver knows an intermediate state that fails its test.
 void fast_face(int hlle, int n, const double* w, const double* bx, double gamma, int* fallback, double* fast,
                double* plain) {
   const Eos eos{gamma, gamma - 1.0, gamma - 2.0};
@@ -140,9 +140,9 @@ void fast_face(int hlle, int n, const double* w, const double* bx, double gamma,
     const Prim1 wl = prim(w + 14 * k), wr = prim(w + 14 * k + 7);
     const Cons1 ul = prim_to_cons(wl, bx[k], eos), ur = prim_to_cons(wr, bx[k], eos);
     Cons1 F;
-    bool known = false;
-    if (!hlle) (void)flux_roe_fast(ul, ur, wl, wr, bx[k], eos, fe.r_gamma_1, F, known);
-    fallback[k] = known;
+    unsigned fails = 0;
+    if (!hlle) (void)flux_roe_fast(ul, ur, wl, wr, bx[k], eos, fe.r_gamma_1, F, fails);
+    fallback[k] = fails != 0;
     put(hlle ? face_flux<kFluxHlle>(ul, ur, wl, wr, bx[k], eos, fe) : face_flux<kFluxRoe>(ul, ur, wl, wr, bx[k], eos, fe),
         fast + 7 * k);
     put(hlle ? riemann<kFluxHlle>(ul, ur, wl, wr, bx[k], eos) : riemann<kFluxRoe>(ul, ur, wl, wr, bx[k], eos),
