@@ -709,13 +709,12 @@ template <class Exec> struct AdjointDriver {
     AdjArgs a = adj_args(Sn, lam[lc], lin);
     a.c = make_coef(hrec[n].dt, G.dx1, G.dx2);
     const int is = G.is, ie = G.ie, js = G.js, je = G.je;
-    // 7 launches where a stage each would make 16: the two sweeps of a stage
-    // run side by side (a small grid's stage leaves most SMs idle), and a
-    // gather too small for a launch is formed by its reader.  With the dt rule
-    // in the sum's launch and nothing cleared beforehand a step of the gradient
-    // makes 18 launches where it made 40: 21 of them took 266 -> 189 us at
-    // 64 x 48 and 504 -> 440 us at 256 x 256 before the stages themselves
-    // became faster
+    // The two sweeps of a stage run side by side (a small grid's stage leaves
+    // most SMs idle), a gather too small for a launch is formed by its reader,
+    // and the dt rule runs in the launch of the sum it needs: 9 launches from here
+    // to the end of this function.  With a launch for every stage and reduction
+    // pass they were 27, and a gradient took 266 us a step at 64 x 48 and 504 at
+    // 256 x 256 instead of 189 and 440, before the stages themselves became faster.
     x.items(full(), AdjFn<R_UPD, FLUX>{a});
     run_items3(x, 0, range_correct_x(is, ie, js, je), AdjFn<R_CORX, FLUX>{a}, range_correct_y(is, ie, js, je),
                AdjFn<R_CORY, FLUX>{a}, range_correct_e(is, ie, js, je), AdjFn<R_CORE, FLUX>{a});

@@ -551,6 +551,7 @@ ATHB_HD void plm_cell_adj(const Prim1& wm, const Prim1& w0, const Prim1& wp, dou
 // A third of the FP64 instructions of plm_cell_adj, no branch around them.
 // ---------------------------------------------------------------------------
 ATHB_HD double mad(double a, double b, double c) { return fma_n(a, b, c); }
+
 // Adjoint of esys_prim_fast: Eb holds the adjoints of the entries (signs as in
 // PrimEigT); db, v1b, .. are set.
 ATHB_HD void esys_prim_reverse(const EsysKeep& K, const PrimLeft& L, double d, double p, double di, double b1,
@@ -1573,8 +1574,6 @@ ATHB_HD void flux_roe_adj(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, con
 // The general form is bound by its chains of divisions and roots with branches
 // around them (255 registers, 8 warps an SM): at 256 x 256 the corrector's
 // launch took 82 us and the predictor's 69 us with it, 42 and 25 us with this.
-// Error against 80-bit arithmetic: mean 2.4e-16 of the largest output (general:
-// 2.6e-16).
 // ---------------------------------------------------------------------------
 
 // Adjoints of the face's averages, speeds and their inputs, set by the parts below.

@@ -1,24 +1,24 @@
 // mhd_fast.cuh -- the hot per-cell and per-face physics of the step with
 // branch-free, correctly rounded divisions and square roots.
 //
-// The functions return the very bits of their counterparts in mhd_physics.cuh
-// (plm_cell, flux_roe, flux_hlle) whenever they report success; a caller whose
-// operands lie outside the ranges below is told so and takes the general
-// function instead.  The ranges let fields and momenta be as small as they
-// come: where a field advects into a region that has none its edge decays by a
-// constant factor per cell, so wide bands of cells hold fields of 1e-50 ..
-// 1e-308, and sending those out of line made the two paths evict each other
-// from the instruction cache (field loop 2048^2 after 200 steps: predictor
-// 2.7 ms, against 1.9 ms for the code before and 1.5 ms at step 5).  Squares
-// of such fields (1e-162 .. 1e-145, the square a denormal or close to one) are
-// scaled into range before a root or a quotient and back after it, exactly;
-// wave speeds that small only count where the flow speed does not absorb them.  What differs is the cost:
-//   * a / b and sqrt(x) as the compiler emits them are each a chain of ~10
-//     dependent FP64 instructions that ends in a test and a call, so the ~150
-//     of them in a zone-cycle cut the code into short blocks that neither
-//     overlap one another nor share work.  Here they are straight-line code
-//     (below), operands with a common denominator share its reciprocal, and
-//     reciprocals of square roots start from the root's own by-product;
+// The functions return the values of their counterparts in mhd_physics.cuh
+// (plm_cell, flux_roe, flux_hlle) bit for bit whenever they report success (a
+// zero may carry the other sign where an input is -0); a caller whose operands
+// lie outside the ranges below is told so and takes the general function
+// instead.  The ranges let fields and momenta be as small as they come: where a
+// field advects into a region that has none its edge decays by a constant
+// factor per cell, so wide bands of cells hold fields of 1e-50 .. 1e-308, and a
+// second code path for them would alternate with the first in the instruction
+// cache.  Squares of such fields (1e-162 .. 1e-145, the square a denormal or
+// close to one) are scaled into range before a root or a quotient and back after
+// it, exactly; wave speeds that small only count where the flow speed does not
+// absorb them.  What differs is the cost:
+//   * the ~150 divisions and square roots of a zone-cycle are straight-line code
+//     (below): operands with a common denominator share its reciprocal, and
+//     reciprocals of square roots start from the root's own by-product.  With
+//     them, and selects for branches, k_predict runs the FP64 pipe at 52% where it
+//     reached 38%, in three quarters of the instructions, and waits on
+//     instruction fetch 0.35 cycles per issue instead of 1.29 (field loop 1024^2);
 //   * products with the sign of the normal field flip a sign bit, and sums that
 //     the reference forms twice with opposite signs are formed once;
 //   * the six intermediate-state tests of the Roe solver are replaced by one
@@ -236,8 +236,8 @@ ATHB_HD Prim1 prim_of(const Cons1& u, double bx, double di, const Eos& eos) {
 }
 // Cell outside the fast functions: densities and pressures within 2^+-120 (8e-37
 // to 1e36; cgs densities of 1e-31 are 2^-103), momenta and fields below 2^100.
-// Nothing formed from these over- or underflows on the way.  A cell outside
-// runs the general functions at 0.6 of the speed the step had with them alone.
+// Nothing formed from these overflows on the way.  A cell outside runs the
+// general functions, at 0.6 of the speed the step had with them alone.
 ATHB_HD bool cell_outside(const Cons1& u, double bx, double p) {
   return outside<-120, 120>(u.d) | outside<-120, 120>(p) | above<100>(u.mx) | above<100>(u.my) | above<100>(u.mz) |
          above<100>(bx) | above<100>(u.by) | above<100>(u.bz);
@@ -808,7 +808,7 @@ ATHB_HD bool flux_roe_fast(const Cons1& Ul, const Cons1& Ur, const Prim1& Wl, co
 // form where a state between two speeds that differ (the reference skips the
 // others) is known to fail, else the general function.  A face that falls back
 // costs its warp this call: noise of order one on every cell, where every warp
-// has such faces, takes 63 us in k_correct at 512 x 384, 88 with the general
+// has such faces, takes 60 us in k_correct at 512 x 384, 88 with the general
 // function alone and 64 without any fast form.  The speeds are formed again here,
 // so that the fast function keeps no more than a mask for the few.
 template <int FLUX>

@@ -299,11 +299,11 @@ __device__ __forceinline__ void predict_y(const GridArgs& g, const PredictGeom& 
   }
 }
 
-// k_predict is bound by the FP64 pipe's latency and by instruction fetch (3
-// warps per scheduler, ~1500 straight-line FP64 instructions per cell and
-// role).  Branch-free divisions, roots and PLM (mhd_fast.cuh), measured on B200:
-// field loop 2048^2 1.90 -> 1.33 ms, blast 1024^2 0.645 -> 0.408 ms (FP64 pipe 38%
-// -> 55% busy), blast 200x300 53 -> 38 us.
+// k_predict is bound by the FP64 pipe's latency (2 warps per scheduler, ~1500
+// straight-line FP64 instructions per cell and role; the pipe 52% busy).
+// Branch-free divisions, roots and PLM (mhd_fast.cuh) and 255 registers took it, on
+// B200, from 1.90 to 1.28 ms (field loop 2048^2), 0.645 to 0.379 ms (blast 1024^2)
+// and 53 to 39 us (blast 200x300).
 //
 // Resident blocks per SM the heavy kernels are compiled for.  k_predict keeps
 // 255 registers per thread and 2 blocks (8 warps) per SM: with the branches

@@ -43,8 +43,8 @@ UNIT = "zone-cycles/s"
 # Algorithmic FP64 operations per zone-cycle of the reference step on the
 # 2048x2048 field loop (every binary + - * / and sqrt on a Real that the
 # reference performs), split by the kernel that performs them.  Counted by
-# `python oracle/opcount.py --problem field_loop --nx 2048 --ny 2048 --steps 3`
-# (profiles/opcount_field_loop_2048.md).  Per launch = value x nx x ny.
+# `python oracle/opcount.py --problem field_loop --nx 2048 --ny 2048 --steps 3`.
+# Per launch = value x nx x ny.
 OPS_PER_ZC = {
     "predict": 3432.2,     # steps 1a-2e and 3 (PLM, MHD source, Roe, emf3_cc)
     "emf_half": 18.0,      # step 4 corner EMF + half-step CT
@@ -54,11 +54,10 @@ OPS_PER_ZC = {
 }
 OPS_STEP = sum(OPS_PER_ZC.values())
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the
-# dominant kernels from single-kernel ncu captures of the 1024x1024 field loop
-# (profiles/k_predict_field_loop_1024.md, k_correct_k_update_field_loop_1024.md),
+# dominant kernels from single-kernel ncu captures of the 1024x1024 field loop,
 # scaled to 2048x2048 by the cell ratio 4.  Applies to the 2048x2048 default
 # workload.
-TRAFFIC_1024 = {"predict": 469.49e6, "correct": 702.56e6, "update_cfl": 241.91e6}
+TRAFFIC_1024 = {"predict": 468.94e6, "correct": 703.54e6, "update_cfl": 242.38e6}
 
 
 def parse():
